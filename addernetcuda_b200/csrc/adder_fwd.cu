@@ -420,12 +420,35 @@ static void choose_fwd_tile(const Geom& g, const TileHint& hint, int& rw, int& r
     else if (rw == 8 && rm == 4) { CALL(KS_, S_, 8, 4) }                                    \
     else if (rw == 4 && rm == 4) { CALL(KS_, S_, 4, 4) }
 
+// Which layers take the gathering kernel (adder_fwd_gather.cu).  Its tile is 64 channels x 128 pixels whatever the plane, but it
+// stages every tap's pixels again, where adder_fwd_kernel shifts one haloed patch: 1x1 kernels have no halo (1024->256 14x14:
+// 1289 -> 928 us at batch 256), a stride-2 patch is mostly halo (128->128 56x56: 791 -> 629 us at batch 64), and with
+// 128 channels, or 64 on planes of 14x14 and more, the staging is small beside the arithmetic (256->256 14x14: 2446 ->
+// 2145 us; but 32->32 16x16: 54 -> 65 us, and 64->64 8x8 too few tiles).  The rule does not look at the batch: the two
+// kernels add in different orders, and an image's result must not depend on its batch.
+static bool fwd_uses_gather(const Geom& g, const TileHint& hint) {
+    TileHint h = hint;
+    h.variant = 0;
+    if (!h.is_default()) return false;
+    if (hint.variant) return hint.variant == 2;
+    if (g.k == 1) return true;
+    const int c = g.Ci < g.Co ? g.Ci : g.Co;
+    return g.stride == 2 ? c >= 64 : c >= 128 || (c >= 64 && g.H * g.W >= 196);
+}
+
 int describe_fwd(const Geom& layer, const TileHint& hint, char* buf, size_t n) {
     const Geom g = flatten_pointwise(layer);
     if (hint.is_default() && pointwise_applicable(g)) {
         snprintf(buf, n, "fwd k=1 s=%d pointwise: one thread per output position, 16 output channels per CTA, threads=256 "
                  "grid=(%d,%d) status=0", g.stride, ceil_div(g.N * g.Ho * g.Wo, 256), ceil_div(g.Co, 16));
         return ADDER_OK;
+    }
+    if (fwd_uses_gather(layer, hint)) {
+        const int w = describe_fwd_gather(conv_geom(layer), buf, n);
+        if (w < 0 || (size_t)w + 16 >= n) return ADDER_OK;
+        buf += w; n -= w;
+        const int w2 = snprintf(buf, n, "; tiled form: ");
+        buf += w2; n -= w2;
     }
     int rw = 8, rm = 8;
     choose_fwd_tile(g, hint, rw, rm);
@@ -446,6 +469,10 @@ int describe_fwd(const Geom& layer, const TileHint& hint, char* buf, size_t n) {
 int fwd_stat_slices(const Geom& layer, const TileHint& hint) {
     const Geom g = flatten_pointwise(layer);
     if (hint.is_default() && pointwise_applicable(g)) return 0;
+    if (fwd_uses_gather(layer, hint)) {
+        const int slices = fwd_gather_stat_slices(conv_geom(layer));
+        return slices > (1 << 20) ? 0 : slices;
+    }
     int rw = 8, rm = 8;
     choose_fwd_tile(g, hint, rw, rm);
     FwdPlan p;
@@ -464,6 +491,7 @@ int launch_fwd(const Geom& layer, const float* x, const float* w, float* out, co
         if (stats != nullptr) return ADDER_ERR_UNSUPPORTED;
         return launch_pointwise_fwd(g, x, w, out, stream);
     }
+    if (fwd_uses_gather(layer, hint)) return launch_fwd_gather(conv_geom(layer), x, w, out, stream, stats, stat_slices);
     int rw = 8, rm = 8;
     choose_fwd_tile(g, hint, rw, rm);
 #define ADDER_FWD_LAUNCH(KS_, S_, RW_, RM_) \

@@ -1,0 +1,428 @@
+// Input gradient of the adder convolution as a channels x pixels tile with a gathered gradient operand (gather.cuh):
+//   gx[n,ci,y,x] = sum over output channels and the taps that read pixel (y, x) of clamp(w - x, -1, 1) * g
+// for 1x1 layers and every kernel extent, stride, padding and dilation.  For a stride S the input pixels fall into S*S
+// classes (y mod S, x mod S) that are read by different taps; a class is a pixel space of its own (blockIdx.z) whose taps
+// are an arithmetic progression, so no thread works on a tap that does not reach its pixel.
+//
+// A thread keeps 4 input channels x 8 pixels of x and of the sums in registers; a k step is three 128-bit loads for
+// 32 terms.  Saturating form: one FFMA.SAT and one FFMA a term, with x' = 1/2 - x/2 in registers:
+// clamp(d,-1,1) = 2*sat(d/2 + 1/2) - 1, and the "-1" is the sum of g over the taps, added up once per pixel while the
+// stages pass by.  Exact form: min.xorsign.abs is the clamp in one instruction (magnitude min(|d|, 1), sign of d),
+// where fminf(fmaxf(d, -1), 1) takes two; the sums are packed pairs of pixels.
+// Both are bound by the register operands they read (5 a term, 2 a cycle and scheduler): 2.6 and 3.4 lane cycles a term
+// with nothing around them.
+#include <cstdio>
+#include "common.cuh"
+#include "gather.cuh"
+#include "kernels.h"
+
+namespace adder {
+
+namespace {
+constexpr int RC = 4;                   // input channels per thread (8 of them, at 3 CTAs per SM, measured 10-15 % slower)
+constexpr int FOLD = 4;                 // chunks per partial sum: at most 64 terms before it is folded into the total
+constexpr int MAX_CLASSES = 9;
+}
+
+struct GxGatherArgs {
+    GatherMap m[MAX_CLASSES];
+    int ry[MAX_CLASSES], rx[MAX_CLASSES];   // first row and column of the class in the input
+    const float* gout;
+    const float* x;
+    const float* w;
+    float* gx;
+    int Ci, H, W, Co, Ho, Wo, KK, CK, sh, sw, accumulate;
+    int w_quads;             // 1x1: rows of w are whole quads and 16-byte aligned
+    int vec_io;              // stride 1, planes are whole quads, x and gx 16-byte aligned
+    int fill_block;          // the other pixels of an sh x sw block belong to no class: write zeros there
+    int fill_quads;          // ... and four blocks of a row can be written as aligned 128-bit words
+};
+
+template <int CG, bool FAST, bool QUADS>
+__global__ void __launch_bounds__(GATHER_THREADS, 4) adder_gx_gather_kernel(const __grid_constant__ GxGatherArgs a) {
+    constexpr int PG = GATHER_THREADS / CG, TC = CG * RC, TP = PG * 8, WP = TC + 4;
+    constexpr int COLS = TP > GATHER_THREADS ? TP / GATHER_THREADS : 1;
+    constexpr int ROWS = TP < GATHER_THREADS ? GATHER_THREADS / TP : 1;
+    constexpr int GS = GATHER_CK * TP, WS = GATHER_CK * WP;
+    extern __shared__ __align__(16) float smem[];
+    float* const Gs = smem;
+    float* const Ws = smem + GATHER_STAGES * GS;
+    float4* const Tot = reinterpret_cast<float4*>(Ws + GATHER_STAGES * WS) + threadIdx.x;    // [8][threads]
+
+    const GatherMap& m = a.m[blockIdx.z];
+    const int p0 = blockIdx.x * TP, ci0 = blockIdx.y * TC;
+    if (p0 >= m.P) return;                       // classes differ by a row and a column
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int cg = (wid % (CG / 4)) * 4 + (lane >> 3), pg = (wid / (CG / 4)) * 8 + (lane & 7);
+    const int ry = a.ry[blockIdx.z], rx = a.rx[blockIdx.z];
+    const size_t image = (size_t)a.Co * a.Ho * a.Wo;
+    const int HW = a.H * a.W;
+
+    GatherPixel px[COLS];
+    if (QUADS) {
+        px[0].decode(m, a.gout, p0 + 4 * (tid % (TP / 4)), image);
+        px[0].base += px[0].row * a.Wo + px[0].col;
+    } else {
+#pragma unroll
+        for (int q = 0; q < COLS; ++q) px[q].decode(m, a.gout, p0 + (COLS > 1 ? tid + q * GATHER_THREADS : tid % TP), image);
+    }
+    GatherChunk fc;
+    const int ck4 = round_up(a.CK, 4);
+    const int nchunks = ceil_div(a.Co, a.CK) * m.ntaps;
+    auto fill = [&](int stage) {
+        const int nch = min(a.CK, a.Co - fc.c0);
+        if (QUADS) gather_quads<TP>(Gs + stage * GS, px[0].base, px[0].ok, a.gout, fc.c0, nch, ck4, a.Ho * a.Wo, tid);
+        else gather_pixels<TP>(Gs + stage * GS, px, a.gout, m, fc, nch, ck4, a.Ho, a.Wo, tid);
+        // weights [output channel of the chunk][input channel of the tile]
+        float* ws = Ws + stage * WS;
+        const float* wsrc = a.w + ((fc.c0 * a.Ci + ci0) * a.KK + m.wt0 + fc.i * m.dwi + fc.j * m.dwj);
+        if (a.w_quads) {
+            constexpr int WQ = TC / 4, WROWS = GATHER_THREADS / WQ;
+            const int q = 4 * (tid % WQ), k0 = tid / WQ;
+            const bool okc = ci0 + q < a.Ci;
+            const float* s = okc ? wsrc + (k0 * a.Ci + q) : a.w;
+            const int step = okc ? WROWS * a.Ci : 0;
+            float* d = ws + k0 * WP + q;
+            if (nch == GATHER_CK && GATHER_CK % WROWS == 0) {
+#pragma unroll
+                for (int k = 0; k < GATHER_CK; k += WROWS, s += step) cp_async16(d + k * WP, s, okc);
+            } else {
+                for (int k = k0; k < ck4; k += WROWS, s += step, d += WROWS * WP) cp_async16(d, k < nch ? s : a.w, okc & (k < nch));
+            }
+        } else {
+            constexpr int WROWS = GATHER_THREADS / TC;
+            const int col = tid % TC;
+            const bool okc = ci0 + col < a.Ci;
+            copy_rows<WROWS, WP>(ws + col, okc ? wsrc + col * a.KK : a.w, okc ? a.Ci * a.KK : 0, okc, tid / TC, nch, ck4);
+        }
+        fc.next(m, a.CK);
+    };
+
+#pragma unroll
+    for (int s = 0; s < GATHER_STAGES - 1; ++s) {
+        if (s < nchunks) fill(s);
+        cp_async_commit();
+    }
+
+    // the thread's 8 pixels: input address (element offset of channel 0) and validity
+    float xv[RC][8];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int p = p0 + h * (TP / 2) + pg * 4;
+        if (a.vec_io) {
+            uint32_t n, r;
+            m.d_phw.divmod(p < m.P ? p : 0, n, r);
+            const float* xs = a.x + ((size_t)n * a.Ci + ci0 + cg * RC) * HW + r;
+#pragma unroll
+            for (int c = 0; c < RC; ++c) {
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (p < m.P && ci0 + cg * RC + c < a.Ci) v = __ldg(reinterpret_cast<const float4*>(xs + (size_t)c * HW));
+                xv[c][4 * h] = v.x; xv[c][4 * h + 1] = v.y; xv[c][4 * h + 2] = v.z; xv[c][4 * h + 3] = v.w;
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                uint32_t n, r, y, x;
+                m.d_phw.divmod(p + j < m.P ? p + j : 0, n, r);
+                m.d_pw.divmod(r, y, x);
+                const float* xs = a.x + ((size_t)n * a.Ci + ci0 + cg * RC) * HW + ((int)y * a.sh + ry) * a.W + (int)x * a.sw + rx;
+#pragma unroll
+                for (int c = 0; c < RC; ++c)
+                    xv[c][4 * h + j] = (p + j < m.P && ci0 + cg * RC + c < a.Ci) ? __ldg(xs + (size_t)c * HW) : 0.f;
+            }
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < RC; ++c)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) xv[c][j] = FAST ? fmaf(xv[c][j], -0.5f, 0.5f) : -xv[c][j];
+
+    float acc[RC][8];
+#pragma unroll
+    for (int c = 0; c < RC; ++c)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[c][j] = 0.f;
+    float box[COLS];
+#pragma unroll
+    for (int q = 0; q < COLS; ++q) box[q] = 0.f;
+
+    GatherChunk cc;
+    int stage = 0, fstage = GATHER_STAGES - 1;
+    for (int c = 0; c < nchunks; ++c) {
+        cp_async_wait<GATHER_STAGES - 2>();
+        __syncthreads();
+        if (c + GATHER_STAGES - 1 < nchunks) fill(fstage);
+        cp_async_commit();
+        const float* gs = Gs + stage * GS + pg * 4;
+        const float* ws = Ws + stage * WS + cg * RC;
+        const int nk = min(ck4, round_up(a.Co - cc.c0, 4));
+#pragma unroll 4
+        for (int k = 0; k < nk; ++k) {
+            const float4 g0 = *reinterpret_cast<const float4*>(gs + k * TP);
+            const float4 g1 = *reinterpret_cast<const float4*>(gs + k * TP + TP / 2);
+            const float4 wq = *reinterpret_cast<const float4*>(ws + k * WP);
+            const float wv[RC] = {wq.x, wq.y, wq.z, wq.w};
+            const float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+            if constexpr (FAST) {
+#pragma unroll
+                for (int r = 0; r < RC; ++r)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) acc[r][j] = fmaf(__saturatef(fmaf(wv[r], 0.5f, xv[r][j])), gv[j], acc[r][j]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; j += 2)
+#pragma unroll
+                    for (int r = 0; r < RC; ++r) {
+                        const uint64_t s = fma2(pack2(clamp_unit(wv[r] + xv[r][j]), clamp_unit(wv[r] + xv[r][j + 1])),
+                                                pack2(gv[j], gv[j + 1]), pack2(acc[r][j], acc[r][j + 1]));
+                        unpack2(s, acc[r][j], acc[r][j + 1]);
+                    }
+            }
+        }
+        if (FAST) {
+            const float* col = Gs + stage * GS + (COLS > 1 ? tid : tid % TP);
+#pragma unroll
+            for (int q = 0; q < COLS; ++q) {
+                const float* cq = col + (tid / TP) * TP + q * GATHER_THREADS;
+                float s = 0.f;
+                if (nk == GATHER_CK) {
+#pragma unroll
+                    for (int k = 0; k < GATHER_CK; k += ROWS) s += cq[k * TP];
+                } else {
+                    for (int k = 0; k < nk; k += ROWS) s += cq[k * TP];
+                }
+                box[q] += s;
+            }
+        }
+        // two-level summation: a long sum over output channels loses far less than one running fp32 accumulator would
+        if (c % FOLD == FOLD - 1 && c + 1 < nchunks) {
+#pragma unroll
+            for (int r = 0; r < RC; ++r)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float4* t = Tot + (r * 2 + h) * GATHER_THREADS;
+                    float4 v = c < FOLD ? make_float4(0.f, 0.f, 0.f, 0.f) : *t;
+                    v.x += acc[r][4 * h]; v.y += acc[r][4 * h + 1]; v.z += acc[r][4 * h + 2]; v.w += acc[r][4 * h + 3];
+                    *t = v;
+                    acc[r][4 * h] = acc[r][4 * h + 1] = acc[r][4 * h + 2] = acc[r][4 * h + 3] = 0.f;
+                }
+        }
+        cc.next(m, a.CK);
+        if (++stage == GATHER_STAGES) stage = 0;
+        if (++fstage == GATHER_STAGES) fstage = 0;
+    }
+    if (nchunks > FOLD) {
+#pragma unroll
+        for (int r = 0; r < RC; ++r)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float4 v = Tot[(r * 2 + h) * GATHER_THREADS];
+                acc[r][4 * h] += v.x; acc[r][4 * h + 1] += v.y; acc[r][4 * h + 2] += v.z; acc[r][4 * h + 3] += v.w;
+            }
+    }
+    if (FAST) {
+        __syncthreads();                         // the stages are free
+        float* bs = smem;                        // [ROWS][TP]
+#pragma unroll
+        for (int q = 0; q < COLS; ++q) bs[tid + q * GATHER_THREADS] = box[q];
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int col = (j >> 2) * (TP / 2) + pg * 4 + (j & 3);
+            float b = bs[col];
+#pragma unroll
+            for (int r = 1; r < ROWS; ++r) b += bs[r * TP + col];
+#pragma unroll
+            for (int r = 0; r < RC; ++r) acc[r][j] = fmaf(2.f, acc[r][j], -b);
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int p = p0 + h * (TP / 2) + pg * 4;
+        if (a.vec_io || a.fill_quads) {
+            if (p >= m.P) continue;
+            uint32_t n, r, y, x;
+            m.d_phw.divmod(p, n, r);
+            m.d_pw.divmod(r, y, x);
+            float* o = a.gx + ((size_t)n * a.Ci + ci0 + cg * RC) * HW + (a.vec_io ? r : (y * 2) * a.W + x * 2);
+#pragma unroll
+            for (int c = 0; c < RC; ++c) {
+                if (ci0 + cg * RC + c >= a.Ci) break;
+                float4* o4 = reinterpret_cast<float4*>(o + (size_t)c * HW);
+                float4 v = make_float4(acc[c][4 * h], acc[c][4 * h + 1], acc[c][4 * h + 2], acc[c][4 * h + 3]);
+                if (a.fill_quads) {              // stride 2, pixels of class (0, 0) only: a zero between them and a row of zeros below
+                    o4[0] = make_float4(v.x, 0.f, v.y, 0.f);
+                    o4[1] = make_float4(v.z, 0.f, v.w, 0.f);
+                    o4 = reinterpret_cast<float4*>(o + (size_t)c * HW + a.W);
+                    o4[0] = o4[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    continue;
+                }
+                if (a.accumulate) {
+                    const float4 old = *o4;
+                    v.x += old.x; v.y += old.y; v.z += old.z; v.w += old.w;
+                }
+                *o4 = v;
+            }
+            continue;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (p + j >= m.P) continue;
+            uint32_t n, r, y, x;
+            m.d_phw.divmod(p + j, n, r);
+            m.d_pw.divmod(r, y, x);
+            const int yi = (int)y * a.sh + ry, xi = (int)x * a.sw + rx;
+            float* o = a.gx + ((size_t)n * a.Ci + ci0 + cg * RC) * HW + yi * a.W + xi;
+#pragma unroll
+            for (int c = 0; c < RC; ++c) {
+                if (ci0 + cg * RC + c >= a.Ci) break;
+                float* oc = o + (size_t)c * HW;
+                const float v = acc[c][4 * h + j];
+                if (a.accumulate) { *oc += v; continue; }
+                *oc = v;
+                if (a.fill_block)
+                    for (int dy = 0; dy < a.sh && yi + dy < a.H; ++dy)
+                        for (int dx = 0; dx < a.sw && xi + dx < a.W; ++dx)
+                            if (dy | dx) oc[dy * a.W + dx] = 0.f;
+            }
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// host side
+// ------------------------------------------------------------------------------------------
+
+namespace {
+
+// CG channel groups of 4 per CTA: 64 channels x 64 pixels, 32 x 128 or 16 x 256 (the cost is explained at choose_tile in
+// adder_fwd_gather.cu; here a term is 2.6 lane cycles).
+int choose_groups(long long P, int classes, int Ci) {
+    static const double rate[4] = {0.5, 0.8, 0.93, 1.0};
+    int best = 16;
+    double best_cost = 1e300;
+    const int sms = sm_count();
+    for (int cg = 16; cg >= 4; cg >>= 1) {
+        const int tc = cg * RC, tp = GATHER_THREADS / cg * 8;
+        const long long tiles = ((P + tp - 1) / tp + classes - 1) * ceil_div(Ci, tc);
+        const long long per_sm = (tiles + sms - 1) / sms;
+        const double cost = per_sm / rate[per_sm < 4 ? per_sm - 1 : 3] * (2.6 * tc * tp + 4.0 * (tc + tp));
+        if (cost < best_cost) { best_cost = cost; best = cg; }
+    }
+    return best;
+}
+
+size_t smem_bytes(int cg) {
+    const int tc = cg * RC, tp = GATHER_THREADS / cg * 8;
+    return ((size_t)GATHER_STAGES * GATHER_CK * (tp + tc + 4) + RC * 8 * GATHER_THREADS) * sizeof(float);
+}
+
+// Taps k of one dimension that reach input positions q*S + r: (r + pad - k*dil) % S == 0.  Output position q + o0 + i*d0.
+struct ClassTaps { int k0, step, count, o0, d0; };
+ClassTaps class_taps(int r, int K, int S, int pad, int dil) {
+    ClassTaps t{0, 1, 0, 0, 0};
+    for (int k = 0; k < K; ++k) {
+        if ((r + pad - k * dil) % S != 0) continue;
+        if (t.count == 0) { t.k0 = k; t.o0 = (r + pad - k * dil) / S; }
+        else if (t.count == 1) { t.step = k - t.k0; t.d0 = (r + pad - k * dil) / S - t.o0; }
+        ++t.count;
+    }
+    return t;
+}
+
+bool fill_classes(const ConvGeom& g, int first, GxGatherArgs& a, int& n, int& total, bool only_first) {
+    n = 0; total = 0;
+    int at = 0;
+    for (int ry = 0; ry < g.sh && ry < g.H; ++ry)
+        for (int rx = 0; rx < g.sw && rx < g.W; ++rx) {
+            if (only_first && (ry | rx)) continue;
+            if (at++ < first || n == MAX_CLASSES) continue;
+            const ClassTaps v = class_taps(ry, g.kh, g.sh, g.ph, g.dh), h = class_taps(rx, g.kw, g.sw, g.pw, g.dw);
+            GatherMap& m = a.m[n];
+            m.PH = ceil_div(g.H - ry, g.sh); m.PW = ceil_div(g.W - rx, g.sw); m.P = g.N * m.PH * m.PW;
+            m.th = v.count; m.tw = h.count; m.ntaps = v.count * h.count;
+            m.sy = m.sx = 1;
+            m.oy0 = v.o0; m.doy = v.d0; m.ox0 = h.o0; m.dox = h.d0;
+            m.wt0 = v.k0 * g.kw + h.k0; m.dwi = v.step * g.kw; m.dwj = h.step;
+            m.d_phw = FastDiv(m.PH * m.PW); m.d_pw = FastDiv(m.PW);
+            a.ry[n] = ry; a.rx[n] = rx;
+            ++n;
+        }
+    total = at;
+    return first + n < total;          // classes left for another launch
+}
+
+// Every tap reaches class (0, 0) only (1x1 kernels, mostly): the other pixels get zeros, written beside their neighbours.
+bool single_class(const ConvGeom& g) {
+    if (g.sh == 1 && g.sw == 1) return false;
+    for (int r = 1; r < g.sh; ++r) if (class_taps(r, g.kh, g.sh, g.ph, g.dh).count) return false;
+    for (int r = 1; r < g.sw; ++r) if (class_taps(r, g.kw, g.sw, g.pw, g.dw).count) return false;
+    return true;
+}
+
+template <int CG, bool FAST, bool QUADS>
+int launch_t(const GxGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
+    auto kern = adder_gx_gather_kernel<CG, FAST, QUADS>;
+    const int se = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
+    if (se != ADDER_OK) return se;
+    kern<<<grid, GATHER_THREADS, smem, stream>>>(a);
+    return launched();
+}
+
+template <bool FAST, bool QUADS>
+int launch_g(int cg, const GxGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
+    if (cg == 16) return launch_t<16, FAST, QUADS>(a, grid, smem, stream);
+    if (cg == 8) return launch_t<8, FAST, QUADS>(a, grid, smem, stream);
+    return launch_t<4, FAST, QUADS>(a, grid, smem, stream);
+}
+
+int plan(const ConvGeom& g, int first, GxGatherArgs& a, dim3& grid, bool& more) {
+    const bool single = single_class(g);
+    int n, total;
+    more = fill_classes(g, first, a, n, total, single);
+    a.Ci = g.Ci; a.H = g.H; a.W = g.W; a.Co = g.Co; a.Ho = g.Ho; a.Wo = g.Wo; a.KK = g.kh * g.kw; a.sh = g.sh; a.sw = g.sw;
+    a.CK = ceil_div(g.Co, ceil_div(g.Co, GATHER_CK));
+    const int cg = choose_groups((long long)a.m[0].P * n, n, g.Ci);
+    grid = dim3((unsigned)ceil_div(a.m[0].P, GATHER_THREADS / cg * 8), (unsigned)ceil_div(g.Ci, cg * RC), (unsigned)n);
+    return cg;
+}
+
+}  // namespace
+
+int describe_gx_gather(const ConvGeom& g, int fast, char* buf, size_t n) {
+    GxGatherArgs a;
+    dim3 grid;
+    bool more;
+    const int cg = plan(g, 0, a, grid, more);
+    return snprintf(buf, n, "gx gather k=%dx%d fast=%d classes=%u TC=%d TP=%d threads=%d smem=%zu grid=(%u,%u) status=0", g.kh, g.kw,
+                    fast, grid.z, cg * RC, GATHER_THREADS / cg * 8, GATHER_THREADS, smem_bytes(cg), grid.x, grid.y);
+}
+
+int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const float* w, float* gx, int fast, int accumulate,
+                     cudaStream_t stream) {
+    bool more = true;
+    for (int first = 0; more; first += MAX_CLASSES) {
+        GxGatherArgs a;
+        dim3 grid;
+        const int cg = plan(g, first, a, grid, more);
+        if (grid.y > 65535) return ADDER_ERR_UNSUPPORTED;
+        a.gout = gout; a.x = x; a.w = w; a.gx = gx; a.accumulate = accumulate;
+        const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gx)) & 15) == 0;
+        const bool unit = g.sh == 1 && g.sw == 1;
+        a.vec_io = unit && (g.H * g.W) % 4 == 0 && aligned;
+        a.w_quads = a.KK == 1 && g.Ci % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
+        a.fill_block = single_class(g) && !accumulate;
+        a.fill_quads = a.fill_block && g.sh == 2 && g.sw == 2 && g.W == 2 * a.m[0].PW && g.H == 2 * a.m[0].PH && a.m[0].PW % 4 == 0 &&
+                       (reinterpret_cast<uintptr_t>(gx) & 15) == 0;
+        // the gradient is read pixel by pixel in order: 1x1 kernels whose class (0, 0) is the output plane
+        const bool quads = g.kh == 1 && g.kw == 1 && g.ph == 0 && g.pw == 0 && a.m[0].PH == g.Ho && a.m[0].PW == g.Wo && grid.z == 1 &&
+                           (g.Ho * g.Wo) % 4 == 0 && (reinterpret_cast<uintptr_t>(gout) & 15) == 0;
+        const size_t smem = smem_bytes(cg);
+        const int st = fast ? (quads ? launch_g<true, true>(cg, a, grid, smem, stream) : launch_g<true, false>(cg, a, grid, smem, stream))
+                            : (quads ? launch_g<false, true>(cg, a, grid, smem, stream) : launch_g<false, false>(cg, a, grid, smem, stream));
+        if (st != ADDER_OK) return st;
+    }
+    return ADDER_OK;
+}
+
+}  // namespace adder

@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(PW_THREADS) adder_pw_gx_kernel(const PwArgs a)
             const float wv[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const float s = FAST ? __saturatef(wv[k] + xv[q + k]) : fminf(fmaxf(wv[k] - xv[q + k], -1.f), 1.f);
+                const float s = FAST ? __saturatef(wv[k] + xv[q + k]) : clamp_unit(wv[k] - xv[q + k]);
                 acc[q + k] = fmaf(s, gv, acc[q + k]);
             }
         }

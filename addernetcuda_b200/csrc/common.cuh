@@ -94,6 +94,14 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
     return r;
 }
 
+// clamp(d, -1, 1), exactly, in one instruction: the smaller magnitude of d and 1 with the sign of d.
+// fminf(fmaxf(d, -1), 1) is two instructions of the half-rate pipe.
+__device__ __forceinline__ float clamp_unit(float d) {
+    float r;
+    asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(r) : "f"(d), "f"(1.0f));
+    return r;
+}
+
 // Loads N consecutive floats from shared memory into registers.  When ALIGNED the address is a
 // multiple of 16 bytes and the run is fetched with 128-/64-bit loads (10 values = 2 x LDS.128 + 1 x
 // LDS.64 instead of 10 scalar loads); otherwise one scalar load per value.

@@ -8,6 +8,14 @@
 
 namespace adder {
 
+// Geometry of a layer with any kernel extent, stride, padding and dilation: what the gathering kernels take.
+struct ConvGeom {
+    int N, Ci, H, W, Co, Ho, Wo, kh, kw, sh, sw, ph, pw, dh, dw;
+};
+inline ConvGeom conv_geom(const Geom& g) {
+    return {g.N, g.Ci, g.H, g.W, g.Co, g.Ho, g.Wo, g.k, g.k, g.stride, g.stride, g.pad, g.pad, 1, 1};
+}
+
 // Optional overrides of the tile heuristics (0 = choose automatically).  Used for tuning sweeps.
 struct TileHint {
     int threads = 0;   // CTA size target
@@ -114,6 +122,15 @@ size_t gw_workspace_bytes(const Geom& g, const TileHint& hint);
 int launch_gw(const Geom& g, const float* gout, const float* x, const float* w, float* gw, float eta,
               float* out_norm, int accumulate, void* workspace, size_t workspace_bytes, const TileHint& hint,
               cudaStream_t s);
+
+// Channels x pixels tiles with a gathered operand (adder_fwd_gather.cu, adder_gx_gather.cu)
+int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* out, cudaStream_t s, double* stats = nullptr,
+                      int stat_slices = 0);
+int fwd_gather_stat_slices(const ConvGeom& g);
+int describe_fwd_gather(const ConvGeom& g, char* buf, size_t n);
+int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const float* w, float* gx, int fast, int accumulate,
+                     cudaStream_t s);
+int describe_gx_gather(const ConvGeom& g, int fast, char* buf, size_t n);
 
 // 1x1 stride-2 layers with at most 64 channels: one thread per output position (adder_pointwise.cu).
 // Chosen automatically unless a tile hint asks for the tiled kernels.
