@@ -893,11 +893,11 @@ static int choose_gx_rw(const Geom& g, const TileHint& hint) {
     else { if (fast) { CALL(KS_, S_, 8, 4, true) } else { CALL(KS_, S_, 8, 4, false) } }
 
 // Which layers take the gathering kernel (adder_gx_gather.cu): see fwd_uses_gather for what the two trade.  1x1 kernels
-// (1024->256 14x14 at batch 256, exact clamp: 2697 -> 1343 us), wide stride-2 layers (128->128 56x56: 2438 -> 888), planes
-// whose rows no segment width divides (27->45 29x31: 240 -> 106), and wide 3x3 layers in the exact form (256->256 14x14: 4988 ->
-// 3312).  The saturating form of adder_gx_kernel with 7-pixel segments is as fast there (2871 against 2954 us) and stays.
-// The rule does not look at the batch: an image's result must not depend on it.
-static bool gx_uses_gather(const Geom& g, int fast, const TileHint& hint) {
+// (1024->256 14x14 at batch 256: 2697 -> 1339 us exact, 2077 -> 1125 saturating), wide stride-2 layers (128->128 56x56 at
+// batch 64: 2438 -> 894), planes whose rows no segment width divides (27->45 29x31: 240 -> 102), and wide 3x3 layers (256->256
+// 14x14: 4988 -> 3342 exact, 2871 -> 2844 saturating; 64->64 56x56: 1365 -> 840 and 805 -> 715).
+// The rule does not look at the batch: the kernels add in different orders, and an image's result must not depend on it.
+static bool gx_uses_gather(const Geom& g, const TileHint& hint) {
     TileHint h = hint;
     h.variant = 0;
     if (!h.is_default()) return false;
@@ -905,10 +905,7 @@ static bool gx_uses_gather(const Geom& g, int fast, const TileHint& hint) {
     if (g.k == 1) return true;
     const int c = g.Ci < g.Co ? g.Ci : g.Co;
     if (g.stride == 2) return c >= 64;
-    const bool sevens = g.W % 8 != 0 && g.W % 7 == 0;
-    if (g.W % 4 != 0 && !sevens) return true;
-    if (fast && sevens) return false;
-    return c >= 128 || (c >= 64 && g.H * g.W >= 196);
+    return (g.W % 4 != 0 && g.W % 7 != 0) || c >= 128 || (c >= 64 && g.H * g.W >= 196);
 }
 
 int describe_gx(const Geom& layer, int fast, const TileHint& hint, char* buf, size_t n) {
@@ -918,7 +915,7 @@ int describe_gx(const Geom& layer, int fast, const TileHint& hint, char* buf, si
                  "grid=(%d,%d) status=0", g.stride, fast, ceil_div(g.N * g.Ho * g.Wo, 256), ceil_div(g.Ci, 16));
         return ADDER_OK;
     }
-    if (gx_uses_gather(layer, fast, hint)) {
+    if (gx_uses_gather(layer, hint)) {
         const int w = describe_gx_gather(conv_geom(layer), fast, buf, n);
         if (w < 0 || (size_t)w + 16 >= n) return ADDER_OK;
         buf += w; n -= w;
@@ -945,7 +942,7 @@ int launch_gx(const Geom& layer, const float* gout, const float* x, const float*
               int accumulate, const TileHint& hint, cudaStream_t stream) {
     const Geom g = flatten_pointwise(layer, true);
     if (hint.is_default() && pointwise_applicable(g)) return launch_pointwise_gx(g, gout, x, w, gx, fast, accumulate, stream);
-    if (gx_uses_gather(layer, fast, hint)) return launch_gx_gather(conv_geom(layer), gout, x, w, gx, fast, accumulate, stream);
+    if (gx_uses_gather(layer, hint)) return launch_gx_gather(conv_geom(layer), gout, x, w, gx, fast, accumulate, stream);
     const int rw = choose_gx_rw(gx_tiling_geom(g), hint);
 #define ADDER_GX_LAUNCH(KS_, S_, RW_, RC_, FAST_) \
     return launch_gx_t<KS_, S_, RW_, RC_, FAST_>(g, gout, x, w, gx, accumulate, hint, stream);

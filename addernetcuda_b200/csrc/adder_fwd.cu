@@ -409,31 +409,28 @@ static void choose_fwd_tile(const Geom& g, const TileHint& hint, int& rw, int& r
     }
 }
 
-#define ADDER_FWD_DISPATCH(CALL)                                                            \
-    if (g.k == 3 && g.stride == 1) { ADDER_FWD_TILES(3, 1, CALL) }                          \
-    else if (g.k == 3 && g.stride == 2) { ADDER_FWD_TILES(3, 2, CALL) }                     \
-    else if (g.k == 1 && g.stride == 1) { ADDER_FWD_TILES(1, 1, CALL) }                     \
-    else if (g.k == 1 && g.stride == 2) { ADDER_FWD_TILES(1, 1, CALL) }
+#define ADDER_FWD_DISPATCH(CALL) if (g.k == 3 && g.stride == 1) { ADDER_FWD_TILES(3, 1, CALL) }
 #define ADDER_FWD_TILES(KS_, S_, CALL)                                                      \
     if (rw == 7) { CALL(KS_, S_, 7, 8) }                                                    \
     else if (rw == 8 && rm == 8) { CALL(KS_, S_, 8, 8) }                                    \
     else if (rw == 8 && rm == 4) { CALL(KS_, S_, 8, 4) }                                    \
     else if (rw == 4 && rm == 4) { CALL(KS_, S_, 4, 4) }
 
-// Which layers take the gathering kernel (adder_fwd_gather.cu).  Its tile is 64 channels x 128 pixels whatever the plane, but it
-// stages every tap's pixels again, where adder_fwd_kernel shifts one haloed patch: 1x1 kernels have no halo (1024->256 14x14:
-// 1289 -> 928 us at batch 256), a stride-2 patch is mostly halo (128->128 56x56: 791 -> 629 us at batch 64), and with
-// 128 channels, or 64 on planes of 14x14 and more, the staging is small beside the arithmetic (256->256 14x14: 2446 ->
-// 2145 us; but 32->32 16x16: 54 -> 65 us, and 64->64 8x8 too few tiles).  The rule does not look at the batch: the two
-// kernels add in different orders, and an image's result must not depend on its batch.
+// Which layers stay with adder_fwd_kernel; every other takes the gathering kernel (adder_fwd_gather.cu), whose tile does not
+// care for the plane but which stages every tap's pixels again where this one shifts one haloed patch.  The two add in the
+// same order, so the choice does not show in the result.  The patch pays for stride-1 3x3 layers whose rows are whole
+// 8-pixel segments, with few enough output channels that staging is a large share of the work (batch 256: 16->16 32x32 47
+// against 57 us, 64->64 8x8 56 against 66; but 64->64 56x56 at batch 64: 679 against 536, 256->256 14x14: 2446 against 2128,
+// 16->32 stride 2: 36 against 30), once the launch has enough outputs to fill the SMs with such tiles (64->64 8x8: 22 against 14 us
+// at batch 32, 23 against 30 at 64).
 static bool fwd_uses_gather(const Geom& g, const TileHint& hint) {
+    if (g.k != 3 || g.stride != 1) return true;
     TileHint h = hint;
     h.variant = 0;
     if (!h.is_default()) return false;
     if (hint.variant) return hint.variant == 2;
-    if (g.k == 1) return true;
-    const int c = g.Ci < g.Co ? g.Ci : g.Co;
-    return g.stride == 2 ? c >= 64 : c >= 128 || (c >= 64 && g.H * g.W >= 196);
+    const bool narrow = g.Co <= 32 || (g.Co <= 64 && g.Ci <= 64 && g.H * g.W < 196);
+    return !(narrow && g.W % 8 == 0 && (long long)g.N * g.Ho * g.Wo * g.Co >= (1 << 18));
 }
 
 int describe_fwd(const Geom& layer, const TileHint& hint, char* buf, size_t n) {

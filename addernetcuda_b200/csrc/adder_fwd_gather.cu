@@ -23,14 +23,23 @@ struct FwdGatherArgs {
     int vec_store;           // planes are whole quads and `out` is 16-byte aligned
 };
 
-template <int RM, int CG, bool QUADS>
-__global__ void __launch_bounds__(GATHER_THREADS, 4) adder_fwd_gather_kernel(const __grid_constant__ FwdGatherArgs a) {
-    constexpr int PG = GATHER_THREADS / CG, TC = CG * RM, TP = PG * 8, WP = TC + 4;
+// RM channels x RP pixels per thread (RP = 8: two quads half a tile apart), CG channel groups, ST stages, MB CTAs per SM.
+template <int RM_, int RP_, int CG_, int ST_, int MB_>
+struct FwdTile {
+    static constexpr int RM = RM_, RP = RP_, CG = CG_, ST = ST_, MB = MB_;
+    static constexpr int PG = GATHER_THREADS / CG, TC = CG * RM, TP = PG * RP, WP = TC + 4;
+    static constexpr int PQ = RP == 8 ? 4 : RP;                 // consecutive pixels of a thread
+};
+
+template <class T, int MODE>
+__global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel(const __grid_constant__ FwdGatherArgs a) {
+    constexpr int RM = T::RM, RP = T::RP, CG = T::CG, PG = T::PG, TC = T::TC, TP = T::TP, WP = T::WP, PQ = T::PQ, ST = T::ST;
     constexpr int COLS = TP > GATHER_THREADS ? TP / GATHER_THREADS : 1;
-    constexpr int XS = GATHER_CK * TP, WS = GATHER_CK * WP;
+    constexpr int CK = MODE == GATHER_NINE ? 9 * GATHER_NINE_CH : GATHER_CK;      // rows of a stage
+    constexpr int XS = CK * TP, WS = CK * WP;
     extern __shared__ __align__(16) float smem[];
     float* const Xs = smem;
-    float* const Ws = smem + GATHER_STAGES * XS;
+    float* const Ws = smem + ST * XS;
 
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int cg = (wid % (CG / 4)) * 4 + (lane >> 3), pg = (wid / (CG / 4)) * 8 + (lane & 7);
@@ -38,79 +47,105 @@ __global__ void __launch_bounds__(GATHER_THREADS, 4) adder_fwd_gather_kernel(con
     const size_t image = (size_t)a.Ci * a.H * a.W;
 
     GatherPixel px[COLS];
-    if (QUADS) {
+    unsigned mask[COLS];
+    if (MODE == GATHER_QUADS) {
         px[0].decode(a.m, a.x, p0 + 4 * (tid % (TP / 4)), image);
         px[0].base += px[0].row * a.W + px[0].col;
     } else {
 #pragma unroll
-        for (int q = 0; q < COLS; ++q) px[q].decode(a.m, a.x, p0 + (COLS > 1 ? tid + q * GATHER_THREADS : tid % TP), image);
+        for (int q = 0; q < COLS; ++q) {
+            px[q].decode(a.m, a.x, p0 + (COLS > 1 ? tid + q * GATHER_THREADS : tid % TP), image);
+            if (MODE == GATHER_NINE) mask[q] = nine_mask(px[q], a.m, a.H, a.W);
+        }
     }
     GatherChunk fc;              // position of the next chunk to stage
     const int ck4 = round_up(a.CK, 4);
     auto fill = [&](int stage) {
-        const int nch = min(a.CK, a.Ci - fc.c0);
-        if (QUADS) gather_quads<TP>(Xs + stage * XS, px[0].base, px[0].ok, a.x, fc.c0, nch, ck4, a.H * a.W, tid);
-        else gather_pixels<TP>(Xs + stage * XS, px, a.x, a.m, fc, nch, ck4, a.H, a.W, tid);
-        // weights [input channel of the chunk][output channel of the tile]: a warp copies 8 channels of 4 outputs
+        int nk, rows, wk;        // reduction steps that exist, rows to stage, and the first one's weight index
+        if constexpr (MODE == GATHER_NINE) {
+            const int nch = min(GATHER_NINE_CH, a.Ci - fc.c0);
+            gather_nine<TP>(Xs + stage * XS, px, mask, a.m, fc.c0, nch, a.H, a.W, tid);
+            nk = nch * 9; rows = CK; wk = fc.c0 * 9;
+        } else {
+            nk = min(a.CK, a.Ci - fc.c0); rows = ck4;
+            if (MODE == GATHER_QUADS) gather_quads<TP>(Xs + stage * XS, px[0].base, px[0].ok, a.x, fc.c0, nk, ck4, a.H * a.W, tid);
+            else gather_pixels<TP>(Xs + stage * XS, px, a.x, a.m, fc, nk, ck4, a.H, a.W, tid);
+            wk = fc.c0 * a.KK + a.m.wt0 + fc.i * a.m.dwi + fc.j * a.m.dwj;
+        }
+        // weights [reduction step][output channel of the tile]: a warp copies 8 steps of 4 outputs
+        const int kstep = MODE == GATHER_NINE ? 1 : a.KK;
         const int k8 = tid & 7, c4 = tid >> 3;
         float* ws = Ws + stage * WS + k8 * WP + c4;
         const int row = a.Ci * a.KK, ncol = a.Co - co0 - c4;
-        const float* wsrc = a.w + ((co0 + c4) * row + (fc.c0 + k8) * a.KK + a.m.wt0 + fc.i * a.m.dwi + fc.j * a.m.dwj);
+        const float* wsrc = a.w + ((co0 + c4) * row + k8 * kstep + wk);
 #pragma unroll
-        for (int kb = 0; kb < GATHER_CK; kb += 8) {
-            if (kb + k8 >= ck4) break;
-            const bool okk = kb + k8 < nch;
+        for (int kb = 0; kb < CK; kb += 8) {
+            if (kb + k8 >= rows) break;
+            const bool okk = kb + k8 < nk;
 #pragma unroll
             for (int c = 0; c < TC; c += GATHER_THREADS / 8) {
+                if (TC % (GATHER_THREADS / 8) != 0 && c + c4 >= TC) break;
                 const bool ok = okk & (c < ncol);
-                cp_async4(ws + kb * WP + c, ok ? wsrc + (c * row + kb * a.KK) : a.w, ok);
+                cp_async4(ws + kb * WP + c, ok ? wsrc + (c * row + kb * kstep) : a.w, ok);
             }
         }
-        fc.next(a.m, a.CK);
+        if (MODE == GATHER_NINE) fc.c0 += GATHER_NINE_CH;
+        else fc.next(a.m, a.CK);
     };
 
-    float acc[RM][8];
+    float acc[RM][RP];
 #pragma unroll
     for (int m = 0; m < RM; ++m)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[m][j] = 0.f;
+        for (int j = 0; j < RP; ++j) acc[m][j] = 0.f;
 
-#pragma unroll
-    for (int s = 0; s < GATHER_STAGES - 1; ++s) {
+#pragma unroll 1
+    for (int s = 0; s < ST - 1; ++s) {
         if (s < a.nchunks) fill(s);
         cp_async_commit();
     }
     GatherChunk cc;
-    int stage = 0, fstage = GATHER_STAGES - 1;
-    for (int c = 0; c < a.nchunks; ++c) {
-        cp_async_wait<GATHER_STAGES - 2>();
-        __syncthreads();
-        if (c + GATHER_STAGES - 1 < a.nchunks) fill(fstage);
-        cp_async_commit();
-        const float* xs = Xs + stage * XS + pg * 4;
-        const float* ws = Ws + stage * WS + cg * RM;
-        const int nk = min(ck4, round_up(a.Ci - cc.c0, 4));
+    int stage = 0, fstage = ST - 1;
 #pragma unroll 1
+    for (int c = 0; c < a.nchunks; ++c) {
+        cp_async_wait<ST - 2>();
+        __syncthreads();
+        if (c + ST - 1 < a.nchunks) fill(fstage);
+        cp_async_commit();
+        const float* xs = Xs + stage * XS + pg * PQ;
+        const float* ws = Ws + stage * WS + cg * RM;
+        const int nk = MODE == GATHER_NINE ? CK : min(ck4, round_up(a.Ci - cc.c0, 4));
+#pragma unroll (RM * RP >= 64 ? 1 : RM * RP >= 32 ? 2 : 4)
         for (int k = 0; k < nk; ++k) {
-            float xv[8], wv[RM];
-            {
-                const float4 q0 = *reinterpret_cast<const float4*>(xs + k * TP);
-                const float4 q1 = *reinterpret_cast<const float4*>(xs + k * TP + TP / 2);
-                xv[0] = q0.x; xv[1] = q0.y; xv[2] = q0.z; xv[3] = q0.w; xv[4] = q1.x; xv[5] = q1.y; xv[6] = q1.z; xv[7] = q1.w;
-            }
+            float xv[RP], wv[RM];
 #pragma unroll
-            for (int m = 0; m < RM; m += 4) {
-                const float4 q = *reinterpret_cast<const float4*>(ws + k * WP + m);
-                wv[m] = q.x; wv[m + 1] = q.y; wv[m + 2] = q.z; wv[m + 3] = q.w;
+            for (int h = 0; h < RP / PQ; ++h) {
+                if constexpr (PQ == 4) {
+                    const float4 q = *reinterpret_cast<const float4*>(xs + k * TP + h * (TP / 2));
+                    xv[4 * h] = q.x; xv[4 * h + 1] = q.y; xv[4 * h + 2] = q.z; xv[4 * h + 3] = q.w;
+                } else {
+                    const float2 q = *reinterpret_cast<const float2*>(xs + k * TP);
+                    xv[0] = q.x; xv[1] = q.y;
+                }
             }
-            uint64_t nx2[8];
+            if constexpr (RM >= 4) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) nx2[j] = pack2(-xv[j], -xv[j]);
+                for (int m = 0; m < RM; m += 4) {
+                    const float4 q = *reinterpret_cast<const float4*>(ws + k * WP + m);
+                    wv[m] = q.x; wv[m + 1] = q.y; wv[m + 2] = q.z; wv[m + 3] = q.w;
+                }
+            } else {
+                const float2 q = *reinterpret_cast<const float2*>(ws + k * WP);
+                wv[0] = q.x; wv[1] = q.y;
+            }
+            uint64_t nx2[RP];
+#pragma unroll
+            for (int j = 0; j < RP; ++j) nx2[j] = pack2(-xv[j], -xv[j]);
 #pragma unroll
             for (int m = 0; m < RM; m += 2) {
                 const uint64_t w2 = pack2(wv[m], wv[m + 1]);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
+                for (int j = 0; j < RP; ++j) {
                     float d0, d1;
                     unpack2(add2(w2, nx2[j]), d0, d1);
                     acc[m][j] += fabsf(d0);
@@ -118,38 +153,40 @@ __global__ void __launch_bounds__(GATHER_THREADS, 4) adder_fwd_gather_kernel(con
                 }
             }
         }
-        cc.next(a.m, a.CK);
-        if (++stage == GATHER_STAGES) stage = 0;
-        if (++fstage == GATHER_STAGES) fstage = 0;
+        if (MODE != GATHER_NINE) cc.next(a.m, a.CK);
+        if (++stage == ST) stage = 0;
+        if (++fstage == ST) fstage = 0;
     }
 
     const int PHW = a.m.PH * a.m.PW;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int p = p0 + h * (TP / 2) + pg * 4;
-        if (a.vec_store) {
-            if (p >= a.m.P) continue;
-            uint32_t n, r;
-            a.m.d_phw.divmod(p, n, r);
-            float* o = a.out + ((size_t)n * a.Co + co0 + cg * RM) * PHW + r;
-#pragma unroll
-            for (int m = 0; m < RM; ++m) {
-                if (co0 + cg * RM + m >= a.Co) break;
-                *reinterpret_cast<float4*>(o + (size_t)m * PHW) =
-                    make_float4(-acc[m][4 * h], -acc[m][4 * h + 1], -acc[m][4 * h + 2], -acc[m][4 * h + 3]);
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (p + j >= a.m.P) continue;
+    for (int h = 0; h < RP / PQ; ++h) {
+        const int p = p0 + h * (TP / 2) + pg * PQ;
+        if constexpr (PQ == 4) {
+            if (a.vec_store) {
+                if (p >= a.m.P) continue;
                 uint32_t n, r;
-                a.m.d_phw.divmod(p + j, n, r);
+                a.m.d_phw.divmod(p, n, r);
                 float* o = a.out + ((size_t)n * a.Co + co0 + cg * RM) * PHW + r;
 #pragma unroll
                 for (int m = 0; m < RM; ++m) {
                     if (co0 + cg * RM + m >= a.Co) break;
-                    o[(size_t)m * PHW] = -acc[m][4 * h + j];
+                    *reinterpret_cast<float4*>(o + (size_t)m * PHW) =
+                        make_float4(-acc[m][4 * h], -acc[m][4 * h + 1], -acc[m][4 * h + 2], -acc[m][4 * h + 3]);
                 }
+                continue;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < PQ; ++j) {
+            if (p + j >= a.m.P) continue;
+            uint32_t n, r;
+            a.m.d_phw.divmod(p + j, n, r);
+            float* o = a.out + ((size_t)n * a.Co + co0 + cg * RM) * PHW + r;
+#pragma unroll
+            for (int m = 0; m < RM; ++m) {
+                if (co0 + cg * RM + m >= a.Co) break;
+                o[(size_t)m * PHW] = -acc[m][PQ * h + j];
             }
         }
     }
@@ -163,8 +200,8 @@ __global__ void __launch_bounds__(GATHER_THREADS, 4) adder_fwd_gather_kernel(con
     for (int m = 0; m < RM; ++m) {
         float s = 0.f, q = 0.f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (p0 + (j >> 2) * (TP / 2) + pg * 4 + (j & 3) < a.m.P) { s -= acc[m][j]; q = fmaf(acc[m][j], acc[m][j], q); }
+        for (int j = 0; j < RP; ++j)
+            if (p0 + (j / PQ) * (TP / 2) + pg * PQ + (j % PQ) < a.m.P) { s -= acc[m][j]; q = fmaf(acc[m][j], acc[m][j], q); }
         st[(cg * RM + m) * (PG + 1) + pg] = make_float2(s, q);
     }
     __syncthreads();
@@ -190,31 +227,43 @@ __global__ void __launch_bounds__(GATHER_THREADS, 4) adder_fwd_gather_kernel(con
 
 namespace {
 
-struct Tile { int rm, cg; };
-constexpr Tile kTiles[] = {{8, 8}, {8, 16}, {8, 4}, {4, 16}, {4, 8}, {4, 4}};
+// The tiles: large ones have the fewest loads per term, small ones give a small layer more threads.  X(RM, RP, CG, ST, MB)
+#define ADDER_FWD_GATHER_TILES(X) \
+    X(8, 8, 8, 2, 4) X(8, 8, 16, 2, 4) X(8, 8, 4, 2, 4) X(4, 8, 16, 3, 4) X(4, 8, 8, 3, 4) X(4, 8, 4, 2, 4) \
+    X(4, 4, 16, 4, 6) X(4, 4, 8, 4, 6) X(4, 4, 4, 4, 6) X(2, 2, 8, 8, 8) X(2, 2, 4, 8, 8)
 
-// What differs between the tiles is how many of their outputs are past the ends of the layer (channels rounded up to TC, pixels
-// to TP), how evenly they fill the SMs, and how much is staged per reduction step (TC + TP values, about 4 lane instructions each
-// against 2.2 per term).  An SM runs its CTAs side by side, so its time is its number of tiles; with fewer than four resident
-// CTAs (16 warps) it does not reach its full rate.
-Tile choose_tile(int P, int Co) {
-    static const double rate[4] = {0.5, 0.8, 0.93, 1.0};
-    Tile best = kTiles[0];
+struct Tile { int rm, rp, cg, st, tc, tp; };
+constexpr Tile kTiles[] = {
+#define X(RM, RP, CG, ST, MB) {RM, RP, CG, ST, RM * CG, RP * GATHER_THREADS / CG},
+    ADDER_FWD_GATHER_TILES(X)
+#undef X
+};
+
+// Time of the layer in cycles per reduction step, for each tile: a thread's step is 2.25 cycles of its scheduler per term, about 6
+// for its loads, and its share of the staging (about 7 instructions per value).  An SM's time is the number of its tiles
+// times that; with one or two tiles, so one or two warps per scheduler, the latency of the loads shows as well (about 28 cycles).
+int choose_tile(int P, int Co) {
+    int best = 0;
     double best_cost = 1e300;
     const int sms = sm_count();
-    for (const Tile& t : kTiles) {
-        const int tc = t.rm * t.cg, tp = GATHER_THREADS / t.cg * 8;
-        const long long tiles = (long long)ceil_div(P, tp) * ceil_div(Co, tc);
+    for (int i = 0; i < (int)(sizeof(kTiles) / sizeof(kTiles[0])); ++i) {
+        const Tile& t = kTiles[i];
+        const long long tiles = (long long)ceil_div(P, t.tp) * ceil_div(Co, t.tc);
         const long long per_sm = (tiles + sms - 1) / sms;
-        const double cost = per_sm / rate[per_sm < 4 ? per_sm - 1 : 3] * (2.2 * tc * tp + 4.0 * (tc + tp));
-        if (cost < best_cost) { best_cost = cost; best = t; }
+        const double step = 2.25 * t.rm * t.rp + 6.0 + 7.0 * (t.tc + t.tp) / GATHER_THREADS;
+        double cost = per_sm * step;
+        if (per_sm <= 2) cost += 28.0;
+        if (cost < best_cost) { best_cost = cost; best = i; }
     }
     return best;
 }
 
-size_t smem_bytes(const Tile& t) {
-    const int tc = t.rm * t.cg, tp = GATHER_THREADS / t.cg * 8;
-    return (size_t)GATHER_STAGES * GATHER_CK * (tp + tc + 4) * sizeof(float);
+int stage_rows(const ConvGeom& g) { return g.kh == 3 && g.kw == 3 ? 9 * GATHER_NINE_CH : GATHER_CK; }
+
+size_t smem_bytes(const Tile& t, int rows) {
+    const size_t stages = (size_t)t.st * rows * (t.tp + t.tc + 4) * sizeof(float);
+    const size_t stats = (size_t)t.tc * (GATHER_THREADS / t.cg + 1) * sizeof(float2);
+    return stages > stats ? stages : stats;
 }
 
 GatherMap fwd_map(const ConvGeom& g) {
@@ -228,40 +277,37 @@ GatherMap fwd_map(const ConvGeom& g) {
     return m;
 }
 
-template <int RM, int CG, bool QUADS>
+template <class T, int MODE>
 int launch_t(const FwdGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
-    auto kern = adder_fwd_gather_kernel<RM, CG, QUADS>;
+    auto kern = adder_fwd_gather_kernel<T, MODE>;
     const int se = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
     if (se != ADDER_OK) return se;
     kern<<<grid, GATHER_THREADS, smem, stream>>>(a);
     return launched();
 }
 
-template <bool QUADS>
-int launch_q(const Tile& t, const FwdGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
-    if (t.rm == 8) {
-        if (t.cg == 16) return launch_t<8, 16, QUADS>(a, grid, smem, stream);
-        if (t.cg == 8) return launch_t<8, 8, QUADS>(a, grid, smem, stream);
-        return launch_t<8, 4, QUADS>(a, grid, smem, stream);
-    }
-    if (t.cg == 16) return launch_t<4, 16, QUADS>(a, grid, smem, stream);
-    if (t.cg == 8) return launch_t<4, 8, QUADS>(a, grid, smem, stream);
-    return launch_t<4, 4, QUADS>(a, grid, smem, stream);
+template <int MODE>
+int launch_mode(int tile, const FwdGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
+    int i = 0;
+#define X(RM, RP, CG, ST, MB) \
+    if (tile == i++) return launch_t<FwdTile<RM, RP, CG, ST, MB>, MODE>(a, grid, smem, stream);
+    ADDER_FWD_GATHER_TILES(X)
+#undef X
+    return ADDER_ERR_INTERNAL;
 }
 
 }  // namespace
 
 int fwd_gather_stat_slices(const ConvGeom& g) {
     const int P = g.N * g.Ho * g.Wo;
-    return ceil_div(P, GATHER_THREADS / choose_tile(P, g.Co).cg * 8);
+    return ceil_div(P, kTiles[choose_tile(P, g.Co)].tp);
 }
 
 int describe_fwd_gather(const ConvGeom& g, char* buf, size_t n) {
     const int P = g.N * g.Ho * g.Wo;
-    const Tile t = choose_tile(P, g.Co);
-    const int tc = t.rm * t.cg, tp = GATHER_THREADS / t.cg * 8;
-    return snprintf(buf, n, "fwd gather k=%dx%d RM=%d TC=%d TP=%d threads=%d smem=%zu grid=(%d,%d) status=0", g.kh, g.kw, t.rm, tc, tp,
-                    GATHER_THREADS, smem_bytes(t), ceil_div(P, tp), ceil_div(g.Co, tc));
+    const Tile& t = kTiles[choose_tile(P, g.Co)];
+    return snprintf(buf, n, "fwd gather k=%dx%d RM=%d RP=%d TC=%d TP=%d threads=%d smem=%zu grid=(%d,%d) status=0", g.kh, g.kw, t.rm,
+                    t.rp, t.tc, t.tp, GATHER_THREADS, smem_bytes(t, stage_rows(g)), ceil_div(P, t.tp), ceil_div(g.Co, t.tc));
 }
 
 int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* out, cudaStream_t stream, double* stats,
@@ -270,18 +316,21 @@ int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* 
     a.m = fwd_map(g);
     a.x = x; a.w = w; a.out = out; a.stats = stats;
     a.Ci = g.Ci; a.H = g.H; a.W = g.W; a.Co = g.Co; a.KK = g.kh * g.kw;
-    const int blocks = ceil_div(g.Ci, GATHER_CK);
-    a.CK = ceil_div(g.Ci, blocks);              // evenly sized channel blocks
-    a.nchunks = ceil_div(g.Ci, a.CK) * a.KK;
+    const bool nine = g.kh == 3 && g.kw == 3;
+    a.CK = nine ? GATHER_NINE_CH : ceil_div(g.Ci, ceil_div(g.Ci, GATHER_CK));              // evenly sized channel blocks
+    a.nchunks = ceil_div(g.Ci, a.CK) * (nine ? 1 : a.KK);
     const bool whole_quads = (g.Ho * g.Wo) % 4 == 0;
     a.vec_store = whole_quads && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
     const bool quads = whole_quads && a.KK == 1 && g.sh == 1 && g.sw == 1 && g.ph == 0 && g.pw == 0 &&
                        (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-    const Tile t = choose_tile(a.m.P, g.Co);
-    const dim3 grid((unsigned)ceil_div(a.m.P, GATHER_THREADS / t.cg * 8), (unsigned)ceil_div(g.Co, t.rm * t.cg));
+    const int tile = choose_tile(a.m.P, g.Co);
+    const Tile& t = kTiles[tile];
+    const dim3 grid((unsigned)ceil_div(a.m.P, t.tp), (unsigned)ceil_div(g.Co, t.tc));
     if (grid.y > 65535) return ADDER_ERR_UNSUPPORTED;
     if (stats != nullptr && stat_slices != (int)grid.x) return ADDER_ERR_WORKSPACE;
-    return quads ? launch_q<true>(t, a, grid, smem_bytes(t), stream) : launch_q<false>(t, a, grid, smem_bytes(t), stream);
+    const size_t smem = smem_bytes(t, stage_rows(g));
+    if (nine) return launch_mode<GATHER_NINE>(tile, a, grid, smem, stream);
+    return quads ? launch_mode<GATHER_QUADS>(tile, a, grid, smem, stream) : launch_mode<GATHER_TAP>(tile, a, grid, smem, stream);
 }
 
 }  // namespace adder

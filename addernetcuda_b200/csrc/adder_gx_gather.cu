@@ -19,7 +19,6 @@
 namespace adder {
 
 namespace {
-constexpr int RC = 4;                   // input channels per thread (8 of them, at 3 CTAs per SM, measured 10-15 % slower)
 constexpr int FOLD = 4;                 // chunks per partial sum: at most 64 terms before it is folded into the total
 constexpr int MAX_CLASSES = 9;
 }
@@ -38,16 +37,25 @@ struct GxGatherArgs {
     int fill_quads;          // ... and four blocks of a row can be written as aligned 128-bit words
 };
 
-template <int CG, bool FAST, bool QUADS>
-__global__ void __launch_bounds__(GATHER_THREADS, 4) adder_gx_gather_kernel(const __grid_constant__ GxGatherArgs a) {
-    constexpr int PG = GATHER_THREADS / CG, TC = CG * RC, TP = PG * 8, WP = TC + 4;
+// RC channels x RP pixels per thread (RP = 8: two quads half a tile apart), CG channel groups, ST stages, MB CTAs per SM.
+// (8 channels x 8 pixels, at 3 CTAs per SM, measured 10-15 % slower than 4 x 8.)
+template <int RC_, int RP_, int CG_, int ST_, int MB_>
+struct GxTile {
+    static constexpr int RC = RC_, RP = RP_, CG = CG_, ST = ST_, MB = MB_;
+    static constexpr int PG = GATHER_THREADS / CG, TC = CG * RC, TP = PG * RP, WP = TC + 4;
+    static constexpr int PQ = RP == 8 ? 4 : RP;                 // consecutive pixels of a thread
+};
+
+template <class T, bool FAST, bool QUADS>
+__global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(const __grid_constant__ GxGatherArgs a) {
+    constexpr int RC = T::RC, RP = T::RP, CG = T::CG, TC = T::TC, TP = T::TP, WP = T::WP, PQ = T::PQ, ST = T::ST;
     constexpr int COLS = TP > GATHER_THREADS ? TP / GATHER_THREADS : 1;
     constexpr int ROWS = TP < GATHER_THREADS ? GATHER_THREADS / TP : 1;
     constexpr int GS = GATHER_CK * TP, WS = GATHER_CK * WP;
     extern __shared__ __align__(16) float smem[];
     float* const Gs = smem;
-    float* const Ws = smem + GATHER_STAGES * GS;
-    float4* const Tot = reinterpret_cast<float4*>(Ws + GATHER_STAGES * WS) + threadIdx.x;    // [8][threads]
+    float* const Ws = smem + ST * GS;
+    float4* const Tot = reinterpret_cast<float4*>(Ws + ST * WS) + threadIdx.x;    // [RC * RP / 4][threads]
 
     const GatherMap& m = a.m[blockIdx.z];
     const int p0 = blockIdx.x * TP, ci0 = blockIdx.y * TC;
@@ -98,79 +106,92 @@ __global__ void __launch_bounds__(GATHER_THREADS, 4) adder_gx_gather_kernel(cons
         fc.next(m, a.CK);
     };
 
-#pragma unroll
-    for (int s = 0; s < GATHER_STAGES - 1; ++s) {
+#pragma unroll 1
+    for (int s = 0; s < ST - 1; ++s) {
         if (s < nchunks) fill(s);
         cp_async_commit();
     }
 
-    // the thread's 8 pixels: input address (element offset of channel 0) and validity
-    float xv[RC][8];
+    // x of the thread's pixels
+    float xv[RC][RP];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int p = p0 + h * (TP / 2) + pg * 4;
-        if (a.vec_io) {
-            uint32_t n, r;
-            m.d_phw.divmod(p < m.P ? p : 0, n, r);
-            const float* xs = a.x + ((size_t)n * a.Ci + ci0 + cg * RC) * HW + r;
+    for (int h = 0; h < RP / PQ; ++h) {
+        const int p = p0 + h * (TP / 2) + pg * PQ;
+        if constexpr (PQ == 4) {
+            if (a.vec_io) {
+                uint32_t n, r;
+                m.d_phw.divmod(p < m.P ? p : 0, n, r);
+                const float* xs = a.x + ((size_t)n * a.Ci + ci0 + cg * RC) * HW + r;
 #pragma unroll
-            for (int c = 0; c < RC; ++c) {
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (p < m.P && ci0 + cg * RC + c < a.Ci) v = __ldg(reinterpret_cast<const float4*>(xs + (size_t)c * HW));
-                xv[c][4 * h] = v.x; xv[c][4 * h + 1] = v.y; xv[c][4 * h + 2] = v.z; xv[c][4 * h + 3] = v.w;
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                uint32_t n, r, y, x;
-                m.d_phw.divmod(p + j < m.P ? p + j : 0, n, r);
-                m.d_pw.divmod(r, y, x);
-                const float* xs = a.x + ((size_t)n * a.Ci + ci0 + cg * RC) * HW + ((int)y * a.sh + ry) * a.W + (int)x * a.sw + rx;
-#pragma unroll
-                for (int c = 0; c < RC; ++c)
-                    xv[c][4 * h + j] = (p + j < m.P && ci0 + cg * RC + c < a.Ci) ? __ldg(xs + (size_t)c * HW) : 0.f;
+                for (int c = 0; c < RC; ++c) {
+                    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (p < m.P && ci0 + cg * RC + c < a.Ci) v = __ldg(reinterpret_cast<const float4*>(xs + (size_t)c * HW));
+                    xv[c][4 * h] = v.x; xv[c][4 * h + 1] = v.y; xv[c][4 * h + 2] = v.z; xv[c][4 * h + 3] = v.w;
+                }
+                continue;
             }
         }
+#pragma unroll
+        for (int j = 0; j < PQ; ++j) {
+            uint32_t n, r, y, x;
+            m.d_phw.divmod(p + j < m.P ? p + j : 0, n, r);
+            m.d_pw.divmod(r, y, x);
+            const float* xs = a.x + ((size_t)n * a.Ci + ci0 + cg * RC) * HW + ((int)y * a.sh + ry) * a.W + (int)x * a.sw + rx;
+#pragma unroll
+            for (int c = 0; c < RC; ++c)
+                xv[c][PQ * h + j] = (p + j < m.P && ci0 + cg * RC + c < a.Ci) ? __ldg(xs + (size_t)c * HW) : 0.f;
+        }
     }
+    float acc[RC][RP];
 #pragma unroll
     for (int c = 0; c < RC; ++c)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) xv[c][j] = FAST ? fmaf(xv[c][j], -0.5f, 0.5f) : -xv[c][j];
-
-    float acc[RC][8];
-#pragma unroll
-    for (int c = 0; c < RC; ++c)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[c][j] = 0.f;
+        for (int j = 0; j < RP; ++j) {
+            xv[c][j] = FAST ? fmaf(xv[c][j], -0.5f, 0.5f) : -xv[c][j];
+            acc[c][j] = 0.f;
+        }
     float box[COLS];
 #pragma unroll
     for (int q = 0; q < COLS; ++q) box[q] = 0.f;
 
     GatherChunk cc;
-    int stage = 0, fstage = GATHER_STAGES - 1;
+    int stage = 0, fstage = ST - 1;
     for (int c = 0; c < nchunks; ++c) {
-        cp_async_wait<GATHER_STAGES - 2>();
+        cp_async_wait<ST - 2>();
         __syncthreads();
-        if (c + GATHER_STAGES - 1 < nchunks) fill(fstage);
+        if (c + ST - 1 < nchunks) fill(fstage);
         cp_async_commit();
-        const float* gs = Gs + stage * GS + pg * 4;
+        const float* gs = Gs + stage * GS + pg * PQ;
         const float* ws = Ws + stage * WS + cg * RC;
         const int nk = min(ck4, round_up(a.Co - cc.c0, 4));
 #pragma unroll 4
         for (int k = 0; k < nk; ++k) {
-            const float4 g0 = *reinterpret_cast<const float4*>(gs + k * TP);
-            const float4 g1 = *reinterpret_cast<const float4*>(gs + k * TP + TP / 2);
-            const float4 wq = *reinterpret_cast<const float4*>(ws + k * WP);
-            const float wv[RC] = {wq.x, wq.y, wq.z, wq.w};
-            const float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+            float gv[RP], wv[RC];
+#pragma unroll
+            for (int h = 0; h < RP / PQ; ++h) {
+                if constexpr (PQ == 4) {
+                    const float4 q = *reinterpret_cast<const float4*>(gs + k * TP + h * (TP / 2));
+                    gv[4 * h] = q.x; gv[4 * h + 1] = q.y; gv[4 * h + 2] = q.z; gv[4 * h + 3] = q.w;
+                } else {
+                    const float2 q = *reinterpret_cast<const float2*>(gs + k * TP);
+                    gv[0] = q.x; gv[1] = q.y;
+                }
+            }
+            if constexpr (RC == 4) {
+                const float4 q = *reinterpret_cast<const float4*>(ws + k * WP);
+                wv[0] = q.x; wv[1] = q.y; wv[2] = q.z; wv[3] = q.w;
+            } else {
+                const float2 q = *reinterpret_cast<const float2*>(ws + k * WP);
+                wv[0] = q.x; wv[1] = q.y;
+            }
             if constexpr (FAST) {
 #pragma unroll
                 for (int r = 0; r < RC; ++r)
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[r][j] = fmaf(__saturatef(fmaf(wv[r], 0.5f, xv[r][j])), gv[j], acc[r][j]);
+                    for (int j = 0; j < RP; ++j) acc[r][j] = fmaf(__saturatef(fmaf(wv[r], 0.5f, xv[r][j])), gv[j], acc[r][j]);
             } else {
 #pragma unroll
-                for (int j = 0; j < 8; j += 2)
+                for (int j = 0; j < RP; j += 2)
 #pragma unroll
                     for (int r = 0; r < RC; ++r) {
                         const uint64_t s = fma2(pack2(clamp_unit(wv[r] + xv[r][j]), clamp_unit(wv[r] + xv[r][j + 1])),
@@ -196,29 +217,27 @@ __global__ void __launch_bounds__(GATHER_THREADS, 4) adder_gx_gather_kernel(cons
         }
         // two-level summation: a long sum over output channels loses far less than one running fp32 accumulator would
         if (c % FOLD == FOLD - 1 && c + 1 < nchunks) {
+            float* av = &acc[0][0];
 #pragma unroll
-            for (int r = 0; r < RC; ++r)
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    float4* t = Tot + (r * 2 + h) * GATHER_THREADS;
-                    float4 v = c < FOLD ? make_float4(0.f, 0.f, 0.f, 0.f) : *t;
-                    v.x += acc[r][4 * h]; v.y += acc[r][4 * h + 1]; v.z += acc[r][4 * h + 2]; v.w += acc[r][4 * h + 3];
-                    *t = v;
-                    acc[r][4 * h] = acc[r][4 * h + 1] = acc[r][4 * h + 2] = acc[r][4 * h + 3] = 0.f;
-                }
+            for (int i = 0; i < RC * RP / 4; ++i) {
+                float4* t = Tot + i * GATHER_THREADS;
+                float4 v = c < FOLD ? make_float4(0.f, 0.f, 0.f, 0.f) : *t;
+                v.x += av[4 * i]; v.y += av[4 * i + 1]; v.z += av[4 * i + 2]; v.w += av[4 * i + 3];
+                *t = v;
+                av[4 * i] = av[4 * i + 1] = av[4 * i + 2] = av[4 * i + 3] = 0.f;
+            }
         }
         cc.next(m, a.CK);
-        if (++stage == GATHER_STAGES) stage = 0;
-        if (++fstage == GATHER_STAGES) fstage = 0;
+        if (++stage == ST) stage = 0;
+        if (++fstage == ST) fstage = 0;
     }
     if (nchunks > FOLD) {
+        float* av = &acc[0][0];
 #pragma unroll
-        for (int r = 0; r < RC; ++r)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const float4 v = Tot[(r * 2 + h) * GATHER_THREADS];
-                acc[r][4 * h] += v.x; acc[r][4 * h + 1] += v.y; acc[r][4 * h + 2] += v.z; acc[r][4 * h + 3] += v.w;
-            }
+        for (int i = 0; i < RC * RP / 4; ++i) {
+            const float4 v = Tot[i * GATHER_THREADS];
+            av[4 * i] += v.x; av[4 * i + 1] += v.y; av[4 * i + 2] += v.z; av[4 * i + 3] += v.w;
+        }
     }
     if (FAST) {
         __syncthreads();                         // the stages are free
@@ -227,8 +246,8 @@ __global__ void __launch_bounds__(GATHER_THREADS, 4) adder_gx_gather_kernel(cons
         for (int q = 0; q < COLS; ++q) bs[tid + q * GATHER_THREADS] = box[q];
         __syncthreads();
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int col = (j >> 2) * (TP / 2) + pg * 4 + (j & 3);
+        for (int j = 0; j < RP; ++j) {
+            const int col = (j / PQ) * (TP / 2) + pg * PQ + (j % PQ);
             float b = bs[col];
 #pragma unroll
             for (int r = 1; r < ROWS; ++r) b += bs[r * TP + col];
@@ -237,36 +256,38 @@ __global__ void __launch_bounds__(GATHER_THREADS, 4) adder_gx_gather_kernel(cons
         }
     }
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int p = p0 + h * (TP / 2) + pg * 4;
-        if (a.vec_io || a.fill_quads) {
-            if (p >= m.P) continue;
-            uint32_t n, r, y, x;
-            m.d_phw.divmod(p, n, r);
-            m.d_pw.divmod(r, y, x);
-            float* o = a.gx + ((size_t)n * a.Ci + ci0 + cg * RC) * HW + (a.vec_io ? r : (y * 2) * a.W + x * 2);
+    for (int h = 0; h < RP / PQ; ++h) {
+        const int p = p0 + h * (TP / 2) + pg * PQ;
+        if constexpr (PQ == 4) {
+            if (a.vec_io || a.fill_quads) {
+                if (p >= m.P) continue;
+                uint32_t n, r, y, x;
+                m.d_phw.divmod(p, n, r);
+                m.d_pw.divmod(r, y, x);
+                float* o = a.gx + ((size_t)n * a.Ci + ci0 + cg * RC) * HW + (a.vec_io ? r : (y * 2) * a.W + x * 2);
 #pragma unroll
-            for (int c = 0; c < RC; ++c) {
-                if (ci0 + cg * RC + c >= a.Ci) break;
-                float4* o4 = reinterpret_cast<float4*>(o + (size_t)c * HW);
-                float4 v = make_float4(acc[c][4 * h], acc[c][4 * h + 1], acc[c][4 * h + 2], acc[c][4 * h + 3]);
-                if (a.fill_quads) {              // stride 2, pixels of class (0, 0) only: a zero between them and a row of zeros below
-                    o4[0] = make_float4(v.x, 0.f, v.y, 0.f);
-                    o4[1] = make_float4(v.z, 0.f, v.w, 0.f);
-                    o4 = reinterpret_cast<float4*>(o + (size_t)c * HW + a.W);
-                    o4[0] = o4[1] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    continue;
+                for (int c = 0; c < RC; ++c) {
+                    if (ci0 + cg * RC + c >= a.Ci) break;
+                    float4* o4 = reinterpret_cast<float4*>(o + (size_t)c * HW);
+                    float4 v = make_float4(acc[c][4 * h], acc[c][4 * h + 1], acc[c][4 * h + 2], acc[c][4 * h + 3]);
+                    if (a.fill_quads) {          // stride 2, pixels of class (0, 0) only: a zero between them and a row of zeros below
+                        o4[0] = make_float4(v.x, 0.f, v.y, 0.f);
+                        o4[1] = make_float4(v.z, 0.f, v.w, 0.f);
+                        o4 = reinterpret_cast<float4*>(o + (size_t)c * HW + a.W);
+                        o4[0] = o4[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        continue;
+                    }
+                    if (a.accumulate) {
+                        const float4 old = *o4;
+                        v.x += old.x; v.y += old.y; v.z += old.z; v.w += old.w;
+                    }
+                    *o4 = v;
                 }
-                if (a.accumulate) {
-                    const float4 old = *o4;
-                    v.x += old.x; v.y += old.y; v.z += old.z; v.w += old.w;
-                }
-                *o4 = v;
+                continue;
             }
-            continue;
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < PQ; ++j) {
             if (p + j >= m.P) continue;
             uint32_t n, r, y, x;
             m.d_phw.divmod(p + j, n, r);
@@ -277,7 +298,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 4) adder_gx_gather_kernel(cons
             for (int c = 0; c < RC; ++c) {
                 if (ci0 + cg * RC + c >= a.Ci) break;
                 float* oc = o + (size_t)c * HW;
-                const float v = acc[c][4 * h + j];
+                const float v = acc[c][PQ * h + j];
                 if (a.accumulate) { *oc += v; continue; }
                 *oc = v;
                 if (a.fill_block)
@@ -295,26 +316,37 @@ __global__ void __launch_bounds__(GATHER_THREADS, 4) adder_gx_gather_kernel(cons
 
 namespace {
 
-// CG channel groups of 4 per CTA: 64 channels x 64 pixels, 32 x 128 or 16 x 256 (the cost is explained at choose_tile in
-// adder_fwd_gather.cu; here a term is 2.6 lane cycles).
-int choose_groups(long long P, int classes, int Ci) {
-    static const double rate[4] = {0.5, 0.8, 0.93, 1.0};
-    int best = 16;
+// X(RC, RP, CG, ST, MB); the choice is explained at choose_tile in adder_fwd_gather.cu, here a term is 2.9 lane
+// cycles, and the longer chain of dependent instructions shows with up to three tiles on an SM.
+#define ADDER_GX_GATHER_TILES(X) \
+    X(4, 8, 16, 2, 4) X(4, 8, 8, 2, 4) X(4, 8, 4, 2, 4) X(4, 4, 16, 4, 6) X(4, 4, 8, 4, 6) X(4, 4, 4, 4, 6) X(2, 2, 8, 8, 8) X(2, 2, 4, 8, 8)
+
+struct Tile { int rc, rp, cg, st, tc, tp; };
+constexpr Tile kTiles[] = {
+#define X(RC, RP, CG, ST, MB) {RC, RP, CG, ST, RC * CG, RP * GATHER_THREADS / CG},
+    ADDER_GX_GATHER_TILES(X)
+#undef X
+};
+
+int choose_tile(const GxGatherArgs& a, int classes, int Ci) {
+    int best = 0;
     double best_cost = 1e300;
     const int sms = sm_count();
-    for (int cg = 16; cg >= 4; cg >>= 1) {
-        const int tc = cg * RC, tp = GATHER_THREADS / cg * 8;
-        const long long tiles = ((P + tp - 1) / tp + classes - 1) * ceil_div(Ci, tc);
+    for (int i = 0; i < (int)(sizeof(kTiles) / sizeof(kTiles[0])); ++i) {
+        const Tile& t = kTiles[i];
+        long long tiles = 0;
+        for (int c = 0; c < classes; ++c) tiles += (long long)ceil_div(a.m[c].P, t.tp) * ceil_div(Ci, t.tc);
         const long long per_sm = (tiles + sms - 1) / sms;
-        const double cost = per_sm / rate[per_sm < 4 ? per_sm - 1 : 3] * (2.6 * tc * tp + 4.0 * (tc + tp));
-        if (cost < best_cost) { best_cost = cost; best = cg; }
+        const double step = 2.9 * t.rc * t.rp + 6.0 + 7.0 * (t.tc + t.tp) / GATHER_THREADS;
+        double cost = per_sm * step;
+        if (per_sm <= 3) cost = 40.0 + (per_sm == 3 ? 1.2 : 1.5) * cost;
+        if (cost < best_cost) { best_cost = cost; best = i; }
     }
     return best;
 }
 
-size_t smem_bytes(int cg) {
-    const int tc = cg * RC, tp = GATHER_THREADS / cg * 8;
-    return ((size_t)GATHER_STAGES * GATHER_CK * (tp + tc + 4) + RC * 8 * GATHER_THREADS) * sizeof(float);
+size_t smem_bytes(const Tile& t) {
+    return ((size_t)t.st * GATHER_CK * (t.tp + t.tc + 4) + (size_t)t.rc * t.rp * GATHER_THREADS) * sizeof(float);
 }
 
 // Taps k of one dimension that reach input positions q*S + r: (r + pad - k*dil) % S == 0.  Output position q + o0 + i*d0.
@@ -360,9 +392,9 @@ bool single_class(const ConvGeom& g) {
     return true;
 }
 
-template <int CG, bool FAST, bool QUADS>
+template <class T, bool FAST, bool QUADS>
 int launch_t(const GxGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
-    auto kern = adder_gx_gather_kernel<CG, FAST, QUADS>;
+    auto kern = adder_gx_gather_kernel<T, FAST, QUADS>;
     const int se = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
     if (se != ADDER_OK) return se;
     kern<<<grid, GATHER_THREADS, smem, stream>>>(a);
@@ -370,10 +402,13 @@ int launch_t(const GxGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream)
 }
 
 template <bool FAST, bool QUADS>
-int launch_g(int cg, const GxGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
-    if (cg == 16) return launch_t<16, FAST, QUADS>(a, grid, smem, stream);
-    if (cg == 8) return launch_t<8, FAST, QUADS>(a, grid, smem, stream);
-    return launch_t<4, FAST, QUADS>(a, grid, smem, stream);
+int launch_tile(int tile, const GxGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
+    int i = 0;
+#define X(RC, RP, CG, ST, MB) \
+    if (tile == i++) return launch_t<GxTile<RC, RP, CG, ST, MB>, FAST, QUADS>(a, grid, smem, stream);
+    ADDER_GX_GATHER_TILES(X)
+#undef X
+    return ADDER_ERR_INTERNAL;
 }
 
 int plan(const ConvGeom& g, int first, GxGatherArgs& a, dim3& grid, bool& more) {
@@ -382,9 +417,9 @@ int plan(const ConvGeom& g, int first, GxGatherArgs& a, dim3& grid, bool& more) 
     more = fill_classes(g, first, a, n, total, single);
     a.Ci = g.Ci; a.H = g.H; a.W = g.W; a.Co = g.Co; a.Ho = g.Ho; a.Wo = g.Wo; a.KK = g.kh * g.kw; a.sh = g.sh; a.sw = g.sw;
     a.CK = ceil_div(g.Co, ceil_div(g.Co, GATHER_CK));
-    const int cg = choose_groups((long long)a.m[0].P * n, n, g.Ci);
-    grid = dim3((unsigned)ceil_div(a.m[0].P, GATHER_THREADS / cg * 8), (unsigned)ceil_div(g.Ci, cg * RC), (unsigned)n);
-    return cg;
+    const int tile = choose_tile(a, n, g.Ci);
+    grid = dim3((unsigned)ceil_div(a.m[0].P, kTiles[tile].tp), (unsigned)ceil_div(g.Ci, kTiles[tile].tc), (unsigned)n);
+    return tile;
 }
 
 }  // namespace
@@ -393,9 +428,9 @@ int describe_gx_gather(const ConvGeom& g, int fast, char* buf, size_t n) {
     GxGatherArgs a;
     dim3 grid;
     bool more;
-    const int cg = plan(g, 0, a, grid, more);
-    return snprintf(buf, n, "gx gather k=%dx%d fast=%d classes=%u TC=%d TP=%d threads=%d smem=%zu grid=(%u,%u) status=0", g.kh, g.kw,
-                    fast, grid.z, cg * RC, GATHER_THREADS / cg * 8, GATHER_THREADS, smem_bytes(cg), grid.x, grid.y);
+    const Tile& t = kTiles[plan(g, 0, a, grid, more)];
+    return snprintf(buf, n, "gx gather k=%dx%d fast=%d classes=%u RC=%d RP=%d TC=%d TP=%d threads=%d smem=%zu grid=(%u,%u) status=0",
+                    g.kh, g.kw, fast, grid.z, t.rc, t.rp, t.tc, t.tp, GATHER_THREADS, smem_bytes(t), grid.x, grid.y);
 }
 
 int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const float* w, float* gx, int fast, int accumulate,
@@ -404,7 +439,7 @@ int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const
     for (int first = 0; more; first += MAX_CLASSES) {
         GxGatherArgs a;
         dim3 grid;
-        const int cg = plan(g, first, a, grid, more);
+        const int tile = plan(g, first, a, grid, more);
         if (grid.y > 65535) return ADDER_ERR_UNSUPPORTED;
         a.gout = gout; a.x = x; a.w = w; a.gx = gx; a.accumulate = accumulate;
         const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gx)) & 15) == 0;
@@ -417,9 +452,9 @@ int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const
         // the gradient is read pixel by pixel in order: 1x1 kernels whose class (0, 0) is the output plane
         const bool quads = g.kh == 1 && g.kw == 1 && g.ph == 0 && g.pw == 0 && a.m[0].PH == g.Ho && a.m[0].PW == g.Wo && grid.z == 1 &&
                            (g.Ho * g.Wo) % 4 == 0 && (reinterpret_cast<uintptr_t>(gout) & 15) == 0;
-        const size_t smem = smem_bytes(cg);
-        const int st = fast ? (quads ? launch_g<true, true>(cg, a, grid, smem, stream) : launch_g<true, false>(cg, a, grid, smem, stream))
-                            : (quads ? launch_g<false, true>(cg, a, grid, smem, stream) : launch_g<false, false>(cg, a, grid, smem, stream));
+        const size_t smem = smem_bytes(kTiles[tile]);
+        const int st = fast ? (quads ? launch_tile<true, true>(tile, a, grid, smem, stream) : launch_tile<true, false>(tile, a, grid, smem, stream))
+                            : (quads ? launch_tile<false, true>(tile, a, grid, smem, stream) : launch_tile<false, false>(tile, a, grid, smem, stream));
         if (st != ADDER_OK) return st;
     }
     return ADDER_OK;

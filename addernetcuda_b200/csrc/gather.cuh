@@ -4,18 +4,21 @@
 // affine tap offsets, so these kernels take every geometry.
 //
 // A CTA of 128 threads owns TC channels x TP pixels; pixels run over the whole batch (image, row, column), so
-// no plane size leaves a ragged tile behind.  The reduction index is (channel block, tap, channel in the
-// block): a chunk of at most GATHER_CK channels of one tap is one shared-memory stage, hence a thread computes
-// the address and the bounds test of its pixel once per chunk and copies a column of channels from there.
-// Two stages, one barrier per chunk.
+// no plane size leaves a ragged tile behind.  A chunk of the reduction is one shared-memory stage:
+//   GATHER_TAP    at most 16 channels of one tap (index order: channel block, tap, channel in the block), so that a
+//                 thread computes the address and the bounds test of its pixel once per chunk;
+//   GATHER_QUADS  the same for 1x1 layers whose operand is read in order: 16-byte copies;
+//   GATHER_NINE   2 channels x the 9 taps of a 3x3 window, in index order (channel, row, column).
+// One barrier per chunk; large tiles keep two stages, small ones as many as hide the latency of a load.
 #pragma once
 #include "common.cuh"
 
 namespace adder {
 
 constexpr int GATHER_CK = 16;
-constexpr int GATHER_STAGES = 2;
+constexpr int GATHER_NINE_CH = 2;        // channels per chunk of GATHER_NINE
 constexpr int GATHER_THREADS = 128;
+enum GatherMode { GATHER_TAP, GATHER_QUADS, GATHER_NINE };
 
 // Where the pixel-side operand of reduction tap (i, j) of pixel (py, px) lives in its source tensor:
 // row py*sy + oy0 + i*doy, column px*sx + ox0 + j*dox; out of bounds reads zero.  wt0 + i*dwi + j*dwj is the tap's
@@ -104,6 +107,39 @@ __device__ __forceinline__ void gather_quads(float* dst, const float* base, bool
         for (int k = 0; k < GATHER_CK; k += ROWS, s += step) cp_async16(d + k * TP, s, ok);
     } else {
         for (int k = k0; k < ck; k += ROWS, s += step, d += ROWS * TP) cp_async16(d, k < nch ? s : src, ok & (k < nch));
+    }
+}
+
+// A bit per tap of the 3x3 window: the tap of this pixel lies inside the plane.
+__device__ __forceinline__ unsigned nine_mask(const GatherPixel& px, const GatherMap& m, int Hs, int Ws) {
+    unsigned mask = 0;
+#pragma unroll
+    for (int t = 0; t < 9; ++t) {
+        const int row = px.row + m.oy0 + (t / 3) * m.doy, col = px.col + m.ox0 + (t % 3) * m.dox;
+        if (px.ok & ((unsigned)row < (unsigned)Hs) & ((unsigned)col < (unsigned)Ws)) mask |= 1u << t;
+    }
+    return mask;
+}
+
+// GATHER_NINE: rows (channel c0 + r/9, tap r%9), r < 18, of the thread's pixels; channels from nch on are zero.
+template <int TP>
+__device__ __forceinline__ void gather_nine(float* dst, const GatherPixel* px, const unsigned* mask, const GatherMap& m, int c0,
+                                            int nch, int Hs, int Ws, int tid) {
+    constexpr int COLS = TP > GATHER_THREADS ? TP / GATHER_THREADS : 1;
+    constexpr int ROWS = TP < GATHER_THREADS ? GATHER_THREADS / TP : 1;
+    const int plane = Hs * Ws;
+#pragma unroll
+    for (int q = 0; q < COLS; ++q) {
+        const float* s = px[q].base + (c0 * plane + (px[q].row + m.oy0) * Ws + px[q].col + m.ox0);
+        float* d = dst + (COLS > 1 ? tid + q * GATHER_THREADS : tid % TP);
+#pragma unroll
+        for (int i = 0; i < (9 * GATHER_NINE_CH + ROWS - 1) / ROWS; ++i) {
+            const int r = i * ROWS + (ROWS > 1 ? tid / TP : 0);
+            if (ROWS > 1 && (9 * GATHER_NINE_CH) % ROWS != 0 && r >= 9 * GATHER_NINE_CH) break;
+            const int c = r / 9, t = r - c * 9;
+            // nothing is read where the predicate is false, so the address may lie outside the tensor there
+            cp_async4(d + r * TP, s + (c * plane + (t / 3) * m.doy * Ws + (t % 3) * m.dox), (mask[q] >> t & 1) & (c < nch));
+        }
     }
 }
 
