@@ -55,6 +55,7 @@ SIGNATURES = {
     "adder_b200_batchnorm_backward": (c_int, [c_void_p] * 10 + [c_int, c_void_p, c_size_t, c_int, c_int, c_int,
                                               c_void_p]),
     "adder_b200_affine_forward": (c_int, [c_void_p] * 5 + [c_int, c_int, c_int, c_int, c_void_p]),
+    "adder_b200_forward_affine": (c_int, [c_void_p] * 5 + [c_int, c_void_p, *_GEOM, c_void_p]),
     "adder_b200_device_status": (c_int, [POINTER(c_int), c_int]),
     "adder_b200_peer_area_bytes": (c_size_t, [c_longlong, c_int]),
     "adder_b200_ipc_export": (c_int, [c_void_p, c_void_p, POINTER(c_ulonglong)]),
@@ -103,6 +104,15 @@ def load() -> ctypes.CDLL:
     return _active
 
 
+def is_product(lib: ctypes.CDLL) -> bool:
+    return lib is _product
+
+
+def _active_changed() -> None:
+    from . import _native
+    _native.sync()
+
+
 class tuning:
     """`with tuning() as lib:` routes every op of this package through libadder_b200_tuning.so, whose
     extra entry points (`lib.adder_b200_set_tile_hint`, `_set_micro_tile`, `_set_variant`) override the
@@ -114,6 +124,7 @@ class tuning:
             _tuning = _open(TUNING_LIB_PATH, {**SIGNATURES, **TUNING_SIGNATURES})
         self._previous = _active
         _active = _tuning
+        _active_changed()
         return _tuning
 
     def __exit__(self, *exc) -> None:
@@ -123,6 +134,7 @@ class tuning:
             _tuning.adder_b200_set_micro_tile(op, 0, 0)
             _tuning.adder_b200_set_variant(op, 0)
         _active = self._previous
+        _active_changed()
 
 
 def check(status: int, what: str) -> None:

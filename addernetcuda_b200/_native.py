@@ -1,0 +1,59 @@
+"""The C++ host path of the eager layer calls (csrc/host.cpp), loaded on the first call with a CUDA tensor.
+
+`layer`, `layer_with_stats`, `layer_affine`, `affine` and `column` return None for whatever they do not take - anything but
+contiguous fp32 CUDA tensors of a geometry the fused kernels are built for - and callers then go on in Python, which handles
+the rest or raises.  They always call the product library; inside a `_lib.tuning()` block they return None.
+"""
+from __future__ import annotations
+
+import ctypes
+import importlib.util
+import sys
+
+import torch
+
+from . import _lib
+
+_NAMES = ("adder_b200_status_string", "adder_b200_forward", "adder_b200_forward_stat_slices", "adder_b200_forward_with_stats",
+          "adder_b200_forward_affine", "adder_b200_affine_forward", "adder_b200_backward_input",
+          "adder_b200_backward_weight_workspace_bytes", "adder_b200_backward_weight")
+_ENTRIES = ("layer", "layer_with_stats", "layer_affine", "affine", "column")
+_mod = None
+
+
+def load() -> None:
+    """Load the extension (built first if necessary), bind it to the product library and put its entry points in place."""
+    global _mod
+    if _mod is None:
+        from . import build
+        if not build.HOST_LIB.exists():
+            build.build()
+        spec = importlib.util.spec_from_file_location("_adder_host", build.HOST_LIB)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        _mod = mod
+        for name in _ENTRIES:
+            globals()[name] = getattr(mod, name)
+    sync()
+
+
+def sync() -> None:
+    """Follow `_lib`: bound to the product library, or off while another one is active."""
+    if _mod is None:
+        return
+    from . import adder, adder_cuda
+    lib = _lib.load()
+    addresses = {n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in _NAMES} if _lib.is_product(lib) else None
+    _mod.bind(addresses, adder.__dict__, adder_cuda.__dict__)
+
+
+def _first_call(name):
+    def call(tensor, *args):
+        if not (isinstance(tensor, torch.Tensor) and tensor.is_cuda):
+            return None
+        load()
+        return getattr(sys.modules[__name__], name)(tensor, *args)
+    return call
+
+
+layer, layer_with_stats, layer_affine, affine, column = (_first_call(n) for n in _ENTRIES)

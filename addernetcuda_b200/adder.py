@@ -14,7 +14,7 @@ import torch
 import torch.nn as nn
 from torch.autograd import Function
 
-from . import adder_cuda
+from . import _native, adder_cuda
 
 # Global switch for the one-instruction clamp in the input gradient (see adder_b200.h).
 FAST_CLAMP = False
@@ -83,9 +83,18 @@ def _adder2d_columns(X, W, stride, padding, dilation):
     return Y.view(co, n, ho, positions // ho).transpose(0, 1).contiguous()
 
 
+def _native_allowed(W) -> bool:
+    """The C++ host path writes gradients into tensors of its own, so not where a data-parallel bucket slot is attached."""
+    return adder_cuda.unpatched() and getattr(W, "_grad_slot", None) is None
+
+
 def adder2d_function(X, W, stride=1, padding=0, dilation=1):
     """Same contract as adder.py:22-41: X[N,Ci,H,W], W[Co,Ci,kh,kw] -> [N,Co,Ho,Wo], differentiable.
     `dilation` is an extension (the reference fixes it to 1)."""
+    if (dilation == 1 or dilation == (1, 1)) and _native_allowed(W):
+        out = _native.layer(X, W, stride, padding)
+        if out is not None:
+            return out
     if _fused_geometry(W, stride, padding, dilation):
         return _Adder2dNCHW.apply(X, W, stride, padding)
     return _adder2d_columns(X, W, stride, padding, dilation)
@@ -94,6 +103,11 @@ def adder2d_function(X, W, stride=1, padding=0, dilation=1):
 class adder(Function):
     """Column-matrix op of adder.py:43-80: `adder.apply(W_col[Co,K], X_col[K,P]) -> [Co,P]`,
     backward returning (rescaled grad_W_col, grad_X_col)."""
+
+    @classmethod
+    def apply(cls, W_col, X_col):
+        out = _native.column(W_col, X_col) if cls is adder else None
+        return out if out is not None else super().apply(W_col, X_col)
 
     @staticmethod
     def forward(ctx, W_col, X_col):
@@ -150,5 +164,15 @@ class adder2d(nn.Module):
         (`adder_cuda.forward(..., stats=True)`), or None where the layer cannot provide them."""
         if self.bias or not x.is_cuda or not _fused_geometry(self.adder, self.stride, self.padding, self.dilation):
             return self.forward(x), None
+        r = _native.layer_with_stats(x, self.adder, self.stride, self.padding) if _native_allowed(self.adder) else None
+        if r is not None:
+            return r[0], (r[1] if r[1].shape[1] > 0 else None)
         out, st = _Adder2dNCHW.apply(x, self.adder, self.stride, self.padding, True)
         return out, (st if st.shape[1] > 0 else None)
+
+    def forward_affine(self, x, scale, shift, residual=None, relu=False):
+        """`relu?(forward(x) * scale[c] + shift[c] + residual)` in one kernel, without autograd: the layer with the folded batch
+        norm behind it (`inference.FoldedBatchNorm2d`).  None where that kernel does not apply."""
+        if self.bias or self.dilation not in (1, (1, 1)) or not _native_allowed(self.adder):
+            return None
+        return _native.layer_affine(x, self.adder, self.stride, self.padding, scale, shift, residual, relu)

@@ -1,4 +1,5 @@
-"""Builds libadder_b200.so in-tree with nvcc for sm_100a (no libtorch, no Python headers).
+"""Builds libadder_b200.so in-tree with nvcc for sm_100a (no libtorch, no Python headers), and the extension _adder_host.so
+on top of it with the C++ compiler (libtorch and Python headers: the host path of the eager layer calls).
 
     python -m addernetcuda_b200.build [--force] [--verbose]
 
@@ -21,6 +22,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 INCLUDE = PKG.parent / "include"
 LIB = PKG / "libadder_b200.so"
+HOST_LIB = PKG / "_adder_host.so"              # csrc/host.cpp
 TUNING_LIB = PKG / "libadder_b200_tuning.so"   # same objects, api.cu compiled with -DADDER_B200_TUNING
 SOURCES = ["api.cu", "adder_fwd.cu", "adder_fwd_gather.cu", "adder_bwd_input.cu", "adder_gx_gather.cu", "adder_bwd_weight.cu", "adder_bwd_weight_pipe.cu", "adder_bwd_weight_tma.cu", "tma_host.cu", "adder_bwd_weight_1x1.cu", "adder_pointwise.cu", "static_scratch.cu", "batchnorm.cu", "peer_allreduce.cu"]
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -34,11 +36,26 @@ def find_nvcc() -> str:
 
 
 def _stale() -> bool:
-    if not LIB.exists() or not TUNING_LIB.exists():
+    libs = (LIB, TUNING_LIB, HOST_LIB)
+    if not all(p.exists() for p in libs):
         return True
-    t = min(LIB.stat().st_mtime, TUNING_LIB.stat().st_mtime)
-    deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + list(INCLUDE.glob("*.h"))
+    t = min(p.stat().st_mtime for p in libs)
+    deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cpp")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + list(INCLUDE.glob("*.h"))
     return any(d.stat().st_mtime > t for d in deps)
+
+
+def _host_command() -> list:
+    """Compile and link csrc/host.cpp against the installed torch."""
+    import sysconfig
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(find_nvcc()).resolve().parent.parent
+    inc = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", cuda / "include", INCLUDE,
+           Path(sysconfig.get_paths()["include"])]
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wno-interference-size",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{p}" for p in inc), str(CSRC / "host.cpp"),
+            "-o", str(HOST_LIB), f"-L{root / 'lib'}", "-lc10", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-lc10_cuda", "-ltorch_cuda",
+            f"-L{cuda / 'lib64'}", "-lcudart"]
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -63,6 +80,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     api_tuning = objdir / "api_tuning.o"
     procs.append(("api.cu (tuning)", subprocess.Popen(common + ["-DADDER_B200_TUNING", "-c", str(CSRC / "api.cu"), "-o", str(api_tuning)],
                                                       stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
+    procs.append(("host.cpp", subprocess.Popen(_host_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
     failed = False
     for src, p in procs:
         out, _ = p.communicate()

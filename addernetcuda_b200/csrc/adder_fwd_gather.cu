@@ -18,9 +18,9 @@ struct FwdGatherArgs {
     const float* x;
     const float* w;
     float* out;
-    double* stats;           // optional [Co][gridDim.x][2]: per pixel tile, the sum of its outputs and of their squares
+    Epilogue ep;
     int Ci, H, W, Co, KK, CK, nchunks;
-    int vec_store;           // planes are whole quads and `out` is 16-byte aligned
+    int vec_store;           // planes are whole quads, `out` and the residual 16-byte aligned
 };
 
 // RM channels x RP pixels per thread (RP = 8: two quads half a tile apart), CG channel groups, ST stages, MB CTAs per SM.
@@ -33,7 +33,7 @@ struct FwdTile {
 
 template <class T, int MODE>
 __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel(const __grid_constant__ FwdGatherArgs a) {
-    constexpr int RM = T::RM, RP = T::RP, CG = T::CG, PG = T::PG, TC = T::TC, TP = T::TP, WP = T::WP, PQ = T::PQ, ST = T::ST;
+    constexpr int RM = T::RM, RP = T::RP, CG = T::CG, TC = T::TC, TP = T::TP, WP = T::WP, PQ = T::PQ, ST = T::ST;
     constexpr int COLS = TP > GATHER_THREADS ? TP / GATHER_THREADS : 1;
     constexpr int CK = MODE == GATHER_NINE ? 9 * GATHER_NINE_CH : GATHER_CK;      // rows of a stage
     constexpr int XS = CK * TP, WS = CK * WP;
@@ -167,12 +167,13 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
                 if (p >= a.m.P) continue;
                 uint32_t n, r;
                 a.m.d_phw.divmod(p, n, r);
-                float* o = a.out + ((size_t)n * a.Co + co0 + cg * RM) * PHW + r;
+                const int c0 = co0 + cg * RM;
+                const size_t at = ((size_t)n * a.Co + c0) * PHW + r;
 #pragma unroll
                 for (int m = 0; m < RM; ++m) {
-                    if (co0 + cg * RM + m >= a.Co) break;
-                    *reinterpret_cast<float4*>(o + (size_t)m * PHW) =
-                        make_float4(-acc[m][4 * h], -acc[m][4 * h + 1], -acc[m][4 * h + 2], -acc[m][4 * h + 3]);
+                    if (c0 + m >= a.Co) break;
+                    const float4 y = make_float4(-acc[m][4 * h], -acc[m][4 * h + 1], -acc[m][4 * h + 2], -acc[m][4 * h + 3]);
+                    *reinterpret_cast<float4*>(a.out + at + (size_t)m * PHW) = finish(a.ep, y, c0 + m, at + (size_t)m * PHW);
                 }
                 continue;
             }
@@ -182,42 +183,14 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
             if (p + j >= a.m.P) continue;
             uint32_t n, r;
             a.m.d_phw.divmod(p + j, n, r);
-            float* o = a.out + ((size_t)n * a.Co + co0 + cg * RM) * PHW + r;
+            const int c0 = co0 + cg * RM;
+            const size_t at = ((size_t)n * a.Co + c0) * PHW + r;
 #pragma unroll
             for (int m = 0; m < RM; ++m) {
-                if (co0 + cg * RM + m >= a.Co) break;
-                o[(size_t)m * PHW] = -acc[m][PQ * h + j];
+                if (c0 + m >= a.Co) break;
+                a.out[at + (size_t)m * PHW] = finish(a.ep, -acc[m][PQ * h + j], c0 + m, at + (size_t)m * PHW);
             }
         }
-    }
-    if (a.stats == nullptr) return;
-
-    // Batch-norm statistics of this pixel tile, as in adder_fwd_kernel: at most 8 values per thread and channel in fp32, then
-    // double in a fixed order.
-    __syncthreads();                                        // the stages are free
-    float2* st = reinterpret_cast<float2*>(smem);           // [TC][PG + 1]
-#pragma unroll
-    for (int m = 0; m < RM; ++m) {
-        float s = 0.f, q = 0.f;
-#pragma unroll
-        for (int j = 0; j < RP; ++j)
-            if (p0 + (j / PQ) * (TP / 2) + pg * PQ + (j % PQ) < a.m.P) { s -= acc[m][j]; q = fmaf(acc[m][j], acc[m][j], q); }
-        st[(cg * RM + m) * (PG + 1) + pg] = make_float2(s, q);
-    }
-    __syncthreads();
-    constexpr int TPC = GATHER_THREADS / TC >= 32 ? 32 : (GATHER_THREADS / TC < 1 ? 1 : GATHER_THREADS / TC);   // threads per channel
-    const int ch = tid / TPC, l = tid % TPC;
-    double ds = 0.0, dq = 0.0;
-    if (ch < TC)
-        for (int e = l; e < PG; e += TPC) { const float2 v = st[ch * (PG + 1) + e]; ds += (double)v.x; dq += (double)v.y; }
-#pragma unroll
-    for (int off = TPC >> 1; off > 0; off >>= 1) {
-        ds += __shfl_xor_sync(0xffffffffu, ds, off);
-        dq += __shfl_xor_sync(0xffffffffu, dq, off);
-    }
-    if (l == 0 && ch < TC && co0 + ch < a.Co) {
-        double* o = a.stats + ((size_t)(co0 + ch) * gridDim.x + blockIdx.x) * 2;
-        o[0] = ds; o[1] = dq;
     }
 }
 
@@ -261,9 +234,7 @@ int choose_tile(int P, int Co) {
 int stage_rows(const ConvGeom& g) { return g.kh == 3 && g.kw == 3 ? 9 * GATHER_NINE_CH : GATHER_CK; }
 
 size_t smem_bytes(const Tile& t, int rows) {
-    const size_t stages = (size_t)t.st * rows * (t.tp + t.tc + 4) * sizeof(float);
-    const size_t stats = (size_t)t.tc * (GATHER_THREADS / t.cg + 1) * sizeof(float2);
-    return stages > stats ? stages : stats;
+    return (size_t)t.st * rows * (t.tp + t.tc + 4) * sizeof(float);
 }
 
 GatherMap fwd_map(const ConvGeom& g) {
@@ -298,11 +269,6 @@ int launch_mode(int tile, const FwdGatherArgs& a, dim3 grid, size_t smem, cudaSt
 
 }  // namespace
 
-int fwd_gather_stat_slices(const ConvGeom& g) {
-    const int P = g.N * g.Ho * g.Wo;
-    return ceil_div(P, kTiles[choose_tile(P, g.Co)].tp);
-}
-
 int describe_fwd_gather(const ConvGeom& g, char* buf, size_t n) {
     const int P = g.N * g.Ho * g.Wo;
     const Tile& t = kTiles[choose_tile(P, g.Co)];
@@ -310,24 +276,22 @@ int describe_fwd_gather(const ConvGeom& g, char* buf, size_t n) {
                     t.rp, t.tc, t.tp, GATHER_THREADS, smem_bytes(t, stage_rows(g)), ceil_div(P, t.tp), ceil_div(g.Co, t.tc));
 }
 
-int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* out, cudaStream_t stream, double* stats,
-                      int stat_slices) {
+int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* out, cudaStream_t stream, const Epilogue& ep) {
     FwdGatherArgs a;
     a.m = fwd_map(g);
-    a.x = x; a.w = w; a.out = out; a.stats = stats;
+    a.x = x; a.w = w; a.out = out; a.ep = ep;
     a.Ci = g.Ci; a.H = g.H; a.W = g.W; a.Co = g.Co; a.KK = g.kh * g.kw;
     const bool nine = g.kh == 3 && g.kw == 3;
     a.CK = nine ? GATHER_NINE_CH : ceil_div(g.Ci, ceil_div(g.Ci, GATHER_CK));              // evenly sized channel blocks
     a.nchunks = ceil_div(g.Ci, a.CK) * (nine ? 1 : a.KK);
     const bool whole_quads = (g.Ho * g.Wo) % 4 == 0;
-    a.vec_store = whole_quads && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    a.vec_store = whole_quads && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(ep.residual)) & 15) == 0;
     const bool quads = whole_quads && a.KK == 1 && g.sh == 1 && g.sw == 1 && g.ph == 0 && g.pw == 0 &&
                        (reinterpret_cast<uintptr_t>(x) & 15) == 0;
     const int tile = choose_tile(a.m.P, g.Co);
     const Tile& t = kTiles[tile];
     const dim3 grid((unsigned)ceil_div(a.m.P, t.tp), (unsigned)ceil_div(g.Co, t.tc));
     if (grid.y > 65535) return ADDER_ERR_UNSUPPORTED;
-    if (stats != nullptr && stat_slices != (int)grid.x) return ADDER_ERR_WORKSPACE;
     const size_t smem = smem_bytes(t, stage_rows(g));
     if (nine) return launch_mode<GATHER_NINE>(tile, a, grid, smem, stream);
     return quads ? launch_mode<GATHER_QUADS>(tile, a, grid, smem, stream) : launch_mode<GATHER_TAP>(tile, a, grid, smem, stream);

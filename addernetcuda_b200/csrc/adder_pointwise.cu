@@ -25,6 +25,7 @@ struct PwArgs {
     float* out;          // forward: [N,Co,Ho,Wo]; input gradient: [N,Ci,H,W]
     int N, Ci, Co, H, W, Ho, Wo, S, P, accumulate, vec2;
     FastDiv d_wo, d_howo;
+    Epilogue ep;         // forward only
 };
 
 bool pointwise_applicable(const Geom& g) {
@@ -79,10 +80,10 @@ __global__ void __launch_bounds__(PW_THREADS) adder_pw_fwd_kernel(const PwArgs a
         }
     }
     const int HoWo = a.Ho * a.Wo;
-    float* o = a.out + ((size_t)n * a.Co + co0) * HoWo + r;
+    const size_t at = ((size_t)n * a.Co + co0) * HoWo + r;
 #pragma unroll
     for (int m = 0; m < PW_CT; ++m)
-        if (co0 + m < a.Co) o[(size_t)m * HoWo] = -acc[m];
+        if (co0 + m < a.Co) a.out[at + (size_t)m * HoWo] = finish(a.ep, -acc[m], co0 + m, at + (size_t)m * HoWo);
 }
 
 // grid (ceil(P/256), ceil(Ci/16)).  FAST: clamp(d,-1,1) = 2*sat(d/2 + 1/2) - 1 with w' = w/2 + 1/2 in
@@ -152,9 +153,9 @@ __global__ void __launch_bounds__(PW_THREADS) adder_pw_gx_kernel(const PwArgs a)
     }
 }
 
-int launch_pointwise_fwd(const Geom& g, const float* x, const float* w, float* out, cudaStream_t stream) {
+int launch_pointwise_fwd(const Geom& g, const float* x, const float* w, float* out, cudaStream_t stream, const Epilogue& ep) {
     PwArgs a = make_pw_args(g);
-    a.x = x; a.w = w; a.out = out;
+    a.x = x; a.w = w; a.out = out; a.ep = ep;
     const dim3 grid(ceil_div(a.P, PW_THREADS), ceil_div(g.Co, PW_CT));
     if (g.Ci <= 16) adder_pw_fwd_kernel<16><<<grid, PW_THREADS, 0, stream>>>(a);
     else if (g.Ci <= 32) adder_pw_fwd_kernel<32><<<grid, PW_THREADS, 0, stream>>>(a);

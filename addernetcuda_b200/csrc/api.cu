@@ -152,6 +152,19 @@ int adder_b200_forward_with_stats(const float* x, const float* w, float* out, do
     return launch_fwd(g, x, w, out, current_hint(0), static_cast<cudaStream_t>(stream), stats, stat_slices);
 }
 
+int adder_b200_forward_affine(const float* x, const float* w, const float* scale, const float* shift, const float* residual,
+                              int relu, float* out, int n, int ci, int h, int wd, int co, int k, int stride, int pad,
+                              void* stream) {
+    Geom g;
+    const int st = make_geom(n, ci, h, wd, co, k, stride, pad, &g);
+    if (st != ADDER_OK) return st;
+    if (n == 0) return ADDER_OK;
+    if (x == nullptr || w == nullptr || out == nullptr || scale == nullptr || shift == nullptr) return ADDER_ERR_NULL_POINTER;
+    Epilogue ep;
+    ep.scale = scale; ep.shift = shift; ep.residual = residual; ep.relu = relu;
+    return launch_fwd(g, x, w, out, current_hint(0), static_cast<cudaStream_t>(stream), nullptr, 0, ep);
+}
+
 int adder_b200_backward_input(const float* grad_out, const float* x, const float* w, float* grad_x, int n, int ci,
                               int h, int wd, int co, int k, int stride, int pad, int flags, void* stream) {
     Geom g;

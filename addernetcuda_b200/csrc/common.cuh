@@ -94,6 +94,33 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
     return r;
 }
 
+// What a forward kernel does with an output before it stores it: nothing (scale == nullptr), or the evaluation-mode batch norm
+// behind the layer, relu?(y * scale[c] + shift[c] + residual).  The same operations in the same order as a pass of their own
+// (adder_b200_affine_forward), without its reads and writes of y.
+struct Epilogue {
+    const float* scale = nullptr;
+    const float* shift = nullptr;
+    const float* residual = nullptr;      // laid out like the output
+    int relu = 0;
+};
+__device__ __forceinline__ float finish(const Epilogue& e, float y, int c, size_t at) {
+    if (e.scale == nullptr) return y;
+    float v = fmaf(y, __ldg(e.scale + c), __ldg(e.shift + c));
+    if (e.residual != nullptr) v += __ldg(e.residual + at);
+    return e.relu ? fmaxf(v, 0.f) : v;
+}
+__device__ __forceinline__ float4 finish(const Epilogue& e, float4 y, int c, size_t at) {
+    if (e.scale == nullptr) return y;
+    const float sc = __ldg(e.scale + c), sh = __ldg(e.shift + c);
+    float4 v = make_float4(fmaf(y.x, sc, sh), fmaf(y.y, sc, sh), fmaf(y.z, sc, sh), fmaf(y.w, sc, sh));
+    if (e.residual != nullptr) {
+        const float4 r = __ldg(reinterpret_cast<const float4*>(e.residual + at));
+        v.x += r.x; v.y += r.y; v.z += r.z; v.w += r.w;
+    }
+    if (e.relu) v = make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
+    return v;
+}
+
 // clamp(d, -1, 1), exactly, in one instruction: the smaller magnitude of d and 1 with the sign of d.
 // fminf(fmaxf(d, -1), 1) is two instructions of the half-rate pipe.
 __device__ __forceinline__ float clamp_unit(float d) {

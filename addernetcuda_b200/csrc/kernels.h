@@ -43,6 +43,7 @@ struct FwdArgs {
     int x_quads;         // 1x1 layers: the halo-free input patch is staged with 16-byte copies
     FastDiv d_xquads;    // divides by the patch's quads per row
     double* stats;       // optional [Co][stat_slices][2]: per pixel tile, the sum of its outputs and of their squares
+    Epilogue ep;
     int stat_slices, stat_tpc;   // slices = pixel tiles of the launch; tpc = threads that share one channel's reduction
     PatchDims pd;        // haloed input patch staged per input-channel chunk
     FastDiv d_tiles_h, d_tiles_w, d_segs, d_spr, d_th, d_tm;
@@ -112,7 +113,7 @@ inline int launched(int n = 1) {
 int ensure_dynamic_smem(const void* kernel, size_t bytes);
 
 int launch_fwd(const Geom& g, const float* x, const float* w, float* out, const TileHint& hint, cudaStream_t s,
-               double* stats = nullptr, int stat_slices = 0);
+               double* stats = nullptr, int stat_slices = 0, const Epilogue& ep = Epilogue());
 // Number of per-channel statistic slices the forward kernel of this geometry writes (one per pixel tile);
 // 0 when that kernel has no fused statistics.
 int fwd_stat_slices(const Geom& g, const TileHint& hint);
@@ -124,9 +125,8 @@ int launch_gw(const Geom& g, const float* gout, const float* x, const float* w, 
               cudaStream_t s);
 
 // Channels x pixels tiles with a gathered operand (adder_fwd_gather.cu, adder_gx_gather.cu)
-int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* out, cudaStream_t s, double* stats = nullptr,
-                      int stat_slices = 0);
-int fwd_gather_stat_slices(const ConvGeom& g);
+int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* out, cudaStream_t s,
+                      const Epilogue& ep = Epilogue());
 int describe_fwd_gather(const ConvGeom& g, char* buf, size_t n);
 int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const float* w, float* gx, int fast, int accumulate,
                      cudaStream_t s);
@@ -135,7 +135,8 @@ int describe_gx_gather(const ConvGeom& g, int fast, char* buf, size_t n);
 // 1x1 stride-2 layers with at most 64 channels: one thread per output position (adder_pointwise.cu).
 // Chosen automatically unless a tile hint asks for the tiled kernels.
 bool pointwise_applicable(const Geom& g);
-int launch_pointwise_fwd(const Geom& g, const float* x, const float* w, float* out, cudaStream_t stream);
+int launch_pointwise_fwd(const Geom& g, const float* x, const float* w, float* out, cudaStream_t stream,
+                         const Epilogue& ep = Epilogue());
 int launch_pointwise_gx(const Geom& g, const float* gout, const float* x, const float* w, float* gx, int fast,
                         int accumulate, cudaStream_t stream);
 int pointwise_gw_splits(const Geom& g);

@@ -16,7 +16,7 @@ from typing import Iterable, Sequence, Tuple
 import torch
 import torch.nn as nn
 
-from . import _lib, adder_cuda
+from . import _lib, _native, adder_cuda
 
 
 def load_reference_checkpoint(model: nn.Module, state_dict: dict, strict: bool = True):
@@ -48,6 +48,9 @@ class FoldedBatchNorm2d(nn.Module):
             if residual is not None:
                 out = out + residual
             return torch.relu(out) if relu else out
+        z = _native.affine(y, self.scale, self.shift, residual, relu)
+        if z is not None:
+            return z
         y = y.contiguous()
         res = residual.contiguous() if residual is not None else None
         n, c, h, w = y.shape

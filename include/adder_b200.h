@@ -199,6 +199,13 @@ ADDER_API int adder_b200_batchnorm_backward(const float* dz, const float* y, con
 ADDER_API int adder_b200_affine_forward(const float* y, const float* scale, const float* shift, const float* residual,
                                         float* z, int relu, int n, int c, int hw, void* stream);
 
+/* The adder layer and that affine map in one kernel: out = y*scale[c] + shift[c] [+ residual] [then ReLU] with
+ * y = the layer's forward, which is not stored.  Same operations in the same order as the two calls.  residual ([n, co, ho, wo])
+ * may be NULL; out must not overlap x. */
+ADDER_API int adder_b200_forward_affine(const float* x, const float* w, const float* scale, const float* shift,
+                                        const float* residual, int relu, float* out, int n, int ci, int h, int wd,
+                                        int co, int k, int stride, int pad, void* stream);
+
 /* Kernels that wait for the copy engine do so with a bounded number of polls; a wait that runs out sets a
  * flag on the device and the kernel returns early (its output is then garbage).  This reads the flag of the
  * current device into *status (0 = never happened) and, with reset != 0, clears it.  Synchronises with
