@@ -200,10 +200,12 @@ __global__ void __launch_bounds__(FIN_THREADS) adder_gw_reduce_flat_kernel(const
         const float* q = a.gsum_part + co;
         double s = 0.0, gs = 0.0;
 #pragma unroll 8
-        for (int sp = 0; sp < a.splits; ++sp) {
+        for (int sp = 0; sp < a.splits; ++sp) {          // gsum_splits >= splits
             s += (double)__ldcg(p + (size_t)sp * a.CoK);
             gs += (double)__ldg(q + (size_t)sp * a.Co);
         }
+#pragma unroll 8
+        for (int sp = a.splits; sp < a.gsum_splits; ++sp) gs += (double)__ldg(q + (size_t)sp * a.Co);
         const float vf = (float)(s - (double)a.w[i] * gs);
         if (a.accumulate) a.gw[i] += vf; else a.gw[i] = vf;
         v2 = (double)vf * (double)vf;
@@ -254,11 +256,14 @@ __global__ void __launch_bounds__(FIN_THREADS) adder_gw_finish_kernel(const GwFi
         const int co = i / a.K;
         const float* p = a.part + i;
         const float* q = a.gsum_part + co;
+        int sp = lane;
 #pragma unroll 4
-        for (int sp = lane; sp < a.splits; sp += FIN_LANES) {
+        for (; sp < a.splits; sp += FIN_LANES) {
             s += (double)p[(size_t)sp * a.CoK];
             gs += (double)q[(size_t)sp * a.Co];
         }
+#pragma unroll 4
+        for (; sp < a.gsum_splits; sp += FIN_LANES) gs += (double)q[(size_t)sp * a.Co];
     }
     s_sum[lane][o] = s;
     s_gs[lane][o] = gs;
@@ -319,6 +324,9 @@ struct GwPlan {
     bool use_1x1 = false;   // 1x1 stride-1 layers with enough channels take the GEMM-style kernel
     bool use_pointwise = false;   // 1x1 stride-2 layers with few channels: adder_pointwise.cu
     bool use_pipe = false;        // 3x3 layers with channels in sixteens: adder_bwd_weight_pipe.cu
+    int gsum_splits() const { return use_mma ? mma_gsum_splits : a.splits; }
+    int mma_gsum_splits = 0;
+    bool use_mma = false;         // tensor cores: adder_gw_mma.cu
     bool use_tma = false;         // ... and stride 1, rows of 8-pixel segments: adder_bwd_weight_tma.cu
 };
 
@@ -437,7 +445,7 @@ static GwPlan plan_gw_t(const Geom& g, const TileHint& hint) {
 
 static GwPlan plan_gw_generic(const Geom& g, const TileHint& hint);
 
-static GwPlan plan_gw(const Geom& g, const TileHint& hint) {
+static GwPlan plan_gw_fp32(const Geom& g, const TileHint& hint) {
     GwPlan p = plan_gw_generic(g, hint);
     if (p.status == ADDER_OK && gw_pipe_applicable(g, hint)) {
         const int sp = gw_pipe_splits(g, hint);
@@ -465,6 +473,34 @@ static GwPlan plan_gw(const Geom& g, const TileHint& hint) {
     return p;
 }
 
+// Which layers take the tensor cores (adder_gw_mma.cu): gradients large enough to fill an instruction of 128 rows (16->16 3x3 at
+// batch 256: 59 against 45 us for the fp32 kernel; 32->32: 44 against 50, 256->256 14x14: 560 against 1526, 1024->256 1x1: 370
+// against 765, 64->64 56x56 at batch 64: 266 against 381), on layers with enough pixels and work to cover the fixed cost of its
+// CTAs (256->256 14x14 at batch 1: 41 against 28 us; at batch 8: 58 against 82).  The warp-tile fp32 kernels keep the layers with
+// up to 64 channels on planes up to 32x32, where they are within 10-20 %: such layers sit in small networks whose training is
+// sensitive to the last bit, and keep their results.
+static bool gw_uses_mma(const Geom& g, bool warp_tile) {
+    const double cok = (double)g.Co * g.Ci * g.k * g.k, pixels = (double)g.N * g.Ho * g.Wo;
+    if (warp_tile && g.Ci <= 64 && g.Co <= 64 && g.H * g.W <= 1024) return false;
+    return cok >= 4096 && pixels >= 512 && cok * pixels >= 5e7;
+}
+
+// The fp32 kernels where the tensor-core kernel does not apply.
+static GwPlan plan_gw(const Geom& g, const TileHint& hint) {
+    TileHint fp32 = hint;
+    if (fp32.variant == 3) fp32.variant = 0;
+    GwPlan p = plan_gw_fp32(g, fp32);
+    if (p.status == ADDER_OK && hint.is_default() && gw_uses_mma(g, p.use_tma || p.use_pipe)) {
+        const int sp = gw_mma_splits(conv_geom(g));
+        if (sp > 0) {
+            p.use_mma = true;
+            p.mma_gsum_splits = gw_mma_gsum_splits(conv_geom(g));
+            p.a.splits = sp;
+        }
+    }
+    return p;
+}
+
 static GwPlan plan_gw_generic(const Geom& g, const TileHint& hint) {
     const bool rw7 = (g.Wo % 8 != 0) && (g.Wo % 7 == 0);
     if (g.k == 3 && g.stride == 1) return rw7 ? plan_gw_t<3, 1, 7, 4, 2>(g, hint) : plan_gw_t<3, 1, 8, 4, 2>(g, hint);
@@ -479,7 +515,17 @@ static GwPlan plan_gw_generic(const Geom& g, const TileHint& hint) {
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 int describe_gw(const Geom& g, const TileHint& hint, char* buf, size_t n) {
-    const GwPlan p = plan_gw(g, hint);
+    TileHint fp32 = hint;
+    if (fp32.variant == 3) fp32.variant = 0;
+    const GwPlan p = plan_gw_fp32(g, fp32);
+    if (p.status == ADDER_OK && hint.is_default() && gw_uses_mma(g, p.use_tma || p.use_pipe)) {
+        const int w = describe_gw_mma(conv_geom(g), buf, n);
+        if (w > 0 && (size_t)w + 16 < n) {
+            buf += w; n -= w;
+            const int w2 = snprintf(buf, n, "; fp32 form: ");
+            buf += w2; n -= w2;
+        }
+    }
     if (p.status == ADDER_OK && p.use_tma) return describe_gw_tma(g, hint, buf, n);
     if (p.status == ADDER_OK && p.use_pipe) return describe_gw_pipe(g, hint, buf, n);
     if (p.status == ADDER_ERR_UNSUPPORTED && !((g.k == 1 || g.k == 3) && (g.stride == 1 || g.stride == 2))) return p.status;
@@ -497,7 +543,7 @@ size_t gw_workspace_bytes(const Geom& g, const TileHint& hint) {
     const GwPlan p = plan_gw(g, hint);
     if (p.status != ADDER_OK) return 0;
     const size_t CoK = (size_t)g.Co * g.Ci * g.k * g.k;
-    size_t floats = align_up((size_t)p.a.splits * CoK, 64) + align_up((size_t)p.a.splits * g.Co, 64) +
+    size_t floats = align_up((size_t)p.a.splits * CoK, 64) + align_up((size_t)p.gsum_splits() * g.Co, 64) +
                     align_up((size_t)p.fin_blocks + 2, 64);
     return floats * sizeof(float);
 }
@@ -515,6 +561,8 @@ int launch_gw(const Geom& g, const float* gout, const float* x, const float* w, 
               float* out_norm, int accumulate, void* workspace, size_t workspace_bytes, const TileHint& hint,
               cudaStream_t stream) {
     GwPlan p = plan_gw(g, hint);
+    TileHint fp32 = hint;
+    if (fp32.variant == 3) fp32.variant = 0;
     if (p.status != ADDER_OK) return p.status;
     const size_t need = gw_workspace_bytes(g, hint);
     if (workspace == nullptr || workspace_bytes < need) return ADDER_ERR_WORKSPACE;
@@ -525,22 +573,23 @@ int launch_gw(const Geom& g, const float* gout, const float* x, const float* w, 
     if ((reinterpret_cast<uintptr_t>(gout) & 15) != 0) p.a.g_quads = 0;
     p.a.part = ws;
     p.a.gsum_part = ws + align_up((size_t)p.a.splits * CoK, 64);
-    float* norm_part = p.a.gsum_part + align_up((size_t)p.a.splits * g.Co, 64);
+    float* norm_part = p.a.gsum_part + align_up((size_t)p.gsum_splits() * g.Co, 64);
     unsigned int* ticket = reinterpret_cast<unsigned int*>(norm_part + p.fin_blocks + 1);
     p.a.ticket = ticket;
 
     const bool rw7 = (g.Wo % 8 != 0) && (g.Wo % 7 == 0);
     int st = ADDER_ERR_UNSUPPORTED;
-    if (p.use_tma) {
-        st = launch_gw_tma(g, gout, x, p.a.part, p.a.gsum_part, ticket, p.a.splits, hint, stream);
+    if (p.use_mma) st = launch_gw_mma(conv_geom(g), gout, x, p.a.part, p.a.gsum_part, ticket, p.a.splits, stream);
+    else if (p.use_tma) {
+        st = launch_gw_tma(g, gout, x, p.a.part, p.a.gsum_part, ticket, p.a.splits, fp32, stream);
         if (st == ADDER_ERR_ALIGNMENT) {
             // no tensor map for these pointers (not 16-byte aligned): the cp.async kernel, same number of slices
-            TileHint h2 = hint;
+            TileHint h2 = fp32;
             h2.ti = p.a.splits;
             st = launch_gw_pipe(g, gout, x, p.a.part, p.a.gsum_part, ticket, p.a.splits, h2, stream);
         }
     }
-    else if (p.use_pipe) st = launch_gw_pipe(g, gout, x, p.a.part, p.a.gsum_part, ticket, p.a.splits, hint, stream);
+    else if (p.use_pipe) st = launch_gw_pipe(g, gout, x, p.a.part, p.a.gsum_part, ticket, p.a.splits, fp32, stream);
     else if (p.use_pointwise) st = launch_pointwise_gw(g, gout, x, p.a.part, p.a.gsum_part, ticket, p.a.splits, stream);
     else if (p.use_1x1) st = launch_gw1x1(g, gout, x, p.a.part, p.a.gsum_part, ticket, p.a.splits, stream);
     else if (g.k == 3 && g.stride == 1) st = rw7 ? launch_main_t<3, 1, 7, 4, 2>(p, stream) : launch_main_t<3, 1, 8, 4, 2>(p, stream);
@@ -551,7 +600,7 @@ int launch_gw(const Geom& g, const float* gout, const float* x, const float* w, 
 
     GwFinishArgs f;
     f.part = p.a.part; f.gsum_part = p.a.gsum_part; f.w = w; f.gw = gw; f.norm_part = norm_part;
-    f.out_norm = out_norm; f.CoK = (int)CoK; f.K = g.Ci * g.k * g.k; f.Co = g.Co; f.splits = p.a.splits;
+    f.out_norm = out_norm; f.CoK = (int)CoK; f.K = g.Ci * g.k * g.k; f.Co = g.Co; f.splits = p.a.splits; f.gsum_splits = p.gsum_splits();
     f.accumulate = accumulate; f.eta = eta;
     const bool need_norm = eta > 0.f || out_norm != nullptr;
     if (need_norm && CoK <= (size_t)FUSED_FINISH_MAX) {

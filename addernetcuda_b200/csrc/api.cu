@@ -272,7 +272,7 @@ int adder_b200_set_tile_hint(int op, int threads, int channel_groups, int tile_r
 }
 
 int adder_b200_set_variant(int op, int variant) {
-    if (op < 0 || op > 2 || variant < 0 || variant > 2) return ADDER_ERR_BAD_SHAPE;
+    if (op < 0 || op > 2 || variant < 0 || variant > 3) return ADDER_ERR_BAD_SHAPE;
     g_hints[op].variant.store(variant);
     return ADDER_OK;
 }

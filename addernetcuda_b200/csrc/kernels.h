@@ -27,7 +27,8 @@ struct TileHint {
     int rw = 0;        // pixels per thread segment (register tile width)
     int rm = 0;        // channels per thread (register tile height)
     int variant = 0;   // weight gradient: 0 = automatic, 1 = the tiled kernel with pixel lanes, 2 = the warp-tile
-                       // kernel that stages with cp.async where the default would use tiled bulk copies
+                       // kernel that stages with cp.async where the default would use tiled bulk copies, 3 = the fp32 kernel that the
+                       // planner would take without the tensor cores; forward and input gradient: 1 = tiled, 2 = gathering
     bool is_default() const { return !(threads | cg | th | ti | ck | smem_kb | rw | rm | variant); }
 };
 
@@ -94,7 +95,7 @@ struct GwFinishArgs {
     float* gw;           // [Co*K] result (scaled when eta > 0)
     float* norm_part;    // [finish blocks] partial sums of squares
     float* out_norm;     // optional: ||gw||_2 before scaling
-    int CoK, K, Co, splits, accumulate;
+    int CoK, K, Co, splits, gsum_splits, accumulate;
     float eta;
 };
 
@@ -156,6 +157,13 @@ int gw_tma_splits(const Geom& g, const TileHint& hint);
 int launch_gw_tma(const Geom& g, const float* gout, const float* x, float* part, float* gsum_part,
                   unsigned int* ticket, int splits, const TileHint& hint, cudaStream_t stream);
 int describe_gw_tma(const Geom& g, const TileHint& hint, char* buf, size_t n);
+
+// Weight gradient on the tensor cores (adder_gw_mma.cu); splits = 0: the geometry does not fit
+int gw_mma_splits(const ConvGeom& g);
+int gw_mma_gsum_splits(const ConvGeom& g);      // slices of the sums of g
+int launch_gw_mma(const ConvGeom& g, const float* gout, const float* x, float* part, float* gsum_part, unsigned int* ticket,
+                  int splits, cudaStream_t stream);
+int describe_gw_mma(const ConvGeom& g, char* buf, size_t n);
 
 bool gw1x1_applicable(const Geom& g);
 int gw1x1_splits(const Geom& g);

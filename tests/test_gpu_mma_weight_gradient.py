@@ -1,0 +1,43 @@
+"""Weight gradient on the tensor cores (csrc/adder_gw_mma.cu): exact three-way bf16 splits with fp32 accumulation.
+
+Compared with a float64 evaluation on the same device, at the edges of its tiles: channels below, at and past a tile, both ways
+of issuing (stacked, split), strides, halos, planes narrower than a step, slices with one chunk, and sums long enough to be
+drained many times.  Bound: a slice's sum loses at most 16 truncations of 2^-23 of the running sum before it is moved (2e-6, reached
+only if all values have one sign; random signs stay near 1e-7), and everything after that is rounded to nearest."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+# (n, ci, co, h, w, k, stride, pad)
+CASES = [(64, 32, 32, 18, 18, 3, 1, 1), (70, 16, 48, 20, 20, 3, 1, 1), (50, 27, 45, 29, 31, 3, 1, 1), (60, 40, 41, 13, 17, 3, 2, 1),
+         (9, 130, 70, 15, 13, 3, 1, 1), (40, 128, 129, 9, 7, 3, 2, 1), (16, 256, 256, 14, 14, 3, 1, 0), (9, 200, 264, 11, 11, 1, 1, 0),
+         (9, 96, 520, 28, 26, 1, 2, 0), (2, 64, 64, 112, 112, 3, 1, 1), (1, 64, 72, 7, 200, 3, 1, 1)]
+
+
+@pytest.mark.parametrize("one_sign", [False, True])
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "n%d_c%dto%d_%dx%d_k%ds%dp%d" % c)
+def test_tensor_core_weight_gradient(case, one_sign):
+    from addernetcuda_b200 import _lib, adder_cuda as ac
+    n, ci, co, h, w, k, s, p = case
+    assert _lib.describe_plan(2, n, ci, h, w, co, k, s, p).startswith("gw mma")
+    gen = torch.Generator(device=DEV).manual_seed(n + ci + co)
+    x = torch.randn(n, ci, h, w, device=DEV, generator=gen)
+    wt = torch.randn(co, ci, k, k, device=DEV, generator=gen)
+    ho, wo = (h + 2 * p - k) // s + 1, (w + 2 * p - k) // s + 1
+    g = torch.randn(n, co, ho, wo, device=DEV, generator=gen)
+    if one_sign:
+        x, g = x.abs() + 1, g.abs() + 1
+    got = ac.backward_weight(g, x, wt, s, p, eta=0.0)
+    want = torch.zeros(co, ci * k * k, device=DEV, dtype=torch.float64)
+    for i in range(n):
+        cols = F.unfold(x[i:i + 1].double(), k, padding=p, stride=s)[0]
+        gi = g[i].double().reshape(co, -1)
+        want += gi @ cols.T - wt.double().reshape(co, -1) * gi.sum(1, keepdim=True)
+    want = want.reshape(wt.shape)
+    rel = float((got.double() - want).norm() / want.norm())
+    print("    rel", rel)
+    assert rel <= (2e-6 if one_sign else 5e-7), rel
+    assert torch.equal(ac.backward_weight(g, x, wt, s, p, eta=0.0), got)     # same bits twice
