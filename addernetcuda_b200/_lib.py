@@ -55,6 +55,10 @@ SIGNATURES = {
     "adder_b200_batchnorm_backward": (c_int, [c_void_p] * 10 + [c_int, c_void_p, c_size_t, c_int, c_int, c_int,
                                               c_void_p]),
     "adder_b200_affine_forward": (c_int, [c_void_p] * 5 + [c_int, c_int, c_int, c_int, c_void_p]),
+    "adder_b200_conv_forward": (c_int, [c_void_p] * 3 + [c_int] * 13 + [c_void_p]),
+    "adder_b200_conv_backward_input": (c_int, [c_void_p] * 4 + [c_int] * 14 + [c_void_p]),
+    "adder_b200_conv_backward_weight_workspace_bytes": (c_size_t, [c_int] * 13),
+    "adder_b200_conv_backward_weight": (c_int, [c_void_p] * 4 + [c_float, c_void_p, c_size_t] + [c_int] * 13 + [c_void_p]),
     "adder_b200_forward_affine": (c_int, [c_void_p] * 5 + [c_int, c_void_p, *_GEOM, c_void_p]),
     "adder_b200_device_status": (c_int, [POINTER(c_int), c_int]),
     "adder_b200_peer_area_bytes": (c_size_t, [c_longlong, c_int]),

@@ -1,7 +1,7 @@
 """The C++ host path of the eager layer calls (csrc/host.cpp), loaded on the first call with a CUDA tensor.
 
-`layer`, `layer_with_stats`, `layer_affine`, `affine` and `column` return None for whatever they do not take - anything but
-contiguous fp32 CUDA tensors of a geometry the fused kernels are built for - and callers then go on in Python, which handles
+`layer`, `conv`, `layer_with_stats`, `layer_affine`, `affine` and `column` return None for whatever they do not take - anything but
+contiguous fp32 CUDA tensors of a geometry the kernels are built for - and callers then go on in Python, which handles
 the rest or raises.  They always call the product library; inside a `_lib.tuning()` block they return None.
 """
 from __future__ import annotations
@@ -16,8 +16,9 @@ from . import _lib
 
 _NAMES = ("adder_b200_status_string", "adder_b200_forward", "adder_b200_forward_stat_slices", "adder_b200_forward_with_stats",
           "adder_b200_forward_affine", "adder_b200_affine_forward", "adder_b200_backward_input",
-          "adder_b200_backward_weight_workspace_bytes", "adder_b200_backward_weight")
-_ENTRIES = ("layer", "layer_with_stats", "layer_affine", "affine", "column")
+          "adder_b200_backward_weight_workspace_bytes", "adder_b200_backward_weight", "adder_b200_conv_forward",
+          "adder_b200_conv_backward_input", "adder_b200_conv_backward_weight_workspace_bytes", "adder_b200_conv_backward_weight")
+_ENTRIES = ("layer", "conv", "layer_with_stats", "layer_affine", "affine", "column")
 _mod = None
 
 
@@ -56,4 +57,4 @@ def _first_call(name):
     return call
 
 
-layer, layer_with_stats, layer_affine, affine, column = (_first_call(n) for n in _ENTRIES)
+layer, conv, layer_with_stats, layer_affine, affine, column = (_first_call(n) for n in _ENTRIES)

@@ -69,16 +69,21 @@ def _fused_geometry(W, stride, padding, dilation) -> bool:
 
 
 def _adder2d_columns(X, W, stride, padding, dilation):
-    """Every other geometry (5x5, 7x7, rectangular kernels, stride 3, dilation ...): the layer as the
-    reference itself computes it, an explicit im2col around the column-matrix op (adder.py:22-41), with this
+    """Every other geometry (5x5, 7x7, rectangular kernels, stride 3, dilation ...).  Almost all of them run on the
+    gathering kernels and the tensor-core weight gradient (`_native.conv`), without a column matrix.  The rest - windows or
+    output rows too wide for the latter, other tensors than contiguous fp32 ones - as the reference itself computes a layer, an explicit im2col around the column-matrix op (adder.py:22-41), with this
     library's column kernels underneath (`adder`) and autograd's fold as col2im.  Columns are ordered
     (image, position), which the op does not care about."""
+    pair = lambda v: (v, v) if isinstance(v, int) else tuple(v)
+    (sh, sw), (ph, pw), (dh, dw) = pair(stride), pair(padding), pair(dilation)
+    if adder_cuda.unpatched():
+        out = _native.conv(X, W, sh, sw, ph, pw, dh, dw)
+        if out is not None:
+            return out
     n, co = X.shape[0], W.shape[0]
     cols = torch.nn.functional.unfold(X, (W.shape[2], W.shape[3]), dilation=dilation, padding=padding, stride=stride)
     k, positions = cols.shape[1], cols.shape[2]
     Y = adder.apply(W.reshape(co, k), cols.transpose(0, 1).reshape(k, n * positions))
-    pair = lambda v: (v, v) if isinstance(v, int) else tuple(v)
-    (sh, _), (ph, _), (dh, _) = pair(stride), pair(padding), pair(dilation)
     ho = (X.shape[2] + 2 * ph - dh * (W.shape[2] - 1) - 1) // sh + 1
     return Y.view(co, n, ho, positions // ho).transpose(0, 1).contiguous()
 

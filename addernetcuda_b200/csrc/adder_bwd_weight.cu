@@ -557,6 +557,28 @@ static int launch_main_t(const GwPlan& p, cudaStream_t stream) {
     return launched();
 }
 
+// Slices -> gradient, its norm and the rescale.
+static int launch_finish(const GwFinishArgs& f, int fin_blocks, unsigned int* ticket, cudaStream_t stream) {
+    const bool need_norm = f.eta > 0.f || f.out_norm != nullptr;
+    if (need_norm && f.CoK <= FUSED_FINISH_MAX) {
+        adder_gw_finish_kernel<<<fin_blocks, FIN_THREADS, 0, stream>>>(f, fin_blocks, ticket);
+        return launched();
+    }
+    const int flat_blocks = ceil_div(f.CoK, FIN_THREADS);      // <= fin_blocks: the norm partials fit their array
+    adder_gw_reduce_flat_kernel<<<flat_blocks, FIN_THREADS, 0, stream>>>(f);
+    if (launched() != ADDER_OK) return ADDER_ERR_CUDA;
+    if (need_norm) {
+        float* scale = f.norm_part + fin_blocks;
+        adder_gw_norm_kernel<<<1, 1024, 0, stream>>>(f, flat_blocks, scale);
+        if (launched() != ADDER_OK) return ADDER_ERR_CUDA;
+        if (f.eta > 0.f) {
+            adder_gw_scale_kernel<<<ceil_div(f.CoK, FIN_THREADS), FIN_THREADS, 0, stream>>>(f.gw, f.CoK, scale);
+            if (launched() != ADDER_OK) return ADDER_ERR_CUDA;
+        }
+    }
+    return ADDER_OK;
+}
+
 int launch_gw(const Geom& g, const float* gout, const float* x, const float* w, float* gw, float eta,
               float* out_norm, int accumulate, void* workspace, size_t workspace_bytes, const TileHint& hint,
               cudaStream_t stream) {
@@ -602,24 +624,45 @@ int launch_gw(const Geom& g, const float* gout, const float* x, const float* w, 
     f.part = p.a.part; f.gsum_part = p.a.gsum_part; f.w = w; f.gw = gw; f.norm_part = norm_part;
     f.out_norm = out_norm; f.CoK = (int)CoK; f.K = g.Ci * g.k * g.k; f.Co = g.Co; f.splits = p.a.splits; f.gsum_splits = p.gsum_splits();
     f.accumulate = accumulate; f.eta = eta;
-    const bool need_norm = eta > 0.f || out_norm != nullptr;
-    if (need_norm && CoK <= (size_t)FUSED_FINISH_MAX) {
-        adder_gw_finish_kernel<<<p.fin_blocks, FIN_THREADS, 0, stream>>>(f, p.fin_blocks, ticket);
-        return launched();
-    }
-    const int flat_blocks = ceil_div((int)CoK, FIN_THREADS);      // <= fin_blocks: the norm partials fit their array
-    adder_gw_reduce_flat_kernel<<<flat_blocks, FIN_THREADS, 0, stream>>>(f);
-    if (launched() != ADDER_OK) return ADDER_ERR_CUDA;
-    if (need_norm) {
-        float* scale = norm_part + p.fin_blocks;
-        adder_gw_norm_kernel<<<1, 1024, 0, stream>>>(f, flat_blocks, scale);
-        if (launched() != ADDER_OK) return ADDER_ERR_CUDA;
-        if (eta > 0.f) {
-            adder_gw_scale_kernel<<<ceil_div((int)CoK, FIN_THREADS), FIN_THREADS, 0, stream>>>(gw, (int)CoK, scale);
-            if (launched() != ADDER_OK) return ADDER_ERR_CUDA;
-        }
-    }
-    return ADDER_OK;
+    return launch_finish(f, p.fin_blocks, ticket, stream);
+}
+
+// A layer with any kernel extent, stride, padding and dilation: the tensor-core kernel alone, which takes all but very wide
+// rows and windows.
+struct ConvGwLayout { size_t gsum, norm, total; int splits, gsum_splits, fin_blocks; };
+
+static bool conv_gw_layout(const ConvGeom& g, ConvGwLayout* l) {
+    l->splits = gw_mma_splits(g);
+    if (l->splits <= 0) return false;
+    l->gsum_splits = gw_mma_gsum_splits(g);
+    const size_t CoK = (size_t)g.Co * g.Ci * g.kh * g.kw;
+    l->fin_blocks = ceil_div((int)CoK, FIN_OUT);
+    l->gsum = align_up((size_t)l->splits * CoK, 64);
+    l->norm = l->gsum + align_up((size_t)l->gsum_splits * g.Co, 64);
+    l->total = l->norm + align_up((size_t)l->fin_blocks + 2, 64);
+    return true;
+}
+
+size_t conv_gw_workspace_bytes(const ConvGeom& g) {
+    ConvGwLayout l;
+    return conv_gw_layout(g, &l) ? l.total * sizeof(float) : 0;
+}
+
+int launch_conv_gw(const ConvGeom& g, const float* gout, const float* x, const float* w, float* gw, float eta, void* workspace,
+                   size_t workspace_bytes, cudaStream_t stream) {
+    ConvGwLayout l;
+    if (!conv_gw_layout(g, &l)) return ADDER_ERR_UNSUPPORTED;
+    if (workspace == nullptr || workspace_bytes < l.total * sizeof(float)) return ADDER_ERR_WORKSPACE;
+    if ((reinterpret_cast<uintptr_t>(workspace) & 255) != 0) return ADDER_ERR_ALIGNMENT;
+    float* ws = static_cast<float*>(workspace);
+    unsigned int* ticket = reinterpret_cast<unsigned int*>(ws + l.norm + l.fin_blocks + 1);
+    const int st = launch_gw_mma(g, gout, x, ws, ws + l.gsum, ticket, l.splits, stream);
+    if (st != ADDER_OK) return st;
+    GwFinishArgs f;
+    f.part = ws; f.gsum_part = ws + l.gsum; f.w = w; f.gw = gw; f.norm_part = ws + l.norm; f.out_norm = nullptr;
+    f.K = g.Ci * g.kh * g.kw; f.CoK = g.Co * f.K; f.Co = g.Co; f.splits = l.splits; f.gsum_splits = l.gsum_splits;
+    f.accumulate = 0; f.eta = eta;
+    return launch_finish(f, l.fin_blocks, ticket, stream);
 }
 
 }  // namespace adder

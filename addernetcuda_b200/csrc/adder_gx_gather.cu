@@ -418,7 +418,9 @@ int plan(const ConvGeom& g, int first, GxGatherArgs& a, dim3& grid, bool& more) 
     a.Ci = g.Ci; a.H = g.H; a.W = g.W; a.Co = g.Co; a.Ho = g.Ho; a.Wo = g.Wo; a.KK = g.kh * g.kw; a.sh = g.sh; a.sw = g.sw;
     a.CK = ceil_div(g.Co, ceil_div(g.Co, GATHER_CK));
     const int tile = choose_tile(a, n, g.Ci);
-    grid = dim3((unsigned)ceil_div(a.m[0].P, kTiles[tile].tp), (unsigned)ceil_div(g.Ci, kTiles[tile].tc), (unsigned)n);
+    int most = 0;
+    for (int c = 0; c < n; ++c) most = a.m[c].P > most ? a.m[c].P : most;
+    grid = dim3((unsigned)ceil_div(most, kTiles[tile].tp), (unsigned)ceil_div(g.Ci, kTiles[tile].tc), (unsigned)n);
     return tile;
 }
 
@@ -450,7 +452,7 @@ int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const
         a.fill_quads = a.fill_block && g.sh == 2 && g.sw == 2 && g.W == 2 * a.m[0].PW && g.H == 2 * a.m[0].PH && a.m[0].PW % 4 == 0 &&
                        (reinterpret_cast<uintptr_t>(gx) & 15) == 0;
         // the gradient is read pixel by pixel in order: 1x1 kernels whose class (0, 0) is the output plane
-        const bool quads = g.kh == 1 && g.kw == 1 && g.ph == 0 && g.pw == 0 && a.m[0].PH == g.Ho && a.m[0].PW == g.Wo && grid.z == 1 &&
+        const bool quads = g.kh == 1 && g.kw == 1 && g.ph == 0 && g.pw == 0 && a.m[0].PH == g.Ho && a.m[0].PW == g.Wo && grid.z == 1 && first == 0 &&
                            (g.Ho * g.Wo) % 4 == 0 && (reinterpret_cast<uintptr_t>(gout) & 15) == 0;
         const size_t smem = smem_bytes(kTiles[tile]);
         const int st = fast ? (quads ? launch_tile<true, true>(tile, a, grid, smem, stream) : launch_tile<true, false>(tile, a, grid, smem, stream))

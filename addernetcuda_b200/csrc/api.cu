@@ -54,6 +54,18 @@ int make_geom(int n, int ci, int h, int wd, int co, int k, int stride, int pad, 
     return ADDER_OK;
 }
 
+int make_conv_geom(int n, int ci, int h, int wd, int co, int kh, int kw, int sh, int sw, int ph, int pw, int dh, int dw, ConvGeom* g) {
+    if (n < 0 || ci <= 0 || h <= 0 || wd <= 0 || co <= 0 || kh <= 0 || kw <= 0 || sh <= 0 || sw <= 0 || ph < 0 || pw < 0 || dh <= 0 || dw <= 0)
+        return ADDER_ERR_BAD_SHAPE;
+    const long long lim = 2147483647LL, eh = (long long)dh * (kh - 1) + 1, ew = (long long)dw * (kw - 1) + 1;
+    if (h + 2LL * ph < eh || wd + 2LL * pw < ew) return ADDER_ERR_BAD_SHAPE;
+    *g = ConvGeom{n, ci, h, wd, co, (int)((h + 2LL * ph - eh) / sh + 1), (int)((wd + 2LL * pw - ew) / sw + 1), kh, kw, sh, sw, ph, pw, dh, dw};
+    if ((long long)n * ci * h * wd > lim || (long long)n * co * g->Ho * g->Wo > lim || (long long)co * ci * kh * kw > lim ||
+        (h + 2LL * ph) * (wd + 2LL * pw) > lim)
+        return ADDER_ERR_UNSUPPORTED;
+    return ADDER_OK;
+}
+
 int make_col_geom(int K, int P, int Co, Geom* g) {
     if (K <= 0 || P < 0 || Co <= 0) return ADDER_ERR_BAD_SHAPE;
     // X[K,P] is an NCHW tensor [1,K,1,P]; W[Co,K] is [Co,K,1,1]; Y[Co,P] is [1,Co,1,P].
@@ -203,6 +215,41 @@ int adder_b200_backward(const float* grad_out, const float* x, const float* w, f
     if (st != ADDER_OK) return st;
     return adder_b200_backward_weight(grad_out, x, w, grad_w, eta, nullptr, workspace, workspace_bytes, n, ci, h, wd,
                                       co, k, stride, pad, flags & ADDER_FLAG_ACCUMULATE, stream);
+}
+
+int adder_b200_conv_forward(const float* x, const float* w, float* out, int n, int ci, int h, int wd, int co, int kh, int kw, int sh, int sw, int ph, int pw, int dh, int dw, void* stream) {
+    ConvGeom g;
+    const int st = make_conv_geom(n, ci, h, wd, co, kh, kw, sh, sw, ph, pw, dh, dw, &g);
+    if (st != ADDER_OK) return st;
+    if (n == 0) return ADDER_OK;
+    if (x == nullptr || w == nullptr || out == nullptr) return ADDER_ERR_NULL_POINTER;
+    return launch_fwd_gather(g, x, w, out, static_cast<cudaStream_t>(stream));
+}
+
+int adder_b200_conv_backward_input(const float* grad_out, const float* x, const float* w, float* grad_x, int n, int ci, int h, int wd, int co, int kh, int kw, int sh, int sw, int ph, int pw, int dh, int dw, int flags, void* stream) {
+    ConvGeom g;
+    const int st = make_conv_geom(n, ci, h, wd, co, kh, kw, sh, sw, ph, pw, dh, dw, &g);
+    if (st != ADDER_OK) return st;
+    if (n == 0) return ADDER_OK;
+    if (grad_out == nullptr || x == nullptr || w == nullptr || grad_x == nullptr) return ADDER_ERR_NULL_POINTER;
+    return launch_gx_gather(g, grad_out, x, w, grad_x, (flags & ADDER_FLAG_FAST_CLAMP) != 0, (flags & ADDER_FLAG_ACCUMULATE) != 0,
+                            static_cast<cudaStream_t>(stream));
+}
+
+size_t adder_b200_conv_backward_weight_workspace_bytes(int n, int ci, int h, int wd, int co, int kh, int kw, int sh, int sw, int ph, int pw, int dh, int dw) {
+    ConvGeom g;
+    if (make_conv_geom(n, ci, h, wd, co, kh, kw, sh, sw, ph, pw, dh, dw, &g) != ADDER_OK || n == 0) return 0;
+    return conv_gw_workspace_bytes(g);
+}
+
+int adder_b200_conv_backward_weight(const float* grad_out, const float* x, const float* w, float* grad_w, float eta, void* workspace,
+                                    size_t workspace_bytes, int n, int ci, int h, int wd, int co, int kh, int kw, int sh, int sw, int ph, int pw, int dh, int dw, void* stream) {
+    ConvGeom g;
+    const int st = make_conv_geom(n, ci, h, wd, co, kh, kw, sh, sw, ph, pw, dh, dw, &g);
+    if (st != ADDER_OK) return st;
+    if (n == 0) return ADDER_ERR_BAD_SHAPE;
+    if (grad_out == nullptr || x == nullptr || w == nullptr || grad_w == nullptr) return ADDER_ERR_NULL_POINTER;
+    return launch_conv_gw(g, grad_out, x, w, grad_w, eta, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
 }
 
 int adder_b200_conv_col(const float* x, const float* w, float* y, int K, int P, int Co, void* stream) {

@@ -29,6 +29,10 @@ struct Api {      // entry points of the loaded libadder_b200.so
     decltype(&adder_b200_backward_input) backward_input = nullptr;
     decltype(&adder_b200_backward_weight_workspace_bytes) backward_weight_workspace_bytes = nullptr;
     decltype(&adder_b200_backward_weight) backward_weight = nullptr;
+    decltype(&adder_b200_conv_forward) conv_forward = nullptr;
+    decltype(&adder_b200_conv_backward_input) conv_backward_input = nullptr;
+    decltype(&adder_b200_conv_backward_weight_workspace_bytes) conv_backward_weight_workspace_bytes = nullptr;
+    decltype(&adder_b200_conv_backward_weight) conv_backward_weight = nullptr;
 };
 Api api;
 PyObject* g_adder_dict = nullptr;          // module dictionaries that hold FAST_CLAMP, OVERLAP_BACKWARD and ETA
@@ -114,11 +118,11 @@ c10::cuda::CUDAStream side_stream(c10::DeviceIndex dev) {
 }
 
 // Both gradients; with `overlap` the weight gradient runs on a side stream beside the input gradient.
-void backward_both(const at::Tensor& g, const at::Tensor& x, const at::Tensor& w, const at::Tensor& gx, const at::Tensor& gw,
-                   const Layer& L, float eta, bool fast, bool overlap) {
+template <class Input, class Weight>
+void run_both(const at::Tensor& x, bool overlap, Input input, Weight weight) {
     if (!overlap) {
-        backward_input(g, x, w, gx, L, fast);
-        backward_weight(g, x, w, gw, L, eta);
+        input();
+        weight();
         return;
     }
     const auto cur = c10::cuda::getCurrentCUDAStream(x.device().index());
@@ -128,11 +132,60 @@ void backward_both(const at::Tensor& g, const at::Tensor& x, const at::Tensor& w
     ready.block(side);
     {
         const c10::cuda::CUDAStreamGuard on_side(side);
-        backward_weight(g, x, w, gw, L, eta);
+        weight();
         done.record(side);
     }
-    backward_input(g, x, w, gx, L, fast);
+    input();
     done.block(cur);
+}
+
+void backward_both(const at::Tensor& g, const at::Tensor& x, const at::Tensor& w, const at::Tensor& gx, const at::Tensor& gw,
+                   const Layer& L, float eta, bool fast, bool overlap) {
+    run_both(x, overlap, [&] { backward_input(g, x, w, gx, L, fast); }, [&] { backward_weight(g, x, w, gw, L, eta); });
+}
+
+// ------------------------------------------------------------------------------------------ any other geometry
+
+// n, ci, h, w, co, kh, kw, sh, sw, ph, pw, dh, dw; then ho, wo
+using Conv = std::array<int, 15>;
+#define ADDER_CONV_GEOM(c) c[0], c[1], c[2], c[3], c[4], c[5], c[6], c[7], c[8], c[9], c[10], c[11], c[12]
+
+bool conv_of(const at::Tensor& x, const at::Tensor& w, const std::array<int64_t, 6>& p, Conv* c) {
+    if (!plain(x) || !plain(w) || x.device() != w.device() || x.dim() != 4 || w.dim() != 4) return false;
+    if (w.size(1) != x.size(1) || x.numel() == 0 || w.numel() == 0) return false;
+    constexpr int64_t lim = 2147483647;
+    for (int i = 0; i < 6; ++i)
+        if (p[i] < (i == 2 || i == 3 ? 0 : 1) || p[i] > (1 << 20)) return false;      // stride, padding, dilation
+    const int64_t h = x.size(2), wd = x.size(3), kh = w.size(2), kw = w.size(3);
+    const int64_t eh = h + 2 * p[2] - p[4] * (kh - 1) - 1, ew = wd + 2 * p[3] - p[5] * (kw - 1) - 1;
+    if (eh < 0 || ew < 0) return false;
+    const int64_t ho = eh / p[0] + 1, wo = ew / p[1] + 1;
+    if (x.numel() > lim || w.numel() > lim || x.size(0) * w.size(0) * ho * wo > lim) return false;
+    *c = Conv{(int)x.size(0), (int)x.size(1), (int)h, (int)wd, (int)w.size(0), (int)kh, (int)kw, (int)p[0], (int)p[1], (int)p[2], (int)p[3],
+              (int)p[4], (int)p[5], (int)ho, (int)wo};
+    return api.conv_backward_weight_workspace_bytes(ADDER_CONV_GEOM((*c))) > 0;
+}
+
+at::Tensor conv_forward(const at::Tensor& x, const at::Tensor& w, const Conv& c) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    at::Tensor out = empty_on(x, {c[0], c[4], c[13], c[14]});
+    check(api.conv_forward(x.const_data_ptr<float>(), w.const_data_ptr<float>(), out.mutable_data_ptr<float>(), ADDER_CONV_GEOM(c),
+                           current_stream(x)), "adder_b200_conv_forward");
+    return out;
+}
+
+void conv_backward_input(const at::Tensor& g, const at::Tensor& x, const at::Tensor& w, const at::Tensor& gx, const Conv& c, bool fast) {
+    check(api.conv_backward_input(g.const_data_ptr<float>(), x.const_data_ptr<float>(), w.const_data_ptr<float>(),
+                                  gx.mutable_data_ptr<float>(), ADDER_CONV_GEOM(c), fast ? ADDER_FLAG_FAST_CLAMP : 0, current_stream(x)),
+          "adder_b200_conv_backward_input");
+}
+
+void conv_backward_weight(const at::Tensor& g, const at::Tensor& x, const at::Tensor& w, const at::Tensor& gw, const Conv& c, float eta) {
+    const int64_t bytes = (int64_t)api.conv_backward_weight_workspace_bytes(ADDER_CONV_GEOM(c));
+    at::Tensor ws = empty_on(x, {bytes}, at::kByte);
+    check(api.conv_backward_weight(g.const_data_ptr<float>(), x.const_data_ptr<float>(), w.const_data_ptr<float>(),
+                                   gw.mutable_data_ptr<float>(), eta, ws.mutable_data_ptr(), (size_t)bytes, ADDER_CONV_GEOM(c),
+                                   current_stream(x)), "adder_b200_conv_backward_weight");
 }
 
 // ------------------------------------------------------------------------------------------ autograd nodes
@@ -188,6 +241,36 @@ struct AdderLayer : public torch::autograd::Function<AdderLayer> {
     }
 };
 
+struct ConvLayer : public torch::autograd::Function<ConvLayer> {
+    static Variable forward(AutogradContext* ctx, const Variable& x, const Variable& w, const std::vector<int64_t>& p) {
+        Conv c;
+        TORCH_CHECK(conv_of(x, w, {p[0], p[1], p[2], p[3], p[4], p[5]}, &c));
+        ctx->save_for_backward({x, w});
+        ctx->saved_data["p"] = p;
+        return conv_forward(x, w, c);
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        const Variable &x = saved[0], &w = saved[1];
+        const auto p = ctx->saved_data["p"].toIntVector();
+        Conv c;
+        TORCH_CHECK(conv_of(x, w, {p[0], p[1], p[2], p[3], p[4], p[5]}, &c));
+        const at::Tensor g = grads[0].contiguous();
+        TORCH_CHECK(g.scalar_type() == at::kFloat && g.device() == x.device(), "grad_out must be a float32 tensor on the layer's device");
+        const c10::cuda::CUDAGuard guard(x.device());
+        const Settings set = settings();
+        at::Tensor gx, gw;
+        if (ctx->needs_input_grad(0)) gx = empty_on(x, x.sizes());
+        if (ctx->needs_input_grad(1)) gw = empty_on(w, w.sizes());
+        auto input = [&] { conv_backward_input(g, x, w, gx, c, set.fast); };
+        auto weight = [&] { conv_backward_weight(g, x, w, gw, c, set.eta); };
+        if (gx.defined() && gw.defined()) run_both(x, set.overlap, input, weight);
+        else if (gx.defined()) input();
+        else if (gw.defined()) weight();
+        return {gx, gw, Variable()};
+    }
+};
+
 // The column-matrix op (adder.py:43-80 of the reference): X[K,P] is the 1x1 layer [1,K,1,P], W[Co,K] its kernel.
 Layer column_layer(const at::Tensor& w, const at::Tensor& x) {
     return {1, (int)x.size(0), 1, (int)x.size(1), (int)w.size(0), 1, 1, 0, 1, (int)x.size(1)};
@@ -237,6 +320,25 @@ PyObject* py_layer(PyObject*, PyObject* const* args, Py_ssize_t n) {
     {
         pybind11::gil_scoped_release no_gil;
         out = needs_node(*x, *w) ? AdderLayer::apply(*x, *w, stride, pad, false)[0] : forward(*x, *w, L);
+    }
+    return THPVariable_Wrap(std::move(out));
+    END_HANDLE_TH_ERRORS
+}
+
+// conv(x, w, sh, sw, ph, pw, dh, dw) -> out, or None
+PyObject* py_conv(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 8 || api.forward == nullptr) Py_RETURN_NONE;
+    const at::Tensor *x = tensor_arg(args[0]), *w = tensor_arg(args[1]);
+    std::array<int64_t, 6> p;
+    for (int i = 0; i < 6; ++i)
+        if (!int_arg(args[2 + i], &p[i])) Py_RETURN_NONE;
+    Conv c;
+    if (x == nullptr || w == nullptr || !conv_of(*x, *w, p, &c)) Py_RETURN_NONE;
+    at::Tensor out;
+    {
+        pybind11::gil_scoped_release no_gil;
+        out = needs_node(*x, *w) ? ConvLayer::apply(*x, *w, std::vector<int64_t>(p.begin(), p.end())) : conv_forward(*x, *w, c);
     }
     return THPVariable_Wrap(std::move(out));
     END_HANDLE_TH_ERRORS
@@ -360,6 +462,10 @@ PyObject* py_bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
         get("adder_b200_backward_input", &a.backward_input);
         get("adder_b200_backward_weight_workspace_bytes", &a.backward_weight_workspace_bytes);
         get("adder_b200_backward_weight", &a.backward_weight);
+        get("adder_b200_conv_forward", &a.conv_forward);
+        get("adder_b200_conv_backward_input", &a.conv_backward_input);
+        get("adder_b200_conv_backward_weight_workspace_bytes", &a.conv_backward_weight_workspace_bytes);
+        get("adder_b200_conv_backward_weight", &a.conv_backward_weight);
     }
     Py_INCREF(args[1]); Py_INCREF(args[2]);
     Py_XDECREF(g_adder_dict); Py_XDECREF(g_cuda_dict);
@@ -370,7 +476,7 @@ PyObject* py_bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 #define ADDER_METHOD(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {ADDER_METHOD("bind", py_bind), ADDER_METHOD("layer", py_layer), ADDER_METHOD("layer_with_stats", py_layer_with_stats),
+PyMethodDef methods[] = {ADDER_METHOD("bind", py_bind), ADDER_METHOD("layer", py_layer), ADDER_METHOD("conv", py_conv), ADDER_METHOD("layer_with_stats", py_layer_with_stats),
                          ADDER_METHOD("layer_affine", py_layer_affine), ADDER_METHOD("affine", py_affine), ADDER_METHOD("column", py_column),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_adder_host", nullptr, -1, methods};

@@ -125,6 +125,11 @@ int launch_gw(const Geom& g, const float* gout, const float* x, const float* w, 
               float* out_norm, int accumulate, void* workspace, size_t workspace_bytes, const TileHint& hint,
               cudaStream_t s);
 
+// Weight gradient of any geometry (tensor cores); 0 bytes: not supported
+size_t conv_gw_workspace_bytes(const ConvGeom& g);
+int launch_conv_gw(const ConvGeom& g, const float* gout, const float* x, const float* w, float* gw, float eta, void* workspace,
+                   size_t workspace_bytes, cudaStream_t stream);
+
 // Channels x pixels tiles with a gathered operand (adder_fwd_gather.cu, adder_gx_gather.cu)
 int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* out, cudaStream_t s,
                       const Epilogue& ep = Epilogue());

@@ -199,6 +199,23 @@ ADDER_API int adder_b200_batchnorm_backward(const float* dz, const float* y, con
 ADDER_API int adder_b200_affine_forward(const float* y, const float* scale, const float* shift, const float* residual,
                                         float* z, int relu, int n, int c, int hw, void* stream);
 
+/* The layer with any kernel extent (kh, kw), stride (sh, sw), padding (ph, pw) and dilation (dh, dw): what the reference computes
+ * through F.unfold around its column kernels (adder.py:22-41), as one kernel per result.  w [co, ci, kh, kw]; the other
+ * tensors, eta and the flags as above.  The weight gradient needs a workspace of the given size (256-byte aligned); a
+ * size of 0 means that it does not take the geometry (windows wider than 12 taps, output rows of several hundred pixels,
+ * an empty batch). */
+ADDER_API int adder_b200_conv_forward(const float* x, const float* w, float* out, int n, int ci, int h, int wd, int co,
+                                      int kh, int kw, int sh, int sw, int ph, int pw, int dh, int dw, void* stream);
+ADDER_API int adder_b200_conv_backward_input(const float* grad_out, const float* x, const float* w, float* grad_x, int n,
+                                             int ci, int h, int wd, int co, int kh, int kw, int sh, int sw, int ph,
+                                             int pw, int dh, int dw, int flags, void* stream);
+ADDER_API size_t adder_b200_conv_backward_weight_workspace_bytes(int n, int ci, int h, int wd, int co, int kh, int kw,
+                                                                 int sh, int sw, int ph, int pw, int dh, int dw);
+ADDER_API int adder_b200_conv_backward_weight(const float* grad_out, const float* x, const float* w, float* grad_w,
+                                              float eta, void* workspace, size_t workspace_bytes, int n, int ci, int h,
+                                              int wd, int co, int kh, int kw, int sh, int sw, int ph, int pw, int dh,
+                                              int dw, void* stream);
+
 /* The adder layer and that affine map in one kernel: out = y*scale[c] + shift[c] [+ residual] [then ReLU] with
  * y = the layer's forward, which is not stored.  Same operations in the same order as the two calls.  residual ([n, co, ho, wo])
  * may be NULL; out must not overlap x. */
