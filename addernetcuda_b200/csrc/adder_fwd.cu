@@ -24,7 +24,8 @@
 
 namespace adder {
 
-template <int KS, int S, int RW, int RM>
+// EP: an epilogue behind the layer (a template parameter: the mere test for it cost 2 % on 16->16 32x32).
+template <int KS, int S, int RW, int RM, bool EP>
 __global__ void __launch_bounds__(256, 2) adder_fwd_kernel(const FwdArgs a) {
     constexpr int KK = KS * KS;
     constexpr int XW = (RW - 1) * S + KS;   // input values one segment touches per (ci, kh)
@@ -162,13 +163,14 @@ __global__ void __launch_bounds__(256, 2) adder_fwd_kernel(const FwdArgs a) {
             const size_t at = (size_t)(n * a.g.Co + co) * HoWo + ho * a.g.Wo + wo0;
             if (RW % 4 == 0 && a.vec_store) {
 #pragma unroll
-                for (int j = 0; j < RW; j += 4)
-                    *reinterpret_cast<float4*>(a.out + at + j) =
-                        finish(a.ep, make_float4(-acc[m][j], -acc[m][j + 1], -acc[m][j + 2], -acc[m][j + 3]), co, at + j);
+                for (int j = 0; j < RW; j += 4) {
+                    const float4 y = make_float4(-acc[m][j], -acc[m][j + 1], -acc[m][j + 2], -acc[m][j + 3]);
+                    *reinterpret_cast<float4*>(a.out + at + j) = EP ? finish(a.ep, y, co, at + j) : y;
+                }
             } else {
 #pragma unroll
                 for (int j = 0; j < RW; ++j)
-                    if (wo0 + j < a.g.Wo) a.out[at + j] = finish(a.ep, -acc[m][j], co, at + j);
+                    if (wo0 + j < a.g.Wo) a.out[at + j] = EP ? finish(a.ep, -acc[m][j], co, at + j) : -acc[m][j];
             }
         }
     }
@@ -385,7 +387,7 @@ static int launch_fwd_t(const Geom& g, const float* x, const float* w, float* ou
         if ((long long)stat_slices != p.gx || p.a.TM * p.a.stat_tpc > p.threads) return ADDER_ERR_WORKSPACE;
         p.a.stats = stats; p.a.stat_slices = stat_slices;
     }
-    auto kern = adder_fwd_kernel<KS, S, RW, RM>;
+    auto kern = ep.scale != nullptr ? adder_fwd_kernel<KS, S, RW, RM, true> : adder_fwd_kernel<KS, S, RW, RM, false>;
     const int se = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), p.smem);
     if (se != ADDER_OK) return se;
     kern<<<dim3((unsigned)p.gx, (unsigned)p.gy), p.threads, p.smem, stream>>>(p.a);

@@ -200,32 +200,27 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
 
 namespace {
 
-// The tiles: large ones have the fewest loads per term, small ones give a small layer more threads.  X(RM, RP, CG, ST, MB)
-#define ADDER_FWD_GATHER_TILES(X) \
-    X(8, 8, 8, 2, 4) X(8, 8, 16, 2, 4) X(8, 8, 4, 2, 4) X(4, 8, 16, 3, 4) X(4, 8, 8, 3, 4) X(4, 8, 4, 2, 4) \
-    X(4, 4, 16, 4, 6) X(4, 4, 8, 4, 6) X(4, 4, 4, 4, 6) X(2, 2, 8, 8, 8) X(2, 2, 4, 8, 8)
+// The tiles: large ones have the fewest loads per term, small ones give a small layer more threads.
+// X(RM, RP, CG, ST, MB, clocks per step: alone, each further CTA, throughput)
+#define ADDER_FWD_GATHER_TILES(X)                                                                                   \
+    X(8, 8, 8, 2, 4, 242, 147, 173) X(8, 8, 16, 2, 4, 241, 74, 186) X(8, 8, 4, 2, 4, 278, 130, 186)                 \
+    X(4, 8, 16, 3, 4, 139, 65, 93) X(4, 8, 8, 3, 4, 139, 65, 93) X(4, 8, 4, 2, 4, 174, 76, 109)                     \
+    X(4, 4, 16, 4, 6, 92, 30, 54) X(4, 4, 8, 4, 6, 92, 30, 54) X(4, 4, 4, 4, 6, 101, 22, 56)                        \
+    X(2, 2, 8, 8, 8, 43, 9, 23) X(2, 2, 4, 8, 8, 49, 10, 26) X(2, 8, 4, 3, 6, 110, 40, 60)
 
-struct Tile { int rm, rp, cg, st, tc, tp; };
+struct Tile { int rm, rp, cg, st, tc, tp; TileCost cost; };
 constexpr Tile kTiles[] = {
-#define X(RM, RP, CG, ST, MB) {RM, RP, CG, ST, RM * CG, RP * GATHER_THREADS / CG},
+#define X(RM, RP, CG, ST, MB, A, M, S) {RM, RP, CG, ST, RM * CG, RP * GATHER_THREADS / CG, {A, M, S}},
     ADDER_FWD_GATHER_TILES(X)
 #undef X
 };
 
-// Time of the layer in cycles per reduction step, for each tile: a thread's step is 2.25 cycles of its scheduler per term, about 6
-// for its loads, and its share of the staging (about 7 instructions per value).  An SM's time is the number of its tiles
-// times that; with one or two tiles, so one or two warps per scheduler, the latency of the loads shows as well (about 28 cycles).
 int choose_tile(int P, int Co) {
     int best = 0;
     double best_cost = 1e300;
     const int sms = sm_count();
     for (int i = 0; i < (int)(sizeof(kTiles) / sizeof(kTiles[0])); ++i) {
-        const Tile& t = kTiles[i];
-        const long long tiles = (long long)ceil_div(P, t.tp) * ceil_div(Co, t.tc);
-        const long long per_sm = (tiles + sms - 1) / sms;
-        const double step = 2.25 * t.rm * t.rp + 6.0 + 7.0 * (t.tc + t.tp) / GATHER_THREADS;
-        double cost = per_sm * step;
-        if (per_sm <= 2) cost += 28.0;
+        const double cost = tile_cost(kTiles[i].cost, (long long)ceil_div(P, kTiles[i].tp) * ceil_div(Co, kTiles[i].tc), sms);
         if (cost < best_cost) { best_cost = cost; best = i; }
     }
     return best;
@@ -260,7 +255,7 @@ int launch_t(const FwdGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream
 template <int MODE>
 int launch_mode(int tile, const FwdGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
     int i = 0;
-#define X(RM, RP, CG, ST, MB) \
+#define X(RM, RP, CG, ST, MB, A, M, S) \
     if (tile == i++) return launch_t<FwdTile<RM, RP, CG, ST, MB>, MODE>(a, grid, smem, stream);
     ADDER_FWD_GATHER_TILES(X)
 #undef X
@@ -282,7 +277,7 @@ int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* 
     a.x = x; a.w = w; a.out = out; a.ep = ep;
     a.Ci = g.Ci; a.H = g.H; a.W = g.W; a.Co = g.Co; a.KK = g.kh * g.kw;
     const bool nine = g.kh == 3 && g.kw == 3;
-    a.CK = nine ? GATHER_NINE_CH : ceil_div(g.Ci, ceil_div(g.Ci, GATHER_CK));              // evenly sized channel blocks
+    a.CK = nine ? GATHER_NINE_CH : g.Ci < GATHER_CK ? g.Ci : GATHER_CK;      // full blocks have the cheaper staging loops
     a.nchunks = ceil_div(g.Ci, a.CK) * (nine ? 1 : a.KK);
     const bool whole_quads = (g.Ho * g.Wo) % 4 == 0;
     a.vec_store = whole_quads && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(ep.residual)) & 15) == 0;

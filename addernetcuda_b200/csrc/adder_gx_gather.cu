@@ -316,19 +316,22 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
 
 namespace {
 
-// X(RC, RP, CG, ST, MB); the choice is explained at choose_tile in adder_fwd_gather.cu, here a term is 2.9 lane
-// cycles, and the longer chain of dependent instructions shows with up to three tiles on an SM.
-#define ADDER_GX_GATHER_TILES(X) \
-    X(4, 8, 16, 2, 4) X(4, 8, 8, 2, 4) X(4, 8, 4, 2, 4) X(4, 4, 16, 4, 6) X(4, 4, 8, 4, 6) X(4, 4, 4, 4, 6) X(2, 2, 8, 8, 8) X(2, 2, 4, 8, 8)
+// X(RC, RP, CG, ST, MB, clocks per step: exact form alone, further, throughput; saturating form the same)
+#define ADDER_GX_GATHER_TILES(X)                                                                                    \
+    X(4, 8, 16, 2, 4, 197, 99, 134, 182, 85, 117) X(4, 8, 8, 2, 4, 196, 112, 134, 182, 85, 118)                     \
+    X(4, 8, 4, 2, 4, 219, 122, 142, 213, 112, 132) X(4, 4, 16, 4, 6, 133, 58, 83, 125, 70, 88)                      \
+    X(4, 4, 8, 4, 6, 128, 56, 80, 120, 49, 70) X(4, 4, 4, 4, 6, 133, 46, 83, 123, 54, 77)                           \
+    X(2, 2, 8, 8, 8, 68, 18, 32, 76, 17, 32) X(2, 2, 4, 8, 8, 70, 18, 33, 80, 18, 33)               \
+    X(2, 8, 4, 3, 6, 140, 60, 80, 140, 60, 80)
 
-struct Tile { int rc, rp, cg, st, tc, tp; };
+struct Tile { int rc, rp, cg, st, tc, tp; TileCost exact, fast; };
 constexpr Tile kTiles[] = {
-#define X(RC, RP, CG, ST, MB) {RC, RP, CG, ST, RC * CG, RP * GATHER_THREADS / CG},
+#define X(RC, RP, CG, ST, MB, A, M, S, FA, FM, FS) {RC, RP, CG, ST, RC * CG, RP * GATHER_THREADS / CG, {A, M, S}, {FA, FM, FS}},
     ADDER_GX_GATHER_TILES(X)
 #undef X
 };
 
-int choose_tile(const GxGatherArgs& a, int classes, int Ci) {
+int choose_tile(const GxGatherArgs& a, int classes, int Ci, bool fast) {
     int best = 0;
     double best_cost = 1e300;
     const int sms = sm_count();
@@ -336,10 +339,7 @@ int choose_tile(const GxGatherArgs& a, int classes, int Ci) {
         const Tile& t = kTiles[i];
         long long tiles = 0;
         for (int c = 0; c < classes; ++c) tiles += (long long)ceil_div(a.m[c].P, t.tp) * ceil_div(Ci, t.tc);
-        const long long per_sm = (tiles + sms - 1) / sms;
-        const double step = 2.9 * t.rc * t.rp + 6.0 + 7.0 * (t.tc + t.tp) / GATHER_THREADS;
-        double cost = per_sm * step;
-        if (per_sm <= 3) cost = 40.0 + (per_sm == 3 ? 1.2 : 1.5) * cost;
+        const double cost = tile_cost(fast ? t.fast : t.exact, tiles, sms);
         if (cost < best_cost) { best_cost = cost; best = i; }
     }
     return best;
@@ -404,20 +404,20 @@ int launch_t(const GxGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream)
 template <bool FAST, bool QUADS>
 int launch_tile(int tile, const GxGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
     int i = 0;
-#define X(RC, RP, CG, ST, MB) \
+#define X(RC, RP, CG, ST, MB, A, M, S, FA, FM, FS) \
     if (tile == i++) return launch_t<GxTile<RC, RP, CG, ST, MB>, FAST, QUADS>(a, grid, smem, stream);
     ADDER_GX_GATHER_TILES(X)
 #undef X
     return ADDER_ERR_INTERNAL;
 }
 
-int plan(const ConvGeom& g, int first, GxGatherArgs& a, dim3& grid, bool& more) {
+int plan(const ConvGeom& g, int first, bool fast, GxGatherArgs& a, dim3& grid, bool& more) {
     const bool single = single_class(g);
     int n, total;
     more = fill_classes(g, first, a, n, total, single);
     a.Ci = g.Ci; a.H = g.H; a.W = g.W; a.Co = g.Co; a.Ho = g.Ho; a.Wo = g.Wo; a.KK = g.kh * g.kw; a.sh = g.sh; a.sw = g.sw;
-    a.CK = ceil_div(g.Co, ceil_div(g.Co, GATHER_CK));
-    const int tile = choose_tile(a, n, g.Ci);
+    a.CK = g.Co < GATHER_CK ? g.Co : GATHER_CK;      // full blocks have the cheaper staging loops, so one ragged block rather than even ones
+    const int tile = choose_tile(a, n, g.Ci, fast);
     int most = 0;
     for (int c = 0; c < n; ++c) most = a.m[c].P > most ? a.m[c].P : most;
     grid = dim3((unsigned)ceil_div(most, kTiles[tile].tp), (unsigned)ceil_div(g.Ci, kTiles[tile].tc), (unsigned)n);
@@ -430,7 +430,7 @@ int describe_gx_gather(const ConvGeom& g, int fast, char* buf, size_t n) {
     GxGatherArgs a;
     dim3 grid;
     bool more;
-    const Tile& t = kTiles[plan(g, 0, a, grid, more)];
+    const Tile& t = kTiles[plan(g, 0, fast != 0, a, grid, more)];
     return snprintf(buf, n, "gx gather k=%dx%d fast=%d classes=%u RC=%d RP=%d TC=%d TP=%d threads=%d smem=%zu grid=(%u,%u) status=0",
                     g.kh, g.kw, fast, grid.z, t.rc, t.rp, t.tc, t.tp, GATHER_THREADS, smem_bytes(t), grid.x, grid.y);
 }
@@ -441,7 +441,7 @@ int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const
     for (int first = 0; more; first += MAX_CLASSES) {
         GxGatherArgs a;
         dim3 grid;
-        const int tile = plan(g, first, a, grid, more);
+        const int tile = plan(g, first, fast != 0, a, grid, more);
         if (grid.y > 65535) return ADDER_ERR_UNSUPPORTED;
         a.gout = gout; a.x = x; a.w = w; a.gx = gx; a.accumulate = accumulate;
         const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gx)) & 15) == 0;
