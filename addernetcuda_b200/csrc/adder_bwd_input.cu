@@ -838,7 +838,8 @@ static int launch_gx_t(const Geom& real, const float* gout, const float* x, cons
                        int accumulate, const TileHint& hint, cudaStream_t stream) {
     GxPlan p;
     const Geom g = gx_tiling_geom(real);
-    const int st = plan_gx_t<KS, S, RW, RC, FAST>(g, hint, p);
+    const int st = hint.is_default() ? cached_plan(g, p, [&](GxPlan& q) { return plan_gx_t<KS, S, RW, RC, FAST>(g, hint, q); })
+                                     : plan_gx_t<KS, S, RW, RC, FAST>(g, hint, p);
     if (st != ADDER_OK) return st;
     p.a.gout = gout; p.a.x = x; p.a.w = w; p.a.gx = gx; p.a.accumulate = accumulate;
     p.a.samp = (KS == 1 && S == 1) ? real.stride : 1;

@@ -486,7 +486,7 @@ static bool gw_uses_mma(const Geom& g, bool warp_tile) {
 }
 
 // The fp32 kernels where the tensor-core kernel does not apply.
-static GwPlan plan_gw(const Geom& g, const TileHint& hint) {
+static GwPlan make_plan_gw(const Geom& g, const TileHint& hint) {
     TileHint fp32 = hint;
     if (fp32.variant == 3) fp32.variant = 0;
     GwPlan p = plan_gw_fp32(g, fp32);
@@ -498,6 +498,13 @@ static GwPlan plan_gw(const Geom& g, const TileHint& hint) {
             p.a.splits = sp;
         }
     }
+    return p;
+}
+
+static GwPlan plan_gw(const Geom& g, const TileHint& hint) {
+    if (!hint.is_default()) return make_plan_gw(g, hint);
+    GwPlan p;
+    cached_plan(g, p, [&](GwPlan& q) { q = make_plan_gw(g, hint); return q.status; });
     return p;
 }
 

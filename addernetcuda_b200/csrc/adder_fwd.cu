@@ -378,8 +378,10 @@ template <int KS, int S, int RW, int RM>
 static int launch_fwd_t(const Geom& g, const float* x, const float* w, float* out, const TileHint& hint,
                         cudaStream_t stream, double* stats, int stat_slices, const Epilogue& ep) {
     FwdPlan p;
-    const int st = plan_fwd_t<KS, S, RW, RM>(g, out, hint, p);
+    const int st = hint.is_default() ? cached_plan(g, p, [&](FwdPlan& q) { return plan_fwd_t<KS, S, RW, RM>(g, nullptr, hint, q); })
+                                     : plan_fwd_t<KS, S, RW, RM>(g, nullptr, hint, p);
     if (st != ADDER_OK) return st;
+    if ((reinterpret_cast<uintptr_t>(out) & 15) != 0) p.a.vec_store = 0;
     p.a.x = x; p.a.w = w; p.a.out = out; p.a.ep = ep;
     if ((reinterpret_cast<uintptr_t>(ep.residual) & 15) != 0) p.a.vec_store = 0;
     if ((reinterpret_cast<uintptr_t>(x) & 15) != 0) p.a.x_quads = 0;

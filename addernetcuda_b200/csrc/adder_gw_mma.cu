@@ -22,7 +22,6 @@
 //   split     many channels: six instructions per tap and 16 pixels, 128 output x up to 192 input channels.
 // One CTA per SM: 11 warps load, split and store, a thread of the twelfth issues the products.  Two shared-memory stages; tcgen05.commit releases a stage when the instructions that read it are done.
 #include <cstdio>
-#include <cstring>
 #include "kernels.h"
 #include "tma.cuh"
 
@@ -561,22 +560,8 @@ bool search(const ConvGeom& g, Plan* best) {
     return true;
 }
 
-// The search above costs some microseconds: each thread keeps its last plans.
 bool plan(const ConvGeom& g, Plan* p) {
-    struct Entry { ConvGeom g; int dev; bool ok; Plan p; };
-    static thread_local Entry kept[32];
-    static thread_local int count = 0, next = 0;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); dev = -1; }
-    for (int i = 0; i < count; ++i)
-        if (kept[i].dev == dev && memcmp(&kept[i].g, &g, sizeof(g)) == 0) { *p = kept[i].p; return kept[i].ok; }
-    Entry& e = kept[next];
-    e.g = g; e.dev = dev;
-    e.ok = search(g, &e.p);
-    next = (next + 1) % 32;
-    if (count < 32) ++count;
-    *p = e.p;
-    return e.ok;
+    return cached_plan(g, *p, [&](Plan& q) { return search(g, &q) ? ADDER_OK : ADDER_ERR_UNSUPPORTED; }) == ADDER_OK;
 }
 
 }  // namespace

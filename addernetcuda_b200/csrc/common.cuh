@@ -2,6 +2,9 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <atomic>
+#include <cstring>
+#include <memory>
 
 namespace adder {
 
@@ -210,10 +213,35 @@ inline int largest_divisor_le(int n, int limit) {
 
 // SM count of the current device (148 when no device is visible, e.g. when only planning on a CPU box).
 inline int sm_count() {
+    static std::atomic<int> known[64];
     int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    sms = known[dev].load(std::memory_order_relaxed);
+    if (sms > 0) return sms;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return 148;
+    known[dev].store(sms, std::memory_order_relaxed);
     return sms;
+}
+
+// A tile plan takes 1-5 us of host time, a small layer's kernel 5: each thread keeps the last 16 plans that `compute` made (one
+// store per call site, by the type of the lambda).  A plan depends on the geometry and the device's SM count alone.
+template <class G, class Plan, class Compute>
+int cached_plan(const G& g, Plan& plan, const Compute& compute) {
+    struct Entry { G g; int sms, status; Plan plan; };
+    constexpr int N = 16;
+    static thread_local std::unique_ptr<Entry[]> kept;
+    static thread_local int count = 0, next = 0;
+    const int sms = sm_count();
+    if (!kept) kept.reset(new Entry[N]);
+    for (int i = 0; i < count; ++i)
+        if (kept[i].sms == sms && std::memcmp(&kept[i].g, &g, sizeof(G)) == 0) { plan = kept[i].plan; return kept[i].status; }
+    Entry& e = kept[next];
+    e.g = g; e.sms = sms;
+    e.status = compute(e.plan);
+    plan = e.plan;
+    next = (next + 1) % N;
+    if (count < N) ++count;
+    return e.status;
 }
 
 }  // namespace adder
