@@ -35,7 +35,7 @@ template <class T, int MODE>
 __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel(const __grid_constant__ FwdGatherArgs a) {
     constexpr int RM = T::RM, RP = T::RP, CG = T::CG, TC = T::TC, TP = T::TP, WP = T::WP, PQ = T::PQ, ST = T::ST;
     constexpr int COLS = TP > GATHER_THREADS ? TP / GATHER_THREADS : 1;
-    constexpr int CK = MODE == GATHER_NINE ? 9 * GATHER_NINE_CH : GATHER_CK;      // rows of a stage
+    constexpr int CK = gather_rows(MODE, ST, TC, TP, 0, T::MB);      // rows of a stage
     constexpr int XS = CK * TP, WS = CK * WP;
     extern __shared__ __align__(16) float smem[];
     float* const Xs = smem;
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
             nk = nch * 9; rows = CK; wk = fc.c0 * 9;
         } else {
             nk = min(a.CK, a.Ci - fc.c0); rows = ck4;
-            if (MODE == GATHER_QUADS) gather_quads<TP>(Xs + stage * XS, px[0].base, px[0].ok, a.x, fc.c0, nk, ck4, a.H * a.W, tid);
+            if (MODE == GATHER_QUADS) gather_quads<TP, CK>(Xs + stage * XS, px[0].base, px[0].ok, a.x, fc.c0, nk, ck4, a.H * a.W, tid);
             else gather_pixels<TP>(Xs + stage * XS, px, a.x, a.m, fc, nk, ck4, a.H, a.W, tid);
             wk = fc.c0 * a.KK + a.m.wt0 + fc.i * a.m.dwi + fc.j * a.m.dwj;
         }
@@ -208,9 +208,9 @@ namespace {
     X(4, 4, 16, 4, 6, 92, 30, 54) X(4, 4, 8, 4, 6, 92, 30, 54) X(4, 4, 4, 4, 6, 101, 22, 56)                        \
     X(2, 2, 8, 8, 8, 43, 9, 23) X(2, 2, 4, 8, 8, 49, 10, 26) X(2, 8, 4, 3, 6, 110, 40, 60)
 
-struct Tile { int rm, rp, cg, st, tc, tp; TileCost cost; };
+struct Tile { int rm, rp, cg, st, mb, tc, tp; TileCost cost; };
 constexpr Tile kTiles[] = {
-#define X(RM, RP, CG, ST, MB, A, M, S) {RM, RP, CG, ST, RM * CG, RP * GATHER_THREADS / CG, {A, M, S}},
+#define X(RM, RP, CG, ST, MB, A, M, S) {RM, RP, CG, ST, MB, RM * CG, RP * GATHER_THREADS / CG, {A, M, S}},
     ADDER_FWD_GATHER_TILES(X)
 #undef X
 };
@@ -226,7 +226,7 @@ int choose_tile(int P, int Co) {
     return best;
 }
 
-int stage_rows(const ConvGeom& g) { return g.kh == 3 && g.kw == 3 ? 9 * GATHER_NINE_CH : GATHER_CK; }
+int stage_rows(const Tile& t, int mode) { return gather_rows(mode, t.st, t.tc, t.tp, 0, t.mb); }
 
 size_t smem_bytes(const Tile& t, int rows) {
     return (size_t)t.st * rows * (t.tp + t.tc + 4) * sizeof(float);
@@ -268,7 +268,7 @@ int describe_fwd_gather(const ConvGeom& g, char* buf, size_t n) {
     const int P = g.N * g.Ho * g.Wo;
     const Tile& t = kTiles[choose_tile(P, g.Co)];
     return snprintf(buf, n, "fwd gather k=%dx%d RM=%d RP=%d TC=%d TP=%d threads=%d smem=%zu grid=(%d,%d) status=0", g.kh, g.kw, t.rm,
-                    t.rp, t.tc, t.tp, GATHER_THREADS, smem_bytes(t, stage_rows(g)), ceil_div(P, t.tp), ceil_div(g.Co, t.tc));
+                    t.rp, t.tc, t.tp, GATHER_THREADS, smem_bytes(t, stage_rows(t, g.kh == 3 && g.kw == 3 ? GATHER_NINE : g.kh * g.kw == 1 ? GATHER_QUADS : GATHER_TAP)), ceil_div(P, t.tp), ceil_div(g.Co, t.tc));
 }
 
 int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* out, cudaStream_t stream, const Epilogue& ep) {
@@ -276,19 +276,20 @@ int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* 
     a.m = fwd_map(g);
     a.x = x; a.w = w; a.out = out; a.ep = ep;
     a.Ci = g.Ci; a.H = g.H; a.W = g.W; a.Co = g.Co; a.KK = g.kh * g.kw;
-    const bool nine = g.kh == 3 && g.kw == 3;
-    a.CK = nine ? GATHER_NINE_CH : g.Ci < GATHER_CK ? g.Ci : GATHER_CK;      // full blocks have the cheaper staging loops
-    a.nchunks = ceil_div(g.Ci, a.CK) * (nine ? 1 : a.KK);
     const bool whole_quads = (g.Ho * g.Wo) % 4 == 0;
     a.vec_store = whole_quads && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(ep.residual)) & 15) == 0;
     const bool quads = whole_quads && a.KK == 1 && g.sh == 1 && g.sw == 1 && g.ph == 0 && g.pw == 0 &&
                        (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    const int mode = g.kh == 3 && g.kw == 3 ? GATHER_NINE : quads ? GATHER_QUADS : GATHER_TAP;
     const int tile = choose_tile(a.m.P, g.Co);
     const Tile& t = kTiles[tile];
+    const int rows = stage_rows(t, mode);
+    a.CK = mode == GATHER_NINE ? GATHER_NINE_CH : g.Ci < rows ? g.Ci : rows;      // full blocks have the cheaper staging loops
+    a.nchunks = ceil_div(g.Ci, a.CK) * (mode == GATHER_NINE ? 1 : a.KK);
     const dim3 grid((unsigned)ceil_div(a.m.P, t.tp), (unsigned)ceil_div(g.Co, t.tc));
     if (grid.y > 65535) return ADDER_ERR_UNSUPPORTED;
-    const size_t smem = smem_bytes(t, stage_rows(g));
-    if (nine) return launch_mode<GATHER_NINE>(tile, a, grid, smem, stream);
+    const size_t smem = smem_bytes(t, rows);
+    if (mode == GATHER_NINE) return launch_mode<GATHER_NINE>(tile, a, grid, smem, stream);
     return quads ? launch_mode<GATHER_QUADS>(tile, a, grid, smem, stream) : launch_mode<GATHER_TAP>(tile, a, grid, smem, stream);
 }
 

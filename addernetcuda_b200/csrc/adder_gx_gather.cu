@@ -19,7 +19,6 @@
 namespace adder {
 
 namespace {
-constexpr int FOLD = 4;                 // chunks per partial sum: at most 64 terms before it is folded into the total
 constexpr int MAX_CLASSES = 9;
 }
 
@@ -51,7 +50,9 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
     constexpr int RC = T::RC, RP = T::RP, CG = T::CG, TC = T::TC, TP = T::TP, WP = T::WP, PQ = T::PQ, ST = T::ST;
     constexpr int COLS = TP > GATHER_THREADS ? TP / GATHER_THREADS : 1;
     constexpr int ROWS = TP < GATHER_THREADS ? GATHER_THREADS / TP : 1;
-    constexpr int GS = GATHER_CK * TP, WS = GATHER_CK * WP;
+    constexpr int CK = gather_rows(QUADS ? GATHER_QUADS : GATHER_TAP, ST, TC, TP, RC * RP * GATHER_THREADS * 4, T::MB);      // rows of a stage
+    constexpr int FOLD = 64 / CK;                // chunks per partial sum: 64 terms before it is folded into the total
+    constexpr int GS = CK * TP, WS = CK * WP;
     extern __shared__ __align__(16) float smem[];
     float* const Gs = smem;
     float* const Ws = smem + ST * GS;
@@ -79,7 +80,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
     const int nchunks = ceil_div(a.Co, a.CK) * m.ntaps;
     auto fill = [&](int stage) {
         const int nch = min(a.CK, a.Co - fc.c0);
-        if (QUADS) gather_quads<TP>(Gs + stage * GS, px[0].base, px[0].ok, a.gout, fc.c0, nch, ck4, a.Ho * a.Wo, tid);
+        if (QUADS) gather_quads<TP, CK>(Gs + stage * GS, px[0].base, px[0].ok, a.gout, fc.c0, nch, ck4, a.Ho * a.Wo, tid);
         else gather_pixels<TP>(Gs + stage * GS, px, a.gout, m, fc, nch, ck4, a.Ho, a.Wo, tid);
         // weights [output channel of the chunk][input channel of the tile]
         float* ws = Ws + stage * WS;
@@ -91,9 +92,9 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
             const float* s = okc ? wsrc + (k0 * a.Ci + q) : a.w;
             const int step = okc ? WROWS * a.Ci : 0;
             float* d = ws + k0 * WP + q;
-            if (nch == GATHER_CK && GATHER_CK % WROWS == 0) {
+            if (nch == CK && CK % WROWS == 0) {
 #pragma unroll
-                for (int k = 0; k < GATHER_CK; k += WROWS, s += step) cp_async16(d + k * WP, s, okc);
+                for (int k = 0; k < CK; k += WROWS, s += step) cp_async16(d + k * WP, s, okc);
             } else {
                 for (int k = k0; k < ck4; k += WROWS, s += step, d += WROWS * WP) cp_async16(d, k < nch ? s : a.w, okc & (k < nch));
             }
@@ -101,7 +102,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
             constexpr int WROWS = GATHER_THREADS / TC;
             const int col = tid % TC;
             const bool okc = ci0 + col < a.Ci;
-            copy_rows<WROWS, WP>(ws + col, okc ? wsrc + col * a.KK : a.w, okc ? a.Ci * a.KK : 0, okc, tid / TC, nch, ck4);
+            copy_rows<WROWS, WP, CK>(ws + col, okc ? wsrc + col * a.KK : a.w, okc ? a.Ci * a.KK : 0, okc, tid / TC, nch, ck4);
         }
         fc.next(m, a.CK);
     };
@@ -206,9 +207,9 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
             for (int q = 0; q < COLS; ++q) {
                 const float* cq = col + (tid / TP) * TP + q * GATHER_THREADS;
                 float s = 0.f;
-                if (nk == GATHER_CK) {
+                if (nk == CK) {
 #pragma unroll
-                    for (int k = 0; k < GATHER_CK; k += ROWS) s += cq[k * TP];
+                    for (int k = 0; k < CK; k += ROWS) s += cq[k * TP];
                 } else {
                     for (int k = 0; k < nk; k += ROWS) s += cq[k * TP];
                 }
@@ -324,9 +325,9 @@ namespace {
     X(2, 2, 8, 8, 8, 68, 18, 32, 76, 17, 32) X(2, 2, 4, 8, 8, 70, 18, 33, 80, 18, 33)               \
     X(2, 8, 4, 3, 6, 140, 60, 80, 140, 60, 80)
 
-struct Tile { int rc, rp, cg, st, tc, tp; TileCost exact, fast; };
+struct Tile { int rc, rp, cg, st, mb, tc, tp; TileCost exact, fast; };
 constexpr Tile kTiles[] = {
-#define X(RC, RP, CG, ST, MB, A, M, S, FA, FM, FS) {RC, RP, CG, ST, RC * CG, RP * GATHER_THREADS / CG, {A, M, S}, {FA, FM, FS}},
+#define X(RC, RP, CG, ST, MB, A, M, S, FA, FM, FS) {RC, RP, CG, ST, MB, RC * CG, RP * GATHER_THREADS / CG, {A, M, S}, {FA, FM, FS}},
     ADDER_GX_GATHER_TILES(X)
 #undef X
 };
@@ -345,8 +346,12 @@ int choose_tile(const GxGatherArgs& a, int classes, int Ci, bool fast) {
     return best;
 }
 
-size_t smem_bytes(const Tile& t) {
-    return ((size_t)t.st * GATHER_CK * (t.tp + t.tc + 4) + (size_t)t.rc * t.rp * GATHER_THREADS) * sizeof(float);
+int stage_rows(const Tile& t, bool quads) {
+    return gather_rows(quads ? GATHER_QUADS : GATHER_TAP, t.st, t.tc, t.tp, t.rc * t.rp * GATHER_THREADS * 4, t.mb);
+}
+
+size_t smem_bytes(const Tile& t, bool quads) {
+    return ((size_t)t.st * stage_rows(t, quads) * (t.tp + t.tc + 4) + (size_t)t.rc * t.rp * GATHER_THREADS) * sizeof(float);
 }
 
 // Taps k of one dimension that reach input positions q*S + r: (r + pad - k*dil) % S == 0.  Output position q + o0 + i*d0.
@@ -416,7 +421,6 @@ int plan(const ConvGeom& g, int first, bool fast, GxGatherArgs& a, dim3& grid, b
     int n, total;
     more = fill_classes(g, first, a, n, total, single);
     a.Ci = g.Ci; a.H = g.H; a.W = g.W; a.Co = g.Co; a.Ho = g.Ho; a.Wo = g.Wo; a.KK = g.kh * g.kw; a.sh = g.sh; a.sw = g.sw;
-    a.CK = g.Co < GATHER_CK ? g.Co : GATHER_CK;      // full blocks have the cheaper staging loops, so one ragged block rather than even ones
     const int tile = choose_tile(a, n, g.Ci, fast);
     int most = 0;
     for (int c = 0; c < n; ++c) most = a.m[c].P > most ? a.m[c].P : most;
@@ -432,7 +436,7 @@ int describe_gx_gather(const ConvGeom& g, int fast, char* buf, size_t n) {
     bool more;
     const Tile& t = kTiles[plan(g, 0, fast != 0, a, grid, more)];
     return snprintf(buf, n, "gx gather k=%dx%d fast=%d classes=%u RC=%d RP=%d TC=%d TP=%d threads=%d smem=%zu grid=(%u,%u) status=0",
-                    g.kh, g.kw, fast, grid.z, t.rc, t.rp, t.tc, t.tp, GATHER_THREADS, smem_bytes(t), grid.x, grid.y);
+                    g.kh, g.kw, fast, grid.z, t.rc, t.rp, t.tc, t.tp, GATHER_THREADS, smem_bytes(t, g.kh * g.kw == 1), grid.x, grid.y);
 }
 
 int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const float* w, float* gx, int fast, int accumulate,
@@ -454,7 +458,9 @@ int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const
         // the gradient is read pixel by pixel in order: 1x1 kernels whose class (0, 0) is the output plane
         const bool quads = g.kh == 1 && g.kw == 1 && g.ph == 0 && g.pw == 0 && a.m[0].PH == g.Ho && a.m[0].PW == g.Wo && grid.z == 1 && first == 0 &&
                            (g.Ho * g.Wo) % 4 == 0 && (reinterpret_cast<uintptr_t>(gout) & 15) == 0;
-        const size_t smem = smem_bytes(kTiles[tile]);
+        const int rows = stage_rows(kTiles[tile], quads);
+        a.CK = g.Co < rows ? g.Co : rows;      // full blocks have the cheaper staging loops, so one ragged block rather than even ones
+        const size_t smem = smem_bytes(kTiles[tile], quads);
         const int st = fast ? (quads ? launch_tile<true, true>(tile, a, grid, smem, stream) : launch_tile<true, false>(tile, a, grid, smem, stream))
                             : (quads ? launch_tile<false, true>(tile, a, grid, smem, stream) : launch_tile<false, false>(tile, a, grid, smem, stream));
         if (st != ADDER_OK) return st;

@@ -20,6 +20,14 @@ constexpr int GATHER_NINE_CH = 2;        // channels per chunk of GATHER_NINE
 constexpr int GATHER_THREADS = 128;
 enum GatherMode { GATHER_TAP, GATHER_QUADS, GATHER_NINE };
 
+// Rows of a stage.  1x1 layers take 32 channels at a time where four CTAs still fit an SM: half the barriers (1024->256 on 75,776
+// pixels: input gradient 1687 -> 1549 us saturating, 2013 -> 1937 exact, forward 1344 -> 1326; 3x3 layers lose 1-6 %, the weights of
+// a chunk being strided).
+__host__ __device__ constexpr int gather_rows(int mode, int stages, int tc, int tp, int more_bytes, int ctas) {
+    if (mode == GATHER_NINE) return 9 * GATHER_NINE_CH;
+    return mode == GATHER_QUADS && ctas <= 4 && stages * 32 * (tp + tc + 4) * 4 + more_bytes <= 56 * 1024 ? 2 * GATHER_CK : GATHER_CK;
+}
+
 // What a tile costs, in clocks per reduction step, measured over 30 layers (n 1-256, 3x3 and 1x1) with every tile forced and fitted
 // within 3-10 %: `alone` for a CTA that has its SM to itself, `more` for each further one beside it while they hide each other's
 // latency, `share` of the SM's throughput.
@@ -73,13 +81,13 @@ struct GatherChunk {
 // Copies rows k0, k0 + STEP, ... of one staged column: row k comes from s + k * stride, rows from nch on are zero.
 // The common full chunk is straight-line code, an address increment and a copy a row; a column that reads zeros has
 // stride 0 and a valid address.
-template <int STEP, int PITCH>
+template <int STEP, int PITCH, int CK = GATHER_CK>
 __device__ __forceinline__ void copy_rows(float* d, const float* s, int stride, bool ok, int k0, int nch, int ck) {
     d += k0 * PITCH;
     s += k0 * stride;
-    if (nch == GATHER_CK) {
+    if (nch == CK) {
 #pragma unroll
-        for (int k = 0; k < GATHER_CK; k += STEP, s += STEP * stride) cp_async4(d + k * PITCH, s, ok);
+        for (int k = 0; k < CK; k += STEP, s += STEP * stride) cp_async4(d + k * PITCH, s, ok);
     } else {
         const float* first = s;
 #pragma unroll 2
@@ -105,7 +113,7 @@ __device__ __forceinline__ void gather_pixels(float* dst, const GatherPixel* px,
 
 // The same for layers whose pixels are the source's own pixels in order (1x1, stride 1, no padding) and whose planes are whole
 // quads: 16-byte copies.  px holds the thread's quad (pixel 4 * (tid % (TP/4)) of the tile).
-template <int TP>
+template <int TP, int CK>
 __device__ __forceinline__ void gather_quads(float* dst, const float* base, bool ok, const float* src, int c0, int nch, int ck,
                                              int plane, int tid) {
     constexpr int QUADS = TP / 4, ROWS = GATHER_THREADS / QUADS;
@@ -113,9 +121,9 @@ __device__ __forceinline__ void gather_quads(float* dst, const float* base, bool
     float* d = dst + k0 * TP + 4 * (tid % QUADS);
     const float* s = ok ? base + (c0 + k0) * plane : src;
     const int step = ok ? ROWS * plane : 0;
-    if (nch == GATHER_CK) {
+    if (nch == CK) {
 #pragma unroll
-        for (int k = 0; k < GATHER_CK; k += ROWS, s += step) cp_async16(d + k * TP, s, ok);
+        for (int k = 0; k < CK; k += ROWS, s += step) cp_async16(d + k * TP, s, ok);
     } else {
         for (int k = k0; k < ck; k += ROWS, s += step, d += ROWS * TP) cp_async16(d, k < nch ? s : src, ok & (k < nch));
     }
