@@ -49,6 +49,7 @@ struct GwMmaArgs {
     int N, Ci, H, W, Co, Ho, Wo, KK;
     int sh, sw, ph, pw;
     int flat;                // 1x1: positions are consecutive output pixels of the batch
+    int quads;               // ... 32 to a chunk, stride 1 and planes of whole quads
     int R, pitch, gpos;      // rows per chunk, positions per row, staged positions of g (a multiple of 16)
     int xrows, xpos, planes, planes_w;       // rows and positions of one plane of x, planes, planes per row of planes
     int chunks, row_blocks, splits;
@@ -107,8 +108,13 @@ __device__ __forceinline__ uint32_t take_bf16(float& a, float& b) {
     return p;
 }
 
-template <bool FLAT, bool STACKED>
+// How positions are read: ROWS of the output with their halo; FLAT, the pixels of the batch in order (1x1 layers); QUADS, the same four
+// at a time, which takes half the instructions.
+enum { ROWS, FLAT_PIXELS, FLAT_QUADS };
+
+template <int MODE, bool STACKED>
 __global__ void __launch_bounds__(THREADS, 1) adder_gw_mma_kernel(const __grid_constant__ GwMmaArgs a, int* error_flag) {
+    constexpr bool FLAT = MODE != ROWS;
     extern __shared__ __align__(128) uint4 smem16[];           // rows of 8 channels
     __shared__ __align__(16) uint4 ones[32];                   // 2 groups of 8 columns x 16 steps: column 0 is one
     __shared__ uint64_t full[2], empty[2], drained;
@@ -239,6 +245,50 @@ __global__ void __launch_bounds__(THREADS, 1) adder_gw_mma_kernel(const __grid_c
                 mma_commit(&empty[s]);
             }
             __syncwarp();
+        }
+    } else if constexpr (MODE == FLAT_QUADS) {
+        // ---- the warps that load, split and store: a thread has four pixels of eight channels.  The reduction's order is free where no
+        // tap shifts it, so pixel 4*l + j of a chunk of 32 is step 8*j + l: eight neighbouring threads store neighbouring rows.
+        const int HoWo = a.Ho * a.Wo, grp = tid >> 3, l = tid & 7;
+        const bool is_x = grp < a.cig, used = grp < a.cig + a.cog;
+        const int C = is_x ? a.Ci : a.Co, ch = is_x ? ci0 + grp * 8 : co0 + (grp - a.cig) * 8, left = used ? C - ch : 0;
+        const float* const tensor = is_x ? a.x : a.g;
+        const int row = (is_x ? 3 * gsplit + grp * 32 : (grp - a.cig) * 32) + l, split_rows = is_x ? xsplit : gsplit;
+        float4 v[8];
+        auto load = [&](int chunk) {
+            const int p = chunk * 32 + 4 * l;
+            const bool in = p < a.N * HoWo;
+            uint32_t im, r;
+            a.d_howo.divmod(in ? p : 0, im, r);
+            const float* src = tensor + ((size_t)im * C + (left > 0 ? ch : 0)) * HoWo + r;
+#pragma unroll
+            for (int q = 0; q < 8; ++q, src += HoWo)
+                v[q] = (in & (q < left)) ? __ldg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        if (n_local > 0) load(c_begin);
+        for (int i = 0; i < n_local; ++i) {
+            const int s = i & 1;
+            if (i >= 2 && !mbar_wait(&empty[s], ((i >> 1) - 1) & 1)) { gave_up = 1; break; }
+            if (used) {
+                uint4* d = smem16 + s * stage_rows + row;
+                auto store = [&](int j, float (&u)[8]) {
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) {
+                        uint4 p;
+                        p.x = take_bf16(u[0], u[1]); p.y = take_bf16(u[2], u[3]);
+                        p.z = take_bf16(u[4], u[5]); p.w = take_bf16(u[6], u[7]);
+                        d[q * split_rows + j * 8] = p;
+                    }
+                };
+                float u0[8], u1[8], u2[8], u3[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) { u0[q] = v[q].x; u1[q] = v[q].y; u2[q] = v[q].z; u3[q] = v[q].w; }
+                store(0, u0); store(1, u1); store(2, u2); store(3, u3);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full[s])) : "memory");
+            if (i + 1 < n_local) load(c_begin + i + 1);
+            if (i > 0 && i % a.drain_chunks == 0 && !drain(i)) { gave_up = 1; break; }
         }
     } else {
         // ---- the warps that load, split and store: each thread has up to TASKS (channel group, position) pairs
@@ -497,7 +547,7 @@ bool shape(const ConvGeom& g, GwMmaArgs a, int rows, Plan* p) {
     const double instr = a.n_instr / 2 + 3 > 36 + a.n_instr / 4 ? a.n_instr / 2 + 3 : 36 + a.n_instr / 4;
     const double sums = (a.stacked ? 42.0 : 126.0) / (a.ci_tiles * a.tap_groups);
     const double products = steps * ((double)a.taps_per_group * (a.stacked ? 1 : 6) * instr + sums) + 250 + 900.0 / a.drain_chunks;
-    const double turn = 1000 + 700.0 * tasks / LOADERS;
+    const double turn = a.quads ? 1800 : 1000 + 700.0 * tasks / LOADERS;
     const double chunk = products > turn ? products : turn;
     const int tiles = a.co_tiles * a.ci_tiles * a.tap_groups, slots = sm_count();
     const int least = ceil_div(a.chunks, (a.stacked ? MAX_STEPS_STACKED : MAX_STEPS_SPLIT) / steps);
@@ -522,6 +572,7 @@ bool search(const ConvGeom& g, Plan* best) {
     a.sh = g.sh; a.sw = g.sw; a.ph = g.ph; a.pw = g.pw;
     a.flat = a.KK == 1 && g.ph == 0 && g.pw == 0;
     a.whole = g.Ci % 8 == 0 && g.Co % 8 == 0;
+    a.quads = a.flat && g.sh == 1 && g.sw == 1 && (g.Ho * g.Wo) % 4 == 0;
     const int co8 = ceil_div(g.Co, 8), ci8 = round_up(ceil_div(g.Ci, 8), 2);
     for (int form = 0; form < 4; ++form)
         for (int by_rows = 0; by_rows < (g.kh > 1 ? 2 : 1); ++by_rows) {
@@ -545,7 +596,7 @@ bool search(const ConvGeom& g, Plan* best) {
                 while (a.tmem_cols < cols) a.tmem_cols *= 2;
                 a.ci_tiles = ceil_div(ceil_div(g.Ci, 8), cig);
                 const int most = a.flat ? 2 : g.Ho;
-                for (int rows = 1; rows <= most; ++rows) {
+                for (int rows = a.quads ? 2 : 1; rows <= most; ++rows) {
                     Plan p;
                     if (!shape(g, a, rows, &p)) break;         // more rows only need more
                     if (p.clocks < best->clocks) *best = p;
@@ -592,8 +643,10 @@ int launch_gw_mma(const ConvGeom& g, const float* gout, const float* x, float* p
     int* flag = nullptr;
     int st = device_error_flag(&flag);
     if (st != ADDER_OK) return st;
-    auto kern = p.a.flat ? (p.a.stacked ? adder_gw_mma_kernel<true, true> : adder_gw_mma_kernel<true, false>)
-                         : (p.a.stacked ? adder_gw_mma_kernel<false, true> : adder_gw_mma_kernel<false, false>);
+    const bool quads = p.a.quads && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gout)) & 15) == 0;
+    auto kern = quads      ? (p.a.stacked ? adder_gw_mma_kernel<FLAT_QUADS, true> : adder_gw_mma_kernel<FLAT_QUADS, false>)
+                : p.a.flat ? (p.a.stacked ? adder_gw_mma_kernel<FLAT_PIXELS, true> : adder_gw_mma_kernel<FLAT_PIXELS, false>)
+                           : (p.a.stacked ? adder_gw_mma_kernel<ROWS, true> : adder_gw_mma_kernel<ROWS, false>);
     st = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), p.smem);
     if (st != ADDER_OK) return st;
     kern<<<dim3((unsigned)splits, (unsigned)(p.a.co_tiles * p.a.ci_tiles * p.a.tap_groups)), THREADS, p.smem, stream>>>(p.a, flag);
