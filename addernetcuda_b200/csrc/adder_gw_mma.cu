@@ -49,7 +49,7 @@ struct GwMmaArgs {
     int N, Ci, H, W, Co, Ho, Wo, KK;
     int sh, sw, ph, pw;
     int flat;                // 1x1: positions are consecutive output pixels of the batch
-    int quads;               // ... 32 to a chunk, stride 1 and planes of whole quads
+    int quads;               // ... 32 to a chunk, in aligned quads (FLAT_QUADS)
     int R, pitch, gpos;      // rows per chunk, positions per row, staged positions of g (a multiple of 16)
     int xrows, xpos, planes, planes_w;       // rows and positions of one plane of x, planes, planes per row of planes
     int chunks, row_blocks, splits;
@@ -260,6 +260,20 @@ __global__ void __launch_bounds__(THREADS, 1) adder_gw_mma_kernel(const __grid_c
             const bool in = p < a.N * HoWo;
             uint32_t im, r;
             a.d_howo.divmod(in ? p : 0, im, r);
+            if (a.sw == 2 && is_x) {                   // every other pixel of every other row
+                uint32_t y, x;
+                a.d_wo.divmod(r, y, x);
+                const int HW = a.H * a.W;
+                const float* src = tensor + ((size_t)im * C + (left > 0 ? ch : 0)) * HW + 2 * y * a.W + 2 * x;
+#pragma unroll
+                for (int q = 0; q < 8; ++q, src += HW) {
+                    const bool ok = in & (q < left);
+                    const float4 lo = ok ? __ldg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float4 hi = ok ? __ldg(reinterpret_cast<const float4*>(src + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    v[q] = make_float4(lo.x, lo.z, hi.x, hi.z);
+                }
+                return;
+            }
             const float* src = tensor + ((size_t)im * C + (left > 0 ? ch : 0)) * HoWo + r;
 #pragma unroll
             for (int q = 0; q < 8; ++q, src += HoWo)
@@ -572,7 +586,8 @@ bool search(const ConvGeom& g, Plan* best) {
     a.sh = g.sh; a.sw = g.sw; a.ph = g.ph; a.pw = g.pw;
     a.flat = a.KK == 1 && g.ph == 0 && g.pw == 0;
     a.whole = g.Ci % 8 == 0 && g.Co % 8 == 0;
-    a.quads = a.flat && g.sh == 1 && g.sw == 1 && (g.Ho * g.Wo) % 4 == 0;
+    // whole aligned quads of output pixels, and of the input pixels under them
+    a.quads = a.flat && (g.Ho * g.Wo) % 4 == 0 && ((g.sh == 1 && g.sw == 1) || (g.sh == 2 && g.sw == 2 && g.Wo % 4 == 0 && g.W == 2 * g.Wo));
     const int co8 = ceil_div(g.Co, 8), ci8 = round_up(ceil_div(g.Ci, 8), 2);
     for (int form = 0; form < 4; ++form)
         for (int by_rows = 0; by_rows < (g.kh > 1 ? 2 : 1); ++by_rows) {
