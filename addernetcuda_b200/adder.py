@@ -71,9 +71,9 @@ def _fused_geometry(W, stride, padding, dilation) -> bool:
 def _adder2d_columns(X, W, stride, padding, dilation):
     """Every other geometry (5x5, 7x7, rectangular kernels, stride 3, dilation ...).  Almost all of them run on the
     gathering kernels and the tensor-core weight gradient (`_native.conv`), without a column matrix.  The rest - windows or
-    output rows too wide for the latter, other tensors than contiguous fp32 ones - as the reference itself computes a layer, an explicit im2col around the column-matrix op (adder.py:22-41), with this
-    library's column kernels underneath (`adder`) and autograd's fold as col2im.  Columns are ordered
-    (image, position), which the op does not care about."""
+    output rows too wide for the latter, other tensors than contiguous fp32 ones - as the reference itself computes a layer:
+    an explicit im2col around the column-matrix op (adder.py:22-41), with this library's column kernels underneath (`adder`)
+    and autograd's fold as col2im.  Columns are ordered (image, position), which the op does not care about."""
     pair = lambda v: (v, v) if isinstance(v, int) else tuple(v)
     (sh, sw), (ph, pw), (dh, dw) = pair(stride), pair(padding), pair(dilation)
     if adder_cuda.unpatched():
@@ -137,8 +137,8 @@ class adder(Function):
 class adder2d(nn.Module):
     """adder.py:83-108.  `depth_wise=True` is rejected: the reference allocates [Co,1,k,k] weights for
     it but its forward ignores the flag, so no caller can rely on it.  3x3 and 1x1 kernels at stride 1 or 2 run
-    on the fused kernels; any other kernel size or stride (and the extensions: a (kh, kw) tuple, `dilation`)
-    runs through the column-matrix kernels behind an explicit im2col."""
+    on the fused kernels; any other kernel size or stride (and the extensions: a (kh, kw) tuple, `dilation`) as
+    `_adder2d_columns` says."""
 
     def __init__(self, input_channel, output_channel, kernel_size, stride=1, padding=0, bias=False,
                  depth_wise=False, dilation=1):

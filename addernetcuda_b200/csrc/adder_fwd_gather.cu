@@ -47,24 +47,23 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
     const size_t image = (size_t)a.Ci * a.H * a.W;
 
     GatherPixel px[COLS];
-    unsigned mask[COLS];
+    constexpr int CH = nine_channels(TC, TP);
+    GatherNine<TP, CH> nine;
     if (MODE == GATHER_QUADS) {
         px[0].decode(a.m, a.x, p0 + 4 * (tid % (TP / 4)), image);
         px[0].base += px[0].row * a.W + px[0].col;
     } else {
 #pragma unroll
-        for (int q = 0; q < COLS; ++q) {
-            px[q].decode(a.m, a.x, p0 + (COLS > 1 ? tid + q * GATHER_THREADS : tid % TP), image);
-            if (MODE == GATHER_NINE) mask[q] = nine_mask(px[q], a.m, a.H, a.W);
-        }
+        for (int q = 0; q < COLS; ++q) px[q].decode(a.m, a.x, p0 + (COLS > 1 ? tid + q * GATHER_THREADS : tid % TP), image);
+        if (MODE == GATHER_NINE) nine.init(px, a.m, a.H, a.W, tid);
     }
     GatherChunk fc;              // position of the next chunk to stage
     const int ck4 = round_up(a.CK, 4);
     auto fill = [&](int stage) {
         int nk, rows, wk;        // reduction steps that exist, rows to stage, and the first one's weight index
         if constexpr (MODE == GATHER_NINE) {
-            const int nch = min(GATHER_NINE_CH, a.Ci - fc.c0);
-            gather_nine<TP>(Xs + stage * XS, px, mask, a.m, fc.c0, nch, a.H, a.W, tid);
+            const int nch = min(CH, a.Ci - fc.c0);
+            nine.fill(Xs + stage * XS, px, a.m, fc.c0, nch, a.H, a.W, tid);
             nk = nch * 9; rows = CK; wk = fc.c0 * 9;
         } else {
             nk = min(a.CK, a.Ci - fc.c0); rows = ck4;
@@ -89,7 +88,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
                 cp_async4(ws + kb * WP + c, ok ? wsrc + (c * row + kb * kstep) : a.w, ok);
             }
         }
-        if (MODE == GATHER_NINE) fc.c0 += GATHER_NINE_CH;
+        if (MODE == GATHER_NINE) fc.c0 += CH;
         else fc.next(a.m, a.CK);
     };
 
@@ -115,7 +114,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
         const float* xs = Xs + stage * XS + pg * PQ;
         const float* ws = Ws + stage * WS + cg * RM;
         const int nk = MODE == GATHER_NINE ? CK : min(ck4, round_up(a.Ci - cc.c0, 4));
-#pragma unroll (RM * RP >= 64 ? 1 : RM * RP >= 32 ? 2 : 4)
+#pragma unroll (RM * RP >= 64 ? 1 : RM * RP >= 32 ? 2 : RM * RP > 1 ? 4 : CK / 2)
         for (int k = 0; k < nk; ++k) {
             float xv[RP], wv[RM];
 #pragma unroll
@@ -123,9 +122,11 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
                 if constexpr (PQ == 4) {
                     const float4 q = *reinterpret_cast<const float4*>(xs + k * TP + h * (TP / 2));
                     xv[4 * h] = q.x; xv[4 * h + 1] = q.y; xv[4 * h + 2] = q.z; xv[4 * h + 3] = q.w;
-                } else {
+                } else if constexpr (PQ == 2) {
                     const float2 q = *reinterpret_cast<const float2*>(xs + k * TP);
                     xv[0] = q.x; xv[1] = q.y;
+                } else {
+                    xv[0] = xs[k * TP];
                 }
             }
             if constexpr (RM >= 4) {
@@ -134,22 +135,26 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
                     const float4 q = *reinterpret_cast<const float4*>(ws + k * WP + m);
                     wv[m] = q.x; wv[m + 1] = q.y; wv[m + 2] = q.z; wv[m + 3] = q.w;
                 }
-            } else {
+            } else if constexpr (RM == 2) {
                 const float2 q = *reinterpret_cast<const float2*>(ws + k * WP);
                 wv[0] = q.x; wv[1] = q.y;
             }
-            uint64_t nx2[RP];
+            if constexpr (RM == 1) {
+                acc[0][0] += fabsf(ws[k * WP] - xv[0]);
+            } else {
+                uint64_t nx2[RP];
 #pragma unroll
-            for (int j = 0; j < RP; ++j) nx2[j] = pack2(-xv[j], -xv[j]);
+                for (int j = 0; j < RP; ++j) nx2[j] = pack2(-xv[j], -xv[j]);
 #pragma unroll
-            for (int m = 0; m < RM; m += 2) {
-                const uint64_t w2 = pack2(wv[m], wv[m + 1]);
+                for (int m = 0; m < RM; m += 2) {
+                    const uint64_t w2 = pack2(wv[m], wv[m + 1]);
 #pragma unroll
-                for (int j = 0; j < RP; ++j) {
-                    float d0, d1;
-                    unpack2(add2(w2, nx2[j]), d0, d1);
-                    acc[m][j] += fabsf(d0);
-                    acc[m + 1][j] += fabsf(d1);
+                    for (int j = 0; j < RP; ++j) {
+                        float d0, d1;
+                        unpack2(add2(w2, nx2[j]), d0, d1);
+                        acc[m][j] += fabsf(d0);
+                        acc[m + 1][j] += fabsf(d1);
+                    }
                 }
             }
         }
@@ -200,13 +205,15 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
 
 namespace {
 
-// The tiles: large ones have the fewest loads per term, small ones give a small layer more threads.
+// The tiles: large ones have the fewest loads per term, small ones give a small layer more threads.  The smallest, an output a
+// thread with 4 channels of a 3x3 window a stage, is for layers of fewer outputs than the chip has threads, whose time is the chain
+// of stages of one CTA (before it: 64->64 8x8 at batch 1 14.1 -> 9.7 us, 32->32 16x16 8.0 -> 5.7, 512->512 7x7 102 -> 79).
 // X(RM, RP, CG, ST, MB, clocks per step: alone, each further CTA, throughput)
 #define ADDER_FWD_GATHER_TILES(X)                                                                                   \
     X(8, 8, 8, 2, 4, 242, 147, 173) X(8, 8, 16, 2, 4, 241, 74, 186) X(8, 8, 4, 2, 4, 278, 130, 186)                 \
     X(4, 8, 16, 3, 4, 139, 65, 93) X(4, 8, 8, 3, 4, 139, 65, 93) X(4, 8, 4, 2, 4, 174, 76, 109)                     \
     X(4, 4, 16, 4, 6, 92, 30, 54) X(4, 4, 8, 4, 6, 92, 30, 54) X(4, 4, 4, 4, 6, 101, 22, 56)                        \
-    X(2, 2, 8, 8, 8, 43, 9, 23) X(2, 2, 4, 8, 8, 49, 10, 26) X(2, 8, 4, 3, 6, 110, 40, 60)
+    X(2, 2, 8, 8, 8, 43, 9, 23) X(2, 2, 4, 8, 8, 49, 10, 26) X(2, 8, 4, 3, 6, 110, 40, 60) X(1, 1, 4, 6, 8, 20, 6, 20)
 
 struct Tile { int rm, rp, cg, st, mb, tc, tp; TileCost cost; };
 constexpr Tile kTiles[] = {
@@ -284,7 +291,7 @@ int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* 
     const int tile = choose_tile(a.m.P, g.Co);
     const Tile& t = kTiles[tile];
     const int rows = stage_rows(t, mode);
-    a.CK = mode == GATHER_NINE ? GATHER_NINE_CH : g.Ci < rows ? g.Ci : rows;      // full blocks have the cheaper staging loops
+    a.CK = mode == GATHER_NINE ? rows / 9 : g.Ci < rows ? g.Ci : rows;      // full blocks have the cheaper staging loops
     a.nchunks = ceil_div(g.Ci, a.CK) * (mode == GATHER_NINE ? 1 : a.KK);
     const dim3 grid((unsigned)ceil_div(a.m.P, t.tp), (unsigned)ceil_div(g.Co, t.tc));
     if (grid.y > 65535) return ADDER_ERR_UNSUPPORTED;

@@ -16,15 +16,17 @@
 namespace adder {
 
 constexpr int GATHER_CK = 16;
-constexpr int GATHER_NINE_CH = 2;        // channels per chunk of GATHER_NINE
 constexpr int GATHER_THREADS = 128;
 enum GatherMode { GATHER_TAP, GATHER_QUADS, GATHER_NINE };
+
+// Channels of a chunk of GATHER_NINE.
+__host__ __device__ constexpr int nine_channels(int tc, int tp) { return tc * tp <= GATHER_THREADS ? 4 : 2; }
 
 // Rows of a stage.  1x1 layers take 32 channels at a time where four CTAs still fit an SM: half the barriers (1024->256 on 75,776
 // pixels: input gradient 1687 -> 1549 us saturating, 2013 -> 1937 exact, forward 1344 -> 1326; 3x3 layers lose 1-6 %, the weights of
 // a chunk being strided).
 __host__ __device__ constexpr int gather_rows(int mode, int stages, int tc, int tp, int more_bytes, int ctas) {
-    if (mode == GATHER_NINE) return 9 * GATHER_NINE_CH;
+    if (mode == GATHER_NINE) return 9 * nine_channels(tc, tp);
     return mode == GATHER_QUADS && ctas <= 4 && stages * 32 * (tp + tc + 4) * 4 + more_bytes <= 56 * 1024 ? 2 * GATHER_CK : GATHER_CK;
 }
 
@@ -140,26 +142,56 @@ __device__ __forceinline__ unsigned nine_mask(const GatherPixel& px, const Gathe
     return mask;
 }
 
-// GATHER_NINE: rows (channel c0 + r/9, tap r%9), r < 18, of the thread's pixels; channels from nch on are zero.
-template <int TP>
-__device__ __forceinline__ void gather_nine(float* dst, const GatherPixel* px, const unsigned* mask, const GatherMap& m, int c0,
-                                            int nch, int Hs, int Ws, int tid) {
-    constexpr int COLS = TP > GATHER_THREADS ? TP / GATHER_THREADS : 1;
-    constexpr int ROWS = TP < GATHER_THREADS ? GATHER_THREADS / TP : 1;
-    const int plane = Hs * Ws;
+// GATHER_NINE: rows (channel c0 + r/9, tap r%9), r < 9 CH, of the thread's pixels; channels from nch on are zero.  Where several
+// threads share a pixel (TP < 128: small layers, whose time is this loop's), a thread's rows are not known at compile time: their
+// offsets are computed once.
+template <int TP, int CH>
+struct GatherNine {
+    static constexpr int COLS = TP > GATHER_THREADS ? TP / GATHER_THREADS : 1;
+    static constexpr int ROWS = TP < GATHER_THREADS ? GATHER_THREADS / TP : 1;
+    static constexpr int N = (9 * CH + ROWS - 1) / ROWS;
+    unsigned mask[COLS];        // a bit per tap; ROWS > 1: a bit per row of this thread
+    int off[ROWS > 1 ? N : 1];
+
+    __device__ __forceinline__ void init(const GatherPixel* px, const GatherMap& m, int Hs, int Ws, int tid) {
 #pragma unroll
-    for (int q = 0; q < COLS; ++q) {
-        const float* s = px[q].base + (c0 * plane + (px[q].row + m.oy0) * Ws + px[q].col + m.ox0);
-        float* d = dst + (COLS > 1 ? tid + q * GATHER_THREADS : tid % TP);
+        for (int q = 0; q < COLS; ++q) mask[q] = nine_mask(px[q], m, Hs, Ws);
+        if constexpr (ROWS > 1) {
+            const unsigned taps = mask[0];
+            mask[0] = 0;
 #pragma unroll
-        for (int i = 0; i < (9 * GATHER_NINE_CH + ROWS - 1) / ROWS; ++i) {
-            const int r = i * ROWS + (ROWS > 1 ? tid / TP : 0);
-            if (ROWS > 1 && (9 * GATHER_NINE_CH) % ROWS != 0 && r >= 9 * GATHER_NINE_CH) break;
-            const int c = r / 9, t = r - c * 9;
-            // nothing is read where the predicate is false, so the address may lie outside the tensor there
-            cp_async4(d + r * TP, s + (c * plane + (t / 3) * m.doy * Ws + (t % 3) * m.dox), (mask[q] >> t & 1) & (c < nch));
+            for (int i = 0; i < N; ++i) {
+                const int r = i * ROWS + tid / TP, c = r / 9, t = r - c * 9;
+                off[i] = c * Hs * Ws + (t / 3) * m.doy * Ws + (t % 3) * m.dox;
+                if (taps >> t & 1) mask[0] |= 1u << i;
+            }
         }
     }
-}
+    __device__ __forceinline__ void fill(float* dst, const GatherPixel* px, const GatherMap& m, int c0, int nch, int Hs, int Ws,
+                                         int tid) const {
+        const int plane = Hs * Ws;
+        if constexpr (ROWS > 1) {
+            const float* s = px[0].base + (c0 * plane + (px[0].row + m.oy0) * Ws + px[0].col + m.ox0);
+            const int rows = 9 * CH - tid / TP, full = 9 * nch - tid / TP;
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                if ((9 * CH) % ROWS != 0 && i == N - 1 && i * ROWS >= rows) break;
+                // nothing is read where the predicate is false, so the address may lie outside the tensor there
+                cp_async4(dst + tid + i * GATHER_THREADS, s + off[i], (mask[0] >> i & 1) & (i * ROWS < full));
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < COLS; ++q) {
+                const float* s = px[q].base + (c0 * plane + (px[q].row + m.oy0) * Ws + px[q].col + m.ox0);
+                float* d = dst + tid + q * GATHER_THREADS;
+#pragma unroll
+                for (int r = 0; r < 9 * CH; ++r) {
+                    const int c = r / 9, t = r - c * 9;
+                    cp_async4(d + r * TP, s + (c * plane + (t / 3) * m.doy * Ws + (t % 3) * m.dox), (mask[q] >> t & 1) & (c < nch));
+                }
+            }
+        }
+    }
+};
 
 }  // namespace adder

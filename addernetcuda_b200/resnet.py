@@ -40,22 +40,23 @@ def _bn_act(bn, y, residual=None, relu=False):
     return torch.relu(out) if relu else out
 
 
-def _hooked(*modules) -> bool:
-    return any(m._forward_hooks or m._forward_pre_hooks for m in modules)
-
-
 def _conv_bn_act(conv, bn, x, residual=None, relu=False):
     """relu?(bn(conv(x)) + residual?).  An adder layer followed by a FusedBatchNorm2d in training mode hands
     the batch statistics over from its own epilogue, so the normalisation reads the layer's output once; one followed by a
     folded batch norm applies it in its own epilogue."""
-    if (bn.__class__.__name__ == "FusedBatchNorm2d" and bn.training and x.is_cuda and x.dtype == torch.float32
+    kind = bn.__class__.__name__
+    if kind == "FoldedBatchNorm2d":
+        # hooks on either module want its own call and output
+        if not (conv._forward_hooks or conv._forward_pre_hooks or bn._forward_hooks or bn._forward_pre_hooks
+                or torch.is_grad_enabled()) and hasattr(conv, "forward_affine"):
+            folded = bn._buffers
+            z = conv.forward_affine(x, folded["scale"], folded["shift"], residual, relu)
+            if z is not None:
+                return z
+    elif (kind == "FusedBatchNorm2d" and bn.training and x.is_cuda and x.dtype == torch.float32
             and hasattr(conv, "forward_with_stats")):
         y, st = conv.forward_with_stats(x)
         return bn(y, residual=residual, relu=relu, stats=st)
-    if bn.__class__.__name__ == "FoldedBatchNorm2d" and hasattr(conv, "forward_affine") and not torch.is_grad_enabled() and not _hooked(conv, bn):
-        z = conv.forward_affine(x, bn.scale, bn.shift, residual, relu)
-        if z is not None:
-            return z
     return _bn_act(bn, conv(x), residual=residual, relu=relu)
 
 
