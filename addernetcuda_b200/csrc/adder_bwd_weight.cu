@@ -180,9 +180,10 @@ __global__ void __launch_bounds__(256, GW_MIN_BLOCKS) adder_gw_kernel(const GwAr
 }
 
 constexpr int FIN_THREADS = 256;
-constexpr int FIN_OUT = 8;                        // gradient elements per reduce block
-constexpr int FIN_LANES = FIN_THREADS / FIN_OUT;  // threads that share one element and split the slices
-constexpr int FUSED_FINISH_MAX = 1 << 17;         // gradients up to this many elements finish in one kernel
+constexpr int FIN_NORM = 8;                       // elements per partial sum of squares
+// Gradients up to this many elements finish in one kernel.  The last block's rescale is a pass of one SM over the gradient (96->96
+// 3x3, 82,944 elements: 67 us with it, 58 with two launches more; 64->64, 36,864: 53 against 56).
+constexpr int FUSED_FINISH_MAX = 1 << 16;
 
 // gw[i] = sum_s part[s][i] - w[i] * sum_s gsum_part[s][co(i)], plus the block's partial of sum gw^2, in double
 // precision and in slice order, so the result does not depend on scheduling.  This is the form for large
@@ -238,70 +239,93 @@ __global__ void __launch_bounds__(1024) adder_gw_norm_kernel(const GwFinishArgs 
     }
 }
 
-// Small gradients: one kernel does all three finishing steps.  Every block reduces its 32 elements
-// and publishes its partial sum of squares; the block that draws the last ticket adds the partials
-// in index order (so the result does not depend on which block that is), derives the scale and
-// applies it to the whole gradient.  The ticket counter is zeroed by the main kernel of the same call.
-__global__ void __launch_bounds__(FIN_THREADS) adder_gw_finish_kernel(const GwFinishArgs a, int nblocks,
-                                                                      unsigned int* ticket) {
-    __shared__ double s_sum[FIN_LANES][FIN_OUT];
-    __shared__ double s_gs[FIN_LANES][FIN_OUT];
-    __shared__ double s_sq[FIN_THREADS];
+// Small gradients: one kernel does all three finishing steps.  Every block reduces OUT elements and publishes its partial
+// sums of squares; the block that draws the last ticket adds the partials in a fixed order (so the result does not depend on
+// which block that is), derives the scale and applies it to the whole gradient.  The ticket counter is zeroed by the main kernel
+// of the same call.  A few MB at most, so latency is what counts: the slices of an element are spread over 256 / OUT threads with
+// eight loads in flight each, and the rescale, which is one block's, keeps eight 16-byte loads a thread in flight (before, with one or
+// two: the whole gradient of 64->64 8x8 at batch 256 63.4 us, now 53; 16->32 1x1 stride 2 20.9 -> 16.5).
+template <int OUT>
+__global__ void __launch_bounds__(FIN_THREADS) adder_gw_finish_kernel(const GwFinishArgs a, int npart, unsigned int* ticket) {
+    constexpr int ROWS = FIN_THREADS / OUT, WARPS = FIN_THREADS / 32;
+    __shared__ double s_sum[WARPS][OUT], s_gs[WARPS][OUT], s_sq[WARPS];
     __shared__ bool s_last;
-    const int o = threadIdx.x & (FIN_OUT - 1);
-    const int lane = threadIdx.x / FIN_OUT;
-    const int i = blockIdx.x * FIN_OUT + o;
-    double s = 0.0, gs = 0.0;
+    const int o = threadIdx.x % OUT, row = threadIdx.x / OUT, warp = threadIdx.x / 32;
+    const int i = blockIdx.x * OUT + o;
+    double t = 0.0, g = 0.0;
+    float wv = 0.f;
     if (i < a.CoK) {
-        const int co = i / a.K;
         const float* p = a.part + i;
-        const float* q = a.gsum_part + co;
-        int sp = lane;
+        const float* q = a.gsum_part + i / a.K;
+        wv = a.w[i];
 #pragma unroll 4
-        for (; sp < a.splits; sp += FIN_LANES) {
-            s += (double)p[(size_t)sp * a.CoK];
-            gs += (double)q[(size_t)sp * a.Co];
+        for (int sp = row; sp < a.gsum_splits; sp += ROWS) {                 // gsum_splits >= splits
+            t += (double)(sp < a.splits ? __ldcg(p + (size_t)sp * a.CoK) : 0.f);
+            g += (double)__ldg(q + (size_t)sp * a.Co);
         }
-#pragma unroll 4
-        for (; sp < a.gsum_splits; sp += FIN_LANES) gs += (double)q[(size_t)sp * a.Co];
     }
-    s_sum[lane][o] = s;
-    s_gs[lane][o] = gs;
-    __syncthreads();
-    double v2 = 0.0;
-    if (lane == 0 && i < a.CoK) {
-        double t = 0.0, g = 0.0;
 #pragma unroll
-        for (int l = 0; l < FIN_LANES; ++l) { t += s_sum[l][o]; g += s_gs[l][o]; }
-        const float vf = (float)(t - (double)a.w[i] * g);
-        if (a.accumulate) a.gw[i] += vf; else a.gw[i] = vf;
-        v2 = (double)vf * (double)vf;
+    for (int off = 16; off >= OUT; off >>= 1) {
+        t += __shfl_xor_sync(0xffffffffu, t, off);
+        g += __shfl_xor_sync(0xffffffffu, g, off);
     }
-    s_sq[threadIdx.x] = (lane == 0) ? v2 : 0.0;
+    if (threadIdx.x % 32 < OUT) { s_sum[warp][o] = t; s_gs[warp][o] = g; }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int k = 0; k < FIN_OUT; ++k) t += s_sq[k];
-        a.norm_part[blockIdx.x] = (float)t;
+    if (warp == 0) {
+        double v2 = 0.0;
+        if (threadIdx.x < OUT && i < a.CoK) {
+            t = g = 0.0;
+#pragma unroll
+            for (int l = 0; l < WARPS; ++l) { t += s_sum[l][o]; g += s_gs[l][o]; }
+            const float vf = (float)(t - (double)wv * g);
+            if (a.accumulate) a.gw[i] += vf; else a.gw[i] = vf;
+            v2 = (double)vf * (double)vf;
+        }
+#pragma unroll
+        for (int off = 1; off < FIN_NORM; off <<= 1) v2 += __shfl_xor_sync(0xffffffffu, v2, off);
+        if (threadIdx.x < OUT && o % FIN_NORM == 0 && i < a.CoK) a.norm_part[i / FIN_NORM] = (float)v2;
         __threadfence();
-        s_last = (atomicAdd(ticket, 1u) == (unsigned)(nblocks - 1));
+        __syncwarp();
+        if (threadIdx.x == 0) s_last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
     }
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    double t = 0.0;
-    for (int k = threadIdx.x; k < nblocks; k += FIN_THREADS) t += (double)__ldcg(a.norm_part + k);
-    s_sq[threadIdx.x] = t;
+    t = 0.0;
+#pragma unroll 8
+    for (int k = threadIdx.x; k < npart; k += FIN_THREADS) t += (double)__ldcg(a.norm_part + k);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+    if (threadIdx.x % 32 == 0) s_sq[warp] = t;
     __syncthreads();
-    for (int off = FIN_THREADS / 2; off > 0; off >>= 1) {
-        if ((int)threadIdx.x < off) s_sq[threadIdx.x] += s_sq[threadIdx.x + off];
-        __syncthreads();
-    }
-    const float nrm = (float)sqrt(s_sq[0]);
+    t = s_sq[0];
+#pragma unroll
+    for (int l = 1; l < WARPS; ++l) t += s_sq[l];
+    const float nrm = (float)sqrt(t);
     if (threadIdx.x == 0 && a.out_norm != nullptr) *a.out_norm = nrm;
     if (a.eta > 0.f) {
+        constexpr int DEEP = 8;
         const float sc = a.eta * sqrtf((float)a.CoK) / fmaxf(nrm, 1e-12f);
-        for (int k = threadIdx.x; k < a.CoK; k += FIN_THREADS) a.gw[k] = __ldcg(a.gw + k) * sc;
+        const int quads = (reinterpret_cast<uintptr_t>(a.gw) & 15) == 0 ? a.CoK / 4 : 0;
+        float4* g4 = reinterpret_cast<float4*>(a.gw);
+        for (int k0 = threadIdx.x; k0 < quads; k0 += DEEP * FIN_THREADS) {
+            float4 v[DEEP];
+#pragma unroll
+            for (int d = 0; d < DEEP; ++d)
+                if (k0 + d * FIN_THREADS < quads) v[d] = __ldcg(g4 + k0 + d * FIN_THREADS);
+#pragma unroll
+            for (int d = 0; d < DEEP; ++d)
+                if (k0 + d * FIN_THREADS < quads) g4[k0 + d * FIN_THREADS] = make_float4(v[d].x * sc, v[d].y * sc, v[d].z * sc, v[d].w * sc);
+        }
+        for (int k0 = 4 * quads + threadIdx.x; k0 < a.CoK; k0 += DEEP * FIN_THREADS) {
+            float v[DEEP];
+#pragma unroll
+            for (int d = 0; d < DEEP; ++d)
+                if (k0 + d * FIN_THREADS < a.CoK) v[d] = __ldcg(a.gw + k0 + d * FIN_THREADS);
+#pragma unroll
+            for (int d = 0; d < DEEP; ++d)
+                if (k0 + d * FIN_THREADS < a.CoK) a.gw[k0 + d * FIN_THREADS] = v[d] * sc;
+        }
     }
 }
 
@@ -319,7 +343,7 @@ struct GwPlan {
     GwArgs a;
     int threads;
     size_t smem;
-    int fin_blocks;
+    int norm_parts;                // partial sums of squares
     int status;
     bool use_1x1 = false;   // 1x1 stride-1 layers with enough channels take the GEMM-style kernel
     bool use_pointwise = false;   // 1x1 stride-2 layers with few channels: adder_pointwise.cu
@@ -439,7 +463,7 @@ static GwPlan plan_gw_t(const Geom& g, const TileHint& hint) {
     a.d_pl = FastDiv(a.PL);
     a.d_cgo = FastDiv(a.CGO);
     a.d_ci_tiles = FastDiv(a.n_ci_tiles);
-    p.fin_blocks = ceil_div(g.Co * g.Ci * KS * KS, FIN_OUT);
+    p.norm_parts = ceil_div(g.Co * g.Ci * KS * KS, FIN_NORM);
     return p;
 }
 
@@ -539,10 +563,10 @@ int describe_gw(const Geom& g, const TileHint& hint, char* buf, size_t n) {
     const GwArgs& a = p.a;
     snprintf(buf, n,
              "gw k=%d s=%d CGO=%d CGC=%d TM=%d TCI=%d PL=%d TI=%d TH=%d SPR=%d SEGS=%d xrows=%d xcols=%d xpitch=%d gpitch=%d "
-             "threads=%d smem=%zu tiles=%d splits=%d tiles_per_split=%d+%d/%d out_tiles=%d fin_blocks=%d gemm1x1=%d pointwise=%d status=%d",
+             "threads=%d smem=%zu tiles=%d splits=%d tiles_per_split=%d+%d/%d out_tiles=%d gemm1x1=%d pointwise=%d status=%d",
              g.k, g.stride, a.CGO, a.CGC, a.TM, a.TCI, a.PL, a.TI, a.TH, a.SPR, a.SEGS, a.pdx.ROWS, a.pdx.COLS, a.pdx.PITCH,
              a.pdg.PITCH, p.threads, p.smem, a.tiles_total, a.splits, a.tiles_per_split, a.tiles_rem, a.splits,
-             ceil_div(g.Co, a.TM) * a.n_ci_tiles, p.fin_blocks, (int)p.use_1x1, (int)p.use_pointwise, p.status);
+             ceil_div(g.Co, a.TM) * a.n_ci_tiles, (int)p.use_1x1, (int)p.use_pointwise, p.status);
     return ADDER_OK;
 }
 
@@ -551,7 +575,7 @@ size_t gw_workspace_bytes(const Geom& g, const TileHint& hint) {
     if (p.status != ADDER_OK) return 0;
     const size_t CoK = (size_t)g.Co * g.Ci * g.k * g.k;
     size_t floats = align_up((size_t)p.a.splits * CoK, 64) + align_up((size_t)p.gsum_splits() * g.Co, 64) +
-                    align_up((size_t)p.fin_blocks + 2, 64);
+                    align_up((size_t)p.norm_parts + 2, 64);
     return floats * sizeof(float);
 }
 
@@ -565,17 +589,19 @@ static int launch_main_t(const GwPlan& p, cudaStream_t stream) {
 }
 
 // Slices -> gradient, its norm and the rescale.
-static int launch_finish(const GwFinishArgs& f, int fin_blocks, unsigned int* ticket, cudaStream_t stream) {
+static int launch_finish(const GwFinishArgs& f, int norm_parts, unsigned int* ticket, cudaStream_t stream) {
     const bool need_norm = f.eta > 0.f || f.out_norm != nullptr;
     if (need_norm && f.CoK <= FUSED_FINISH_MAX) {
-        adder_gw_finish_kernel<<<fin_blocks, FIN_THREADS, 0, stream>>>(f, fin_blocks, ticket);
+        // 32 elements a block read whole 128-byte lines, where that still makes a block an SM; else 8
+        if (ceil_div(f.CoK, 32) >= sm_count()) adder_gw_finish_kernel<32><<<ceil_div(f.CoK, 32), FIN_THREADS, 0, stream>>>(f, norm_parts, ticket);
+        else adder_gw_finish_kernel<8><<<ceil_div(f.CoK, 8), FIN_THREADS, 0, stream>>>(f, norm_parts, ticket);
         return launched();
     }
-    const int flat_blocks = ceil_div(f.CoK, FIN_THREADS);      // <= fin_blocks: the norm partials fit their array
+    const int flat_blocks = ceil_div(f.CoK, FIN_THREADS);      // <= norm_parts: the norm partials fit their array
     adder_gw_reduce_flat_kernel<<<flat_blocks, FIN_THREADS, 0, stream>>>(f);
     if (launched() != ADDER_OK) return ADDER_ERR_CUDA;
     if (need_norm) {
-        float* scale = f.norm_part + fin_blocks;
+        float* scale = f.norm_part + norm_parts;
         adder_gw_norm_kernel<<<1, 1024, 0, stream>>>(f, flat_blocks, scale);
         if (launched() != ADDER_OK) return ADDER_ERR_CUDA;
         if (f.eta > 0.f) {
@@ -603,7 +629,7 @@ int launch_gw(const Geom& g, const float* gout, const float* x, const float* w, 
     p.a.part = ws;
     p.a.gsum_part = ws + align_up((size_t)p.a.splits * CoK, 64);
     float* norm_part = p.a.gsum_part + align_up((size_t)p.gsum_splits() * g.Co, 64);
-    unsigned int* ticket = reinterpret_cast<unsigned int*>(norm_part + p.fin_blocks + 1);
+    unsigned int* ticket = reinterpret_cast<unsigned int*>(norm_part + p.norm_parts + 1);
     p.a.ticket = ticket;
 
     const bool rw7 = (g.Wo % 8 != 0) && (g.Wo % 7 == 0);
@@ -631,22 +657,22 @@ int launch_gw(const Geom& g, const float* gout, const float* x, const float* w, 
     f.part = p.a.part; f.gsum_part = p.a.gsum_part; f.w = w; f.gw = gw; f.norm_part = norm_part;
     f.out_norm = out_norm; f.CoK = (int)CoK; f.K = g.Ci * g.k * g.k; f.Co = g.Co; f.splits = p.a.splits; f.gsum_splits = p.gsum_splits();
     f.accumulate = accumulate; f.eta = eta;
-    return launch_finish(f, p.fin_blocks, ticket, stream);
+    return launch_finish(f, p.norm_parts, ticket, stream);
 }
 
 // A layer with any kernel extent, stride, padding and dilation: the tensor-core kernel alone, which takes all but very wide
 // rows and windows.
-struct ConvGwLayout { size_t gsum, norm, total; int splits, gsum_splits, fin_blocks; };
+struct ConvGwLayout { size_t gsum, norm, total; int splits, gsum_splits, norm_parts; };
 
 static bool conv_gw_layout(const ConvGeom& g, ConvGwLayout* l) {
     l->splits = gw_mma_splits(g);
     if (l->splits <= 0) return false;
     l->gsum_splits = gw_mma_gsum_splits(g);
     const size_t CoK = (size_t)g.Co * g.Ci * g.kh * g.kw;
-    l->fin_blocks = ceil_div((int)CoK, FIN_OUT);
+    l->norm_parts = ceil_div((int)CoK, FIN_NORM);
     l->gsum = align_up((size_t)l->splits * CoK, 64);
     l->norm = l->gsum + align_up((size_t)l->gsum_splits * g.Co, 64);
-    l->total = l->norm + align_up((size_t)l->fin_blocks + 2, 64);
+    l->total = l->norm + align_up((size_t)l->norm_parts + 2, 64);
     return true;
 }
 
@@ -662,14 +688,14 @@ int launch_conv_gw(const ConvGeom& g, const float* gout, const float* x, const f
     if (workspace == nullptr || workspace_bytes < l.total * sizeof(float)) return ADDER_ERR_WORKSPACE;
     if ((reinterpret_cast<uintptr_t>(workspace) & 255) != 0) return ADDER_ERR_ALIGNMENT;
     float* ws = static_cast<float*>(workspace);
-    unsigned int* ticket = reinterpret_cast<unsigned int*>(ws + l.norm + l.fin_blocks + 1);
+    unsigned int* ticket = reinterpret_cast<unsigned int*>(ws + l.norm + l.norm_parts + 1);
     const int st = launch_gw_mma(g, gout, x, ws, ws + l.gsum, ticket, l.splits, stream);
     if (st != ADDER_OK) return st;
     GwFinishArgs f;
     f.part = ws; f.gsum_part = ws + l.gsum; f.w = w; f.gw = gw; f.norm_part = ws + l.norm; f.out_norm = nullptr;
     f.K = g.Ci * g.kh * g.kw; f.CoK = g.Co * f.K; f.Co = g.Co; f.splits = l.splits; f.gsum_splits = l.gsum_splits;
     f.accumulate = 0; f.eta = eta;
-    return launch_finish(f, l.fin_blocks, ticket, stream);
+    return launch_finish(f, l.norm_parts, ticket, stream);
 }
 
 }  // namespace adder

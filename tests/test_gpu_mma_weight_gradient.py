@@ -41,3 +41,24 @@ def test_tensor_core_weight_gradient(case, one_sign):
     print("    rel", rel)
     assert rel <= (2e-6 if one_sign else 5e-7), rel
     assert torch.equal(ac.backward_weight(g, x, wt, s, p, eta=0.0), got)     # same bits twice
+
+
+# gradients of 9 to 65,790 elements: both block widths of the one-launch finish, its largest size and the first beyond it, with remainders
+@pytest.mark.parametrize("ci,co", [(1, 1), (16, 29), (17, 31), (85, 85), (85, 86)])
+def test_finish_of_the_weight_gradient(ci, co):
+    """Norm and rescale.  The slices are added in double, so what the sums of 192 products lose before that (192 u of their
+    size, u = 2^-24) and the roundings of scale and product bound the norm of the error."""
+    from addernetcuda_b200 import adder_cuda as ac
+    gen = torch.Generator(device=DEV).manual_seed(ci + co)
+    x = torch.randn(3, ci, 8, 8, device=DEV, generator=gen)
+    w = torch.randn(co, ci, 3, 3, device=DEV, generator=gen)
+    g = torch.randn(3, co, 8, 8, device=DEV, generator=gen)
+    got, norm = ac.backward_weight(g, x, w, 1, 1, eta=0.2, return_norm=True)
+    cols = F.unfold(x.double(), 3, padding=1)
+    g64 = g.double().reshape(3, co, -1)
+    want = torch.einsum("ncp,nkp->ck", g64, cols) - w.double().reshape(co, -1) * g64.sum((0, 2))[:, None]
+    size = torch.einsum("ncp,nkp->ck", g64.abs(), cols.abs()) + w.double().reshape(co, -1).abs() * g64.abs().sum((0, 2))[:, None]
+    bound = float((192 + 8) * 2.0 ** -24 * size.norm() / want.norm())
+    assert abs(float(norm) - float(want.norm())) <= bound * float(want.norm())
+    want *= 0.2 * want.numel() ** 0.5 / want.norm()
+    assert float((got.double().reshape(co, -1) - want).norm()) <= 2 * bound * float(want.norm())
