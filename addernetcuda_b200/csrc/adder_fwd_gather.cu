@@ -20,6 +20,7 @@ struct FwdGatherArgs {
     float* out;
     Epilogue ep;
     int Ci, H, W, Co, KK, CK, nchunks;
+    int vec_w;               // rows of w are whole, aligned quads in the order of the reduction
     int vec_store;           // planes are whole quads, `out` and the residual 16-byte aligned
 };
 
@@ -29,13 +30,14 @@ struct FwdTile {
     static constexpr int RM = RM_, RP = RP_, CG = CG_, ST = ST_, MB = MB_;
     static constexpr int PG = GATHER_THREADS / CG, TC = CG * RM, TP = PG * RP, WP = TC + 4;
     static constexpr int PQ = RP == 8 ? 4 : RP;                 // consecutive pixels of a thread
+    static constexpr bool THIN = RM <= 2 && RP <= 2;
 };
 
 template <class T, int MODE>
 __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel(const __grid_constant__ FwdGatherArgs a) {
     constexpr int RM = T::RM, RP = T::RP, CG = T::CG, TC = T::TC, TP = T::TP, WP = T::WP, PQ = T::PQ, ST = T::ST;
     constexpr int COLS = TP > GATHER_THREADS ? TP / GATHER_THREADS : 1;
-    constexpr int CK = gather_rows(MODE, ST, TC, TP, 0, T::MB);      // rows of a stage
+    constexpr int CK = gather_rows(MODE, ST, TC, TP, 0, T::MB, T::THIN);      // rows of a stage
     constexpr int XS = CK * TP, WS = CK * WP;
     extern __shared__ __align__(16) float smem[];
     float* const Xs = smem;
@@ -47,7 +49,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
     const size_t image = (size_t)a.Ci * a.H * a.W;
 
     GatherPixel px[COLS];
-    constexpr int CH = nine_channels(TC, TP);
+    constexpr int CH = nine_channels(T::THIN);
     GatherNine<TP, CH> nine;
     if (MODE == GATHER_QUADS) {
         px[0].decode(a.m, a.x, p0 + 4 * (tid % (TP / 4)), image);
@@ -68,24 +70,46 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
         } else {
             nk = min(a.CK, a.Ci - fc.c0); rows = ck4;
             if (MODE == GATHER_QUADS) gather_quads<TP, CK>(Xs + stage * XS, px[0].base, px[0].ok, a.x, fc.c0, nk, ck4, a.H * a.W, tid);
-            else gather_pixels<TP>(Xs + stage * XS, px, a.x, a.m, fc, nk, ck4, a.H, a.W, tid);
+            else gather_pixels<TP, CK>(Xs + stage * XS, px, a.x, a.m, fc, nk, ck4, a.H, a.W, tid);
             wk = fc.c0 * a.KK + a.m.wt0 + fc.i * a.m.dwi + fc.j * a.m.dwj;
         }
-        // weights [reduction step][output channel of the tile]: a warp copies 8 steps of 4 outputs
-        const int kstep = MODE == GATHER_NINE ? 1 : a.KK;
-        const int k8 = tid & 7, c4 = tid >> 3;
-        float* ws = Ws + stage * WS + k8 * WP + c4;
-        const int row = a.Ci * a.KK, ncol = a.Co - co0 - c4;
-        const float* wsrc = a.w + ((co0 + c4) * row + k8 * kstep + wk);
+        const int kstep = MODE == GATHER_NINE ? 1 : a.KK, row = a.Ci * a.KK;
+        if constexpr (T::THIN) {
+            // weights [output channel of the tile][reduction step]: a thread copies 4 steps
 #pragma unroll
-        for (int kb = 0; kb < CK; kb += 8) {
-            if (kb + k8 >= rows) break;
-            const bool okk = kb + k8 < nk;
+            for (int i0 = 0; i0 < TC * CK / 4; i0 += GATHER_THREADS) {
+                const int c = (i0 + tid) / (CK / 4), k = (i0 + tid) % (CK / 4) * 4;
+                if ((TC * CK / 4) % GATHER_THREADS != 0 && c >= TC) break;
+                float* ws = Ws + stage * WS + c * (CK + 4) + k;
+                const bool okc = co0 + c < a.Co;
+                const float* wsrc = a.w + (okc ? (co0 + c) * row + wk : 0);
+                if (a.vec_w) {
+                    const bool ok = okc & (k < nk);
+                    cp_async16(ws, ok ? wsrc + k : a.w, ok);
+                } else {
 #pragma unroll
-            for (int c = 0; c < TC; c += GATHER_THREADS / 8) {
-                if (TC % (GATHER_THREADS / 8) != 0 && c + c4 >= TC) break;
-                const bool ok = okk & (c < ncol);
-                cp_async4(ws + kb * WP + c, ok ? wsrc + (c * row + kb * kstep) : a.w, ok);
+                    for (int i = 0; i < 4; ++i) {
+                        const bool ok = okc & (k + i < nk);
+                        cp_async4(ws + i, ok ? wsrc + (k + i) * kstep : a.w, ok);
+                    }
+                }
+            }
+        } else {
+            // weights [reduction step][output channel of the tile]: a warp copies 8 steps of 4 outputs
+            const int k8 = tid & 7, c4 = tid >> 3;
+            float* ws = Ws + stage * WS + k8 * WP + c4;
+            const int ncol = a.Co - co0 - c4;
+            const float* wsrc = a.w + ((co0 + c4) * row + k8 * kstep + wk);
+#pragma unroll
+            for (int kb = 0; kb < CK; kb += 8) {
+                if (kb + k8 >= rows) break;
+                const bool okk = kb + k8 < nk;
+#pragma unroll
+                for (int c = 0; c < TC; c += GATHER_THREADS / 8) {
+                    if (TC % (GATHER_THREADS / 8) != 0 && c + c4 >= TC) break;
+                    const bool ok = okk & (c < ncol);
+                    cp_async4(ws + kb * WP + c, ok ? wsrc + (c * row + kb * kstep) : a.w, ok);
+                }
             }
         }
         if (MODE == GATHER_NINE) fc.c0 += CH;
@@ -112,36 +136,54 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
         if (c + ST - 1 < a.nchunks) fill(fstage);
         cp_async_commit();
         const float* xs = Xs + stage * XS + pg * PQ;
-        const float* ws = Ws + stage * WS + cg * RM;
         const int nk = MODE == GATHER_NINE ? CK : min(ck4, round_up(a.Ci - cc.c0, 4));
-#pragma unroll (RM * RP >= 64 ? 1 : RM * RP >= 32 ? 2 : RM * RP > 1 ? 4 : CK / 2)
-        for (int k = 0; k < nk; ++k) {
-            float xv[RP], wv[RM];
+        if constexpr (T::THIN) {
+            const float* ws = Ws + stage * WS + cg * RM * (CK + 4);
+#pragma unroll (RM == 1 ? CK / 4 : 2)
+            for (int k = 0; k < CK; k += 4) {
+                if (MODE != GATHER_NINE && k >= nk) break;
+                float4 wq[RM];
+                float xv[4][RP];
 #pragma unroll
-            for (int h = 0; h < RP / PQ; ++h) {
-                if constexpr (PQ == 4) {
+                for (int m = 0; m < RM; ++m) wq[m] = *reinterpret_cast<const float4*>(ws + m * (CK + 4) + k);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if constexpr (RP == 2) {
+                        const float2 q = *reinterpret_cast<const float2*>(xs + (k + i) * TP);
+                        xv[i][0] = q.x; xv[i][1] = q.y;
+                    } else {
+                        xv[i][0] = xs[(k + i) * TP];
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int m = 0; m < RM; ++m) {
+                        const float wv = i == 0 ? wq[m].x : i == 1 ? wq[m].y : i == 2 ? wq[m].z : wq[m].w;
+#pragma unroll
+                        for (int j = 0; j < RP; ++j) acc[m][j] += fabsf(wv - xv[i][j]);
+                    }
+            }
+        } else {
+            const float* ws = Ws + stage * WS + cg * RM;
+#pragma unroll (RM * RP >= 64 ? 1 : RM * RP >= 32 ? 2 : 4)
+            for (int k = 0; k < nk; ++k) {
+                float xv[RP], wv[RM];
+#pragma unroll
+                for (int h = 0; h < RP / PQ; ++h) {
                     const float4 q = *reinterpret_cast<const float4*>(xs + k * TP + h * (TP / 2));
                     xv[4 * h] = q.x; xv[4 * h + 1] = q.y; xv[4 * h + 2] = q.z; xv[4 * h + 3] = q.w;
-                } else if constexpr (PQ == 2) {
-                    const float2 q = *reinterpret_cast<const float2*>(xs + k * TP);
-                    xv[0] = q.x; xv[1] = q.y;
-                } else {
-                    xv[0] = xs[k * TP];
                 }
-            }
-            if constexpr (RM >= 4) {
+                if constexpr (RM >= 4) {
 #pragma unroll
-                for (int m = 0; m < RM; m += 4) {
-                    const float4 q = *reinterpret_cast<const float4*>(ws + k * WP + m);
-                    wv[m] = q.x; wv[m + 1] = q.y; wv[m + 2] = q.z; wv[m + 3] = q.w;
+                    for (int m = 0; m < RM; m += 4) {
+                        const float4 q = *reinterpret_cast<const float4*>(ws + k * WP + m);
+                        wv[m] = q.x; wv[m + 1] = q.y; wv[m + 2] = q.z; wv[m + 3] = q.w;
+                    }
+                } else {
+                    const float2 q = *reinterpret_cast<const float2*>(ws + k * WP);
+                    wv[0] = q.x; wv[1] = q.y;
                 }
-            } else if constexpr (RM == 2) {
-                const float2 q = *reinterpret_cast<const float2*>(ws + k * WP);
-                wv[0] = q.x; wv[1] = q.y;
-            }
-            if constexpr (RM == 1) {
-                acc[0][0] += fabsf(ws[k * WP] - xv[0]);
-            } else {
                 uint64_t nx2[RP];
 #pragma unroll
                 for (int j = 0; j < RP; ++j) nx2[j] = pack2(-xv[j], -xv[j]);
@@ -205,15 +247,17 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
 
 namespace {
 
-// The tiles: large ones have the fewest loads per term, small ones give a small layer more threads.  The smallest, an output a
-// thread with 4 channels of a 3x3 window a stage, is for layers of fewer outputs than the chip has threads, whose time is the chain
-// of stages of one CTA (before it: 64->64 8x8 at batch 1 14.1 -> 9.7 us, 32->32 16x16 8.0 -> 5.7, 512->512 7x7 102 -> 79).
+// The tiles: large ones have the fewest loads per term, small ones give a small layer more threads.  The last three (THIN) are
+// bound by the instructions around a term in a CTA's chain of stages, few CTAs being resident: they keep their weights as
+// [channel][step], which takes 16-byte copies and gives four steps a load, and have stages twice as long.  At batch 1, with the
+// 2x2 tiles built like the large ones -> now: 64->64 8x8 14.1 -> 7.5 us, 256->256 14x14 52 -> 43.5, 512->512 7x7 102 -> 63,
+// 1024->256 14x14 33 -> 22, 2048->512 7x7 69 -> 41.
 // X(RM, RP, CG, ST, MB, clocks per step: alone, each further CTA, throughput)
 #define ADDER_FWD_GATHER_TILES(X)                                                                                   \
     X(8, 8, 8, 2, 4, 242, 147, 173) X(8, 8, 16, 2, 4, 241, 74, 186) X(8, 8, 4, 2, 4, 278, 130, 186)                 \
     X(4, 8, 16, 3, 4, 139, 65, 93) X(4, 8, 8, 3, 4, 139, 65, 93) X(4, 8, 4, 2, 4, 174, 76, 109)                     \
     X(4, 4, 16, 4, 6, 92, 30, 54) X(4, 4, 8, 4, 6, 92, 30, 54) X(4, 4, 4, 4, 6, 101, 22, 56)                        \
-    X(2, 2, 8, 8, 8, 43, 9, 23) X(2, 2, 4, 8, 8, 49, 10, 26) X(2, 8, 4, 3, 6, 110, 40, 60) X(1, 1, 4, 6, 8, 20, 6, 20)
+    X(2, 8, 4, 3, 6, 110, 40, 60) X(2, 2, 8, 4, 8, 35, 10, 20) X(2, 2, 4, 4, 6, 38, 12, 23) X(1, 1, 4, 6, 8, 16, 9, 11)
 
 struct Tile { int rm, rp, cg, st, mb, tc, tp; TileCost cost; };
 constexpr Tile kTiles[] = {
@@ -233,7 +277,7 @@ int choose_tile(int P, int Co) {
     return best;
 }
 
-int stage_rows(const Tile& t, int mode) { return gather_rows(mode, t.st, t.tc, t.tp, 0, t.mb); }
+int stage_rows(const Tile& t, int mode) { return gather_rows(mode, t.st, t.tc, t.tp, 0, t.mb, t.rm <= 2 && t.rp <= 2); }
 
 size_t smem_bytes(const Tile& t, int rows) {
     return (size_t)t.st * rows * (t.tp + t.tc + 4) * sizeof(float);
@@ -284,6 +328,7 @@ int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* 
     a.x = x; a.w = w; a.out = out; a.ep = ep;
     a.Ci = g.Ci; a.H = g.H; a.W = g.W; a.Co = g.Co; a.KK = g.kh * g.kw;
     const bool whole_quads = (g.Ho * g.Wo) % 4 == 0;
+    a.vec_w = (a.KK == 1 || (g.kh == 3 && g.kw == 3)) && (g.Ci * a.KK) % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
     a.vec_store = whole_quads && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(ep.residual)) & 15) == 0;
     const bool quads = whole_quads && a.KK == 1 && g.sh == 1 && g.sw == 1 && g.ph == 0 && g.pw == 0 &&
                        (reinterpret_cast<uintptr_t>(x) & 15) == 0;

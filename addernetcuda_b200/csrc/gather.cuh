@@ -19,14 +19,16 @@ constexpr int GATHER_CK = 16;
 constexpr int GATHER_THREADS = 128;
 enum GatherMode { GATHER_TAP, GATHER_QUADS, GATHER_NINE };
 
-// Channels of a chunk of GATHER_NINE.
-__host__ __device__ constexpr int nine_channels(int tc, int tp) { return tc * tp <= GATHER_THREADS ? 4 : 2; }
+// Channels of a chunk of GATHER_NINE; thin tiles (a few outputs a thread) spend their time on the instructions around a stage
+// rather than on its terms, so their stages are twice as long.
+__host__ __device__ constexpr int nine_channels(bool thin) { return thin ? 4 : 2; }
 
 // Rows of a stage.  1x1 layers take 32 channels at a time where four CTAs still fit an SM: half the barriers (1024->256 on 75,776
 // pixels: input gradient 1687 -> 1549 us saturating, 2013 -> 1937 exact, forward 1344 -> 1326; 3x3 layers lose 1-6 %, the weights of
 // a chunk being strided).
-__host__ __device__ constexpr int gather_rows(int mode, int stages, int tc, int tp, int more_bytes, int ctas) {
-    if (mode == GATHER_NINE) return 9 * nine_channels(tc, tp);
+__host__ __device__ constexpr int gather_rows(int mode, int stages, int tc, int tp, int more_bytes, int ctas, bool thin = false) {
+    if (mode == GATHER_NINE) return 9 * nine_channels(thin);
+    if (thin) return 2 * GATHER_CK;
     return mode == GATHER_QUADS && ctas <= 4 && stages * 32 * (tp + tc + 4) * 4 + more_bytes <= 56 * 1024 ? 2 * GATHER_CK : GATHER_CK;
 }
 
@@ -98,7 +100,7 @@ __device__ __forceinline__ void copy_rows(float* d, const float* s, int stride, 
 }
 
 // Stages one chunk of the pixel-side operand as [channel][TP pixels].
-template <int TP>
+template <int TP, int CK = GATHER_CK>
 __device__ __forceinline__ void gather_pixels(float* dst, const GatherPixel* px, const float* src, const GatherMap& m,
                                               const GatherChunk& c, int nch, int ck, int Hs, int Ws, int tid) {
     constexpr int COLS = TP > GATHER_THREADS ? TP / GATHER_THREADS : 1;      // pixels per thread
@@ -108,7 +110,7 @@ __device__ __forceinline__ void gather_pixels(float* dst, const GatherPixel* px,
     for (int q = 0; q < COLS; ++q) {
         const int row = px[q].row + m.oy0 + c.i * m.doy, col = px[q].col + m.ox0 + c.j * m.dox;
         const bool ok = px[q].ok & ((unsigned)row < (unsigned)Hs) & ((unsigned)col < (unsigned)Ws);
-        copy_rows<ROWS, TP>(dst + (COLS > 1 ? tid + q * GATHER_THREADS : tid % TP), ok ? px[q].base + (c.c0 * plane + row * Ws + col) : src,
+        copy_rows<ROWS, TP, CK>(dst + (COLS > 1 ? tid + q * GATHER_THREADS : tid % TP), ok ? px[q].base + (c.c0 * plane + row * Ws + col) : src,
                             ok ? plane : 0, ok, tid / TP, nch, ck);
     }
 }
