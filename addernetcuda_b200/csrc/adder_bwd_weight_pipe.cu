@@ -90,11 +90,11 @@ __global__ void __launch_bounds__(GWP_WARPS * 32, 2) adder_gw_pipe_kernel(const 
         (void)item_rows(cur, n, r0);
         float* xs = smem + stage * a.stage_floats;
         float* gs = xs + a.xs_stage;
-        fill_patch<false>(xs, a.x, a.pdx, n, ci0, r0 * S - a.g.pad, -a.g.pad, a.g.N, a.g.Ci, a.g.H, a.g.W, tid, nthreads);
+        fill_patch(xs, a.x, a.pdx, n, ci0, r0 * S - a.g.pad, -a.g.pad, a.g.N, a.g.Ci, a.g.H, a.g.W, tid, nthreads);
         if (a.g_quads)
             fill_patch_quads(gs, a.gout, a.pdg, a.d_gquads, n, co0, r0, 0, a.g.N, a.g.Co, a.g.Ho, a.g.Wo, tid, nthreads);
         else
-            fill_patch<false>(gs, a.gout, a.pdg, n, co0, r0, 0, a.g.N, a.g.Co, a.g.Ho, a.g.Wo, tid, nthreads);
+            fill_patch(gs, a.gout, a.pdg, n, co0, r0, 0, a.g.N, a.g.Co, a.g.Ho, a.g.Wo, tid, nthreads);
     };
 
     float acc[RM][RC][KK];

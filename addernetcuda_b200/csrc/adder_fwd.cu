@@ -41,9 +41,9 @@ __global__ void __launch_bounds__(256, 2) adder_fwd_kernel(const FwdArgs a) {
     const int n0 = tn * a.TI;
     const int ho0 = th * a.TH;
     const int wo_t0 = tw * (a.SPR * RW);      // first output column of this tile
-    const int wi0 = wo_t0 * S * a.pd.GS - a.g.pad;      // input column of patch column 0
+    const int wi0 = wo_t0 * S - a.g.pad;      // input column of patch column 0
     const int co0 = blockIdx.y * (a.CG * RM);
-    const int hi0 = ho0 * S * a.pd.GS - a.g.pad;       // input row of patch row 0
+    const int hi0 = ho0 * S - a.g.pad;       // input row of patch row 0
 
     // thread role: (channel group, segment); segment -> (image, tile row, segment within row)
     uint32_t cg, seg, t2, ws, img, hr;
@@ -65,11 +65,7 @@ __global__ void __launch_bounds__(256, 2) adder_fwd_kernel(const FwdArgs a) {
 
     auto fill = [&](int chunk, int stage) {
         const int ci0 = chunk * a.CK;
-        if (KS == 1 && a.x_quads)
-            fill_patch_quads(Xs + stage * a.xs_stage, a.x, a.pd, a.d_xquads, n0, ci0, hi0, wi0, a.g.N, a.g.Ci, a.g.H, a.g.W,
-                             tid, nthreads);
-        else
-            fill_patch(Xs + stage * a.xs_stage, a.x, a.pd, n0, ci0, hi0, wi0, a.g.N, a.g.Ci, a.g.H, a.g.W, tid, nthreads);
+        fill_patch(Xs + stage * a.xs_stage, a.x, a.pd, n0, ci0, hi0, wi0, a.g.N, a.g.Ci, a.g.H, a.g.W, tid, nthreads);
         float* wsm = Ws + stage * a.ws_stage;
         const int kbase = ci0 * KK;
         const int kk_lim = a.CK * KK;
@@ -253,12 +249,6 @@ static int plan_fwd_t(const Geom& g, const float* out, const TileHint& hint, Fwd
         // CTA, so that every staged input patch is used twice as often (60 -> 56 us on that layer) - as long as
         // that still leaves about one CTA per SM.
         TileHint h2 = hint;
-        if (KS == 1 && g.Co >= 64) {
-            // 1x1 layers: one tap per staged input value, so twice the channels per CTA pays on every size
-            // (1024->256 14x14: 429 -> 380 us)
-            h2.threads = 256;
-            if (plan_fwd_t<KS, S, RW, RM>(g, out, h2, p) == ADDER_OK) return ADDER_OK;
-        }
         h2.threads = 128;
         const int st = plan_fwd_t<KS, S, RW, RM>(g, out, h2, p);
         if (st == ADDER_OK && p.gx * p.gy < 2LL * sm_count() && g.Co > p.a.TM) {
@@ -316,22 +306,15 @@ static int plan_fwd_t(const Geom& g, const float* out, const TileHint& hint, Fwd
     a.ROWS_PITCH = a.IN_ROWS * a.PITCH;
     a.pd.TI = a.TI; a.pd.ROWS = a.IN_ROWS; a.pd.COLS = a.IN_COLS; a.pd.PITCH = a.PITCH; a.pd.ROWS_PITCH = a.ROWS_PITCH;
     a.pd.d_cols = FastDiv(a.IN_COLS); a.pd.d_rows = FastDiv(a.IN_ROWS);
-    // A strided 1x1 layer is a stride-1 layer on the sampled pixels: the kernel runs its stride-1 form (S = 1)
-    // and the patch fill gathers every g.stride-th row and column, so nothing unsampled is staged.
-    a.pd.GS = (KS == 1 && S == 1) ? g.stride : 1;
-    // 1x1 stride-1 layers have no halo: where rows and tiles are whole quads the patch moves in 16-byte copies
-    a.x_quads = (KS == 1 && S == 1 && g.stride == 1 && g.pad == 0 && a.IN_COLS % 4 == 0 && a.PITCH % 4 == 0 && g.W % 4 == 0 &&
-                 (a.SPR * RW) % 4 == 0) ? 1 : 0;
-    a.d_xquads = FastDiv(a.IN_COLS >= 4 ? a.IN_COLS / 4 : 1);
     a.CH_STRIDE = a.TI * a.ROWS_PITCH;
     // channel chunk: fill the shared-memory budget (two CTAs per SM) without exceeding Ci
     // shared memory per CTA in proportion to its threads, so that about 16 warps stay resident per SM
     const int budget_floats = (hint.smem_kb > 0 ? hint.smem_kb : 100) * 1024 / 4;
-    int ck = hint.ck > 0 ? hint.ck : (KS == 1 ? 32 : 16);
+    int ck = hint.ck > 0 ? hint.ck : 16;
     if (ck > g.Ci) ck = g.Ci;
     // All input channels in ONE chunk need no second stage; where that fits the budget it is taken (no chunk barrier).
     bool whole = false;
-    if (hint.ck <= 0 && KS == 3 && g.Ci <= 64 &&
+    if (hint.ck <= 0 && g.Ci <= 64 &&
         round_up(g.Ci * ti_budget * a.ROWS_PITCH, 4) + g.Ci * KS * KS * a.TM <= budget_floats) {
         ck = g.Ci;
         whole = true;
@@ -384,7 +367,6 @@ static int launch_fwd_t(const Geom& g, const float* x, const float* w, float* ou
     if ((reinterpret_cast<uintptr_t>(out) & 15) != 0) p.a.vec_store = 0;
     p.a.x = x; p.a.w = w; p.a.out = out; p.a.ep = ep;
     if ((reinterpret_cast<uintptr_t>(ep.residual) & 15) != 0) p.a.vec_store = 0;
-    if ((reinterpret_cast<uintptr_t>(x) & 15) != 0) p.a.x_quads = 0;
     if (stats != nullptr) {
         if ((long long)stat_slices != p.gx || p.a.TM * p.a.stat_tpc > p.threads) return ADDER_ERR_WORKSPACE;
         p.a.stats = stats; p.a.stat_slices = stat_slices;

@@ -1,5 +1,5 @@
 // Cooperative asynchronous copy of a zero-filled rectangular patch of an NCHW tensor into shared
-// memory: dst[(c*TI + i)*ROWS_PITCH + r*PITCH + q] = src[n0+i, c0+c, row0+r*GS, col0+q*GS], or 0 where
+// memory: dst[(c*TI + i)*ROWS_PITCH + r*PITCH + q] = src[n0+i, c0+c, row0+r, col0+q], or 0 where
 // any index falls outside the tensor (that is how padding and ragged tile edges are produced).
 #pragma once
 #include "common.cuh"
@@ -9,14 +9,9 @@ namespace adder {
 struct PatchDims {
     int CH, TI, ROWS, COLS, PITCH, ROWS_PITCH;   // patch extents and shared-memory pitches
     int CHS = 0;                                 // channel stride if it is not TI*ROWS_PITCH (padded planes)
-    int GS = 1;                                  // gather stride: patch position (r, q) reads src[row0 + r*GS, col0 + q*GS]
     FastDiv d_cols, d_rows;
 };
 
-// With DUP every value is stored twice in a row (dst[... + r*PITCH + 2*q] and the word after it; PITCH then
-// counts the doubled row), so that a 64-bit shared-memory load yields the pair (v, v) a packed f32x2
-// instruction wants as its broadcast operand, without any register moves.
-template <bool DUP = false>
 __device__ __forceinline__ void fill_patch(float* dst, const float* __restrict__ src, const PatchDims& p,
                                            int n0, int c0, int row0, int col0, int N, int C, int Hs, int Ws,
                                            int tid, int nthreads) {
@@ -30,16 +25,14 @@ __device__ __forceinline__ void fill_patch(float* dst, const float* __restrict__
         uint32_t rho, q, i, r;
         p.d_cols.divmod(e, rho, q);
         p.d_rows.divmod(rho, i, r);
-        const int n = n0 + (int)i, row = row0 + (int)r * p.GS, col = col0 + (int)q * p.GS;
+        const int n = n0 + (int)i, row = row0 + (int)r, col = col0 + (int)q;
         const bool ok = (n < N) & (row >= 0) & (row < Hs) & (col >= 0) & (col < Ws);
         const float* s = ok ? src + ((size_t)(n * C + c0) * plane + row * Ws + col) : src;
-        float* d = dst + i * p.ROWS_PITCH + r * p.PITCH + (DUP ? 2 * q : q);
+        float* d = dst + i * p.ROWS_PITCH + r * p.PITCH + q;
 #pragma unroll 4
         for (int c = 0; c < p.CH; ++c) {
             const bool okc = ok & (c < nch);
-            const float* sc = okc ? s + (size_t)c * plane : src;
-            cp_async4(d + c * ch_stride, sc, okc);
-            if (DUP) cp_async4(d + c * ch_stride + 1, sc, okc);
+            cp_async4(d + c * ch_stride, okc ? s + (size_t)c * plane : src, okc);
         }
     }
 }
