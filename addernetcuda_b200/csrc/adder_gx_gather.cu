@@ -7,7 +7,8 @@
 // A thread keeps 4 input channels x 8 pixels of x and of the sums in registers; a k step is three 128-bit loads for
 // 32 terms.  Saturating form: one FFMA.SAT and one FFMA a term, with x' = 1/2 - x/2 in registers:
 // clamp(d,-1,1) = 2*sat(d/2 + 1/2) - 1, and the "-1" is the sum of g over the taps, added up once per pixel while the
-// stages pass by.  Exact form: min.xorsign.abs is the clamp in one instruction (magnitude min(|d|, 1), sign of d),
+// stages pass by: in four partial sums, of rows r, r + 4, r + 8 and r + 12 of every 16, whichever threads share the pixel, so that
+// the tile - which follows the size of the batch - does not show in the result.  Exact form: min.xorsign.abs is the clamp in one instruction (magnitude min(|d|, 1), sign of d),
 // where fminf(fmaxf(d, -1), 1) takes two; the sums are packed pairs of pixels.
 // Both are bound by the register operands they read (5 a term, 2 a cycle and scheduler): 2.6 and 3.4 lane cycles a term
 // with nothing around them.
@@ -50,6 +51,8 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
     constexpr int RC = T::RC, RP = T::RP, CG = T::CG, TC = T::TC, TP = T::TP, WP = T::WP, PQ = T::PQ, ST = T::ST;
     constexpr int COLS = TP > GATHER_THREADS ? TP / GATHER_THREADS : 1;
     constexpr int ROWS = TP < GATHER_THREADS ? GATHER_THREADS / TP : 1;
+    constexpr int PARTS = 4, MINE = PARTS / ROWS;      // partial sums of g per pixel, and those of one thread
+    static_assert(PARTS % ROWS == 0, "whole partial sums per thread");
     constexpr int CK = gather_rows(QUADS ? GATHER_QUADS : GATHER_TAP, ST, TC, TP, RC * RP * GATHER_THREADS * 4, T::MB);      // rows of a stage
     constexpr int FOLD = 64 / CK;                // chunks per partial sum: 64 terms before it is folded into the total
     constexpr int GS = CK * TP, WS = CK * WP;
@@ -151,9 +154,11 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
             xv[c][j] = FAST ? fmaf(xv[c][j], -0.5f, 0.5f) : -xv[c][j];
             acc[c][j] = 0.f;
         }
-    float box[COLS];
+    float box[COLS][MINE];
 #pragma unroll
-    for (int q = 0; q < COLS; ++q) box[q] = 0.f;
+    for (int q = 0; q < COLS; ++q)
+#pragma unroll
+        for (int i = 0; i < MINE; ++i) box[q][i] = 0.f;
 
     GatherChunk cc;
     int stage = 0, fstage = ST - 1;
@@ -202,18 +207,29 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
             }
         }
         if (FAST) {
-            const float* col = Gs + stage * GS + (COLS > 1 ? tid : tid % TP);
+            const float* col = Gs + stage * GS + (COLS > 1 ? tid : tid % TP) + (ROWS > 1 ? tid / TP : 0) * TP;
 #pragma unroll
             for (int q = 0; q < COLS; ++q) {
-                const float* cq = col + (tid / TP) * TP + q * GATHER_THREADS;
-                float s = 0.f;
+                const float* cq = col + q * GATHER_THREADS;
                 if (nk == CK) {
 #pragma unroll
-                    for (int k = 0; k < CK; k += ROWS) s += cq[k * TP];
+                    for (int kb = 0; kb < CK; kb += 16)
+#pragma unroll
+                        for (int i = 0; i < MINE; ++i) {
+                            float s = 0.f;
+#pragma unroll
+                            for (int k = kb + i * ROWS; k < kb + 16; k += PARTS) s += cq[k * TP];
+                            box[q][i] += s;
+                        }
                 } else {
-                    for (int k = 0; k < nk; k += ROWS) s += cq[k * TP];
+                    for (int kb = 0; kb < nk; kb += 16)
+#pragma unroll
+                        for (int i = 0; i < MINE; ++i) {
+                            float s = 0.f;
+                            for (int k = kb; k < kb + 16 && k < nk; k += PARTS) s += cq[(k + i * ROWS) * TP];      // nk is a multiple of 4
+                            box[q][i] += s;
+                        }
                 }
-                box[q] += s;
             }
         }
         // two-level summation: a long sum over output channels loses far less than one running fp32 accumulator would
@@ -242,16 +258,19 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
     }
     if (FAST) {
         __syncthreads();                         // the stages are free
-        float* bs = smem;                        // [ROWS][TP]
+        float* bs = smem;                        // [PARTS][TP]
 #pragma unroll
-        for (int q = 0; q < COLS; ++q) bs[tid + q * GATHER_THREADS] = box[q];
+        for (int q = 0; q < COLS; ++q)
+#pragma unroll
+            for (int i = 0; i < MINE; ++i)
+                bs[((ROWS > 1 ? tid / TP : 0) + i * ROWS) * TP + (COLS > 1 ? tid + q * GATHER_THREADS : tid % TP)] = box[q][i];
         __syncthreads();
 #pragma unroll
         for (int j = 0; j < RP; ++j) {
             const int col = (j / PQ) * (TP / 2) + pg * PQ + (j % PQ);
             float b = bs[col];
 #pragma unroll
-            for (int r = 1; r < ROWS; ++r) b += bs[r * TP + col];
+            for (int r = 1; r < PARTS; ++r) b += bs[r * TP + col];
 #pragma unroll
             for (int r = 0; r < RC; ++r) acc[r][j] = fmaf(2.f, acc[r][j], -b);
         }
