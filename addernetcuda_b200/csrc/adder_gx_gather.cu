@@ -51,9 +51,9 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
     constexpr int RC = T::RC, RP = T::RP, CG = T::CG, TC = T::TC, TP = T::TP, WP = T::WP, PQ = T::PQ, ST = T::ST;
     constexpr int COLS = TP > GATHER_THREADS ? TP / GATHER_THREADS : 1;
     constexpr int ROWS = TP < GATHER_THREADS ? GATHER_THREADS / TP : 1;
-    constexpr int PARTS = 4, MINE = PARTS / ROWS;      // partial sums of g per pixel, and those of one thread
-    static_assert(PARTS % ROWS == 0, "whole partial sums per thread");
     constexpr int CK = gather_rows(QUADS ? GATHER_QUADS : GATHER_TAP, ST, TC, TP, RC * RP * GATHER_THREADS * 4, T::MB);      // rows of a stage
+    constexpr int PARTS = 4, MINE = PARTS / ROWS;      // partial sums of g per pixel, and those of one thread
+    static_assert(PARTS % ROWS == 0 && (PARTS > ROWS || CK == 16), "whole partial sums per thread, a stage at a time");
     constexpr int FOLD = 64 / CK;                // chunks per partial sum: 64 terms before it is folded into the total
     constexpr int GS = CK * TP, WS = CK * WP;
     extern __shared__ __align__(16) float smem[];
@@ -207,28 +207,47 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
             }
         }
         if (FAST) {
-            const float* col = Gs + stage * GS + (COLS > 1 ? tid : tid % TP) + (ROWS > 1 ? tid / TP : 0) * TP;
-#pragma unroll
-            for (int q = 0; q < COLS; ++q) {
-                const float* cq = col + q * GATHER_THREADS;
+            const float* col = Gs + stage * GS + (COLS > 1 ? tid : tid % TP);
+            if constexpr (MINE == 1) {               // small tiles: a thread has one of the four
+                const float* cq = col + (tid / TP) * TP;
+                float s = 0.f;
                 if (nk == CK) {
 #pragma unroll
-                    for (int kb = 0; kb < CK; kb += 16)
-#pragma unroll
-                        for (int i = 0; i < MINE; ++i) {
-                            float s = 0.f;
-#pragma unroll
-                            for (int k = kb + i * ROWS; k < kb + 16; k += PARTS) s += cq[k * TP];
-                            box[q][i] += s;
-                        }
+                    for (int k = 0; k < CK; k += ROWS) s += cq[k * TP];
                 } else {
-                    for (int kb = 0; kb < nk; kb += 16)
+                    for (int k = 0; k < nk; k += ROWS) s += cq[k * TP];
+                }
+                box[0][0] += s;
+            } else {
 #pragma unroll
-                        for (int i = 0; i < MINE; ++i) {
-                            float s = 0.f;
-                            for (int k = kb; k < kb + 16 && k < nk; k += PARTS) s += cq[(k + i * ROWS) * TP];      // nk is a multiple of 4
-                            box[q][i] += s;
+                for (int q = 0; q < COLS; ++q) {
+                    const float* cq = col + (ROWS > 1 ? tid / TP : 0) * TP + q * GATHER_THREADS;
+                    if (nk == CK) {
+#pragma unroll
+                        for (int kb = 0; kb < CK; kb += 16) {
+                            float s[MINE];
+#pragma unroll
+                            for (int k = 0; k < 16 / ROWS; ++k) {
+                                const float v = cq[(kb + k * ROWS) * TP];
+                                s[k % MINE] = k < MINE ? v : s[k % MINE] + v;
+                            }
+#pragma unroll
+                            for (int i = 0; i < MINE; ++i) box[q][i] += s[i];
                         }
+                    } else {
+#pragma unroll 1
+                        for (int kb = 0; kb < nk; kb += 16) {
+                            float s[MINE];
+#pragma unroll
+                            for (int i = 0; i < MINE; ++i) s[i] = 0.f;
+#pragma unroll 1
+                            for (int k = kb; k < min(kb + 16, nk); k += PARTS)      // nk is a multiple of 4
+#pragma unroll
+                                for (int i = 0; i < MINE; ++i) s[i] += cq[(k + i * ROWS) * TP];
+#pragma unroll
+                            for (int i = 0; i < MINE; ++i) box[q][i] += s[i];
+                        }
+                    }
                 }
             }
         }
