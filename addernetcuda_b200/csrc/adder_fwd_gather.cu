@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
     const int ck4 = round_up(a.CK, 4);
     auto fill = [&](int stage) {
         int nk, rows, wk;        // reduction steps that exist, rows to stage, and the first one's weight index
+        int nk2 = 0, wk2 = 0;    // GATHER_HALVES: of the second block
         if constexpr (MODE == GATHER_NINE) {
             const int nch = min(CH, a.Ci - fc.c0);
             nine.fill(Xs + stage * XS, px, a.m, fc.c0, nch, a.H, a.W, tid);
@@ -70,8 +71,15 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
         } else {
             nk = min(a.CK, a.Ci - fc.c0); rows = ck4;
             if (MODE == GATHER_QUADS) gather_quads<TP, CK>(Xs + stage * XS, px[0].base, px[0].ok, a.x, fc.c0, nk, ck4, a.H * a.W, tid);
-            else gather_pixels<TP, CK>(Xs + stage * XS, px, a.x, a.m, fc, nk, ck4, a.H, a.W, tid);
+            else gather_pixels<TP, MODE == GATHER_HALVES ? GATHER_CK : CK>(Xs + stage * XS, px, a.x, a.m, fc, nk, ck4, a.H, a.W, tid);
             wk = fc.c0 * a.KK + a.m.wt0 + fc.i * a.m.dwi + fc.j * a.m.dwj;
+            if constexpr (MODE == GATHER_HALVES) {
+                fc.next(a.m, GATHER_CK);
+                GatherChunk f2 = fc;
+                if (fc.c0 >= a.Ci) f2.c0 = 0;                    // none left: zeros, from an address within the tensor
+                else { nk2 = min(GATHER_CK, a.Ci - fc.c0); wk2 = fc.c0 * a.KK + a.m.wt0 + fc.i * a.m.dwi + fc.j * a.m.dwj; }
+                gather_pixels<TP>(Xs + stage * XS + GATHER_CK * TP, px, a.x, a.m, f2, nk2, GATHER_CK, a.H, a.W, tid);
+            }
         }
         const int kstep = MODE == GATHER_NINE ? 1 : a.KK, row = a.Ci * a.KK;
         if constexpr (T::THIN) {
@@ -82,15 +90,17 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
                 if ((TC * CK / 4) % GATHER_THREADS != 0 && c >= TC) break;
                 float* ws = Ws + stage * WS + c * (CK + 4) + k;
                 const bool okc = co0 + c < a.Co;
-                const float* wsrc = a.w + (okc ? (co0 + c) * row + wk : 0);
-                if (a.vec_w) {
-                    const bool ok = okc & (k < nk);
-                    cp_async16(ws, ok ? wsrc + k : a.w, ok);
+                const bool second = MODE == GATHER_HALVES && k >= GATHER_CK;
+                const int kr = second ? k - GATHER_CK : k, nkr = second ? nk2 : nk;
+                const float* wsrc = a.w + (okc ? (co0 + c) * row + (second ? wk2 : wk) : 0);
+                if (MODE != GATHER_HALVES && a.vec_w) {
+                    const bool ok = okc & (kr < nkr);
+                    cp_async16(ws, ok ? wsrc + kr : a.w, ok);
                 } else {
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        const bool ok = okc & (k + i < nk);
-                        cp_async4(ws + i, ok ? wsrc + (k + i) * kstep : a.w, ok);
+                        const bool ok = okc & (kr + i < nkr);
+                        cp_async4(ws + i, ok ? wsrc + (kr + i) * kstep : a.w, ok);
                     }
                 }
             }
@@ -136,12 +146,12 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
         if (c + ST - 1 < a.nchunks) fill(fstage);
         cp_async_commit();
         const float* xs = Xs + stage * XS + pg * PQ;
-        const int nk = MODE == GATHER_NINE ? CK : min(ck4, round_up(a.Ci - cc.c0, 4));
+        const int nk = MODE == GATHER_NINE || MODE == GATHER_HALVES ? CK : min(ck4, round_up(a.Ci - cc.c0, 4));
         if constexpr (T::THIN) {
             const float* ws = Ws + stage * WS + cg * RM * (CK + 4);
 #pragma unroll (RM == 1 ? CK / 4 : 2)
             for (int k = 0; k < CK; k += 4) {
-                if (MODE != GATHER_NINE && k >= nk) break;
+                if (MODE != GATHER_NINE && MODE != GATHER_HALVES && k >= nk) break;
                 float4 wq[RM];
                 float xv[4][RP];
 #pragma unroll
@@ -307,7 +317,10 @@ template <int MODE>
 int launch_mode(int tile, const FwdGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
     int i = 0;
 #define X(RM, RP, CG, ST, MB, A, M, S) \
-    if (tile == i++) return launch_t<FwdTile<RM, RP, CG, ST, MB>, MODE>(a, grid, smem, stream);
+    if (tile == i++) {                                                                                 \
+        using T = FwdTile<RM, RP, CG, ST, MB>;                                                         \
+        if constexpr (MODE != GATHER_HALVES || T::THIN) return launch_t<T, MODE>(a, grid, smem, stream); \
+    }
     ADDER_FWD_GATHER_TILES(X)
 #undef X
     return ADDER_ERR_INTERNAL;
@@ -336,12 +349,17 @@ int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* 
     const int tile = choose_tile(a.m.P, g.Co);
     const Tile& t = kTiles[tile];
     const int rows = stage_rows(t, mode);
-    a.CK = mode == GATHER_NINE ? rows / 9 : g.Ci < rows ? g.Ci : rows;      // full blocks have the cheaper staging loops
+    // Windows of several taps are added up in the order (block of 16 channels, tap, channel) by every tile: the tile follows the batch,
+    // and an image's result must not.  A thin tile, whose stages have 32 rows, takes two such blocks a stage.
+    const bool halves = mode == GATHER_TAP && a.KK > 1 && g.Ci > GATHER_CK && rows > GATHER_CK;
+    a.CK = mode == GATHER_NINE ? rows / 9 : halves ? GATHER_CK : g.Ci < rows ? g.Ci : rows;      // full blocks have the cheaper staging loops
     a.nchunks = ceil_div(g.Ci, a.CK) * (mode == GATHER_NINE ? 1 : a.KK);
+    if (halves) a.nchunks = ceil_div(a.nchunks, 2);
     const dim3 grid((unsigned)ceil_div(a.m.P, t.tp), (unsigned)ceil_div(g.Co, t.tc));
     if (grid.y > 65535) return ADDER_ERR_UNSUPPORTED;
     const size_t smem = smem_bytes(t, rows);
     if (mode == GATHER_NINE) return launch_mode<GATHER_NINE>(tile, a, grid, smem, stream);
+    if (halves) return launch_mode<GATHER_HALVES>(tile, a, grid, smem, stream);
     return quads ? launch_mode<GATHER_QUADS>(tile, a, grid, smem, stream) : launch_mode<GATHER_TAP>(tile, a, grid, smem, stream);
 }
 

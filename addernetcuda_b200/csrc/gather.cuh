@@ -8,6 +8,7 @@
 //   GATHER_TAP    at most 16 channels of one tap (index order: channel block, tap, channel in the block), so that a
 //                 thread computes the address and the bounds test of its pixel once per chunk;
 //   GATHER_QUADS  the same for 1x1 layers whose operand is read in order: 16-byte copies;
+//   GATHER_HALVES two such blocks in one stage of a thin tile;
 //   GATHER_NINE   2 channels x the 9 taps of a 3x3 window, in index order (channel, row, column).
 // One barrier per chunk; large tiles keep two stages, small ones as many as hide the latency of a load.
 #pragma once
@@ -17,7 +18,7 @@ namespace adder {
 
 constexpr int GATHER_CK = 16;
 constexpr int GATHER_THREADS = 128;
-enum GatherMode { GATHER_TAP, GATHER_QUADS, GATHER_NINE };
+enum GatherMode { GATHER_TAP, GATHER_QUADS, GATHER_NINE, GATHER_HALVES };
 
 // Channels of a chunk of GATHER_NINE; thin tiles (a few outputs a thread) spend their time on the instructions around a stage
 // rather than on its terms, so their stages are twice as long.

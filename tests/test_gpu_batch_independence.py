@@ -11,7 +11,9 @@ DEV = "cuda:0"
 CASES = [(128, 128, 14, 14, 3, 1, 1, (1, 8, 16, 64)), (64, 64, 15, 15, 3, 1, 1, (1, 8, 64)), (256, 256, 14, 14, 3, 1, 1, (1, 8, 64)),
          (40, 72, 9, 11, 3, 1, 1, (1, 5, 64)), (96, 64, 16, 16, 3, 2, 1, (1, 8, 100)), (256, 64, 14, 14, 1, 1, 0, (1, 8, 64)),
          (100, 60, 7, 9, 1, 1, 0, (1, 8, 64)), (64, 128, 28, 28, 1, 2, 0, (1, 8, 64)), (16, 16, 32, 32, 3, 1, 1, (1, 8, 64))]
-OTHER = [(16, 24, 21, 23, 7, 2, 3, (1, 8, 64))]      # beyond the standard geometries
+# beyond the standard geometries: blocks of channels below, at and past 16 and 32, even and odd numbers of taps
+OTHER = [(48, 40, 20, 20, 5, 1, 2, (1, 6, 64)), (36, 33, 18, 18, 2, 2, 0, (1, 16, 64)), (16, 24, 21, 23, 7, 2, 3, (1, 8, 64)),
+         (17, 20, 12, 12, 5, 1, 2, (1, 8, 128)), (64, 64, 14, 14, 4, 1, 1, (1, 8, 64))]
 
 
 @pytest.mark.parametrize("fast", [False, True], ids=["exact", "saturating"])
