@@ -44,6 +44,18 @@ def _stale() -> bool:
     return any(d.stat().st_mtime > t for d in deps)
 
 
+def _shared_libstdcxx() -> list:
+    """The C++ runtime that torch runs on, named before the compiler's own.  A compiler that has only a static one would put a
+    second copy into the extension, and streams of one copy cannot format with the locale of the other: an error
+    message with a number in it ended the process."""
+    import torch  # noqa: F401  (loads it)
+    try:
+        maps = Path("/proc/self/maps").read_text()
+    except OSError:
+        return []
+    return sorted({line.split()[-1] for line in maps.splitlines() if "/libstdc++.so" in line})[:1]
+
+
 def _host_command() -> list:
     """Compile and link csrc/host.cpp against the installed torch."""
     import sysconfig
@@ -54,7 +66,7 @@ def _host_command() -> list:
            Path(sysconfig.get_paths()["include"])]
     return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wno-interference-size",
             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{p}" for p in inc), str(CSRC / "host.cpp"),
-            "-o", str(HOST_LIB), f"-L{root / 'lib'}", "-lc10", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-lc10_cuda", "-ltorch_cuda",
+            "-o", str(HOST_LIB), *_shared_libstdcxx(), f"-L{root / 'lib'}", "-lc10", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-lc10_cuda", "-ltorch_cuda",
             f"-L{cuda / 'lib64'}", "-lcudart"]
 
 

@@ -39,8 +39,11 @@ Api api;
 PyObject* g_adder_dict = nullptr;          // module dictionaries that hold FAST_CLAMP, OVERLAP_BACKWARD and ETA
 PyObject* g_cuda_dict = nullptr;
 
+// ValueError for what the caller can mend, RuntimeError otherwise, as _lib.check raises.
 void check(int status, const char* what) {
-    TORCH_CHECK(status == ADDER_OK, what, ": ", api.status_string(status), " (status ", status, ")");
+    const bool runtime = status == ADDER_ERR_CUDA || status == ADDER_ERR_INTERNAL || status == ADDER_ERR_TIMEOUT;
+    TORCH_CHECK(status == ADDER_OK || !runtime, what, ": ", api.status_string(status), " (status ", status, ")");
+    TORCH_CHECK_VALUE(status == ADDER_OK, what, ": ", api.status_string(status), " (status ", status, ")");
 }
 
 cudaStream_t current_stream(const at::Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }

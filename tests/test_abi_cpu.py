@@ -151,3 +151,14 @@ def test_reference_model_files_import_unchanged_on_the_dropin():
         sys.path.remove(REFERENCE_DIR)
         for mod in ("adder", "adder_cuda", "resnet20", "resnet50", "vgg", "densenet"):
             sys.modules.pop(mod, None)
+
+
+def test_host_extension_runs_on_torchs_cxx_runtime():
+    """With a C++ runtime of its own (linked statically) the extension cannot format a number into an error message."""
+    from addernetcuda_b200 import build
+    if not build._shared_libstdcxx():
+        pytest.skip("no shared libstdc++ in this process")
+    build.build()
+    image = build.HOST_LIB.read_bytes()
+    assert b"\0libstdc++.so.6\0" in image and b"\0_ZNSolsEi\0" in image      # needed, and operator<<(int) among its imports
+    assert b"locale::facet::_S_create_c_locale name not valid" not in image  # a text of the runtime itself

@@ -1,0 +1,39 @@
+"""The C++ host path of the eager layer calls (csrc/host.cpp) beside what torch and the caller may do around a layer."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _rand(*shape, seed=0):
+    return torch.randn(*shape, device=DEV, generator=torch.Generator(device=DEV).manual_seed(seed + sum(shape)))
+
+
+def _calls():
+    """(name, function of an input that requires grad, shape of the input) of every autograd node the path makes."""
+    from addernetcuda_b200 import adder
+    l3, l5 = (adder.adder2d(6, 8, k, padding=k // 2).to(DEV) for k in (3, 5))
+    w = torch.nn.Parameter(_rand(8, 24))
+    return [("3x3", l3, l3.adder, (2, 6, 9, 10)), ("5x5", l5, l5.adder, (2, 6, 9, 10)),
+            ("columns", lambda x: adder.adder.apply(w, x), w, (24, 70))]
+
+
+def _grads(x, w):
+    r = x.grad.clone(), w.grad.clone()
+    x.grad = w.grad = None
+    return r
+
+
+def test_a_refused_call_raises():
+    """A status other than 0 is a ValueError with the library's words, in forward and in backward: more channels than a launch has rows
+    of blocks."""
+    from addernetcuda_b200 import adder
+    n = 4_500_000
+    one = torch.ones(1, 1, device=DEV)
+    with pytest.raises(ValueError, match="adder_b200_forward: .*status 3"):
+        adder.adder.apply(torch.ones(n, 1, device=DEV), one)
+    x = torch.ones(n, 1, device=DEV, requires_grad=True)
+    out = adder.adder.apply(torch.zeros(1, n, device=DEV), x)
+    with pytest.raises(ValueError, match="adder_b200_backward_input: .*status 3"):
+        out.backward(one)
