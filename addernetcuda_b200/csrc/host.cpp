@@ -14,6 +14,7 @@
 #include <c10/cuda/CUDAGuard.h>
 
 #include <array>
+#include <atomic>
 #include <mutex>
 
 #include "../../include/adder_b200.h"
@@ -35,7 +36,10 @@ struct Api {      // entry points of the loaded libadder_b200.so
     decltype(&adder_b200_conv_backward_weight_workspace_bytes) conv_backward_weight_workspace_bytes = nullptr;
     decltype(&adder_b200_conv_backward_weight) conv_backward_weight = nullptr;
 };
+// Written once, by the first bind to the product library, which is never unloaded: autograd nodes made by this path call through it
+// for as long as they live, from any thread.  `enabled` is what bind() switches, and only the Python entry points look at it.
 Api api;
+std::atomic<bool> enabled{false};
 PyObject* g_adder_dict = nullptr;          // module dictionaries that hold FAST_CLAMP, OVERLAP_BACKWARD and ETA
 PyObject* g_cuda_dict = nullptr;
 
@@ -319,7 +323,7 @@ bool needs_node(const at::Tensor& a, const at::Tensor& b) { return at::GradMode:
 // layer(x, w, stride, padding) -> out, or None
 PyObject* py_layer(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 4 || api.forward == nullptr) Py_RETURN_NONE;
+    if (n != 4 || !enabled.load(std::memory_order_acquire)) Py_RETURN_NONE;
     const at::Tensor *x = tensor_arg(args[0]), *w = tensor_arg(args[1]);
     int64_t stride, pad;
     Layer L;
@@ -336,7 +340,7 @@ PyObject* py_layer(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // conv(x, w, sh, sw, ph, pw, dh, dw) -> out, or None
 PyObject* py_conv(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 8 || api.forward == nullptr) Py_RETURN_NONE;
+    if (n != 8 || !enabled.load(std::memory_order_acquire)) Py_RETURN_NONE;
     const at::Tensor *x = tensor_arg(args[0]), *w = tensor_arg(args[1]);
     std::array<int64_t, 6> p;
     for (int i = 0; i < 6; ++i)
@@ -355,7 +359,7 @@ PyObject* py_conv(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // layer_with_stats(x, w, stride, padding) -> (out, statistics), or None
 PyObject* py_layer_with_stats(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 4 || api.forward == nullptr) Py_RETURN_NONE;
+    if (n != 4 || !enabled.load(std::memory_order_acquire)) Py_RETURN_NONE;
     const at::Tensor *x = tensor_arg(args[0]), *w = tensor_arg(args[1]);
     int64_t stride, pad;
     Layer L;
@@ -387,7 +391,7 @@ bool affine_args(PyObject* scale, PyObject* shift, PyObject* residual, const at:
 // layer_affine(x, w, stride, padding, scale, shift, residual, relu) -> relu?(layer * scale + shift + residual) without autograd, or None
 PyObject* py_layer_affine(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 8 || api.forward == nullptr) Py_RETURN_NONE;
+    if (n != 8 || !enabled.load(std::memory_order_acquire)) Py_RETURN_NONE;
     const at::Tensor *x = tensor_arg(args[0]), *w = tensor_arg(args[1]), *sc, *sh, *res;
     int64_t stride, pad;
     Layer L;
@@ -412,7 +416,7 @@ PyObject* py_layer_affine(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // affine(y, scale, shift, residual, relu) -> the same behind a tensor, or None
 PyObject* py_affine(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 5 || api.forward == nullptr) Py_RETURN_NONE;
+    if (n != 5 || !enabled.load(std::memory_order_acquire)) Py_RETURN_NONE;
     const at::Tensor *y = tensor_arg(args[0]), *sc, *sh, *res;
     if (y == nullptr || !plain(*y) || y->dim() != 4 || y->numel() == 0 || y->numel() > 2147483647) Py_RETURN_NONE;
     if (!affine_args(args[1], args[2], args[3], *y, y->size(1), y->sizes(), &sc, &sh, &res)) Py_RETURN_NONE;
@@ -433,7 +437,7 @@ PyObject* py_affine(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // column(W[Co,K], X[K,P]) -> [Co,P], or None
 PyObject* py_column(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 2 || api.forward == nullptr) Py_RETURN_NONE;
+    if (n != 2 || !enabled.load(std::memory_order_acquire)) Py_RETURN_NONE;
     const at::Tensor *w = tensor_arg(args[0]), *x = tensor_arg(args[1]);
     if (w == nullptr || x == nullptr || !plain(*w) || !plain(*x) || w->dim() != 2 || x->dim() != 2 || w->size(1) != x->size(0) ||
         w->numel() == 0 || x->numel() == 0 || w->device() != x->device())
@@ -450,12 +454,14 @@ PyObject* py_column(PyObject*, PyObject* const* args, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// bind({name: address}, adder module dict, adder_cuda module dict); bind(None, ...) switches the entry points off
+// bind({name: address}, adder module dict, adder_cuda module dict) switches the entry points on, bind(None, ...) off
 PyObject* py_bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     TORCH_CHECK(n == 3 && PyDict_Check(args[1]) && PyDict_Check(args[2]), "bind(addresses, dict, dict)");
-    Api a;
-    if (args[0] != Py_None) {
+    enabled.store(false, std::memory_order_release);
+    const bool on = args[0] != Py_None;
+    if (on && api.forward == nullptr) {
+        Api a;
         auto get = [&](const char* name, auto* fn) {
             PyObject* v = PyDict_GetItemString(args[0], name);
             TORCH_CHECK(v != nullptr && PyLong_Check(v), "no address for ", name);
@@ -474,11 +480,12 @@ PyObject* py_bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
         get("adder_b200_conv_backward_input", &a.conv_backward_input);
         get("adder_b200_conv_backward_weight_workspace_bytes", &a.conv_backward_weight_workspace_bytes);
         get("adder_b200_conv_backward_weight", &a.conv_backward_weight);
+        api = a;
     }
     Py_INCREF(args[1]); Py_INCREF(args[2]);
     Py_XDECREF(g_adder_dict); Py_XDECREF(g_cuda_dict);
     g_adder_dict = args[1]; g_cuda_dict = args[2];
-    api = a;
+    enabled.store(on, std::memory_order_release);
     Py_RETURN_NONE;
     END_HANDLE_TH_ERRORS
 }

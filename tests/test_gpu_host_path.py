@@ -37,3 +37,23 @@ def test_a_refused_call_raises():
     out = adder.adder.apply(torch.zeros(1, n, device=DEV), x)
     with pytest.raises(ValueError, match="adder_b200_backward_input: .*status 3"):
         out.backward(one)
+
+
+@pytest.mark.parametrize("i", range(3), ids=["3x3", "5x5", "columns"])
+def test_a_forward_before_a_tuning_block_may_run_its_backward_inside(i):
+    """The nodes keep the product library's entry points while another library is active."""
+    from addernetcuda_b200 import _lib
+    _, call, w, shape = _calls()[i]
+    x = _rand(*shape).requires_grad_()
+    out = call(x)
+    g = _rand(*out.shape, seed=1)
+    out.backward(g)
+    want = _grads(x, w)
+    out = call(x)
+    with _lib.tuning():
+        out.backward(g)
+    got = _grads(x, w)
+    call(x).backward(g)                                  # and the path is on again behind it
+    again = _grads(x, w)
+    for a, b, c in zip(want, got, again):
+        assert torch.equal(a, b) and torch.equal(a, c)
