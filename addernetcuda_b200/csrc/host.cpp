@@ -7,6 +7,7 @@
 #include <torch/extension.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/EmptyTensor.h>
@@ -42,6 +43,9 @@ Api api;
 std::atomic<bool> enabled{false};
 PyObject* g_adder_dict = nullptr;          // module dictionaries that hold FAST_CLAMP, OVERLAP_BACKWARD and ETA
 PyObject* g_cuda_dict = nullptr;
+
+// A torch.jit trace records the Python layer's autograd functions as operators; what runs here would leave a constant in it.
+bool available() { return enabled.load(std::memory_order_acquire) && !torch::jit::tracer::isTracing(); }
 
 // ValueError for what the caller can mend, RuntimeError otherwise, as _lib.check raises.
 void check(int status, const char* what) {
@@ -323,7 +327,7 @@ bool needs_node(const at::Tensor& a, const at::Tensor& b) { return at::GradMode:
 // layer(x, w, stride, padding) -> out, or None
 PyObject* py_layer(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 4 || !enabled.load(std::memory_order_acquire)) Py_RETURN_NONE;
+    if (n != 4 || !available()) Py_RETURN_NONE;
     const at::Tensor *x = tensor_arg(args[0]), *w = tensor_arg(args[1]);
     int64_t stride, pad;
     Layer L;
@@ -340,7 +344,7 @@ PyObject* py_layer(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // conv(x, w, sh, sw, ph, pw, dh, dw) -> out, or None
 PyObject* py_conv(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 8 || !enabled.load(std::memory_order_acquire)) Py_RETURN_NONE;
+    if (n != 8 || !available()) Py_RETURN_NONE;
     const at::Tensor *x = tensor_arg(args[0]), *w = tensor_arg(args[1]);
     std::array<int64_t, 6> p;
     for (int i = 0; i < 6; ++i)
@@ -359,7 +363,7 @@ PyObject* py_conv(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // layer_with_stats(x, w, stride, padding) -> (out, statistics), or None
 PyObject* py_layer_with_stats(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 4 || !enabled.load(std::memory_order_acquire)) Py_RETURN_NONE;
+    if (n != 4 || !available()) Py_RETURN_NONE;
     const at::Tensor *x = tensor_arg(args[0]), *w = tensor_arg(args[1]);
     int64_t stride, pad;
     Layer L;
@@ -391,7 +395,7 @@ bool affine_args(PyObject* scale, PyObject* shift, PyObject* residual, const at:
 // layer_affine(x, w, stride, padding, scale, shift, residual, relu) -> relu?(layer * scale + shift + residual) without autograd, or None
 PyObject* py_layer_affine(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 8 || !enabled.load(std::memory_order_acquire)) Py_RETURN_NONE;
+    if (n != 8 || !available()) Py_RETURN_NONE;
     const at::Tensor *x = tensor_arg(args[0]), *w = tensor_arg(args[1]), *sc, *sh, *res;
     int64_t stride, pad;
     Layer L;
@@ -416,7 +420,7 @@ PyObject* py_layer_affine(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // affine(y, scale, shift, residual, relu) -> the same behind a tensor, or None
 PyObject* py_affine(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 5 || !enabled.load(std::memory_order_acquire)) Py_RETURN_NONE;
+    if (n != 5 || !available()) Py_RETURN_NONE;
     const at::Tensor *y = tensor_arg(args[0]), *sc, *sh, *res;
     if (y == nullptr || !plain(*y) || y->dim() != 4 || y->numel() == 0 || y->numel() > 2147483647) Py_RETURN_NONE;
     if (!affine_args(args[1], args[2], args[3], *y, y->size(1), y->sizes(), &sc, &sh, &res)) Py_RETURN_NONE;
@@ -437,7 +441,7 @@ PyObject* py_affine(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // column(W[Co,K], X[K,P]) -> [Co,P], or None
 PyObject* py_column(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 2 || !enabled.load(std::memory_order_acquire)) Py_RETURN_NONE;
+    if (n != 2 || !available()) Py_RETURN_NONE;
     const at::Tensor *w = tensor_arg(args[0]), *x = tensor_arg(args[1]);
     if (w == nullptr || x == nullptr || !plain(*w) || !plain(*x) || w->dim() != 2 || x->dim() != 2 || w->size(1) != x->size(0) ||
         w->numel() == 0 || x->numel() == 0 || w->device() != x->device())

@@ -57,3 +57,25 @@ def test_a_forward_before_a_tuning_block_may_run_its_backward_inside(i):
     again = _grads(x, w)
     for a, b, c in zip(want, got, again):
         assert torch.equal(a, b) and torch.equal(a, c)
+
+
+@pytest.mark.parametrize("grad", [False, True], ids=["no_grad", "grad"])
+@pytest.mark.parametrize("i", range(3), ids=["3x3", "5x5", "columns"])
+def test_a_trace_records_the_operation(i, grad):
+    """torch.jit.trace: the traced module follows a new input instead of returning the output of the traced one."""
+    _, call, w, shape = _calls()[i]
+
+    class Net(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.w = w
+
+        def forward(self, x):
+            return call(x)
+
+    net, a, b = Net(), _rand(*shape), _rand(*shape, seed=1)
+    with torch.set_grad_enabled(grad):
+        traced = torch.jit.trace(net, a, check_trace=False)
+        # (a traced 5x5 layer runs as columns, which adds in another order)
+        torch.testing.assert_close(traced(b), net(b), rtol=1e-5, atol=1e-4)
+        assert float((traced(b) - traced(a)).abs().max()) > 1.0
