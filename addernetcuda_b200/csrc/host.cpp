@@ -65,11 +65,14 @@ struct Layer {      // geometry arguments of the C interface
 };
 #define ADDER_GEOM(L) (L).n, (L).ci, (L).h, (L).w, (L).co, (L).k, (L).stride, (L).pad
 
+// What the kernels take.  A dual tensor of forward-mode differentiation is left to the Python layer, which refuses it: without a node,
+// its tangent would be dropped without a word.
 bool plain(const at::Tensor& t) {
     static const c10::DispatchKeySet wrapped({c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
                                               c10::DispatchKey::Functionalize, c10::DispatchKey::Python,
                                               c10::DispatchKey::Conjugate, c10::DispatchKey::Negative});
-    return t.is_cuda() && t.scalar_type() == at::kFloat && t.layout() == at::kStrided && t.is_contiguous() && !t.key_set().has_any(wrapped);
+    return t.is_cuda() && t.scalar_type() == at::kFloat && t.layout() == at::kStrided && t.is_contiguous() && !t.key_set().has_any(wrapped) &&
+           !t._fw_grad(0).defined();
 }
 
 bool layer_of(const at::Tensor& x, const at::Tensor& w, int64_t stride, int64_t pad, Layer* L) {

@@ -79,3 +79,16 @@ def test_a_trace_records_the_operation(i, grad):
         # (a traced 5x5 layer runs as columns, which adds in another order)
         torch.testing.assert_close(traced(b), net(b), rtol=1e-5, atol=1e-4)
         assert float((traced(b) - traced(a)).abs().max()) > 1.0
+
+
+@pytest.mark.parametrize("i", range(3), ids=["3x3", "5x5", "columns"])
+def test_forward_mode_is_refused(i):
+    """No derivative is defined for it, so a dual input is an error, whether or not a gradient is wanted as well."""
+    import torch.autograd.forward_ad as fw
+    _, call, w, shape = _calls()[i]
+    for grad, frozen in ((True, False), (True, True), (False, False)):
+        w.requires_grad_(not frozen)
+        with torch.set_grad_enabled(grad), fw.dual_level():
+            x = fw.make_dual(_rand(*shape), torch.ones(shape, device=DEV))
+            with pytest.raises(NotImplementedError, match="jvp"):
+                call(x)
