@@ -209,6 +209,20 @@ void conv_backward_weight(const at::Tensor& g, const at::Tensor& x, const at::Te
 
 // ------------------------------------------------------------------------------------------ autograd nodes
 
+using torch::autograd::AutogradContext;
+using torch::autograd::Variable;
+using torch::autograd::variable_list;
+
+// What a saved-tensor hook hands back need not be what it was given: every backward looks at its tensors again.
+constexpr const char* SAVED = "the saved tensors came back in another form: contiguous float32 CUDA tensors of the forward's shapes are needed";
+
+at::Tensor gradient(const Variable& grad, const at::Tensor& x, at::IntArrayRef shape) {
+    const at::Tensor g = grad.contiguous();
+    TORCH_CHECK(g.scalar_type() == at::kFloat && g.device() == x.device(), "grad_out must be a float32 tensor on the layer's device");
+    TORCH_CHECK(g.sizes() == shape, "grad_out has shape ", g.sizes(), ", expected ", shape);
+    return g;
+}
+
 struct Settings { bool fast, overlap; float eta; };
 
 // The module-level switches are read when the backward runs, as the Python layer reads them.
@@ -222,9 +236,6 @@ Settings settings() {
     return {flag(g_adder_dict, "FAST_CLAMP"), flag(g_adder_dict, "OVERLAP_BACKWARD"), eta != nullptr ? (float)PyFloat_AsDouble(eta) : 0.2f};
 }
 
-using torch::autograd::AutogradContext;
-using torch::autograd::Variable;
-using torch::autograd::variable_list;
 
 // adder2d on NCHW tensors (adder.py:22-80 of the reference).
 struct AdderLayer : public torch::autograd::Function<AdderLayer> {
@@ -245,9 +256,8 @@ struct AdderLayer : public torch::autograd::Function<AdderLayer> {
         const auto saved = ctx->get_saved_variables();
         const Variable &x = saved[0], &w = saved[1];
         Layer L;
-        TORCH_CHECK(layer_of(x, w, ctx->saved_data["stride"].toInt(), ctx->saved_data["pad"].toInt(), &L));
-        const at::Tensor g = grads[0].contiguous();
-        TORCH_CHECK(g.scalar_type() == at::kFloat && g.device() == x.device(), "grad_out must be a float32 tensor on the layer's device");
+        TORCH_CHECK(layer_of(x, w, ctx->saved_data["stride"].toInt(), ctx->saved_data["pad"].toInt(), &L), SAVED);
+        const at::Tensor g = gradient(grads[0], x, {L.n, L.co, L.ho, L.wo});
         const c10::cuda::CUDAGuard guard(x.device());
         const Settings set = settings();
         at::Tensor gx, gw;
@@ -273,9 +283,8 @@ struct ConvLayer : public torch::autograd::Function<ConvLayer> {
         const Variable &x = saved[0], &w = saved[1];
         const auto p = ctx->saved_data["p"].toIntVector();
         Conv c;
-        TORCH_CHECK(conv_of(x, w, {p[0], p[1], p[2], p[3], p[4], p[5]}, &c));
-        const at::Tensor g = grads[0].contiguous();
-        TORCH_CHECK(g.scalar_type() == at::kFloat && g.device() == x.device(), "grad_out must be a float32 tensor on the layer's device");
+        TORCH_CHECK(conv_of(x, w, {p[0], p[1], p[2], p[3], p[4], p[5]}, &c), SAVED);
+        const at::Tensor g = gradient(grads[0], x, {c[0], c[4], c[13], c[14]});
         const c10::cuda::CUDAGuard guard(x.device());
         const Settings set = settings();
         at::Tensor gx, gw;
@@ -291,23 +300,30 @@ struct ConvLayer : public torch::autograd::Function<ConvLayer> {
 };
 
 // The column-matrix op (adder.py:43-80 of the reference): X[K,P] is the 1x1 layer [1,K,1,P], W[Co,K] its kernel.
-Layer column_layer(const at::Tensor& w, const at::Tensor& x) {
-    return {1, (int)x.size(0), 1, (int)x.size(1), (int)w.size(0), 1, 1, 0, 1, (int)x.size(1)};
+bool column_of(const at::Tensor& w, const at::Tensor& x, Layer* L) {
+    if (!plain(w) || !plain(x) || w.dim() != 2 || x.dim() != 2 || w.size(1) != x.size(0) || w.numel() == 0 || x.numel() == 0 ||
+        w.device() != x.device())
+        return false;
+    constexpr int64_t lim = 2147483647;
+    if (w.numel() > lim || x.numel() > lim || w.size(0) * x.size(1) > lim) return false;
+    *L = Layer{1, (int)x.size(0), 1, (int)x.size(1), (int)w.size(0), 1, 1, 0, 1, (int)x.size(1)};
+    return true;
 }
 
 struct AdderColumn : public torch::autograd::Function<AdderColumn> {
     static Variable forward(AutogradContext* ctx, const Variable& w, const Variable& x) {
+        Layer L;
+        TORCH_CHECK(column_of(w, x, &L));
         ctx->save_for_backward({w, x});
-        const Layer L = column_layer(w, x);
         return ::forward(x, w, L).view({L.co, L.w});
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
         const auto saved = ctx->get_saved_variables();
         const Variable &w = saved[0], &x = saved[1];
-        const at::Tensor g = grads[0].contiguous();
-        TORCH_CHECK(g.scalar_type() == at::kFloat && g.device() == x.device(), "grad_output must be a float32 tensor on the op's device");
+        Layer L;
+        TORCH_CHECK(column_of(w, x, &L), SAVED);
+        const at::Tensor g = gradient(grads[0], x, {L.co, L.w});
         const c10::cuda::CUDAGuard guard(x.device());
-        const Layer L = column_layer(w, x);
         at::Tensor gx = empty_on(x, x.sizes()), gw = empty_on(w, w.sizes());
         backward_both(g, x, w, gx, gw, L, 0.2f, false, true);
         return {gw, gx};
@@ -446,16 +462,13 @@ PyObject* py_column(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     if (n != 2 || !available()) Py_RETURN_NONE;
     const at::Tensor *w = tensor_arg(args[0]), *x = tensor_arg(args[1]);
-    if (w == nullptr || x == nullptr || !plain(*w) || !plain(*x) || w->dim() != 2 || x->dim() != 2 || w->size(1) != x->size(0) ||
-        w->numel() == 0 || x->numel() == 0 || w->device() != x->device())
-        Py_RETURN_NONE;
-    constexpr int64_t lim = 2147483647;
-    if (w->numel() > lim || x->numel() > lim || w->size(0) * x->size(1) > lim) Py_RETURN_NONE;
+    Layer L;
+    if (w == nullptr || x == nullptr || !column_of(*w, *x, &L)) Py_RETURN_NONE;
     at::Tensor out;
     {
         pybind11::gil_scoped_release no_gil;
         if (needs_node(*w, *x)) out = AdderColumn::apply(*w, *x);
-        else { const Layer L = column_layer(*w, *x); out = forward(*x, *w, L).view({L.co, L.w}); }
+        else out = forward(*x, *w, L).view({L.co, L.w});
     }
     return THPVariable_Wrap(std::move(out));
     END_HANDLE_TH_ERRORS

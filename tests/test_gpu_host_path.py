@@ -92,3 +92,24 @@ def test_forward_mode_is_refused(i):
             x = fw.make_dual(_rand(*shape), torch.ones(shape, device=DEV))
             with pytest.raises(NotImplementedError, match="jvp"):
                 call(x)
+
+
+@pytest.mark.parametrize("change", [lambda t: t.cpu(), lambda t: t.double(), lambda t: t.mT.contiguous().mT, lambda t: t[:-1].contiguous()],
+                         ids=["cpu", "double", "strided", "shorter"])
+@pytest.mark.parametrize("i", range(3), ids=["3x3", "5x5", "columns"])
+def test_backward_looks_at_what_saved_tensor_hooks_return(i, change):
+    """Tensors in another form than the kernels take are an error, not an address."""
+    _, call, w, shape = _calls()[i]
+    x = _rand(*shape).requires_grad_()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, change):
+        out = call(x)
+    with pytest.raises((RuntimeError, TypeError, ValueError)):
+        out.backward(_rand(*out.shape))
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.cpu(), lambda t: t.to(DEV)):
+        out = call(x)
+    g = _rand(*out.shape)
+    out.backward(g)
+    got = _grads(x, w)
+    call(x).backward(g)
+    for a, b in zip(got, _grads(x, w)):
+        assert torch.equal(a, b)
