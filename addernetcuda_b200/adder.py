@@ -111,7 +111,7 @@ class adder(Function):
 
     @classmethod
     def apply(cls, W_col, X_col):
-        out = _native.column(W_col, X_col) if cls is adder else None
+        out = _native.column(W_col, X_col) if cls is adder and adder_cuda.unpatched() else None
         return out if out is not None else super().apply(W_col, X_col)
 
     @staticmethod

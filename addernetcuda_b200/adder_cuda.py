@@ -191,15 +191,6 @@ def backward(grad_out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, stride: i
     return gx, gw
 
 
-def unpatched() -> bool:
-    """No caller has replaced one of the four operations of this module (to record or wrap what the layers call): only
-    then may a layer go through the C++ host path, which does not come by here."""
-    return (forward is _own[0] and backward is _own[1] and backward_input is _own[2] and backward_weight is _own[3])
-
-
-_own = (forward, backward, backward_input, backward_weight)
-
-
 def _expect_grad_shape(grad_out, g):
     ho, wo = output_size(g[2], g[3], g[5], g[6], g[7])
     want = (g[0], g[4], ho, wo)
@@ -276,3 +267,13 @@ def ADDER_BACKWARD(grad_y, x, w, grad_w, grad_i):
         _lib.check(lib.adder_b200_backward_col(grad_y.data_ptr(), x.data_ptr(), w.data_ptr(), grad_w.data_ptr(),
                                                grad_i.data_ptr(), K, P, Co, ws.data_ptr(), ws.numel(), _stream(dev)),
                    "adder_b200_backward_col")
+
+
+_own = (forward, backward, backward_input, backward_weight, ADDER_CONV, ADDER_BACKWARD)
+
+
+def unpatched() -> bool:
+    """No caller has replaced one of the operations of this module that layers and the column op call (to record or wrap
+    them): only then may a call go through the C++ host path, which does not come by here."""
+    return (forward is _own[0] and backward is _own[1] and backward_input is _own[2] and backward_weight is _own[3]
+            and ADDER_CONV is _own[4] and ADDER_BACKWARD is _own[5])

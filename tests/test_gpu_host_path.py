@@ -113,3 +113,26 @@ def test_backward_looks_at_what_saved_tensor_hooks_return(i, change):
     call(x).backward(g)
     for a, b in zip(got, _grads(x, w)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("i,names", [(0, ("forward", "backward")), (1, ("ADDER_CONV", "ADDER_BACKWARD")), (2, ("ADDER_CONV", "ADDER_BACKWARD"))],
+                         ids=["3x3", "5x5", "columns"])
+def test_replaced_operations_are_called(i, names, monkeypatch):
+    """Code that wraps the operations of `adder_cuda` sees the calls of layers and of the column op."""
+    from addernetcuda_b200 import adder_cuda
+    _, call, w, shape = _calls()[i]
+    x = _rand(*shape).requires_grad_()
+    out = call(x)
+    out.backward(_rand(*out.shape, seed=1))
+    want, seen = _grads(x, w), []
+
+    def wrapped(name, fn):
+        return lambda *a, **kw: (seen.append(name), fn(*a, **kw))[1]
+    for name in names:
+        monkeypatch.setattr(adder_cuda, name, wrapped(name, getattr(adder_cuda, name)))
+    again = call(x)
+    again.backward(_rand(*out.shape, seed=1))
+    assert seen == list(names)
+    torch.testing.assert_close(again, out, rtol=1e-5, atol=1e-4)
+    for a, b in zip(_grads(x, w), want):
+        torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-4)
