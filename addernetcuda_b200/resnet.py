@@ -15,10 +15,13 @@ import math
 import numpy as np
 import torch
 import torch.nn as nn
+from torch.nn.modules import module as _nn_module
+
+from .adder import adder2d
+from .inference import FoldedBatchNorm2d
 
 
 def _default_conv():
-    from .adder import adder2d
     return adder2d
 
 
@@ -40,15 +43,23 @@ def _bn_act(bn, y, residual=None, relu=False):
     return torch.relu(out) if relu else out
 
 
+def _folds(conv, bn) -> bool:
+    """The layer and the folded batch norm behind it may run as one call, because nobody wants either's own: no hooks on the
+    two or on every module, and no forward but that of their classes."""
+    if conv.__class__.forward is not adder2d.forward or bn.__class__ is not FoldedBatchNorm2d or torch.is_grad_enabled():
+        return False
+    c, b = conv.__dict__, bn.__dict__
+    return not (c["_forward_hooks"] or c["_forward_pre_hooks"] or b["_forward_hooks"] or b["_forward_pre_hooks"] or "forward" in c
+                or "forward" in b or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks)
+
+
 def _conv_bn_act(conv, bn, x, residual=None, relu=False):
     """relu?(bn(conv(x)) + residual?).  An adder layer followed by a FusedBatchNorm2d in training mode hands
     the batch statistics over from its own epilogue, so the normalisation reads the layer's output once; one followed by a
     folded batch norm applies it in its own epilogue."""
     kind = bn.__class__.__name__
     if kind == "FoldedBatchNorm2d":
-        # hooks on either module want its own call and output
-        if not (conv._forward_hooks or conv._forward_pre_hooks or bn._forward_hooks or bn._forward_pre_hooks
-                or torch.is_grad_enabled()) and hasattr(conv, "forward_affine"):
+        if _folds(conv, bn):
             folded = bn._buffers
             z = conv.forward_affine(x, folded["scale"], folded["shift"], residual, relu)
             if z is not None:

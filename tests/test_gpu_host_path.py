@@ -136,3 +136,44 @@ def test_replaced_operations_are_called(i, names, monkeypatch):
     torch.testing.assert_close(again, out, rtol=1e-5, atol=1e-4)
     for a, b in zip(_grads(x, w), want):
         torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-4)
+
+
+def test_a_folded_network_runs_the_modules_that_someone_looks_at():
+    """A layer and the folded batch norm behind it are one call only while nothing hangs on the call of either: global hooks, hooks
+    on a module, a forward of a subclass or of an instance are seen as without that."""
+    from addernetcuda_b200 import adder, inference, resnet
+    torch.manual_seed(0)
+    net, images = resnet.resnet20().to(DEV), _rand(8, 3, 32, 32)
+    for m in net.modules():                              # statistics of these images: outputs on both sides of the ReLU
+        if isinstance(m, torch.nn.BatchNorm2d):
+            m.momentum = 1.0
+    with torch.no_grad():
+        net.train()(images)
+    inference.fold_batchnorm(net)
+    block = net.layer1[0]
+
+    class Doubled(adder.adder2d):
+        def forward(self, x):
+            return 2.0 * super().forward(x)
+
+    with torch.no_grad():
+        want = net(images)
+        assert not torch.equal(want, net(_rand(8, 3, 32, 32, seed=1)))
+        seen = []
+        hook = torch.nn.modules.module.register_module_forward_hook(lambda m, i, o: seen.append(m))
+        assert torch.equal(net(images), want)
+        hook.remove()
+        assert {m for m in net.modules() if isinstance(m, (adder.adder2d, inference.FoldedBatchNorm2d))} <= set(seen)
+        for m in (block.conv1, block.bn1):
+            hook = m.register_forward_hook(lambda m, i, o: 2.0 * o)
+            doubled = net(images)
+            assert not torch.equal(doubled, want)
+            hook.remove()
+            own = m.forward
+            m.forward = lambda *a, **kw: 2.0 * own(*a, **kw)
+            assert torch.equal(net(images), doubled)
+            del m.forward
+        block.conv1.__class__ = Doubled
+        assert not torch.equal(net(images), want)
+        block.conv1.__class__ = adder.adder2d
+        assert torch.equal(net(images), want)
