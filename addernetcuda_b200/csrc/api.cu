@@ -37,6 +37,12 @@ TileHint current_hint(int) { return TileHint(); }
 #endif
 std::atomic<unsigned long long> g_launches{0};
 
+// The fp32 kernel that the planner takes without the tensor cores (TileHint::variant).
+TileHint fp32_hint() {
+    TileHint h;
+    h.variant = 3;
+    return h;
+}
 
 // Validates a layer geometry and fills Geom.  Every tensor must have fewer than 2^31 elements
 // (the kernels index tiles with 32-bit integers and element offsets with 64-bit ones).
@@ -102,6 +108,21 @@ int ensure_dynamic_smem(const void* kernel, size_t bytes) {
         it = granted.emplace(std::make_pair(kernel, dev), (size_t)dyn).first;
     }
     return bytes <= it->second ? ADDER_OK : ADDER_ERR_UNSUPPORTED;
+}
+
+size_t backward_weight_fp32_bytes(int n, int ci, int h, int wd, int co, int k, int stride, int pad) {
+    Geom g;
+    if (make_geom(n, ci, h, wd, co, k, stride, pad, &g) != ADDER_OK) return 0;
+    if (n == 0) g.N = 1;
+    return gw_workspace_bytes(g, fp32_hint());
+}
+
+int backward_weight_fp32(const float* grad_out, const float* x, const float* w, float* grad_w, float eta, float* out_norm, void* workspace,
+                         size_t workspace_bytes, int n, int ci, int h, int wd, int co, int k, int stride, int pad, cudaStream_t stream) {
+    Geom g;
+    const int st = make_geom(n, ci, h, wd, co, k, stride, pad, &g);
+    if (st != ADDER_OK) return st;
+    return launch_gw(g, grad_out, x, w, grad_w, eta, out_norm, 0, workspace, workspace_bytes, fp32_hint(), stream);
 }
 }  // namespace adder
 

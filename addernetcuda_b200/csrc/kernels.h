@@ -123,6 +123,12 @@ int launch_gw(const Geom& g, const float* gout, const float* x, const float* w, 
               float* out_norm, int accumulate, void* workspace, size_t workspace_bytes, const TileHint& hint,
               cudaStream_t s);
 
+// The weight gradient on the fp32 kernels alone, whose slices take less scratch than the tensor-core kernel's: a size of 0 means an
+// invalid geometry, which the call reports (api.cu).
+size_t backward_weight_fp32_bytes(int n, int ci, int h, int wd, int co, int k, int stride, int pad);
+int backward_weight_fp32(const float* grad_out, const float* x, const float* w, float* grad_w, float eta, float* out_norm, void* workspace,
+                         size_t workspace_bytes, int n, int ci, int h, int wd, int co, int k, int stride, int pad, cudaStream_t stream);
+
 // Weight gradient of any geometry (tensor cores); 0 bytes: not supported
 size_t conv_gw_workspace_bytes(const ConvGeom& g);
 int launch_conv_gw(const ConvGeom& g, const float* gout, const float* x, const float* w, float* gw, float eta, void* workspace,

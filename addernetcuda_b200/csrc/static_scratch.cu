@@ -9,9 +9,10 @@
 // adder_b200_backward_weight() wants.  Those callers pass inputs and outputs only.
 //
 // Limits and sharing.  The array is ADDER_B200_STATIC_SCRATCH_BYTES (8 MiB) per GPU that loads the
-// library, held until the process exits.  A geometry whose partial sums do not fit is refused with
-// ADDER_ERR_TOO_LARGE (all 20 adder layers of ResNet-20 at batch 256 fit; the wide ResNet-50 layers
-// do not).  Every call on a device uses the same array and finds the previous call's contents in
+// library, held until the process exits.  Where the tensor-core kernel's partial sums do not fit, the fp32
+// kernels, which make fewer slices, compute the layer (128->128 28x28 at batch 8: 14.3 MB and 5.4).  A geometry
+// whose partial sums do not fit either way is refused with ADDER_ERR_TOO_LARGE (all 20 adder layers of ResNet-20
+// at batch 256 fit; the wide ResNet-50 layers do not).  Every call on a device uses the same array and finds the previous call's contents in
 // it; that is harmless, because the kernels write every scratch word they later read (each CTA
 // stores its whole slice of partial sums, including CTAs that had no pixels to process), so nothing
 // has to be cleared.  For the same reason two calls that run on the GPU at the same time (different
@@ -63,10 +64,14 @@ int adder_b200_backward_weight_static(const float* grad_out, const float* x, con
     if (need == 0)   // invalid geometry or no plan: the workspace-taking entry point reports which (it cannot launch without scratch)
         return adder_b200_backward_weight(grad_out, x, w, grad_w, eta, out_norm, nullptr, 0, n, ci, h, wd, co, k, stride,
                                           pad, 0, stream);
-    if (need > kScratchBytes) return ADDER_ERR_TOO_LARGE;
+    const bool fp32 = need > kScratchBytes;
+    if (fp32 && adder::backward_weight_fp32_bytes(n, ci, h, wd, co, k, stride, pad) > kScratchBytes) return ADDER_ERR_TOO_LARGE;
     void* scratch = nullptr;
     const int st = scratch_address(&scratch);
     if (st != ADDER_OK) return st;
+    if (fp32)
+        return adder::backward_weight_fp32(grad_out, x, w, grad_w, eta, out_norm, scratch, kScratchBytes, n, ci, h, wd, co, k, stride, pad,
+                                           static_cast<cudaStream_t>(stream));
     return adder_b200_backward_weight(grad_out, x, w, grad_w, eta, out_norm, scratch, kScratchBytes, n, ci, h, wd, co,
                                       k, stride, pad, 0, stream);
 }

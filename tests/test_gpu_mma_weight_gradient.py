@@ -62,3 +62,28 @@ def test_finish_of_the_weight_gradient(ci, co):
     assert abs(float(norm) - float(want.norm())) <= bound * float(want.norm())
     want *= 0.2 * want.numel() ** 0.5 / want.norm()
     assert float((got.double().reshape(co, -1) - want).norm()) <= 2 * bound * float(want.norm())
+
+
+@pytest.mark.parametrize("case", [(8, 128, 128, 28, 28, 3, 1, 1), (8, 256, 256, 14, 14, 3, 1, 1), (1, 128, 128, 32, 32, 3, 1, 1)],
+                         ids=lambda c: "n%d_c%dto%d_%dx%d_k%ds%dp%d" % c)
+def test_fixed_scratch_takes_layers_whose_tensor_core_slices_do_not_fit(case):
+    """The entry point with 8 MiB of its own falls back to the fp32 kernels, which need less.  K = n ho wo products added in fp32, in
+    slices that are added in double: (K + 8) u of their size (u = 2^-24) bounds the error, as below for the finish."""
+    from addernetcuda_b200 import _lib
+    n, ci, co, h, w, k, s, p = case
+    lib = _lib.load()
+    assert lib.adder_b200_backward_weight_workspace_bytes(n, ci, h, w, co, k, s, p) > lib.adder_b200_static_scratch_bytes()
+    gen = torch.Generator(device=DEV).manual_seed(n + ci)
+    x = torch.randn(n, ci, h, w, device=DEV, generator=gen)
+    wt = torch.randn(co, ci, k, k, device=DEV, generator=gen)
+    g = torch.randn(n, co, h, w, device=DEV, generator=gen)
+    got, want, size = torch.full_like(wt, 7.0), 0.0, 0.0
+    stream = torch.cuda.current_stream().cuda_stream
+    status = lib.adder_b200_backward_weight_static(g.data_ptr(), x.data_ptr(), wt.data_ptr(), got.data_ptr(), 0.0, None, n, ci, h, w, co,
+                                                   k, s, p, stream)
+    assert status == 0, status
+    for i in range(n):
+        cols, gi, w64 = F.unfold(x[i:i + 1].double(), k, padding=p)[0], g[i].double().reshape(co, -1), wt.double().reshape(co, -1)
+        want += gi @ cols.T - w64 * gi.sum(1, keepdim=True)
+        size += gi.abs() @ cols.abs().T + w64.abs() * gi.abs().sum(1, keepdim=True)
+    assert ((got.double().reshape(co, -1) - want).abs() <= (n * h * w + 8) * 2.0 ** -24 * size).all()
