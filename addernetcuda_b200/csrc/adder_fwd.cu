@@ -433,7 +433,7 @@ int describe_fwd(const Geom& layer, const TileHint& hint, char* buf, size_t n) {
     }
     if (fwd_uses_gather(layer, hint)) {
         const int w = describe_fwd_gather(conv_geom(layer), buf, n);
-        if (w < 0 || (size_t)w + 16 >= n) return ADDER_OK;
+        if (layer.k == 1 || w < 0 || (size_t)w + 16 >= n) return ADDER_OK;      // the tiled kernel has no 1x1 form
         buf += w; n -= w;
         const int w2 = snprintf(buf, n, "; tiled form: ");
         buf += w2; n -= w2;

@@ -328,11 +328,18 @@ int launch_mode(int tile, const FwdGatherArgs& a, dim3 grid, size_t smem, cudaSt
 
 }  // namespace
 
+static int fwd_mode(const ConvGeom& g, bool aligned) {
+    if (g.kh == 3 && g.kw == 3) return GATHER_NINE;
+    const bool in_order = g.kh * g.kw == 1 && g.sh == 1 && g.sw == 1 && g.ph == 0 && g.pw == 0;
+    return in_order && aligned && (g.Ho * g.Wo) % 4 == 0 ? GATHER_QUADS : GATHER_TAP;
+}
+
 int describe_fwd_gather(const ConvGeom& g, char* buf, size_t n) {
     const int P = g.N * g.Ho * g.Wo;
     const Tile& t = kTiles[choose_tile(P, g.Co)];
-    return snprintf(buf, n, "fwd gather k=%dx%d RM=%d RP=%d TC=%d TP=%d threads=%d smem=%zu grid=(%d,%d) status=0", g.kh, g.kw, t.rm,
-                    t.rp, t.tc, t.tp, GATHER_THREADS, smem_bytes(t, stage_rows(t, g.kh == 3 && g.kw == 3 ? GATHER_NINE : g.kh * g.kw == 1 ? GATHER_QUADS : GATHER_TAP)), ceil_div(P, t.tp), ceil_div(g.Co, t.tc));
+    const size_t smem = smem_bytes(t, stage_rows(t, fwd_mode(g, true)));
+    return snprintf(buf, n, "fwd gather k=%dx%d RM=%d RP=%d TC=%d TP=%d threads=%d smem=%zu grid=(%d,%d) status=%d", g.kh, g.kw, t.rm,
+                    t.rp, t.tc, t.tp, GATHER_THREADS, smem, ceil_div(P, t.tp), ceil_div(g.Co, t.tc), gather_status(ceil_div(g.Co, t.tc), smem));
 }
 
 int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* out, cudaStream_t stream, const Epilogue& ep) {
@@ -343,9 +350,7 @@ int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* 
     const bool whole_quads = (g.Ho * g.Wo) % 4 == 0;
     a.vec_w = (a.KK == 1 || (g.kh == 3 && g.kw == 3)) && (g.Ci * a.KK) % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
     a.vec_store = whole_quads && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(ep.residual)) & 15) == 0;
-    const bool quads = whole_quads && a.KK == 1 && g.sh == 1 && g.sw == 1 && g.ph == 0 && g.pw == 0 &&
-                       (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-    const int mode = g.kh == 3 && g.kw == 3 ? GATHER_NINE : quads ? GATHER_QUADS : GATHER_TAP;
+    const int mode = fwd_mode(g, (reinterpret_cast<uintptr_t>(x) & 15) == 0);
     const int tile = choose_tile(a.m.P, g.Co);
     const Tile& t = kTiles[tile];
     const int rows = stage_rows(t, mode);
@@ -356,11 +361,11 @@ int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* 
     a.nchunks = ceil_div(g.Ci, a.CK) * (mode == GATHER_NINE ? 1 : a.KK);
     if (halves) a.nchunks = ceil_div(a.nchunks, 2);
     const dim3 grid((unsigned)ceil_div(a.m.P, t.tp), (unsigned)ceil_div(g.Co, t.tc));
-    if (grid.y > 65535) return ADDER_ERR_UNSUPPORTED;
     const size_t smem = smem_bytes(t, rows);
+    if (gather_status((int)grid.y, smem) != ADDER_OK) return ADDER_ERR_UNSUPPORTED;
     if (mode == GATHER_NINE) return launch_mode<GATHER_NINE>(tile, a, grid, smem, stream);
     if (halves) return launch_mode<GATHER_HALVES>(tile, a, grid, smem, stream);
-    return quads ? launch_mode<GATHER_QUADS>(tile, a, grid, smem, stream) : launch_mode<GATHER_TAP>(tile, a, grid, smem, stream);
+    return mode == GATHER_QUADS ? launch_mode<GATHER_QUADS>(tile, a, grid, smem, stream) : launch_mode<GATHER_TAP>(tile, a, grid, smem, stream);
 }
 
 }  // namespace adder

@@ -646,8 +646,9 @@ int describe_gw_mma(const ConvGeom& g, char* buf, size_t n) {
     Plan p;
     if (!plan(g, &p)) return 0;
     const GwMmaArgs& a = p.a;
-    return snprintf(buf, n, "gw mma %s co=%d ci=%d taps=%d R=%d K=%d smem=%zu cols=%d tiles=%d splits=%d", a.stacked ? "stacked" : "split",
-                    a.cog * 8, a.cig * 8, a.taps_per_group, a.R, a.gpos, p.smem, a.tmem_cols, a.co_tiles * a.ci_tiles * a.tap_groups, a.splits);
+    return snprintf(buf, n, "gw mma %s co=%d ci=%d taps=%d R=%d K=%d threads=%d smem=%zu cols=%d grid=(%d,%d) splits=%d status=0",
+                    a.stacked ? "stacked" : "split", a.cog * 8, a.cig * 8, a.taps_per_group, a.R, a.gpos, THREADS, p.smem, a.tmem_cols,
+                    a.splits, a.co_tiles * a.ci_tiles * a.tap_groups, a.splits);
 }
 
 int launch_gw_mma(const ConvGeom& g, const float* gout, const float* x, float* part, float* gsum_part, unsigned int* ticket, int splits,

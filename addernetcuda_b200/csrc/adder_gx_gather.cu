@@ -468,13 +468,20 @@ int plan(const ConvGeom& g, int first, bool fast, GxGatherArgs& a, dim3& grid, b
 
 }  // namespace
 
+// The gradient is read pixel by pixel in order: 1x1 kernels whose class (0, 0) is the output plane.
+static bool gx_quads(const ConvGeom& g, const GxGatherArgs& a, const dim3& grid, int first, bool aligned) {
+    return g.kh == 1 && g.kw == 1 && g.ph == 0 && g.pw == 0 && a.m[0].PH == g.Ho && a.m[0].PW == g.Wo && grid.z == 1 && first == 0 &&
+           (g.Ho * g.Wo) % 4 == 0 && aligned;
+}
+
 int describe_gx_gather(const ConvGeom& g, int fast, char* buf, size_t n) {
     GxGatherArgs a;
     dim3 grid;
     bool more;
     const Tile& t = kTiles[plan(g, 0, fast != 0, a, grid, more)];
-    return snprintf(buf, n, "gx gather k=%dx%d fast=%d classes=%u RC=%d RP=%d TC=%d TP=%d threads=%d smem=%zu grid=(%u,%u) status=0",
-                    g.kh, g.kw, fast, grid.z, t.rc, t.rp, t.tc, t.tp, GATHER_THREADS, smem_bytes(t, g.kh * g.kw == 1), grid.x, grid.y);
+    const size_t smem = smem_bytes(t, gx_quads(g, a, grid, 0, true));
+    return snprintf(buf, n, "gx gather k=%dx%d fast=%d classes=%u RC=%d RP=%d TC=%d TP=%d threads=%d smem=%zu grid=(%u,%u) status=%d",
+                    g.kh, g.kw, fast, grid.z, t.rc, t.rp, t.tc, t.tp, GATHER_THREADS, smem, grid.x, grid.y, gather_status((int)grid.y, smem));
 }
 
 int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const float* w, float* gx, int fast, int accumulate,
@@ -484,7 +491,6 @@ int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const
         GxGatherArgs a;
         dim3 grid;
         const int tile = plan(g, first, fast != 0, a, grid, more);
-        if (grid.y > 65535) return ADDER_ERR_UNSUPPORTED;
         a.gout = gout; a.x = x; a.w = w; a.gx = gx; a.accumulate = accumulate;
         const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gx)) & 15) == 0;
         const bool unit = g.sh == 1 && g.sw == 1;
@@ -493,12 +499,11 @@ int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const
         a.fill_block = single_class(g) && !accumulate;
         a.fill_quads = a.fill_block && g.sh == 2 && g.sw == 2 && g.W == 2 * a.m[0].PW && g.H == 2 * a.m[0].PH && a.m[0].PW % 4 == 0 &&
                        (reinterpret_cast<uintptr_t>(gx) & 15) == 0;
-        // the gradient is read pixel by pixel in order: 1x1 kernels whose class (0, 0) is the output plane
-        const bool quads = g.kh == 1 && g.kw == 1 && g.ph == 0 && g.pw == 0 && a.m[0].PH == g.Ho && a.m[0].PW == g.Wo && grid.z == 1 && first == 0 &&
-                           (g.Ho * g.Wo) % 4 == 0 && (reinterpret_cast<uintptr_t>(gout) & 15) == 0;
+        const bool quads = gx_quads(g, a, grid, first, (reinterpret_cast<uintptr_t>(gout) & 15) == 0);
         const int rows = stage_rows(kTiles[tile], quads);
         a.CK = g.Co < rows ? g.Co : rows;      // full blocks have the cheaper staging loops, so one ragged block rather than even ones
         const size_t smem = smem_bytes(kTiles[tile], quads);
+        if (gather_status((int)grid.y, smem) != ADDER_OK) return ADDER_ERR_UNSUPPORTED;
         const int st = fast ? (quads ? launch_tile<true, true>(tile, a, grid, smem, stream) : launch_tile<true, false>(tile, a, grid, smem, stream))
                             : (quads ? launch_tile<false, true>(tile, a, grid, smem, stream) : launch_tile<false, false>(tile, a, grid, smem, stream));
         if (st != ADDER_OK) return st;

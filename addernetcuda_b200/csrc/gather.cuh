@@ -13,6 +13,7 @@
 // One barrier per chunk; large tiles keep two stages, small ones as many as hide the latency of a load.
 #pragma once
 #include "common.cuh"
+#include "../../include/adder_b200.h"
 
 namespace adder {
 
@@ -43,6 +44,9 @@ inline double tile_cost(const TileCost& t, long long tiles, int sms) {
     const double a = t.alone + t.more * (double)(p - 1), b = (double)t.share * (double)p;
     return a > b ? a : b;
 }
+
+// Whether a launch of the gathering kernels can be made: the extent of the grid and the shared memory of a CTA.
+inline int gather_status(int grid_y, size_t smem) { return grid_y > 65535 || smem > 227 * 1024 ? ADDER_ERR_UNSUPPORTED : ADDER_OK; }
 
 // Where the pixel-side operand of reduction tap (i, j) of pixel (py, px) lives in its source tensor:
 // row py*sy + oy0 + i*doy, column px*sx + ox0 + j*dox; out of bounds reads zero.  wt0 + i*dwi + j*dwj is the tap's
