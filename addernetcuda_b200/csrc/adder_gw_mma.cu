@@ -208,10 +208,11 @@ __global__ void __launch_bounds__(THREADS, 1) adder_gw_mma_kernel(const __grid_c
         const uint32_t id_main = idesc | ((uint32_t)(a.n_instr >> 3) << 17), id_sum = idesc | (2u << 17);
         const uint32_t a_hi = desc_hi((uint32_t)a.gpos * 16u), b_hi = desc_hi((uint32_t)xrows_all * 16u);
         const uint32_t ones_lo = desc_lo(smem_u32(ones)), ones_hi = desc_hi(256);
-        for (int i = 0; i < n_local; ++i) {
+        int i = 0;
+        for (; i < n_local; ++i) {
             const int s = i & 1;
-            if (!mbar_wait(&full[s], (i >> 1) & 1)) { gave_up = 1; break; }
-            if (i > 0 && i % a.drain_chunks == 0 && (!drain(i) || !mbar_wait(&drained, (i / a.drain_chunks - 1) & 1))) { gave_up = 1; break; }
+            if (!mbar_wait(&full[s], (i >> 1) & 1)) break;
+            if (i > 0 && i % a.drain_chunks == 0 && (!drain(i) || !mbar_wait(&drained, (i / a.drain_chunks - 1) & 1))) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const bool sums = (c_begin + i) % sharers == share;
             if (elect_one()) {
@@ -245,6 +246,11 @@ __global__ void __launch_bounds__(THREADS, 1) adder_gw_mma_kernel(const __grid_c
                 mma_commit(&empty[s]);
             }
             __syncwarp();
+        }
+        if (i < n_local) {
+            gave_up = 1;
+            // what was issued still reads this CTA's shared memory and writes the accumulators that it is about to free
+            if (i > 0) mbar_wait(&empty[(i - 1) & 1], ((i - 1) >> 1) & 1);
         }
     } else if constexpr (MODE == FLAT_QUADS) {
         // ---- the warps that load, split and store: a thread has four pixels of eight channels.  The reduction's order is free where no

@@ -45,7 +45,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 
 // Waits for the phase with the given parity, at most MBAR_WAIT_LIMIT polls (each poll already blocks for a
 // while inside the hardware).  Returns false when it gave up: the caller reports that and leaves.
-constexpr int MBAR_WAIT_LIMIT = 1 << 18;      // about a second
+// The limit is some 16 s: a caller that runs on gets a result from scratch that nothing wrote, so it must outlast a GPU that is shared
+// with another process in time slices.
+constexpr int MBAR_WAIT_LIMIT = 1 << 22;
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     for (int i = 0; i < MBAR_WAIT_LIMIT; ++i) {
         if (mbar_try_wait(bar, parity)) return true;

@@ -158,3 +158,11 @@ def test_imagenet_plane_rules():
     for hw in (32, 56, 28, 14):
         assert _field(_launched(1, 64, 128, hw, hw, 128, 3, 2, 1, 1), "classes") == 4
         assert _field(_launched(1, 64, 32, hw, hw, 32, 3, 2, 1, 1), "segs/thread") == 2
+
+
+def test_waits_for_the_copy_engine_outlast_a_time_slice():
+    """A kernel whose wait runs out leaves its result unwritten and a flag on the device, which a caller need not read: the bound
+    is for a copy that never lands, not for a GPU that another process has for a second (2^18 polls)."""
+    from addernetcuda_b200 import build
+    text = (build.CSRC / "tma.cuh").read_text()
+    assert int(re.search(r"MBAR_WAIT_LIMIT = 1 << (\d+);", text).group(1)) >= 22
