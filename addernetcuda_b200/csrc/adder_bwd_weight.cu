@@ -185,6 +185,12 @@ constexpr int FIN_NORM = 8;                       // elements per partial sum of
 // 3x3, 82,944 elements: 67 us with it, 58 with two launches more; 64->64, 36,864: 53 against 56).
 constexpr int FUSED_FINISH_MAX = 1 << 16;
 
+// The factor of the adaptive rescale.  A norm that is not a number stays one, as in the reference's clamp: fmaxf(nrm, 1e-12f) would
+// make 1e-12 of it and blow up what is finite of the gradient (the tensor-core kernel has no infinities: one in x or g makes NaN).
+__device__ __forceinline__ float rescale(const GwFinishArgs& a, float nrm) {
+    return a.eta * sqrtf((float)a.CoK) / (nrm < 1e-12f ? 1e-12f : nrm);
+}
+
 // gw[i] = sum_s part[s][i] - w[i] * sum_s gsum_part[s][co(i)], plus the block's partial of sum gw^2, in double
 // precision and in slice order, so the result does not depend on scheduling.  This is the form for large
 // gradients (more elements than FUSED_FINISH_MAX), whose slices are few and long: one thread per element, so a
@@ -235,7 +241,7 @@ __global__ void __launch_bounds__(1024) adder_gw_norm_kernel(const GwFinishArgs 
     if (threadIdx.x == 0) {
         const float nrm = (float)sqrt(red[0]);
         if (a.out_norm != nullptr) *a.out_norm = nrm;
-        *scale_out = a.eta * sqrtf((float)a.CoK) / fmaxf(nrm, 1e-12f);
+        *scale_out = rescale(a, nrm);
     }
 }
 
@@ -305,7 +311,7 @@ __global__ void __launch_bounds__(FIN_THREADS) adder_gw_finish_kernel(const GwFi
     if (threadIdx.x == 0 && a.out_norm != nullptr) *a.out_norm = nrm;
     if (a.eta > 0.f) {
         constexpr int DEEP = 8;
-        const float sc = a.eta * sqrtf((float)a.CoK) / fmaxf(nrm, 1e-12f);
+        const float sc = rescale(a, nrm);
         const int quads = (reinterpret_cast<uintptr_t>(a.gw) & 15) == 0 ? a.CoK / 4 : 0;
         float4* g4 = reinterpret_cast<float4*>(a.gw);
         for (int k0 = threadIdx.x; k0 < quads; k0 += DEEP * FIN_THREADS) {

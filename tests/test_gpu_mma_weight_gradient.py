@@ -87,3 +87,19 @@ def test_fixed_scratch_takes_layers_whose_tensor_core_slices_do_not_fit(case):
         want += gi @ cols.T - w64 * gi.sum(1, keepdim=True)
         size += gi.abs() @ cols.abs().T + w64.abs() * gi.abs().sum(1, keepdim=True)
     assert ((got.double().reshape(co, -1) - want).abs() <= (n * h * w + 8) * 2.0 ** -24 * size).all()
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("case", [(9, 130, 70, 15, 13, 3, 1, 1), (40, 128, 129, 9, 7, 3, 2, 1), (3, 16, 16, 8, 8, 3, 1, 1), (3, 85, 86, 8, 8, 3, 1, 1)],
+                         ids=lambda c: "n%d_c%dto%d_%dx%d_k%ds%dp%d" % c)
+def test_a_value_that_is_not_finite_does_not_blow_up_the_gradient(case, value):
+    """adder.py:78 of the reference divides by norm(p=2).clamp(min=1e-12): a norm of NaN gives NaN everywhere, one of infinity zero for
+    what is finite.  Tensor-core and fp32 kernels, finish in one launch and in three."""
+    from addernetcuda_b200 import adder_cuda as ac
+    n, ci, co, h, w, k, s, p = case
+    gen = torch.Generator(device=DEV).manual_seed(ci)
+    x = torch.randn(n, ci, h, w, device=DEV, generator=gen)
+    g = torch.randn(n, co, (h + 2 * p - k) // s + 1, (w + 2 * p - k) // s + 1, device=DEV, generator=gen)
+    x[0, 0, h // 2, w // 2] = value
+    got = ac.backward_weight(g, x, torch.randn(co, ci, k, k, device=DEV, generator=gen), s, p)
+    assert got.isnan().any() and (got[~got.isnan()] == 0).all()
