@@ -406,13 +406,26 @@ static void choose_fwd_tile(const Geom& g, const TileHint& hint, int& rw, int& r
     else if (rw == 8 && rm == 4) { CALL(KS_, S_, 8, 4) }                                    \
     else if (rw == 4 && rm == 4) { CALL(KS_, S_, 4, 4) }
 
+// Time of adder_fwd_kernel in clocks per reduction step, fitted to 430 stride-1 layers (n 1-256, 3-512 channels): within 6 % for half
+// of them.  A CTA's terms go through at 0.66 clocks per warp and term when several CTAs share an SM, slower by a share when few do; a
+// CTA whose warps do not spread evenly over the four schedulers takes as long as the fullest one.
+static double tiled_fwd_clocks(const FwdPlan& p) {
+    const int sms = sm_count(), warps = p.threads / 32;
+    const double ctas = (double)p.gx * p.gy, waves = (double)(((long long)ctas + sms - 1) / sms);
+    const double share = p.rw == 4 ? 0.72 + 0.32 / waves : 0.66 + (warps <= 4 ? 0.18 : 0.07) / waves;
+    double uneven = warps < 4 ? 4.0 / warps : ceil_div(warps, 4) * 4.0 / warps;
+    if (warps == 1) uneven *= 1.25;
+    const double cta = (double)p.rw * p.rm * warps * share;
+    return waves <= 8 ? waves * cta * uneven : ctas / sms * cta * (1 + 0.2 * (uneven - 1));      // many CTAs come and go: no waves
+}
+
 // Which layers stay with adder_fwd_kernel; every other takes the gathering kernel (adder_fwd_gather.cu), whose tile does not
 // care for the plane but which stages every tap's pixels again where this one shifts one haloed patch.  The two add in the
-// same order, so the choice does not show in the result.  The patch pays for stride-1 3x3 layers whose rows are whole
-// 8-pixel segments, with few enough output channels that staging is a large share of the work (batch 256: 16->16 32x32 47
-// against 57 us, 64->64 8x8 56 against 66; but 64->64 56x56 at batch 64: 679 against 536, 256->256 14x14: 2446 against 2128,
-// 16->32 stride 2: 36 against 30), once the launch has enough outputs to fill the SMs with such tiles (64->64 8x8: 22 against 14 us
-// at batch 32, 23 against 30 at 64).  Where batch-norm statistics are asked for, this kernel makes them in its epilogue.
+// same order, so the choice does not show in the result.  1x1 kernels and stride 2 (16->32 at batch 256: 36 against 30 us) are the
+// gathering kernel's; of the stride-1 3x3 layers each kernel takes those it is predicted to be faster on.  Over 430 drawn ones the time
+// lost against the better of the two is 0.2 % on average; 7 are more than 5 % slower than with this kernel (with a rule on channels and
+// plane before: 20, the worst 16->40 60x60 at batch 147 404 against 323 us, 416->33 10x24 at batch 241 1190 against 825).  Where
+// batch-norm statistics are asked for, this kernel makes them in its epilogue.
 static bool fwd_uses_gather(const Geom& g, const TileHint& hint) {
     if (g.k != 3) return true;
     TileHint h = hint;
@@ -420,8 +433,19 @@ static bool fwd_uses_gather(const Geom& g, const TileHint& hint) {
     if (!h.is_default()) return false;
     if (hint.variant) return hint.variant == 2;
     if (g.stride != 1) return true;
-    const bool narrow = g.Co <= 32 || (g.Co <= 64 && g.Ci <= 64 && g.H * g.W < 196);
-    return !(narrow && g.W % 8 == 0 && (long long)g.N * g.Ho * g.Wo * g.Co >= (1 << 18));
+    bool gather = true;
+    cached_plan(g, gather, [&](bool& use) {
+        int rw = 8, rm = 8;
+        choose_fwd_tile(g, hint, rw, rm);
+        FwdPlan p;
+        int st = ADDER_ERR_UNSUPPORTED;
+#define ADDER_FWD_PLAN(KS_, S_, RW_, RM_) st = plan_fwd_t<KS_, S_, RW_, RM_>(g, nullptr, hint, p);
+        ADDER_FWD_DISPATCH(ADDER_FWD_PLAN)
+#undef ADDER_FWD_PLAN
+        use = st != ADDER_OK || tiled_fwd_clocks(p) >= fwd_gather_clocks(conv_geom(g));
+        return ADDER_OK;
+    });
+    return gather;
 }
 
 int describe_fwd(const Geom& layer, const TileHint& hint, char* buf, size_t n) {

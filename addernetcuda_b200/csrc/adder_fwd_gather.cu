@@ -328,6 +328,12 @@ int launch_mode(int tile, const FwdGatherArgs& a, dim3 grid, size_t smem, cudaSt
 
 }  // namespace
 
+double fwd_gather_clocks(const ConvGeom& g) {
+    const int P = g.N * g.Ho * g.Wo;
+    const Tile& t = kTiles[choose_tile(P, g.Co)];
+    return tile_cost(t.cost, (long long)ceil_div(P, t.tp) * ceil_div(g.Co, t.tc), sm_count());
+}
+
 static int fwd_mode(const ConvGeom& g, bool aligned) {
     if (g.kh == 3 && g.kw == 3) return GATHER_NINE;
     const bool in_order = g.kh * g.kw == 1 && g.sh == 1 && g.sw == 1 && g.ph == 0 && g.pw == 0;

@@ -137,6 +137,7 @@ int launch_conv_gw(const ConvGeom& g, const float* gout, const float* x, const f
 // Channels x pixels tiles with a gathered operand (adder_fwd_gather.cu, adder_gx_gather.cu)
 int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* out, cudaStream_t s,
                       const Epilogue& ep = Epilogue());
+double fwd_gather_clocks(const ConvGeom& g);      // predicted time of its launch, in clocks per reduction step
 int describe_fwd_gather(const ConvGeom& g, char* buf, size_t n);
 int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const float* w, float* gx, int fast, int accumulate,
                      cudaStream_t s);

@@ -166,3 +166,13 @@ def test_waits_for_the_copy_engine_outlast_a_time_slice():
     from addernetcuda_b200 import build
     text = (build.CSRC / "tma.cuh").read_text()
     assert int(re.search(r"MBAR_WAIT_LIMIT = 1 << (\d+);", text).group(1)) >= 22
+
+
+def test_forward_kernel_by_predicted_time():
+    """Stride-1 3x3 forwards: the tiled kernel where it is the faster one - few input channels, or output channels that fill a
+    fraction of the gathering kernel's tiles - and the gathering kernel for wide layers, ragged planes and small launches."""
+    for shape in ((147, 16, 60, 60, 40), (241, 416, 10, 24, 33), (231, 112, 15, 57, 19), (31, 425, 62, 62, 5), (256, 16, 32, 32, 16),
+                  (256, 64, 8, 8, 64)):
+        assert "gather" not in _launched(0, *shape, 3, 1, 1), shape
+    for shape in ((64, 64, 56, 56, 64), (256, 256, 14, 14, 256), (50, 27, 29, 31, 45), (1, 16, 32, 32, 16), (1, 512, 7, 7, 512)):
+        assert "gather" in _launched(0, *shape, 3, 1, 1), shape
