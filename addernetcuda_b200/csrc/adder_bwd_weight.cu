@@ -504,15 +504,17 @@ static GwPlan plan_gw_fp32(const Geom& g, const TileHint& hint) {
 }
 
 // Which layers take the tensor cores (adder_gw_mma.cu): gradients large enough to fill an instruction of 128 rows (16->16 3x3 at
-// batch 256: 59 against 45 us for the fp32 kernel; 32->32: 44 against 50, 256->256 14x14: 560 against 1526, 1024->256 1x1: 370
-// against 765, 64->64 56x56 at batch 64: 266 against 381), on layers with enough pixels and work to cover the fixed cost of its
-// CTAs (256->256 14x14 at batch 1: 41 against 28 us; at batch 8: 58 against 82).  The warp-tile fp32 kernels keep the layers with
-// up to 64 channels on planes up to 32x32, where they are within 10-20 %: such layers sit in small networks whose training is
-// sensitive to the last bit, and keep their results.
+// batch 256: 59 against 45 us for the fp32 kernel; 256->256 14x14: 560 against 1526, 1024->256 1x1: 370 against 765, 64->64 56x56 at
+// batch 64: 266 against 381) with more than 8 output channels (304->7 32x32 at batch 40: 136 against 99, 244 against 174 beside the
+// input gradient), on layers with enough pixels and work to cover the fixed cost of its CTAs (256->256 14x14 at batch 1: 41
+// against 28 us; at batch 8: 58 against 82).  On planes up to 32x32 with up to 64 channels, where the warp-tile kernels are at their
+// best, that takes more work: with 6e8 products (64->64) 8x8 at batch 256 takes 49 against 53 us, 102 against 109 beside the input
+// gradient, but 16x16 at batch 64 49 against 52 and 157 against 123; with 1.2e9 16x16 68 against 81 and 182 against 209, with 9.7e9
+// (32x32 at batch 256) 331 against 481 and 1211 against 1341.
 static bool gw_uses_mma(const Geom& g, bool warp_tile) {
     const double cok = (double)g.Co * g.Ci * g.k * g.k, pixels = (double)g.N * g.Ho * g.Wo;
-    if (warp_tile && g.Ci <= 64 && g.Co <= 64 && g.H * g.W <= 1024) return false;
-    return cok >= 4096 && pixels >= 512 && cok * pixels >= 5e7;
+    const bool small_planes = warp_tile && g.Ci <= 64 && g.Co <= 64 && g.H * g.W <= 1024;
+    return g.Co > 8 && cok >= 4096 && pixels >= 512 && cok * pixels >= (small_planes ? 8e8 : 5e7);
 }
 
 // The fp32 kernels where the tensor-core kernel does not apply.

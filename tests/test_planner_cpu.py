@@ -176,3 +176,11 @@ def test_forward_kernel_by_predicted_time():
         assert "gather" not in _launched(0, *shape, 3, 1, 1), shape
     for shape in ((64, 64, 56, 56, 64), (256, 256, 14, 14, 256), (50, 27, 29, 31, 45), (1, 16, 32, 32, 16), (1, 512, 7, 7, 512)):
         assert "gather" in _launched(0, *shape, 3, 1, 1), shape
+
+
+def test_weight_gradient_kernel_by_size():
+    """Tensor cores: more than 8 output channels, and on small planes with few channels more work than elsewhere."""
+    for shape in ((40, 304, 32, 32, 7), (244, 112, 29, 29, 6), (64, 64, 16, 16, 64), (256, 64, 8, 8, 64)):
+        assert not _launched(2, *shape, 3, 1, 1).startswith("gw mma"), shape
+    for shape in ((40, 304, 32, 32, 9), (115, 8, 32, 32, 282), (128, 64, 16, 16, 64), (400, 64, 8, 8, 64), (64, 64, 36, 36, 64)):
+        assert _launched(2, *shape, 3, 1, 1).startswith("gw mma"), shape
