@@ -45,8 +45,9 @@ static PwArgs make_pw_args(const Geom& g) {
     return a;
 }
 
-// grid (ceil(P/256), ceil(Co/16)); CIT = input channels held in registers (Ci rounded up to 16).
-template <int CIT>
+// grid (ceil(P/256), ceil(Co/16)); CIT = input channels held in registers (Ci rounded up to 16); EP: an epilogue behind the layer (the
+// test for it, and the parameters it needs, cost 0.2 us of 3.5 on 16->32 15x20).
+template <int CIT, bool EP>
 __global__ void __launch_bounds__(PW_THREADS) adder_pw_fwd_kernel(const PwArgs a) {
     __shared__ __align__(16) float ws[CIT * PW_CT];       // [ci][co of the group]
     const int co0 = blockIdx.y * PW_CT;
@@ -81,9 +82,10 @@ __global__ void __launch_bounds__(PW_THREADS) adder_pw_fwd_kernel(const PwArgs a
     }
     const int HoWo = a.Ho * a.Wo;
     const size_t at = ((size_t)n * a.Co + co0) * HoWo + r;
+    float* o = a.out + at;
 #pragma unroll
     for (int m = 0; m < PW_CT; ++m)
-        if (co0 + m < a.Co) a.out[at + (size_t)m * HoWo] = finish(a.ep, -acc[m], co0 + m, at + (size_t)m * HoWo);
+        if (co0 + m < a.Co) o[(size_t)m * HoWo] = EP ? finish(a.ep, -acc[m], co0 + m, at + (size_t)m * HoWo) : -acc[m];
 }
 
 // grid (ceil(P/256), ceil(Ci/16)).  FAST: clamp(d,-1,1) = 2*sat(d/2 + 1/2) - 1 with w' = w/2 + 1/2 in
@@ -157,9 +159,9 @@ int launch_pointwise_fwd(const Geom& g, const float* x, const float* w, float* o
     PwArgs a = make_pw_args(g);
     a.x = x; a.w = w; a.out = out; a.ep = ep;
     const dim3 grid(ceil_div(a.P, PW_THREADS), ceil_div(g.Co, PW_CT));
-    if (g.Ci <= 16) adder_pw_fwd_kernel<16><<<grid, PW_THREADS, 0, stream>>>(a);
-    else if (g.Ci <= 32) adder_pw_fwd_kernel<32><<<grid, PW_THREADS, 0, stream>>>(a);
-    else adder_pw_fwd_kernel<64><<<grid, PW_THREADS, 0, stream>>>(a);
+    auto kern = ep.scale != nullptr ? (g.Ci <= 16 ? adder_pw_fwd_kernel<16, true> : g.Ci <= 32 ? adder_pw_fwd_kernel<32, true> : adder_pw_fwd_kernel<64, true>)
+                                    : (g.Ci <= 16 ? adder_pw_fwd_kernel<16, false> : g.Ci <= 32 ? adder_pw_fwd_kernel<32, false> : adder_pw_fwd_kernel<64, false>);
+    kern<<<grid, PW_THREADS, 0, stream>>>(a);
     return launched();
 }
 
