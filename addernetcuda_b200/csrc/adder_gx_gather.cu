@@ -35,6 +35,7 @@ struct GxGatherArgs {
     int vec_io;              // stride 1, planes are whole quads, x and gx 16-byte aligned
     int fill_block;          // the other pixels of an sh x sw block belong to no class: write zeros there
     int fill_quads;          // ... and four blocks of a row can be written as aligned 128-bit words
+    int fill_pairs;          // ... or, rows being even, each block as two aligned 64-bit words
 };
 
 // RC channels x RP pixels per thread (RP = 8: two quads half a tile apart), CG channel groups, ST stages, MB CTAs per SM.
@@ -325,6 +326,26 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
                 continue;
             }
         }
+        if (a.fill_pairs) {                      // stride 2, pixels of class (0, 0) only, rows of an even length
+#pragma unroll 1
+            for (int j = 0; j < PQ && p + j < m.P; ++j) {
+                uint32_t n, r, y, x;
+                m.d_phw.divmod(p + j, n, r);
+                m.d_pw.divmod(r, y, x);
+                float* o = a.gx + ((size_t)n * a.Ci + ci0 + cg * RC) * HW + 2 * y * a.W + 2 * x;
+                const bool below = 2 * (int)y + 1 < a.H;
+#pragma unroll
+                for (int c = 0; c < RC; ++c) {
+                    if (ci0 + cg * RC + c >= a.Ci) break;
+                    float v = acc[c][PQ * h];
+#pragma unroll
+                    for (int q = 1; q < PQ; ++q) v = j == q ? acc[c][PQ * h + q] : v;
+                    *reinterpret_cast<float2*>(o + (size_t)c * HW) = make_float2(v, 0.f);
+                    if (below) *reinterpret_cast<float2*>(o + (size_t)c * HW + a.W) = make_float2(0.f, 0.f);
+                }
+            }
+            continue;
+        }
 #pragma unroll
         for (int j = 0; j < PQ; ++j) {
             if (p + j >= m.P) continue;
@@ -499,6 +520,8 @@ int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const
         a.fill_block = single_class(g) && !accumulate;
         a.fill_quads = a.fill_block && g.sh == 2 && g.sw == 2 && g.W == 2 * a.m[0].PW && g.H == 2 * a.m[0].PH && a.m[0].PW % 4 == 0 &&
                        (reinterpret_cast<uintptr_t>(gx) & 15) == 0;
+        // (planes of an odd height keep an even number of values, so that every plane starts aligned)
+        a.fill_pairs = a.fill_block && !a.fill_quads && g.sh == 2 && g.sw == 2 && g.W % 2 == 0 && (reinterpret_cast<uintptr_t>(gx) & 7) == 0;
         const bool quads = gx_quads(g, a, grid, first, (reinterpret_cast<uintptr_t>(gout) & 15) == 0);
         const int rows = stage_rows(kTiles[tile], quads);
         a.CK = g.Co < rows ? g.Co : rows;      // full blocks have the cheaper staging loops, so one ragged block rather than even ones

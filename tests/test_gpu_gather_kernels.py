@@ -20,6 +20,7 @@ CASES = [(1, 16, 16, 32, 32, 3, 1, 1), (1, 5, 7, 5, 5, 3, 1, 1), (1, 66, 67, 8, 
          (2, 27, 45, 29, 31, 3, 1, 1), (6, 130, 129, 14, 14, 3, 1, 1), (40, 65, 70, 15, 13, 3, 2, 1), (2, 64, 72, 16, 16, 3, 2, 1),
          (1, 33, 36, 4, 4, 1, 1, 0), (3, 70, 130, 12, 12, 1, 1, 0), (20, 100, 260, 11, 11, 1, 1, 0), (2, 64, 96, 28, 28, 1, 2, 0),
          (3, 40, 33, 13, 15, 1, 2, 0), (300, 3, 20, 20, 20, 3, 1, 1), (64, 160, 24, 28, 28, 1, 1, 0), (2, 9, 12, 17, 19, 5, 1, 2),
+         (3, 40, 16, 14, 14, 1, 2, 0), (3, 40, 16, 13, 14, 1, 2, 0), (2, 70, 16, 34, 34, 1, 2, 0),
          (1, 6, 33, 23, 30, 3, 4, 1), (2, 20, 18, 12, 16, 2, 2, 0), (1, 3, 40, 33, 33, 7, 2, 3)]
 
 
