@@ -177,3 +177,22 @@ def test_a_folded_network_runs_the_modules_that_someone_looks_at():
         assert not torch.equal(net(images), want)
         block.conv1.__class__ = adder.adder2d
         assert torch.equal(net(images), want)
+
+
+def test_wide_strides_go_through_columns():
+    """Strides whose input gradient is nearly all zeros: same results, from the path that is faster on them."""
+    from addernetcuda_b200 import _native, adder
+    for stride, native in ((16, True), (25, False), ((1, 601), False)):
+        layer = adder.adder2d(3, 4, 2, stride=stride).to(DEV)
+        sh, sw = (stride, stride) if isinstance(stride, int) else stride
+        x = _rand(2, 3, 40, 320 if sw < 320 else 620).requires_grad_()
+        assert (_native.conv(x, layer.adder, sh, sw, 0, 0, 1, 1) is not None) == native
+        out = layer(x)
+        g = _rand(*out.shape, seed=1)
+        out.backward(g)
+        cols = torch.nn.functional.unfold(x.detach().double(), 2, stride=stride).requires_grad_()
+        d = layer.adder.detach().double().reshape(4, 12, 1) - cols[:, None]
+        torch.testing.assert_close(out.double().reshape(2, 4, -1), -d.abs().sum(2), rtol=1e-5, atol=1e-5)
+        gc = (d.clamp(-1, 1) * g.double().reshape(2, 4, 1, -1)).sum(1)
+        want = torch.nn.functional.fold(gc.detach(), x.shape[2:], 2, stride=stride)
+        torch.testing.assert_close(x.grad.double(), want, rtol=1e-5, atol=1e-5)
