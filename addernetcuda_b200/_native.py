@@ -9,6 +9,7 @@ from __future__ import annotations
 import ctypes
 import importlib.util
 import sys
+import warnings
 
 import torch
 
@@ -23,19 +24,37 @@ _mod = None
 
 
 def load() -> None:
-    """Load the extension (built first if necessary), bind it to the product library and put its entry points in place."""
+    """Load the extension (built first if it is missing or was linked with another torch), bind it to the product library and put
+    its entry points in place.  Where that fails, callers get None and a warning: the Python layer needs the library alone."""
     global _mod
     if _mod is None:
-        from . import build
-        if not build.HOST_LIB.exists():
-            build.build()
-        spec = importlib.util.spec_from_file_location("_adder_host", build.HOST_LIB)
-        mod = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(mod)
+        mod = _import()
+        if mod is None:
+            for name in _ENTRIES:
+                globals()[name] = _absent
+            return
         _mod = mod
         for name in _ENTRIES:
             globals()[name] = getattr(mod, name)
     sync()
+
+
+def _import():
+    from . import build
+    if not build.host_usable() and not build.build_host():
+        return None
+    spec = importlib.util.spec_from_file_location("_adder_host", build.HOST_LIB)
+    try:
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+    except ImportError as e:
+        warnings.warn(f"{build.HOST_LIB.name} does not load ({e}): eager layer calls go through the Python layer")
+        return None
+    return mod
+
+
+def _absent(*args):
+    return None
 
 
 def sync() -> None:

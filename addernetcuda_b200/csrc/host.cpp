@@ -522,4 +522,13 @@ PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_adder_host", nullptr, -1, met
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__adder_host() { return PyModule_Create(&module_def); }
+#ifndef ADDER_HOST_MARK
+#define ADDER_HOST_MARK ""
+#endif
+
+// The mark says which torch this file was linked with; build.py looks for it before it is loaded.
+PyMODINIT_FUNC PyInit__adder_host() {
+    PyObject* m = PyModule_Create(&module_def);
+    if (m != nullptr) PyModule_AddStringConstant(m, "built_for", ADDER_HOST_MARK);
+    return m;
+}

@@ -162,3 +162,30 @@ def test_host_extension_runs_on_torchs_cxx_runtime():
     image = build.HOST_LIB.read_bytes()
     assert b"\0libstdc++.so.6\0" in image and b"\0_ZNSolsEi\0" in image      # needed, and operator<<(int) among its imports
     assert b"locale::facet::_S_create_c_locale name not valid" not in image  # a text of the runtime itself
+
+
+def test_a_missing_host_extension_costs_speed_only(monkeypatch, tmp_path):
+    """No compiler, no header, another torch: a warning, entry points that return None (callers go on in Python), and no file
+    where one is half written.  The C library does not depend on any of it."""
+    from addernetcuda_b200 import _native, build
+    kept = {n: getattr(_native, n) for n in (*_native._ENTRIES, "_mod")}
+    try:
+        monkeypatch.setattr(_native, "_mod", None)
+        monkeypatch.setattr(build, "HOST_LIB", tmp_path / "_adder_host.so")
+        monkeypatch.setenv("CXX", str(tmp_path / "no-compiler"))
+        assert not build.host_usable()
+        with pytest.warns(UserWarning, match="not built"):
+            _native.load()
+        assert all(getattr(_native, n)(None, None) is None for n in _native._ENTRIES) and _native._mod is None
+        build.HOST_LIB.write_bytes(b"linked with something else")
+        assert not build.host_usable()                   # another torch: built again, not loaded
+        build.HOST_LIB.write_bytes(build._host_mark().encode())
+        with pytest.warns(UserWarning, match="does not load"):
+            _native.load()
+        monkeypatch.setenv("CXX", "false")               # a compiler that fails
+        with pytest.warns(UserWarning, match="not built"):
+            assert not build.build_host()
+        assert [p.name for p in tmp_path.iterdir()] == ["_adder_host.so"]
+    finally:
+        for n, v in kept.items():
+            setattr(_native, n, v)
