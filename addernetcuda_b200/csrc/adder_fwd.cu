@@ -531,7 +531,7 @@ int fwd_stat_slices(const Geom& layer, const TileHint& hint) {
     if (hint.is_default() && pointwise_applicable(g)) return 0;
     int rw = 8, rm = 8;
     choose_fwd_tile(g, hint, rw, rm);
-    if (stats_apart(layer, hint)) return segment_stat_slices(g, rw);
+    if (stats_apart(layer, hint)) return g.Co <= 65535 ? segment_stat_slices(g, rw) : 0;      // a row of blocks per channel
     FwdPlan p;
     int st = ADDER_ERR_UNSUPPORTED;
 #define ADDER_FWD_PLAN(KS_, S_, RW_, RM_) st = plan_fwd_t<KS_, S_, RW_, RM_>(g, nullptr, hint, p);

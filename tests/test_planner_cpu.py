@@ -184,3 +184,11 @@ def test_weight_gradient_kernel_by_size():
         assert not _launched(2, *shape, 3, 1, 1).startswith("gw mma"), shape
     for shape in ((40, 304, 32, 32, 9), (115, 8, 32, 32, 282), (128, 64, 16, 16, 64), (400, 64, 8, 8, 64), (64, 64, 36, 36, 64)):
         assert _launched(2, *shape, 3, 1, 1).startswith("gw mma"), shape
+
+
+def test_statistics_pass_has_a_row_of_blocks_per_channel():
+    """Beyond the rows of a grid there are no fused statistics (the batch norm reads the output itself), not a launch that fails."""
+    lib = _lib.load()
+    for co, some in ((65535, True), (65536, False)):
+        assert (lib.adder_b200_forward_stat_slices(8, 4, 3, 3, co, 1, 1, 0) > 0) == some
+        assert (lib.adder_b200_forward_stat_slices(8, 128, 3, 3, co, 3, 1, 1) > 0) == some
