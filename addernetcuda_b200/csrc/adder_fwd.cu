@@ -407,7 +407,7 @@ static void choose_fwd_tile(const Geom& g, const TileHint& hint, int& rw, int& r
     else if (rw == 4 && rm == 4) { CALL(KS_, S_, 4, 4) }
 
 // Time of adder_fwd_kernel in clocks per reduction step, fitted to 430 stride-1 layers (n 1-256, 3-512 channels): within 6 % for half
-// of them.  A CTA's terms go through at 0.66 clocks per warp and term when several CTAs share an SM, slower by a share when few do; a
+// of those, and of 1400 others.  A CTA's terms go through at 0.66 clocks per warp and term when several CTAs share an SM, slower by a share when few do; a
 // CTA whose warps do not spread evenly over the four schedulers takes as long as the fullest one.
 static double tiled_fwd_clocks(const FwdPlan& p) {
     const int sms = sm_count(), warps = p.threads / 32;
@@ -416,15 +416,15 @@ static double tiled_fwd_clocks(const FwdPlan& p) {
     double uneven = warps < 4 ? 4.0 / warps : ceil_div(warps, 4) * 4.0 / warps;
     if (warps == 1) uneven *= 1.25;
     const double cta = (double)p.rw * p.rm * warps * share;
-    return waves <= 8 ? waves * cta * uneven : ctas / sms * cta * (1 + 0.2 * (uneven - 1));      // many CTAs come and go: no waves
+    return waves <= 8 ? waves * cta * uneven : ctas / sms * cta * (1.04 + 0.2 * (uneven - 1));      // many CTAs come and go: no waves
 }
 
 // Which layers stay with adder_fwd_kernel; every other takes the gathering kernel (adder_fwd_gather.cu), whose tile does not
 // care for the plane but which stages every tap's pixels again where this one shifts one haloed patch.  The two add in the
 // same order, so the choice does not show in the result.  1x1 kernels and stride 2 (16->32 at batch 256: 36 against 30 us) are the
-// gathering kernel's; of the stride-1 3x3 layers each kernel takes those it is predicted to be faster on.  Over 430 drawn ones the time
-// lost against the better of the two is 0.2 % on average; 7 are more than 5 % slower than with this kernel (with a rule on channels and
-// plane before: 20, the worst 16->40 60x60 at batch 147 404 against 323 us, 416->33 10x24 at batch 241 1190 against 825).  Where
+// gathering kernel's; of the stride-1 3x3 layers each kernel takes those it is predicted to be faster on.  Over 1400 drawn ones the
+// time lost against the better of the two is 0.23 % on average; 15 are more than 5 % slower than with this kernel (20 of 430 with a rule
+// on channels and plane before, the worst 16->40 60x60 at batch 147 404 against 323 us, 416->33 10x24 at batch 241 1190 against 825).  Where
 // batch-norm statistics are asked for, this kernel makes them in its epilogue.
 static bool fwd_uses_gather(const Geom& g, const TileHint& hint) {
     if (g.k != 3) return true;

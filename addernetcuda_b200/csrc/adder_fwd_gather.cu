@@ -267,7 +267,7 @@ namespace {
     X(8, 8, 8, 2, 4, 242, 147, 173) X(8, 8, 16, 2, 4, 241, 74, 186) X(8, 8, 4, 2, 4, 278, 130, 186)                 \
     X(4, 8, 16, 3, 4, 139, 65, 93) X(4, 8, 8, 3, 4, 139, 65, 93) X(4, 8, 4, 2, 4, 174, 76, 109)                     \
     X(4, 4, 16, 4, 6, 92, 30, 54) X(4, 4, 8, 4, 6, 92, 30, 54) X(4, 4, 4, 4, 6, 101, 22, 56)                        \
-    X(2, 8, 4, 3, 6, 110, 40, 60) X(2, 2, 8, 4, 8, 35, 10, 20) X(2, 2, 4, 4, 6, 38, 12, 23) X(1, 1, 4, 6, 8, 16, 9, 11)
+    X(2, 8, 4, 3, 6, 110, 75, 81) X(2, 2, 8, 4, 8, 35, 10, 20) X(2, 2, 4, 4, 6, 38, 12, 23) X(1, 1, 4, 6, 8, 16, 9, 11)
 
 struct Tile { int rm, rp, cg, st, mb, tc, tp; TileCost cost; };
 constexpr Tile kTiles[] = {
