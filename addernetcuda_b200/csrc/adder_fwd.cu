@@ -407,8 +407,8 @@ static void choose_fwd_tile(const Geom& g, const TileHint& hint, int& rw, int& r
     else if (rw == 4 && rm == 4) { CALL(KS_, S_, 4, 4) }
 
 // Time of adder_fwd_kernel in clocks per reduction step, fitted to 430 stride-1 layers (n 1-256, 3-512 channels): within 6 % for half
-// of those, and of 1400 others.  A CTA's terms go through at 0.66 clocks per warp and term when several CTAs share an SM, slower by a share when few do; a
-// CTA whose warps do not spread evenly over the four schedulers takes as long as the fullest one.
+// of those, and of 1400 others.  A CTA's terms go through at 0.66 clocks per warp and term when several CTAs share an SM, slower by a
+// share when few do; a CTA whose warps do not spread evenly over the four schedulers takes as long as the fullest one.
 static double tiled_fwd_clocks(const FwdPlan& p) {
     const int sms = sm_count(), warps = p.threads / 32;
     const double ctas = (double)p.gx * p.gy, waves = (double)(((long long)ctas + sms - 1) / sms);

@@ -176,6 +176,10 @@ def test_forward_kernel_by_predicted_time():
         assert "gather" not in _launched(0, *shape, 3, 1, 1), shape
     for shape in ((64, 64, 56, 56, 64), (256, 256, 14, 14, 256), (50, 27, 29, 31, 45), (1, 16, 32, 32, 16), (1, 512, 7, 7, 512)):
         assert "gather" in _launched(0, *shape, 3, 1, 1), shape
+    # the 2x8 tile of 8 channels only where nothing better fits (it cost half of what it takes)
+    for shape in ((256, 32, 16, 16, 21), (80, 64, 30, 30, 24), (72, 24, 38, 38, 24)):
+        plan = _launched(0, *shape, 3, 1, 1)
+        assert not (_field(plan, "RM") == 2 and _field(plan, "RP") == 8), plan
 
 
 def test_weight_gradient_kernel_by_size():
