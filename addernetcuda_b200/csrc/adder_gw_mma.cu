@@ -3,12 +3,17 @@
 // (grad_w = part - w * gsum; the finish kernels of adder_bwd_weight.cu add the slices, as for the fp32 kernels).
 //
 // This is a matrix product whose reduction runs over pixels, so it belongs on the tensor cores, but it must keep fp32
-// accuracy.  Every value is split exactly into three bf16 numbers, v = v1 + v2 + v3 (8 bits of significand each, 24
-// together), and the products v_i * u_j with i + j <= 4 are accumulated in fp32 in tensor memory: what is dropped is below
-// 2^-25 of a product, less than the rounding of one fp32 multiplication.  The tensor core rounds its running sums toward
-// zero, which loses about 1.3e-8 of a sum per accumulation (measured), so the leading products v1*u1 have an accumulator of their
-// own, and after every 16 accumulations it is moved into fp32 registers (rounded to nearest) and cleared.  The others are 2^-8
-// smaller and stay.  Against float64 the result is as close as the fp32 kernels' (1e-7 to 4e-7).
+// accuracy.  Every value is split into three bf16 numbers, v = v1 + v2 + v3 (8 bits of significand each, 24 together; exact for
+// magnitudes from 2^-110 up to the largest bf16, 3.39e38 - smaller values lose bits of v3, larger ones and infinities become
+// NaN).  The split form accumulates the products v_i * u_j with i + j <= 4 in fp32 in tensor memory: what it drops, v2*u3 + v3*u2 +
+// v3*u3, is at most 2^-24 of a product, about one fp32 rounding; the stacked form drops nothing.  The tensor core rounds its
+// running sums toward zero, which loses about 1.3e-8 of a sum per accumulation (measured), so the leading products v1*u1 have an
+// accumulator of their own, and after every 16 accumulations it is moved into fp32 registers (rounded to nearest) and cleared.  The
+// others are 2^-8 smaller and stay.  Against float64 the result is as close as the fp32 kernels' (1e-7 to 4e-7).
+//
+// What bounds it: the loading warps' turn, not a pipe.  On 256->256 14x14 at batch 384 (832 us) the tensor pipe is active 39 % of the
+// cycles, issue slots 38 %, the shared-memory pipe 10 %; the warps wait for their loads and for the conversion's chain of
+// dependent instructions, 11 of them an SM.  Each value is read and split by every CTA that shares it (x six times there, g twelve).
 //
 // Operands.  Threads read x and g in fp32 (eight channels of one pixel each; neighbouring lanes take neighbouring pixels), split
 // them and store 16-byte rows of 8 channels: shared memory holds [split][channel group of 8][position] rows, the

@@ -5,11 +5,11 @@
 //
 // A CTA of 128 threads owns TC channels x TP pixels; pixels run over the whole batch (image, row, column), so
 // no plane size leaves a ragged tile behind.  A chunk of the reduction is one shared-memory stage:
-//   GATHER_TAP    at most 16 channels of one tap (index order: channel block, tap, channel in the block), so that a
-//                 thread computes the address and the bounds test of its pixel once per chunk;
-//   GATHER_QUADS  the same for 1x1 layers whose operand is read in order: 16-byte copies;
-//   GATHER_HALVES two such blocks in one stage of a thin tile;
-//   GATHER_NINE   2 channels x the 9 taps of a 3x3 window, in index order (channel, row, column).
+//   GATHER_TAP    16 channels of one tap (index order: channel block, tap, channel in the block), so that a thread computes the
+//                 address and the bounds test of its pixel once per chunk (32 of a 1x1 layer in the thin tiles);
+//   GATHER_HALVES two blocks of 16 channels and one tap each in one stage of a thin tile;
+//   GATHER_QUADS  1x1 layers whose operand is read in order: 16-byte copies, 16 or 32 channels;
+//   GATHER_NINE   2 channels (4 in the thin tiles) x the 9 taps of a 3x3 window, in index order (channel, row, column).
 // One barrier per chunk; large tiles keep two stages, small ones as many as hide the latency of a load.
 #pragma once
 #include "common.cuh"

@@ -133,8 +133,12 @@ c10::cuda::CUDAStream side_stream(c10::DeviceIndex dev) {
 }
 
 // Both gradients; with `overlap` the weight gradient runs on a side stream beside the input gradient.
-// Below about 150 M terms the kernels (10-25 us each) gain nothing from running side by side and the events cost 6 us of host time;
-// inside a graph capture they cost nothing.
+// What that gives depends on what else runs.  Among other passes (250 drawn layers) it saves 4 % from 1.5e8 to 2.5e8 terms, 2 % up to
+// 1e9, less above.  A pass that is waited for gains or loses: where the input gradient is one long chain on few CTAs, the weight
+// gradient's CTAs, each of which fills an SM, may take the SMs first and leave it crowded on the rest (256->256 14x14 at batch 2:
+// 356 us, 200 one after the other; the other order loses as much on 256->512 14x14 stride 2 at batch 4, 596 against 250).  Below 1.5e8
+// terms one after the other is the faster on average there, and the events cost 6 us of host time; inside a graph capture they
+// cost nothing.
 constexpr double OVERLAP_TERMS = 1.5e8;
 
 template <class Input, class Weight>
