@@ -24,15 +24,12 @@
 #include "patch_fill.cuh"
 #include <cstdio>
 
-#ifndef GX_PACKED
-#define GX_PACKED 1
-#endif
 namespace adder {
 
 template <bool FAST>
 __device__ __forceinline__ float gx_term(float wv, float xv) {
     if (FAST) return __saturatef(wv + xv);                 // wv = w/2+1/2, xv = -x/2
-    return clamp_unit(wv - xv);
+    return clamp_unit(wv + xv);                            // xv = -x
 }
 
 // Stride-2 taps of one output channel for a thread whose pixels have row phase PH = (y+pad) mod 2 and
@@ -168,7 +165,8 @@ __global__ void __launch_bounds__(256, MB) adder_gx_kernel(const GxArgs a) {
     const int q0 = wq0 + ws * RW;                  // class-pixel index of the thread's first pixel
     const int HW = a.g.H * a.g.W;
 
-    constexpr bool PACKED = GX_PACKED && FAST && S == 1 && (RC % 2 == 0);
+    constexpr bool PACKED = S == 1;                // sums of two channels in one register pair
+    static_assert(RC % 2 == 0, "pairs of channels");
     float xv[RC][RW];
     float acc[RC][RW];
     uint64_t acc2[RC / 2][RW];
@@ -187,10 +185,10 @@ __global__ void __launch_bounds__(256, MB) adder_gx_kernel(const GxArgs a) {
             for (int j = 0; j < RW; j += 4) {
                 float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (okr && q0 + j < a.g.W) v = __ldg(reinterpret_cast<const float4*>(xr + j));
-                xv[c][j] = FAST ? -0.5f * v.x : v.x;
-                xv[c][j + 1] = FAST ? -0.5f * v.y : v.y;
-                xv[c][j + 2] = FAST ? -0.5f * v.z : v.z;
-                xv[c][j + 3] = FAST ? -0.5f * v.w : v.w;
+                xv[c][j] = FAST ? -0.5f * v.x : -v.x;
+                xv[c][j + 1] = FAST ? -0.5f * v.y : -v.y;
+                xv[c][j + 2] = FAST ? -0.5f * v.z : -v.z;
+                xv[c][j + 3] = FAST ? -0.5f * v.w : -v.w;
             }
 #pragma unroll
             for (int j = 0; j < RW; ++j) acc[c][j] = 0.f;
@@ -201,7 +199,7 @@ __global__ void __launch_bounds__(256, MB) adder_gx_kernel(const GxArgs a) {
             const int wi = (q0 + j) * S + pw;
             const bool ok = active && n < a.g.N && ci < a.g.Ci && hi < a.g.H && wi < a.g.W;
             const float v = ok ? __ldg(a.x + ((size_t)(n * a.g.Ci + ci) * a.x_plane + hi * a.x_row + wi * a.samp)) : 0.f;
-            xv[c][j] = FAST ? -0.5f * v : v;
+            xv[c][j] = FAST ? -0.5f * v : -v;
             acc[c][j] = 0.f;
         }
     }
@@ -260,33 +258,29 @@ __global__ void __launch_bounds__(256, MB) adder_gx_kernel(const GxArgs a) {
                     for (int kh = 0; kh < KS; ++kh, gr -= a.pd.PITCH) {
                         float gv[RW + KS - 1];
                         load_run<RW + KS - 1, (RW % 4 == 0)>(gv, gr);
-                        if constexpr (PACKED) {
-                            // two channels per fused multiply-add: (s0, s1) * (g, g) + (acc0, acc1)
-                            uint64_t g2[RW + KS - 1];
+                        // two channels per fused multiply-add: (s0, s1) * (g, g) + (acc0, acc1)
+                        uint64_t g2[RW + KS - 1];
 #pragma unroll
-                            for (int i = 0; i < RW + KS - 1; ++i) g2[i] = pack2(gv[i], gv[i]);
-#pragma unroll
-                            for (int kw = 0; kw < KS; ++kw) {
-                                const float4 t = *reinterpret_cast<const float4*>(wch + (kh * KS + kw) * RC);
-                                const float wv[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-                                for (int cc = 0; cc < RC; cc += 2)
-#pragma unroll
-                                    for (int j = 0; j < RW; ++j)
-                                        acc2[cc / 2][j] = fma2(pack2(gx_term<true>(wv[cc], xv[cc][j]), gx_term<true>(wv[cc + 1], xv[cc + 1][j])),
-                                                               g2[j + KS - 1 - kw], acc2[cc / 2][j]);
-                            }
-                        } else {
+                        for (int i = 0; i < RW + KS - 1; ++i) g2[i] = pack2(gv[i], gv[i]);
 #pragma unroll
                         for (int kw = 0; kw < KS; ++kw) {
                             const float4 t = *reinterpret_cast<const float4*>(wch + (kh * KS + kw) * RC);
                             const float wv[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
-                            for (int cc = 0; cc < RC; ++cc)
+                            for (int cc = 0; cc < RC; cc += 2)
 #pragma unroll
-                                for (int j = 0; j < RW; ++j)
-                                    acc[cc][j] = fmaf(gx_term<FAST>(wv[cc], xv[cc][j]), gv[j + KS - 1 - kw], acc[cc][j]);
-                        }
+                                for (int j = 0; j < RW; ++j) {
+                                    float s0, s1;
+                                    if constexpr (FAST) {
+                                        s0 = gx_term<true>(wv[cc], xv[cc][j]);
+                                        s1 = gx_term<true>(wv[cc + 1], xv[cc + 1][j]);
+                                    } else {         // (one packed subtraction: 16->16 32x32 at batch 256 74.3 -> 65.2 us, 64->64 8x8 83.3 -> 78.0)
+                                        unpack2(add2(pack2(wv[cc], wv[cc + 1]), pack2(xv[cc][j], xv[cc + 1][j])), s0, s1);
+                                        s0 = clamp_unit(s0);
+                                        s1 = clamp_unit(s1);
+                                    }
+                                    acc2[cc / 2][j] = fma2(pack2(s0, s1), g2[j + KS - 1 - kw], acc2[cc / 2][j]);
+                                }
                         }
                     }
                 } else if constexpr (S == 2 && RC == 4) {
@@ -519,7 +513,7 @@ __global__ void __launch_bounds__(256, 2) adder_gx_s2pair_kernel(const GxArgs a)
                 const int wi = (q0 + j) * S + pwv[sg];
                 const bool ok = active && n < a.g.N && ci < a.g.Ci && hiv[sg] < a.g.H && wi < a.g.W;
                 const float v = ok ? __ldg(a.x + ((size_t)(n * a.g.Ci + ci) * HW + hiv[sg] * a.g.W + wi)) : 0.f;
-                xv[sg][c][j] = FAST ? -0.5f * v : v;
+                xv[sg][c][j] = FAST ? -0.5f * v : -v;
                 acc[sg][c][j] = 0.f;
             }
         }

@@ -9,8 +9,8 @@
 // clamp(d,-1,1) = 2*sat(d/2 + 1/2) - 1, and the "-1" is the sum of g over the taps, added up once per pixel while the
 // stages pass by: in four partial sums, of rows r, r + 4, r + 8 and r + 12 of every 16, whichever threads share the pixel, so that
 // the tile - which follows the size of the batch - does not show in the result.  Exact form: min.xorsign.abs is the clamp in one instruction (magnitude min(|d|, 1), sign of d),
-// where fminf(fmaxf(d, -1), 1) takes two; the sums are packed pairs of pixels.
-// Both are bound by the register operands they read (5 a term, 2 a cycle and scheduler): 2.6 and 3.4 lane cycles a term
+// where fminf(fmaxf(d, -1), 1) takes two; differences (large tiles) and sums are packed pairs of pixels.
+// Both are bound by the register operands they read (5 a term, 2 a cycle and scheduler): 2.5 and 3.0 lane cycles a term
 // with nothing around them.
 #include <cstdio>
 #include "common.cuh"
@@ -196,7 +196,21 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
                 for (int r = 0; r < RC; ++r)
 #pragma unroll
                     for (int j = 0; j < RP; ++j) acc[r][j] = fmaf(__saturatef(fmaf(wv[r], 0.5f, xv[r][j])), gv[j], acc[r][j]);
-            } else {
+            } else if constexpr (RP == 8 && CG >= 8) {
+                // both steps of a pair of pixels packed but the clamp: 2.97 lane-clocks a term with nothing around it, 3.31 with a scalar
+                // subtraction (1024->256 14x14 at batch 256: 1308 -> 1179 us)
+#pragma unroll
+                for (int r = 0; r < RC; ++r) {
+                    const uint64_t w2 = pack2(wv[r], wv[r]);
+#pragma unroll
+                    for (int j = 0; j < RP; j += 2) {
+                        float d0, d1;
+                        unpack2(add2(w2, pack2(xv[r][j], xv[r][j + 1])), d0, d1);
+                        const uint64_t s = fma2(pack2(clamp_unit(d0), clamp_unit(d1)), pack2(gv[j], gv[j + 1]), pack2(acc[r][j], acc[r][j + 1]));
+                        unpack2(s, acc[r][j], acc[r][j + 1]);
+                    }
+                }
+            } else {                             // (small launches are a chain of latencies: a packed operation is the longer one)
 #pragma unroll
                 for (int j = 0; j < RP; j += 2)
 #pragma unroll
