@@ -30,6 +30,8 @@ SIGNATURES = {
     "adder_b200_output_size": (c_int, [c_int, c_int, c_int, c_int, c_int, POINTER(c_int), POINTER(c_int)]),
     "adder_b200_forward": (c_int, [c_void_p, c_void_p, c_void_p, *_GEOM, c_void_p]),
     "adder_b200_backward_input": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, *_GEOM, c_int, c_void_p]),
+    "adder_b200_backward_input_workspace_bytes": (c_size_t, [*_GEOM]),
+    "adder_b200_backward_input_with_workspace": (c_int, [c_void_p] * 5 + [c_size_t, *_GEOM, c_int, c_void_p]),
     "adder_b200_backward_weight_workspace_bytes": (c_size_t, [*_GEOM]),
     "adder_b200_backward_weight": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p,
                                            c_size_t, *_GEOM, c_int, c_void_p]),
@@ -57,6 +59,8 @@ SIGNATURES = {
     "adder_b200_affine_forward": (c_int, [c_void_p] * 5 + [c_int, c_int, c_int, c_int, c_void_p]),
     "adder_b200_conv_forward": (c_int, [c_void_p] * 3 + [c_int] * 13 + [c_void_p]),
     "adder_b200_conv_backward_input": (c_int, [c_void_p] * 4 + [c_int] * 14 + [c_void_p]),
+    "adder_b200_conv_backward_input_workspace_bytes": (c_size_t, [c_int] * 13),
+    "adder_b200_conv_backward_input_with_workspace": (c_int, [c_void_p] * 5 + [c_size_t] + [c_int] * 14 + [c_void_p]),
     "adder_b200_conv_backward_weight_workspace_bytes": (c_size_t, [c_int] * 13),
     "adder_b200_conv_backward_weight": (c_int, [c_void_p] * 4 + [c_float, c_void_p, c_size_t] + [c_int] * 13 + [c_void_p]),
     "adder_b200_forward_affine": (c_int, [c_void_p] * 5 + [c_int, c_void_p, *_GEOM, c_void_p]),

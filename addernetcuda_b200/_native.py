@@ -16,9 +16,11 @@ import torch
 from . import _lib
 
 _NAMES = ("adder_b200_status_string", "adder_b200_forward", "adder_b200_forward_stat_slices", "adder_b200_forward_with_stats",
-          "adder_b200_forward_affine", "adder_b200_affine_forward", "adder_b200_backward_input",
+          "adder_b200_forward_affine", "adder_b200_affine_forward",
+          "adder_b200_backward_input_workspace_bytes", "adder_b200_backward_input_with_workspace",
           "adder_b200_backward_weight_workspace_bytes", "adder_b200_backward_weight", "adder_b200_conv_forward",
-          "adder_b200_conv_backward_input", "adder_b200_conv_backward_weight_workspace_bytes", "adder_b200_conv_backward_weight")
+          "adder_b200_conv_backward_input_workspace_bytes", "adder_b200_conv_backward_input_with_workspace",
+          "adder_b200_conv_backward_weight_workspace_bytes", "adder_b200_conv_backward_weight")
 _ENTRIES = ("layer", "conv", "layer_with_stats", "layer_affine", "affine", "column")
 _mod = None
 

@@ -124,9 +124,12 @@ def backward_input(grad_out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, str
     gx = torch.empty_like(x)
     flags = _lib.FLAG_FAST_CLAMP if fast_clamp else 0
     with torch.cuda.device(dev):
-        _lib.check(_lib.load().adder_b200_backward_input(grad_out.data_ptr(), x.data_ptr(), w.data_ptr(),
-                                                         gx.data_ptr(), *g, flags, _stream(dev)),
-                   "adder_b200_backward_input")
+        lib = _lib.load()
+        nbytes = lib.adder_b200_backward_input_workspace_bytes(*g)
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
+        _lib.check(lib.adder_b200_backward_input_with_workspace(
+            grad_out.data_ptr(), x.data_ptr(), w.data_ptr(), gx.data_ptr(), ws.data_ptr() if nbytes else None, nbytes, *g, flags,
+            _stream(dev)), "adder_b200_backward_input")
     return gx
 
 

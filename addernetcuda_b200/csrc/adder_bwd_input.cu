@@ -933,11 +933,16 @@ int describe_gx(const Geom& layer, int fast, const TileHint& hint, char* buf, si
     return ADDER_OK;
 }
 
+size_t gx_workspace_bytes(const Geom& layer, const TileHint& hint) {
+    if (hint.is_default() && pointwise_applicable(flatten_pointwise(layer, true))) return 0;
+    return gx_uses_gather(layer, hint) ? gx_gather_workspace_bytes(conv_geom(layer)) : 0;
+}
+
 int launch_gx(const Geom& layer, const float* gout, const float* x, const float* w, float* gx, int fast,
-              int accumulate, const TileHint& hint, cudaStream_t stream) {
+              int accumulate, const TileHint& hint, cudaStream_t stream, void* workspace, size_t workspace_bytes) {
     const Geom g = flatten_pointwise(layer, true);
     if (hint.is_default() && pointwise_applicable(g)) return launch_pointwise_gx(g, gout, x, w, gx, fast, accumulate, stream);
-    if (gx_uses_gather(layer, hint)) return launch_gx_gather(conv_geom(layer), gout, x, w, gx, fast, accumulate, stream);
+    if (gx_uses_gather(layer, hint)) return launch_gx_gather(conv_geom(layer), gout, x, w, gx, fast, accumulate, stream, workspace, workspace_bytes);
     const int rw = choose_gx_rw(gx_tiling_geom(g), hint);
 #define ADDER_GX_LAUNCH(KS_, S_, RW_, RC_, FAST_) \
     return launch_gx_t<KS_, S_, RW_, RC_, FAST_>(g, gout, x, w, gx, accumulate, hint, stream);

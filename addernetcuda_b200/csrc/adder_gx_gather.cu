@@ -11,7 +11,8 @@
 // the tile - which follows the size of the batch - does not show in the result.  Exact form: min.xorsign.abs is the clamp in one instruction (magnitude min(|d|, 1), sign of d),
 // where fminf(fmaxf(d, -1), 1) takes two; differences (large tiles) and sums are packed pairs of pixels.
 // Both are bound by the register operands they read (5 a term, 2 a cycle and scheduler): 2.5 and 3.0 lane cycles a term
-// with nothing around them.
+// with nothing around them.  What stands around them is the staging: without it the saturating form of 256->256 14x14 at batch 256
+// takes 2.90 lane cycles a term, with it 3.43 from w as it lies and 3.27 from a copy by taps (gx_gather_workspace_bytes).
 #include <cstdio>
 #include "common.cuh"
 #include "gather.cuh"
@@ -28,7 +29,7 @@ struct GxGatherArgs {
     int ry[MAX_CLASSES], rx[MAX_CLASSES];   // first row and column of the class in the input
     const float* gout;
     const float* x;
-    const float* w;
+    const float* w;          // [Co][Ci][KK]; GATHER_TAP_ROWS: [KK][Co][Ci]
     float* gx;
     int Ci, H, W, Co, Ho, Wo, KK, CK, sh, sw, accumulate;
     int w_quads;             // 1x1: rows of w are whole quads and 16-byte aligned
@@ -47,12 +48,13 @@ struct GxTile {
     static constexpr int PQ = RP == 8 ? 4 : RP;                 // consecutive pixels of a thread
 };
 
-template <class T, bool FAST, bool QUADS>
+template <class T, bool FAST, int MODE>
 __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(const __grid_constant__ GxGatherArgs a) {
     constexpr int RC = T::RC, RP = T::RP, CG = T::CG, TC = T::TC, TP = T::TP, WP = T::WP, PQ = T::PQ, ST = T::ST;
     constexpr int COLS = TP > GATHER_THREADS ? TP / GATHER_THREADS : 1;
     constexpr int ROWS = TP < GATHER_THREADS ? GATHER_THREADS / TP : 1;
-    constexpr int CK = gather_rows(QUADS ? GATHER_QUADS : GATHER_TAP, ST, TC, TP, RC * RP * GATHER_THREADS * 4, T::MB);      // rows of a stage
+    constexpr bool QUADS = MODE == GATHER_QUADS, TAP_ROWS = MODE == GATHER_TAP_ROWS;
+    constexpr int CK = gather_rows(MODE, ST, TC, TP, RC * RP * GATHER_THREADS * 4, T::MB);      // rows of a stage
     constexpr int PARTS = 4, MINE = PARTS / ROWS;      // partial sums of g per pixel, and those of one thread
     static_assert(PARTS % ROWS == 0 && (PARTS > ROWS || CK == 16), "whole partial sums per thread, a stage at a time");
     constexpr int FOLD = 64 / CK;                // chunks per partial sum: 64 terms before it is folded into the total
@@ -88,8 +90,10 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
         else gather_pixels<TP>(Gs + stage * GS, px, a.gout, m, fc, nch, ck4, a.Ho, a.Wo, tid);
         // weights [output channel of the chunk][input channel of the tile]
         float* ws = Ws + stage * WS;
-        const float* wsrc = a.w + ((fc.c0 * a.Ci + ci0) * a.KK + m.wt0 + fc.i * m.dwi + fc.j * m.dwj);
-        if (a.w_quads) {
+        const float* wsrc;
+        if constexpr (TAP_ROWS) wsrc = a.w + (((m.wt0 + fc.i * m.dwi + fc.j * m.dwj) * a.Co + fc.c0) * a.Ci + ci0);
+        else wsrc = a.w + ((fc.c0 * a.Ci + ci0) * a.KK + m.wt0 + fc.i * m.dwi + fc.j * m.dwj);
+        if (TAP_ROWS || a.w_quads) {
             constexpr int WQ = TC / 4, WROWS = GATHER_THREADS / WQ;
             const int q = 4 * (tid % WQ), k0 = tid / WQ;
             const bool okc = ci0 + q < a.Ci;
@@ -419,12 +423,12 @@ int choose_tile(const GxGatherArgs& a, int classes, int Ci, bool fast) {
     return best;
 }
 
-int stage_rows(const Tile& t, bool quads) {
-    return gather_rows(quads ? GATHER_QUADS : GATHER_TAP, t.st, t.tc, t.tp, t.rc * t.rp * GATHER_THREADS * 4, t.mb);
+int stage_rows(const Tile& t, int mode) {
+    return gather_rows(mode, t.st, t.tc, t.tp, t.rc * t.rp * GATHER_THREADS * 4, t.mb);
 }
 
-size_t smem_bytes(const Tile& t, bool quads) {
-    return ((size_t)t.st * stage_rows(t, quads) * (t.tp + t.tc + 4) + (size_t)t.rc * t.rp * GATHER_THREADS) * sizeof(float);
+size_t smem_bytes(const Tile& t, int mode) {
+    return ((size_t)t.st * stage_rows(t, mode) * (t.tp + t.tc + 4) + (size_t)t.rc * t.rp * GATHER_THREADS) * sizeof(float);
 }
 
 // Taps k of one dimension that reach input positions q*S + r: (r + pad - k*dil) % S == 0.  Output position q + o0 + i*d0.
@@ -470,23 +474,29 @@ bool single_class(const ConvGeom& g) {
     return true;
 }
 
-template <class T, bool FAST, bool QUADS>
+template <class T, bool FAST, int MODE>
 int launch_t(const GxGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
-    auto kern = adder_gx_gather_kernel<T, FAST, QUADS>;
+    auto kern = adder_gx_gather_kernel<T, FAST, MODE>;
     const int se = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
     if (se != ADDER_OK) return se;
     kern<<<grid, GATHER_THREADS, smem, stream>>>(a);
     return launched();
 }
 
-template <bool FAST, bool QUADS>
+template <bool FAST, int MODE>
 int launch_tile(int tile, const GxGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
     int i = 0;
 #define X(RC, RP, CG, ST, MB, A, M, S, FA, FM, FS) \
-    if (tile == i++) return launch_t<GxTile<RC, RP, CG, ST, MB>, FAST, QUADS>(a, grid, smem, stream);
+    if (tile == i++) return launch_t<GxTile<RC, RP, CG, ST, MB>, FAST, MODE>(a, grid, smem, stream);
     ADDER_GX_GATHER_TILES(X)
 #undef X
     return ADDER_ERR_INTERNAL;
+}
+
+template <bool FAST>
+int launch_mode(int mode, int tile, const GxGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
+    if (mode == GATHER_TAP_ROWS) return launch_tile<FAST, GATHER_TAP_ROWS>(tile, a, grid, smem, stream);
+    return mode == GATHER_QUADS ? launch_tile<FAST, GATHER_QUADS>(tile, a, grid, smem, stream) : launch_tile<FAST, GATHER_TAP>(tile, a, grid, smem, stream);
 }
 
 int plan(const ConvGeom& g, int first, bool fast, GxGatherArgs& a, dim3& grid, bool& more) {
@@ -514,13 +524,45 @@ int describe_gx_gather(const ConvGeom& g, int fast, char* buf, size_t n) {
     dim3 grid;
     bool more;
     const Tile& t = kTiles[plan(g, 0, fast != 0, a, grid, more)];
-    const size_t smem = smem_bytes(t, gx_quads(g, a, grid, 0, true));
+    const size_t smem = smem_bytes(t, gx_quads(g, a, grid, 0, true) ? GATHER_QUADS : GATHER_TAP);
     return snprintf(buf, n, "gx gather k=%dx%d fast=%d classes=%u RC=%d RP=%d TC=%d TP=%d threads=%d smem=%zu grid=(%u,%u) status=%d",
                     g.kh, g.kw, fast, grid.z, t.rc, t.rp, t.tc, t.tp, GATHER_THREADS, smem, grid.x, grid.y, gather_status((int)grid.y, smem));
 }
 
+// w[Co][Ci][KK] -> [KK][Co][Ci]: a block has 64 input channels of one output channel, which are consecutive on both sides.
+__global__ void __launch_bounds__(256) by_taps_kernel(const float* __restrict__ w, float* __restrict__ wt, int Co, int Ci, int KK) {
+    extern __shared__ float taps[];              // [64][KK]
+    const int co = blockIdx.x, ci0 = blockIdx.y * 64, n = min(64, Ci - ci0);
+    const float* src = w + ((size_t)co * Ci + ci0) * KK;
+    for (int e = threadIdx.x; e < n * KK; e += 256) taps[e] = __ldg(src + e);
+    __syncthreads();
+    const int c = threadIdx.x & 63;
+    if (c < n)
+        for (int t = threadIdx.x >> 6; t < KK; t += 4) wt[((size_t)t * Co + co) * Ci + ci0 + c] = taps[c * KK + t];
+}
+
+// Windows of several taps: bytes of the copy of w by taps, whose rows a stage takes in 16-byte copies; 0 where the layer does
+// without.  As they lie, a stage's weights are 4-byte copies KK words apart, a sector of L2 each.  256->256 14x14 at batch 256: 2790 ->
+// 2657 us with the copy's own launch, 128->128 56x56 stride 2 at batch 64: 783 -> 729, 512->512 14x14 stride 2: 771 -> 716.  The launch
+// takes 3 to 8 us, which a layer of 3e9 terms (230 us) wins back; 176->176 8x8 at batch 47 (8e8) lost 8 us of 150.  The order of addition
+// is the same, so the result is.
+size_t gx_gather_workspace_bytes(const ConvGeom& g) {
+    const int KK = g.kh * g.kw;
+    const double terms = (double)g.N * g.Ho * g.Wo * g.Co * g.Ci * KK;
+    if (KK == 1 || KK > 128 || g.Ci % 4 != 0 || g.Co > 65535 * 32 || g.Ci > 65535 * 64 || terms < 3e9) return 0;
+    return (size_t)KK * g.Co * g.Ci * sizeof(float);
+}
+
 int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const float* w, float* gx, int fast, int accumulate,
-                     cudaStream_t stream) {
+                     cudaStream_t stream, void* workspace, size_t workspace_bytes) {
+    float* by_taps = nullptr;
+    const size_t need = gx_gather_workspace_bytes(g);
+    if (workspace != nullptr && need > 0 && workspace_bytes >= need && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0) {
+        by_taps = static_cast<float*>(workspace);
+        by_taps_kernel<<<dim3((unsigned)g.Co, (unsigned)ceil_div(g.Ci, 64)), 256, (size_t)64 * g.kh * g.kw * sizeof(float), stream>>>(w, by_taps, g.Co, g.Ci, g.kh * g.kw);
+        const int st = launched();
+        if (st != ADDER_OK) return st;
+    }
     bool more = true;
     for (int first = 0; more; first += MAX_CLASSES) {
         GxGatherArgs a;
@@ -530,6 +572,7 @@ int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const
         const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gx)) & 15) == 0;
         const bool unit = g.sh == 1 && g.sw == 1;
         a.vec_io = unit && (g.H * g.W) % 4 == 0 && aligned;
+        if (by_taps != nullptr) a.w = by_taps;
         a.w_quads = a.KK == 1 && g.Ci % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
         a.fill_block = single_class(g) && !accumulate;
         a.fill_quads = a.fill_block && g.sh == 2 && g.sw == 2 && g.W == 2 * a.m[0].PW && g.H == 2 * a.m[0].PH && a.m[0].PW % 4 == 0 &&
@@ -537,12 +580,12 @@ int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const
         // (planes of an odd height keep an even number of values, so that every plane starts aligned)
         a.fill_pairs = a.fill_block && !a.fill_quads && g.sh == 2 && g.sw == 2 && g.W % 2 == 0 && (reinterpret_cast<uintptr_t>(gx) & 7) == 0;
         const bool quads = gx_quads(g, a, grid, first, (reinterpret_cast<uintptr_t>(gout) & 15) == 0);
-        const int rows = stage_rows(kTiles[tile], quads);
+        const int mode = by_taps != nullptr ? GATHER_TAP_ROWS : quads ? GATHER_QUADS : GATHER_TAP;
+        const int rows = stage_rows(kTiles[tile], mode);
         a.CK = g.Co < rows ? g.Co : rows;      // full blocks have the cheaper staging loops, so one ragged block rather than even ones
-        const size_t smem = smem_bytes(kTiles[tile], quads);
+        const size_t smem = smem_bytes(kTiles[tile], mode);
         if (gather_status((int)grid.y, smem) != ADDER_OK) return ADDER_ERR_UNSUPPORTED;
-        const int st = fast ? (quads ? launch_tile<true, true>(tile, a, grid, smem, stream) : launch_tile<true, false>(tile, a, grid, smem, stream))
-                            : (quads ? launch_tile<false, true>(tile, a, grid, smem, stream) : launch_tile<false, false>(tile, a, grid, smem, stream));
+        const int st = fast ? launch_mode<true>(mode, tile, a, grid, smem, stream) : launch_mode<false>(mode, tile, a, grid, smem, stream);
         if (st != ADDER_OK) return st;
     }
     return ADDER_OK;

@@ -198,15 +198,27 @@ int adder_b200_forward_affine(const float* x, const float* w, const float* scale
     return launch_fwd(g, x, w, out, current_hint(0), static_cast<cudaStream_t>(stream), nullptr, 0, ep);
 }
 
-int adder_b200_backward_input(const float* grad_out, const float* x, const float* w, float* grad_x, int n, int ci,
-                              int h, int wd, int co, int k, int stride, int pad, int flags, void* stream) {
+size_t adder_b200_backward_input_workspace_bytes(int n, int ci, int h, int wd, int co, int k, int stride, int pad) {
+    Geom g;
+    if (make_geom(n, ci, h, wd, co, k, stride, pad, &g) != ADDER_OK || n == 0) return 0;
+    return gx_workspace_bytes(g, current_hint(1));
+}
+
+int adder_b200_backward_input_with_workspace(const float* grad_out, const float* x, const float* w, float* grad_x, void* workspace,
+                                             size_t workspace_bytes, int n, int ci, int h, int wd, int co, int k, int stride, int pad,
+                                             int flags, void* stream) {
     Geom g;
     const int st = make_geom(n, ci, h, wd, co, k, stride, pad, &g);
     if (st != ADDER_OK) return st;
     if (n == 0) return ADDER_OK;
     if (grad_out == nullptr || x == nullptr || w == nullptr || grad_x == nullptr) return ADDER_ERR_NULL_POINTER;
     return launch_gx(g, grad_out, x, w, grad_x, (flags & ADDER_FLAG_FAST_CLAMP) != 0,
-                     (flags & ADDER_FLAG_ACCUMULATE) != 0, current_hint(1), static_cast<cudaStream_t>(stream));
+                     (flags & ADDER_FLAG_ACCUMULATE) != 0, current_hint(1), static_cast<cudaStream_t>(stream), workspace, workspace_bytes);
+}
+
+int adder_b200_backward_input(const float* grad_out, const float* x, const float* w, float* grad_x, int n, int ci,
+                              int h, int wd, int co, int k, int stride, int pad, int flags, void* stream) {
+    return adder_b200_backward_input_with_workspace(grad_out, x, w, grad_x, nullptr, 0, n, ci, h, wd, co, k, stride, pad, flags, stream);
 }
 
 size_t adder_b200_backward_weight_workspace_bytes(int n, int ci, int h, int wd, int co, int k, int stride, int pad) {
@@ -247,14 +259,25 @@ int adder_b200_conv_forward(const float* x, const float* w, float* out, int n, i
     return launch_fwd_gather(g, x, w, out, static_cast<cudaStream_t>(stream));
 }
 
-int adder_b200_conv_backward_input(const float* grad_out, const float* x, const float* w, float* grad_x, int n, int ci, int h, int wd, int co, int kh, int kw, int sh, int sw, int ph, int pw, int dh, int dw, int flags, void* stream) {
+size_t adder_b200_conv_backward_input_workspace_bytes(int n, int ci, int h, int wd, int co, int kh, int kw, int sh, int sw, int ph, int pw, int dh, int dw) {
+    ConvGeom g;
+    if (make_conv_geom(n, ci, h, wd, co, kh, kw, sh, sw, ph, pw, dh, dw, &g) != ADDER_OK || n == 0) return 0;
+    return gx_gather_workspace_bytes(g);
+}
+
+int adder_b200_conv_backward_input_with_workspace(const float* grad_out, const float* x, const float* w, float* grad_x, void* workspace,
+                                                  size_t workspace_bytes, int n, int ci, int h, int wd, int co, int kh, int kw, int sh, int sw, int ph, int pw, int dh, int dw, int flags, void* stream) {
     ConvGeom g;
     const int st = make_conv_geom(n, ci, h, wd, co, kh, kw, sh, sw, ph, pw, dh, dw, &g);
     if (st != ADDER_OK) return st;
     if (n == 0) return ADDER_OK;
     if (grad_out == nullptr || x == nullptr || w == nullptr || grad_x == nullptr) return ADDER_ERR_NULL_POINTER;
     return launch_gx_gather(g, grad_out, x, w, grad_x, (flags & ADDER_FLAG_FAST_CLAMP) != 0, (flags & ADDER_FLAG_ACCUMULATE) != 0,
-                            static_cast<cudaStream_t>(stream));
+                            static_cast<cudaStream_t>(stream), workspace, workspace_bytes);
+}
+
+int adder_b200_conv_backward_input(const float* grad_out, const float* x, const float* w, float* grad_x, int n, int ci, int h, int wd, int co, int kh, int kw, int sh, int sw, int ph, int pw, int dh, int dw, int flags, void* stream) {
+    return adder_b200_conv_backward_input_with_workspace(grad_out, x, w, grad_x, nullptr, 0, n, ci, h, wd, co, kh, kw, sh, sw, ph, pw, dh, dw, flags, stream);
 }
 
 size_t adder_b200_conv_backward_weight_workspace_bytes(int n, int ci, int h, int wd, int co, int kh, int kw, int sh, int sw, int ph, int pw, int dh, int dw) {

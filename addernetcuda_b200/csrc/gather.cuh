@@ -10,6 +10,7 @@
 //   GATHER_HALVES two blocks of 16 channels and one tap each in one stage of a thin tile;
 //   GATHER_QUADS  1x1 layers whose operand is read in order: 16-byte copies, 16 or 32 channels;
 //   GATHER_NINE   2 channels (4 in the thin tiles) x the 9 taps of a 3x3 window, in index order (channel, row, column).
+//   GATHER_TAP_ROWS (input gradient) GATHER_TAP with the weights from a copy by taps, in 16-byte copies.
 // One barrier per chunk; large tiles keep two stages, small ones as many as hide the latency of a load.
 #pragma once
 #include "common.cuh"
@@ -19,7 +20,7 @@ namespace adder {
 
 constexpr int GATHER_CK = 16;
 constexpr int GATHER_THREADS = 128;
-enum GatherMode { GATHER_TAP, GATHER_QUADS, GATHER_NINE, GATHER_HALVES };
+enum GatherMode { GATHER_TAP, GATHER_QUADS, GATHER_NINE, GATHER_HALVES, GATHER_TAP_ROWS };
 
 // Channels of a chunk of GATHER_NINE; thin tiles (a few outputs a thread) spend their time on the instructions around a stage
 // rather than on its terms, so their stages are twice as long.

@@ -29,11 +29,13 @@ struct Api {      // entry points of the loaded libadder_b200.so
     decltype(&adder_b200_forward_with_stats) forward_with_stats = nullptr;
     decltype(&adder_b200_forward_affine) forward_affine = nullptr;
     decltype(&adder_b200_affine_forward) affine_forward = nullptr;
-    decltype(&adder_b200_backward_input) backward_input = nullptr;
+    decltype(&adder_b200_backward_input_workspace_bytes) backward_input_workspace_bytes = nullptr;
+    decltype(&adder_b200_backward_input_with_workspace) backward_input_with_workspace = nullptr;
     decltype(&adder_b200_backward_weight_workspace_bytes) backward_weight_workspace_bytes = nullptr;
     decltype(&adder_b200_backward_weight) backward_weight = nullptr;
     decltype(&adder_b200_conv_forward) conv_forward = nullptr;
-    decltype(&adder_b200_conv_backward_input) conv_backward_input = nullptr;
+    decltype(&adder_b200_conv_backward_input_workspace_bytes) conv_backward_input_workspace_bytes = nullptr;
+    decltype(&adder_b200_conv_backward_input_with_workspace) conv_backward_input_with_workspace = nullptr;
     decltype(&adder_b200_conv_backward_weight_workspace_bytes) conv_backward_weight_workspace_bytes = nullptr;
     decltype(&adder_b200_conv_backward_weight) conv_backward_weight = nullptr;
 };
@@ -109,13 +111,17 @@ std::pair<at::Tensor, at::Tensor> forward_with_stats(const at::Tensor& x, const 
     return {out, st};
 }
 
-void backward_input(const at::Tensor& g, const at::Tensor& x, const at::Tensor& w, const at::Tensor& gx, const Layer& L, bool fast) {
-    check(api.backward_input(g.const_data_ptr<float>(), x.const_data_ptr<float>(), w.const_data_ptr<float>(), gx.mutable_data_ptr<float>(),
-                             ADDER_GEOM(L), fast ? ADDER_FLAG_FAST_CLAMP : 0, current_stream(x)), "adder_b200_backward_input");
-}
-
 // The scratch comes from torch's caching allocator on the current stream: a cached block most of the time, safe with any number
 // of threads and streams, and part of the graph's own pool under capture.
+void backward_input(const at::Tensor& g, const at::Tensor& x, const at::Tensor& w, const at::Tensor& gx, const Layer& L, bool fast) {
+    const size_t bytes = api.backward_input_workspace_bytes(ADDER_GEOM(L));
+    at::Tensor ws;
+    if (bytes > 0) ws = empty_on(x, {(int64_t)bytes}, at::kByte);
+    check(api.backward_input_with_workspace(g.const_data_ptr<float>(), x.const_data_ptr<float>(), w.const_data_ptr<float>(), gx.mutable_data_ptr<float>(),
+                                            bytes > 0 ? ws.mutable_data_ptr() : nullptr, bytes, ADDER_GEOM(L), fast ? ADDER_FLAG_FAST_CLAMP : 0,
+                                            current_stream(x)), "adder_b200_backward_input");
+}
+
 void backward_weight(const at::Tensor& g, const at::Tensor& x, const at::Tensor& w, const at::Tensor& gw, const Layer& L, float eta) {
     const int64_t bytes = (int64_t)api.backward_weight_workspace_bytes(ADDER_GEOM(L));
     at::Tensor ws = empty_on(x, {bytes}, at::kByte);
@@ -202,9 +208,12 @@ at::Tensor conv_forward(const at::Tensor& x, const at::Tensor& w, const Conv& c)
 }
 
 void conv_backward_input(const at::Tensor& g, const at::Tensor& x, const at::Tensor& w, const at::Tensor& gx, const Conv& c, bool fast) {
-    check(api.conv_backward_input(g.const_data_ptr<float>(), x.const_data_ptr<float>(), w.const_data_ptr<float>(),
-                                  gx.mutable_data_ptr<float>(), ADDER_CONV_GEOM(c), fast ? ADDER_FLAG_FAST_CLAMP : 0, current_stream(x)),
-          "adder_b200_conv_backward_input");
+    const size_t bytes = api.conv_backward_input_workspace_bytes(ADDER_CONV_GEOM(c));
+    at::Tensor ws;
+    if (bytes > 0) ws = empty_on(x, {(int64_t)bytes}, at::kByte);
+    check(api.conv_backward_input_with_workspace(g.const_data_ptr<float>(), x.const_data_ptr<float>(), w.const_data_ptr<float>(),
+                                                 gx.mutable_data_ptr<float>(), bytes > 0 ? ws.mutable_data_ptr() : nullptr, bytes, ADDER_CONV_GEOM(c),
+                                                 fast ? ADDER_FLAG_FAST_CLAMP : 0, current_stream(x)), "adder_b200_conv_backward_input");
 }
 
 void conv_backward_weight(const at::Tensor& g, const at::Tensor& x, const at::Tensor& w, const at::Tensor& gw, const Conv& c, float eta) {
@@ -501,11 +510,13 @@ PyObject* py_bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
         get("adder_b200_forward_with_stats", &a.forward_with_stats);
         get("adder_b200_forward_affine", &a.forward_affine);
         get("adder_b200_affine_forward", &a.affine_forward);
-        get("adder_b200_backward_input", &a.backward_input);
+        get("adder_b200_backward_input_workspace_bytes", &a.backward_input_workspace_bytes);
+        get("adder_b200_backward_input_with_workspace", &a.backward_input_with_workspace);
         get("adder_b200_backward_weight_workspace_bytes", &a.backward_weight_workspace_bytes);
         get("adder_b200_backward_weight", &a.backward_weight);
         get("adder_b200_conv_forward", &a.conv_forward);
-        get("adder_b200_conv_backward_input", &a.conv_backward_input);
+        get("adder_b200_conv_backward_input_workspace_bytes", &a.conv_backward_input_workspace_bytes);
+        get("adder_b200_conv_backward_input_with_workspace", &a.conv_backward_input_with_workspace);
         get("adder_b200_conv_backward_weight_workspace_bytes", &a.conv_backward_weight_workspace_bytes);
         get("adder_b200_conv_backward_weight", &a.conv_backward_weight);
         api = a;

@@ -117,7 +117,8 @@ int launch_fwd(const Geom& g, const float* x, const float* w, float* out, const 
 // 0 when that kernel has no fused statistics.
 int fwd_stat_slices(const Geom& g, const TileHint& hint);
 int launch_gx(const Geom& g, const float* gout, const float* x, const float* w, float* gx, int fast,
-              int accumulate, const TileHint& hint, cudaStream_t s);
+              int accumulate, const TileHint& hint, cudaStream_t s, void* workspace = nullptr, size_t workspace_bytes = 0);
+size_t gx_workspace_bytes(const Geom& g, const TileHint& hint);      // optional scratch of the input gradient; 0: none
 size_t gw_workspace_bytes(const Geom& g, const TileHint& hint);
 int launch_gw(const Geom& g, const float* gout, const float* x, const float* w, float* gw, float eta,
               float* out_norm, int accumulate, void* workspace, size_t workspace_bytes, const TileHint& hint,
@@ -140,7 +141,8 @@ int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* 
 double fwd_gather_clocks(const ConvGeom& g);      // predicted time of its launch, in clocks per reduction step
 int describe_fwd_gather(const ConvGeom& g, char* buf, size_t n);
 int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const float* w, float* gx, int fast, int accumulate,
-                     cudaStream_t s);
+                     cudaStream_t s, void* workspace = nullptr, size_t workspace_bytes = 0);
+size_t gx_gather_workspace_bytes(const ConvGeom& g);
 int describe_gx_gather(const ConvGeom& g, int fast, char* buf, size_t n);
 
 // 1x1 stride-2 layers with at most 64 channels: one thread per output position (adder_pointwise.cu).

@@ -86,6 +86,13 @@ ADDER_API int adder_b200_forward(const float* x, const float* w, float* out, int
 ADDER_API int adder_b200_backward_input(const float* grad_out, const float* x, const float* w, float* grad_x, int n, int ci,
                               int h, int wd, int co, int k, int stride, int pad, int flags, void* stream);
 
+/* The same with optional scratch (16-byte aligned; NULL or too small: as without): a copy of w in the order in which the kernel stages
+ * it.  The result is the same, bit for bit.  The size is 0 for layers that do without. */
+ADDER_API size_t adder_b200_backward_input_workspace_bytes(int n, int ci, int h, int wd, int co, int k, int stride, int pad);
+ADDER_API int adder_b200_backward_input_with_workspace(const float* grad_out, const float* x, const float* w, float* grad_x,
+                              void* workspace, size_t workspace_bytes, int n, int ci, int h, int wd, int co, int k, int stride,
+                              int pad, int flags, void* stream);
+
 /* Bytes of scratch the weight-gradient entry points need for this geometry on the current device. */
 ADDER_API size_t adder_b200_backward_weight_workspace_bytes(int n, int ci, int h, int wd, int co, int k, int stride, int pad);
 
@@ -210,6 +217,12 @@ ADDER_API int adder_b200_conv_forward(const float* x, const float* w, float* out
 ADDER_API int adder_b200_conv_backward_input(const float* grad_out, const float* x, const float* w, float* grad_x, int n,
                                              int ci, int h, int wd, int co, int kh, int kw, int sh, int sw, int ph,
                                              int pw, int dh, int dw, int flags, void* stream);
+ADDER_API size_t adder_b200_conv_backward_input_workspace_bytes(int n, int ci, int h, int wd, int co, int kh, int kw, int sh,
+                                                                int sw, int ph, int pw, int dh, int dw);
+ADDER_API int adder_b200_conv_backward_input_with_workspace(const float* grad_out, const float* x, const float* w, float* grad_x,
+                                                            void* workspace, size_t workspace_bytes, int n, int ci, int h,
+                                                            int wd, int co, int kh, int kw, int sh, int sw, int ph, int pw,
+                                                            int dh, int dw, int flags, void* stream);
 ADDER_API size_t adder_b200_conv_backward_weight_workspace_bytes(int n, int ci, int h, int wd, int co, int kh, int kw,
                                                                  int sh, int sw, int ph, int pw, int dh, int dw);
 ADDER_API int adder_b200_conv_backward_weight(const float* grad_out, const float* x, const float* w, float* grad_w,
