@@ -24,21 +24,32 @@ struct FwdGatherArgs {
     int vec_store;           // planes are whole quads, `out` and the residual 16-byte aligned
 };
 
+// Tiles that may take the weights as they lie (ROWS), where rows of w are whole aligned quads: 16-byte copies instead of four times as many
+// that transpose, 5 to 9 % of a tile of 16 x 4 channels (512->512 7x7 3x3 at batch 64: 697 -> 639 us, 512->128 28x28: 250 -> 232).
+// Tiles of fewer channels spend their staging on pixels and gain nothing; eight channels a thread have no registers for several steps of
+// each at a time and lose 1 to 6 %.
+__host__ __device__ constexpr bool takes_rows(int rm, int cg) { return rm == 4 && cg == 16; }
+
 // RM channels x RP pixels per thread (RP = 8: two quads half a tile apart), CG channel groups, ST stages, MB CTAs per SM.
 template <int RM_, int RP_, int CG_, int ST_, int MB_>
 struct FwdTile {
     static constexpr int RM = RM_, RP = RP_, CG = CG_, ST = ST_, MB = MB_;
     static constexpr int PG = GATHER_THREADS / CG, TC = CG * RM, TP = PG * RP, WP = TC + 4;
     static constexpr int PQ = RP == 8 ? 4 : RP;                 // consecutive pixels of a thread
-    static constexpr bool THIN = RM <= 2 && RP <= 2;
+    static constexpr bool THIN = RM <= 2 && RP <= 2, TAKES_ROWS = takes_rows(RM, CG);
 };
+
+// ROWS: weights [channel][step], the floats of a row.  The 18 steps of two channels of a 3x3 window come as the 80 aligned bytes around
+// them: they start at the third float for every other pair of channels.
+__host__ __device__ constexpr int weight_row(int mode, int rows) { return mode == GATHER_NINE_ROWS ? 20 : rows; }
 
 template <class T, int MODE>
 __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel(const __grid_constant__ FwdGatherArgs a) {
     constexpr int RM = T::RM, RP = T::RP, CG = T::CG, TC = T::TC, TP = T::TP, WP = T::WP, PQ = T::PQ, ST = T::ST;
     constexpr int COLS = TP > GATHER_THREADS ? TP / GATHER_THREADS : 1;
     constexpr int CK = gather_rows(MODE, ST, TC, TP, 0, T::MB, T::THIN);      // rows of a stage
-    constexpr int XS = CK * TP, WS = CK * WP;
+    constexpr bool NINE = MODE == GATHER_NINE || MODE == GATHER_NINE_ROWS, ROWS = MODE == GATHER_QUADS_ROWS || MODE == GATHER_NINE_ROWS;
+    constexpr int XS = CK * TP, WK = weight_row(MODE, CK), WS = ROWS ? TC * WK : CK * WP;
     extern __shared__ __align__(16) float smem[];
     float* const Xs = smem;
     float* const Ws = smem + ST * XS;
@@ -51,26 +62,26 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
     GatherPixel px[COLS];
     constexpr int CH = nine_channels(T::THIN);
     GatherNine<TP, CH> nine;
-    if (MODE == GATHER_QUADS) {
+    if (MODE == GATHER_QUADS || MODE == GATHER_QUADS_ROWS) {
         px[0].decode(a.m, a.x, p0 + 4 * (tid % (TP / 4)), image);
         px[0].base += px[0].row * a.W + px[0].col;
     } else {
 #pragma unroll
         for (int q = 0; q < COLS; ++q) px[q].decode(a.m, a.x, p0 + (COLS > 1 ? tid + q * GATHER_THREADS : tid % TP), image);
-        if (MODE == GATHER_NINE) nine.init(px, a.m, a.H, a.W, tid);
+        if (NINE) nine.init(px, a.m, a.H, a.W, tid);
     }
     GatherChunk fc;              // position of the next chunk to stage
     const int ck4 = round_up(a.CK, 4);
     auto fill = [&](int stage) {
         int nk, rows, wk;        // reduction steps that exist, rows to stage, and the first one's weight index
         int nk2 = 0, wk2 = 0;    // GATHER_HALVES: of the second block
-        if constexpr (MODE == GATHER_NINE) {
+        if constexpr (NINE) {
             const int nch = min(CH, a.Ci - fc.c0);
             nine.fill(Xs + stage * XS, px, a.m, fc.c0, nch, a.H, a.W, tid);
             nk = nch * 9; rows = CK; wk = fc.c0 * 9;
         } else {
             nk = min(a.CK, a.Ci - fc.c0); rows = ck4;
-            if (MODE == GATHER_QUADS) gather_quads<TP, CK>(Xs + stage * XS, px[0].base, px[0].ok, a.x, fc.c0, nk, ck4, a.H * a.W, tid);
+            if (MODE == GATHER_QUADS || MODE == GATHER_QUADS_ROWS) gather_quads<TP, CK>(Xs + stage * XS, px[0].base, px[0].ok, a.x, fc.c0, nk, ck4, a.H * a.W, tid);
             else gather_pixels<TP, MODE == GATHER_HALVES ? GATHER_CK : CK>(Xs + stage * XS, px, a.x, a.m, fc, nk, ck4, a.H, a.W, tid);
             wk = fc.c0 * a.KK + a.m.wt0 + fc.i * a.m.dwi + fc.j * a.m.dwj;
             if constexpr (MODE == GATHER_HALVES) {
@@ -81,8 +92,18 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
                 gather_pixels<TP>(Xs + stage * XS + GATHER_CK * TP, px, a.x, a.m, f2, nk2, GATHER_CK, a.H, a.W, tid);
             }
         }
-        const int kstep = MODE == GATHER_NINE ? 1 : a.KK, row = a.Ci * a.KK;
-        if constexpr (T::THIN) {
+        const int kstep = NINE ? 1 : a.KK, row = a.Ci * a.KK;
+        if constexpr (ROWS) {
+            constexpr int WQ = WK / 4;               // 16-byte words of a row
+            const float* wsrc = a.w + (co0 * row + (NINE ? wk - (fc.c0 & 2) : wk));
+#pragma unroll
+            for (int i0 = 0; i0 < TC * WQ; i0 += GATHER_THREADS) {
+                const int c = (i0 + tid) / WQ, k = (i0 + tid) % WQ * 4;
+                if ((TC * WQ) % GATHER_THREADS != 0 && c >= TC) break;
+                const bool ok = co0 + c < a.Co && (NINE || k < nk);
+                cp_async16(Ws + stage * WS + c * WK + k, ok ? wsrc + (c * row + k) : a.w, ok);
+            }
+        } else if constexpr (T::THIN) {
             // weights [output channel of the tile][reduction step]: a thread copies 4 steps
 #pragma unroll
             for (int i0 = 0; i0 < TC * CK / 4; i0 += GATHER_THREADS) {
@@ -122,7 +143,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
                 }
             }
         }
-        if (MODE == GATHER_NINE) fc.c0 += CH;
+        if (NINE) fc.c0 += CH;
         else fc.next(a.m, a.CK);
     };
 
@@ -146,7 +167,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
         if (c + ST - 1 < a.nchunks) fill(fstage);
         cp_async_commit();
         const float* xs = Xs + stage * XS + pg * PQ;
-        const int nk = MODE == GATHER_NINE || MODE == GATHER_HALVES ? CK : min(ck4, round_up(a.Ci - cc.c0, 4));
+        const int nk = NINE || MODE == GATHER_HALVES ? CK : min(ck4, round_up(a.Ci - cc.c0, 4));
         if constexpr (T::THIN) {
             const float* ws = Ws + stage * WS + cg * RM * (CK + 4);
 #pragma unroll (RM == 1 ? CK / 4 : 2)
@@ -173,6 +194,44 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
 #pragma unroll
                         for (int j = 0; j < RP; ++j) acc[m][j] += fabsf(wv - xv[i][j]);
                     }
+            }
+        } else if constexpr (ROWS) {
+            // SW steps a load of w; pairs of pixels, as two channels of a step are not neighbours here
+            constexpr int SW = NINE ? 2 : 4;
+            const float* ws = Ws + stage * WS + cg * RM * WK + (NINE ? 2 * (c & 1) : 0);
+#pragma unroll 1
+            for (int k = 0; k < nk; k += SW) {
+                float wv[RM][SW];
+#pragma unroll
+                for (int m = 0; m < RM; ++m) {
+                    if constexpr (SW == 4) {
+                        const float4 q = *reinterpret_cast<const float4*>(ws + m * WK + k);
+                        wv[m][0] = q.x; wv[m][1] = q.y; wv[m][2] = q.z; wv[m][3] = q.w;
+                    } else {
+                        const float2 q = *reinterpret_cast<const float2*>(ws + m * WK + k);
+                        wv[m][0] = q.x; wv[m][1] = q.y;
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < SW; ++i) {
+                    uint64_t x2[RP / 2];
+#pragma unroll
+                    for (int h = 0; h < RP / PQ; ++h) {
+                        const float4 q = *reinterpret_cast<const float4*>(xs + (k + i) * TP + h * (TP / 2));
+                        x2[2 * h] = pack2(q.x, q.y); x2[2 * h + 1] = pack2(q.z, q.w);
+                    }
+#pragma unroll
+                    for (int m = 0; m < RM; ++m) {
+                        const uint64_t nw2 = pack2(-wv[m][i], -wv[m][i]);
+#pragma unroll
+                        for (int j = 0; j < RP / 2; ++j) {
+                            float d0, d1;
+                            unpack2(add2(x2[j], nw2), d0, d1);
+                            acc[m][2 * j] += fabsf(d0);
+                            acc[m][2 * j + 1] += fabsf(d1);
+                        }
+                    }
+                }
             }
         } else {
             const float* ws = Ws + stage * WS + cg * RM;
@@ -210,7 +269,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_fwd_gather_kernel
                 }
             }
         }
-        if (MODE != GATHER_NINE) cc.next(a.m, a.CK);
+        if (!NINE) cc.next(a.m, a.CK);
         if (++stage == ST) stage = 0;
         if (++fstage == ST) fstage = 0;
     }
@@ -276,21 +335,33 @@ constexpr Tile kTiles[] = {
 #undef X
 };
 
-int choose_tile(int P, int Co) {
+// `rows`: rows of w are whole aligned quads (takes_rows), which takes 5 % off what a tile costs that profits.
+int choose_tile(int P, int Co, bool rows) {
     int best = 0;
     double best_cost = 1e300;
     const int sms = sm_count();
     for (int i = 0; i < (int)(sizeof(kTiles) / sizeof(kTiles[0])); ++i) {
-        const double cost = tile_cost(kTiles[i].cost, (long long)ceil_div(P, kTiles[i].tp) * ceil_div(Co, kTiles[i].tc), sms);
+        const Tile& t = kTiles[i];
+        const double cost = tile_cost(t.cost, (long long)ceil_div(P, t.tp) * ceil_div(Co, t.tc), sms) * (rows && takes_rows(t.rm, t.cg) ? 0.95 : 1.0);
         if (cost < best_cost) { best_cost = cost; best = i; }
     }
     return best;
 }
 
-int stage_rows(const Tile& t, int mode) { return gather_rows(mode, t.st, t.tc, t.tp, 0, t.mb, t.rm <= 2 && t.rp <= 2); }
+// Layers whose weights can be staged as they lie: 3x3, and 1x1 whose pixels are the input's in order.  The plan looks at the sizes alone,
+// the launch at the alignment too.
+bool row_layer(const ConvGeom& g) {
+    const bool in_order = g.kh * g.kw == 1 && g.sh == 1 && g.sw == 1 && g.ph == 0 && g.pw == 0 && (g.Ho * g.Wo) % 4 == 0;
+    const int K = g.Ci * g.kh * g.kw;            // (a row of fewer steps is mostly padding of the stage: 4->336 16x16 at batch 11 3.0 -> 3.4 us)
+    return K % 4 == 0 && K >= 32 && (in_order || (g.kh == 3 && g.kw == 3));
+}
 
-size_t smem_bytes(const Tile& t, int rows) {
-    return (size_t)t.st * rows * (t.tp + t.tc + 4) * sizeof(float);
+bool thin(const Tile& t) { return t.rm <= 2 && t.rp <= 2; }
+int stage_rows(const Tile& t, int mode) { return gather_rows(mode, t.st, t.tc, t.tp, 0, t.mb, thin(t)); }
+
+size_t smem_bytes(const Tile& t, int mode) {
+    const int rows = stage_rows(t, mode);
+    return (size_t)t.st * (rows * t.tp + (mode > GATHER_HALVES ? t.tc * weight_row(mode, rows) : rows * (t.tc + 4))) * sizeof(float);
 }
 
 GatherMap fwd_map(const ConvGeom& g) {
@@ -319,7 +390,7 @@ int launch_mode(int tile, const FwdGatherArgs& a, dim3 grid, size_t smem, cudaSt
 #define X(RM, RP, CG, ST, MB, A, M, S) \
     if (tile == i++) {                                                                                 \
         using T = FwdTile<RM, RP, CG, ST, MB>;                                                         \
-        if constexpr (MODE != GATHER_HALVES || T::THIN) return launch_t<T, MODE>(a, grid, smem, stream); \
+        if constexpr (MODE == GATHER_HALVES ? T::THIN : MODE < GATHER_HALVES || T::TAKES_ROWS) return launch_t<T, MODE>(a, grid, smem, stream); \
     }
     ADDER_FWD_GATHER_TILES(X)
 #undef X
@@ -330,20 +401,23 @@ int launch_mode(int tile, const FwdGatherArgs& a, dim3 grid, size_t smem, cudaSt
 
 double fwd_gather_clocks(const ConvGeom& g) {
     const int P = g.N * g.Ho * g.Wo;
-    const Tile& t = kTiles[choose_tile(P, g.Co)];
-    return tile_cost(t.cost, (long long)ceil_div(P, t.tp) * ceil_div(g.Co, t.tc), sm_count());
+    const bool rows = row_layer(g);
+    const Tile& t = kTiles[choose_tile(P, g.Co, rows)];
+    return tile_cost(t.cost, (long long)ceil_div(P, t.tp) * ceil_div(g.Co, t.tc), sm_count()) * (rows && takes_rows(t.rm, t.cg) ? 0.95 : 1.0);
 }
 
-static int fwd_mode(const ConvGeom& g, bool aligned) {
-    if (g.kh == 3 && g.kw == 3) return GATHER_NINE;
+static int fwd_mode(const ConvGeom& g, const Tile& t, bool aligned, bool w_quads) {
+    const bool rows = w_quads && takes_rows(t.rm, t.cg);
+    if (g.kh == 3 && g.kw == 3) return rows ? GATHER_NINE_ROWS : GATHER_NINE;
     const bool in_order = g.kh * g.kw == 1 && g.sh == 1 && g.sw == 1 && g.ph == 0 && g.pw == 0;
-    return in_order && aligned && (g.Ho * g.Wo) % 4 == 0 ? GATHER_QUADS : GATHER_TAP;
+    if (!in_order || !aligned || (g.Ho * g.Wo) % 4 != 0) return GATHER_TAP;
+    return rows ? GATHER_QUADS_ROWS : GATHER_QUADS;
 }
 
 int describe_fwd_gather(const ConvGeom& g, char* buf, size_t n) {
     const int P = g.N * g.Ho * g.Wo;
-    const Tile& t = kTiles[choose_tile(P, g.Co)];
-    const size_t smem = smem_bytes(t, stage_rows(t, fwd_mode(g, true)));
+    const Tile& t = kTiles[choose_tile(P, g.Co, row_layer(g))];
+    const size_t smem = smem_bytes(t, fwd_mode(g, t, true, row_layer(g)));
     return snprintf(buf, n, "fwd gather k=%dx%d RM=%d RP=%d TC=%d TP=%d threads=%d smem=%zu grid=(%d,%d) status=%d", g.kh, g.kw, t.rm,
                     t.rp, t.tc, t.tp, GATHER_THREADS, smem, ceil_div(P, t.tp), ceil_div(g.Co, t.tc), gather_status(ceil_div(g.Co, t.tc), smem));
 }
@@ -356,20 +430,23 @@ int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* 
     const bool whole_quads = (g.Ho * g.Wo) % 4 == 0;
     a.vec_w = (a.KK == 1 || (g.kh == 3 && g.kw == 3)) && (g.Ci * a.KK) % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
     a.vec_store = whole_quads && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(ep.residual)) & 15) == 0;
-    const int mode = fwd_mode(g, (reinterpret_cast<uintptr_t>(x) & 15) == 0);
-    const int tile = choose_tile(a.m.P, g.Co);
+    const int tile = choose_tile(a.m.P, g.Co, row_layer(g));
     const Tile& t = kTiles[tile];
+    const int mode = fwd_mode(g, t, (reinterpret_cast<uintptr_t>(x) & 15) == 0, a.vec_w && row_layer(g));
     const int rows = stage_rows(t, mode);
     // Windows of several taps are added up in the order (block of 16 channels, tap, channel) by every tile: the tile follows the batch,
     // and an image's result must not.  A thin tile, whose stages have 32 rows, takes two such blocks a stage.
     const bool halves = mode == GATHER_TAP && a.KK > 1 && g.Ci > GATHER_CK && rows > GATHER_CK;
-    a.CK = mode == GATHER_NINE ? rows / 9 : halves ? GATHER_CK : g.Ci < rows ? g.Ci : rows;      // full blocks have the cheaper staging loops
-    a.nchunks = ceil_div(g.Ci, a.CK) * (mode == GATHER_NINE ? 1 : a.KK);
+    const bool nine = mode == GATHER_NINE || mode == GATHER_NINE_ROWS;
+    a.CK = nine ? rows / 9 : halves ? GATHER_CK : g.Ci < rows ? g.Ci : rows;      // full blocks have the cheaper staging loops
+    a.nchunks = ceil_div(g.Ci, a.CK) * (nine ? 1 : a.KK);
     if (halves) a.nchunks = ceil_div(a.nchunks, 2);
     const dim3 grid((unsigned)ceil_div(a.m.P, t.tp), (unsigned)ceil_div(g.Co, t.tc));
-    const size_t smem = smem_bytes(t, rows);
+    const size_t smem = smem_bytes(t, mode);
     if (gather_status((int)grid.y, smem) != ADDER_OK) return ADDER_ERR_UNSUPPORTED;
     if (mode == GATHER_NINE) return launch_mode<GATHER_NINE>(tile, a, grid, smem, stream);
+    if (mode == GATHER_NINE_ROWS) return launch_mode<GATHER_NINE_ROWS>(tile, a, grid, smem, stream);
+    if (mode == GATHER_QUADS_ROWS) return launch_mode<GATHER_QUADS_ROWS>(tile, a, grid, smem, stream);
     if (halves) return launch_mode<GATHER_HALVES>(tile, a, grid, smem, stream);
     return mode == GATHER_QUADS ? launch_mode<GATHER_QUADS>(tile, a, grid, smem, stream) : launch_mode<GATHER_TAP>(tile, a, grid, smem, stream);
 }

@@ -10,6 +10,7 @@
 //   GATHER_HALVES two blocks of 16 channels and one tap each in one stage of a thin tile;
 //   GATHER_QUADS  1x1 layers whose operand is read in order: 16-byte copies, 16 or 32 channels;
 //   GATHER_NINE   2 channels (4 in the thin tiles) x the 9 taps of a 3x3 window, in index order (channel, row, column).
+//   GATHER_QUADS_ROWS, GATHER_NINE_ROWS (forward, takes_rows) the same with the weights left as they lie, in 16-byte copies;
 //   GATHER_TAP_ROWS (input gradient) GATHER_TAP with the weights from a copy by taps, in 16-byte copies.
 // One barrier per chunk; large tiles keep two stages, small ones as many as hide the latency of a load.
 #pragma once
@@ -20,7 +21,7 @@ namespace adder {
 
 constexpr int GATHER_CK = 16;
 constexpr int GATHER_THREADS = 128;
-enum GatherMode { GATHER_TAP, GATHER_QUADS, GATHER_NINE, GATHER_HALVES, GATHER_TAP_ROWS };
+enum GatherMode { GATHER_TAP, GATHER_QUADS, GATHER_NINE, GATHER_HALVES, GATHER_QUADS_ROWS, GATHER_NINE_ROWS, GATHER_TAP_ROWS };
 
 // Channels of a chunk of GATHER_NINE; thin tiles (a few outputs a thread) spend their time on the instructions around a stage
 // rather than on its terms, so their stages are twice as long.
@@ -30,9 +31,9 @@ __host__ __device__ constexpr int nine_channels(bool thin) { return thin ? 4 : 2
 // pixels: input gradient 1687 -> 1549 us saturating, 2013 -> 1937 exact, forward 1344 -> 1326; 3x3 layers lose 1-6 %, the weights of
 // a chunk being strided).
 __host__ __device__ constexpr int gather_rows(int mode, int stages, int tc, int tp, int more_bytes, int ctas, bool thin = false) {
-    if (mode == GATHER_NINE) return 9 * nine_channels(thin);
+    if (mode == GATHER_NINE || mode == GATHER_NINE_ROWS) return 9 * nine_channels(thin);
     if (thin) return 2 * GATHER_CK;
-    return mode == GATHER_QUADS && ctas <= 4 && stages * 32 * (tp + tc + 4) * 4 + more_bytes <= 56 * 1024 ? 2 * GATHER_CK : GATHER_CK;
+    return (mode == GATHER_QUADS || mode == GATHER_QUADS_ROWS) && ctas <= 4 && stages * 32 * (tp + tc + 4) * 4 + more_bytes <= 56 * 1024 ? 2 * GATHER_CK : GATHER_CK;
 }
 
 // What a tile costs, in clocks per reduction step, measured over 30 layers (n 1-256, 3x3 and 1x1) with every tile forced and fitted

@@ -1,5 +1,5 @@
-"""Staging of the weights in 16-byte copies: the input gradient's copy by taps.  It does not change the order of addition, so it is
-compared bit for bit with the form without scratch, and with the oracle."""
+"""Staging of the weights in 16-byte copies: the forward's rows as they lie, the input gradient's copy by taps.  Neither changes the
+order of addition, so both are compared bit for bit with the forms that a misaligned or missing buffer takes, and with the oracle."""
 import pytest
 import torch
 
@@ -15,6 +15,27 @@ def _tensors(n, ci, co, h, w, k, s, p):
     wt = torch.randn(co, ci, k, k, device=DEV, generator=gen)
     g = torch.randn(n, co, (h + 2 * p - k) // s + 1, (w + 2 * p - k) // s + 1, device=DEV, generator=gen)
     return x, wt, g
+
+
+def _shifted(t):
+    """The same values at an address that is no multiple of 16 bytes."""
+    buf = torch.empty(t.numel() + 1, device=t.device)
+    buf[1:] = t.flatten()
+    return buf[1:].view(t.shape)
+
+
+# one block of channels and less, ragged outputs and inputs, odd and even numbers of channel pairs, several blocks
+@pytest.mark.parametrize("shape", [(64, 64, 64, 14, 14, 3, 1, 1), (40, 36, 100, 17, 9, 3, 1, 1), (64, 128, 128, 28, 28, 3, 1, 1),
+                                   (20, 32, 64, 20, 20, 1, 1, 0), (64, 512, 128, 14, 14, 1, 1, 0), (48, 68, 60, 12, 20, 1, 1, 0)],
+                         ids=lambda s: "n%d_c%dto%d_%dx%d_k%ds%dp%d" % s)
+def test_forward_rows(shape):
+    from addernetcuda_b200 import adder_cuda as ac
+    x, w, _ = _tensors(*shape)
+    s, p = shape[6:]
+    out = ac.forward(x, w, s, p)
+    assert torch.equal(out, ac.forward(x, _shifted(w), s, p))
+    ok, _, msg = O.compare("out", out[:2], O.adder2d_forward_direct(x[:2].cpu(), w.cpu(), s, p))
+    assert ok, msg
 
 
 @pytest.mark.parametrize("fast", [False, True], ids=["exact", "saturating"])
