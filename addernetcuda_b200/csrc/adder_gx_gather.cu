@@ -39,6 +39,10 @@ struct GxGatherArgs {
     int fill_pairs;          // ... or, rows being even, each block as two aligned 64-bit words
 };
 
+// Tiles that may stage their weights from the copy by taps: with 8 and most of those with 16 input channels a row is too short to share
+// the 16-byte copies among the threads, and the launch loses up to 11 %, its copy not counted (copy_share).
+__host__ __device__ constexpr bool takes_copy(int rc, int rp, int cg) { return rc * cg >= 32 || (rp == 2 && cg == 8); }
+
 // RC channels x RP pixels per thread (RP = 8: two quads half a tile apart), CG channel groups, ST stages, MB CTAs per SM.
 // (8 channels x 8 pixels, at 3 CTAs per SM, measured 10-15 % slower than 4 x 8.)
 template <int RC_, int RP_, int CG_, int ST_, int MB_>
@@ -46,6 +50,7 @@ struct GxTile {
     static constexpr int RC = RC_, RP = RP_, CG = CG_, ST = ST_, MB = MB_;
     static constexpr int PG = GATHER_THREADS / CG, TC = CG * RC, TP = PG * RP, WP = TC + 4;
     static constexpr int PQ = RP == 8 ? 4 : RP;                 // consecutive pixels of a thread
+    static constexpr bool TAKES_COPY = takes_copy(RC, RP, CG);
 };
 
 template <class T, bool FAST, int MODE>
@@ -409,15 +414,19 @@ constexpr Tile kTiles[] = {
 #undef X
 };
 
+long long tile_count(const GxGatherArgs& a, int classes, int Ci, const Tile& t) {
+    long long tiles = 0;
+    for (int c = 0; c < classes; ++c) tiles += (long long)ceil_div(a.m[c].P, t.tp) * ceil_div(Ci, t.tc);
+    return tiles;
+}
+
 int choose_tile(const GxGatherArgs& a, int classes, int Ci, bool fast) {
     int best = 0;
     double best_cost = 1e300;
     const int sms = sm_count();
     for (int i = 0; i < (int)(sizeof(kTiles) / sizeof(kTiles[0])); ++i) {
         const Tile& t = kTiles[i];
-        long long tiles = 0;
-        for (int c = 0; c < classes; ++c) tiles += (long long)ceil_div(a.m[c].P, t.tp) * ceil_div(Ci, t.tc);
-        const double cost = tile_cost(fast ? t.fast : t.exact, tiles, sms);
+        const double cost = tile_cost(fast ? t.fast : t.exact, tile_count(a, classes, Ci, t), sms);
         if (cost < best_cost) { best_cost = cost; best = i; }
     }
     return best;
@@ -487,7 +496,10 @@ template <bool FAST, int MODE>
 int launch_tile(int tile, const GxGatherArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
     int i = 0;
 #define X(RC, RP, CG, ST, MB, A, M, S, FA, FM, FS) \
-    if (tile == i++) return launch_t<GxTile<RC, RP, CG, ST, MB>, FAST, MODE>(a, grid, smem, stream);
+    if (tile == i++) {                                                                                        \
+        using T = GxTile<RC, RP, CG, ST, MB>;                                                                 \
+        if constexpr (MODE != GATHER_TAP_ROWS || T::TAKES_COPY) return launch_t<T, FAST, MODE>(a, grid, smem, stream); \
+    }
     ADDER_GX_GATHER_TILES(X)
 #undef X
     return ADDER_ERR_INTERNAL;
@@ -541,23 +553,59 @@ __global__ void __launch_bounds__(256) by_taps_kernel(const float* __restrict__ 
         for (int t = threadIdx.x >> 6; t < KK; t += 4) wt[((size_t)t * Co + co) * Ci + ci0 + c] = taps[c * KK + t];
 }
 
-// Windows of several taps: bytes of the copy of w by taps, whose rows a stage takes in 16-byte copies; 0 where the layer does
-// without.  As they lie, a stage's weights are 4-byte copies KK words apart, a sector of L2 each.  256->256 14x14 at batch 256: 2790 ->
-// 2657 us with the copy's own launch, 128->128 56x56 stride 2 at batch 64: 783 -> 729, 512->512 14x14 stride 2: 771 -> 716.  The launch
-// takes 3 to 8 us, which a layer of 3e9 terms (230 us) wins back; 176->176 8x8 at batch 47 (8e8) lost 8 us of 150.  The order of addition
-// is the same, so the result is.
-size_t gx_gather_workspace_bytes(const ConvGeom& g) {
+namespace {
+
+// What a launch saves by staging from the copy by taps, as a share of its time and without the copy's own: about the lower quartile of
+// 700 layers (2x2 to 7x7 windows, 64-2000 input channels, 25 to 98,000 output positions), measured with and without.  As w lies, a stage's
+// weights are 4-byte copies KK words apart: from 9 taps on each fetches a sector of L2 for itself, and the larger w is the less of it
+// stays close.  Medians, exact and saturating form: 64 channels x 64 pixels 0.04 and 0.07 at 3x3, 0.17 and 0.24 at 5x5, 0.27 and 0.32 at
+// 7x7; 32 x 64 0.05, 0.10; 0.23, 0.29; 0.34, 0.38; 32 x 128 0.01, 0.04; 0.04, 0.10; 0.07, 0.11; 16 x 32 -0.04, 0.01; 0.19, 0.22
+// (-0.03 where CTAs have an SM each); 0.25, 0.27.  The other tiles of 8 and 16 channels lose or gain 0.02 at most.
+double copy_share(const Tile& t, bool fast, int KK, bool alone) {
+    const double nine = t.rp == 8 ? (fast ? 0.04 : 0.025) : alone ? 0.01 : fast ? 0.07 : 0.04;
+    const double s = KK < 9 ? 0.015 : KK < 25 ? nine : KK < 49 ? 0.15 : 0.22;
+    if (t.rp == 8 && t.tc == 32) return KK < 25 ? (fast ? 0.02 : 0.0) : fast ? 0.09 : 0.035;
+    if (t.tc >= 32) return s;
+    return takes_copy(t.rc, t.rp, t.tc / t.rc) && KK >= 25 && !alone ? s : 0.0;
+}
+
+// Whether the copy pays for itself.  It reads and writes every weight at 2.7 TB/s behind a launch of 4 us, so it takes outputs to share it:
+// 2048->2048 7x7 at batch 2 lost 5 % of 1240 us by it, 4096->4096 5x5 at batch 1 20 to 30 %.  256->256 14x14 at batch 256: 2790 -> 2657 us,
+// 128->128 56x56 stride 2 at batch 64 783 -> 729, 512->512 14x14 stride 2 771 -> 716, 5x5 256->256 14x14 at batch 16 982 -> 680.  Layers below
+// 3e9 terms do without; of 506 measured above that the rule takes 359, none of which loses more than 3 %.  (Classes beyond the first
+// launch's, of strides above 3, are not counted.)
+bool copy_pays(const ConvGeom& g, const GxGatherArgs& a, int classes, const Tile& t, bool fast) {
+    const int sms = sm_count(), KK = g.kh * g.kw;
+    const long long tiles = tile_count(a, classes, g.Ci, t);
+    int taps = 0;
+    for (int c = 0; c < classes; ++c) taps += a.m[c].ntaps;
+    const double us = tile_cost(fast ? t.fast : t.exact, tiles, sms) * g.Co * taps / classes / 1965.0;
+    return 4.0 + 8.0 * KK * g.Co * g.Ci / 2.7e6 <= copy_share(t, fast, KK, tiles <= sms) * us;
+}
+
+}  // namespace
+
+static bool uses_copy(const ConvGeom& g, bool fast) {
     const int KK = g.kh * g.kw;
     const double terms = (double)g.N * g.Ho * g.Wo * g.Co * g.Ci * KK;
-    if (KK == 1 || KK > 128 || g.Ci % 4 != 0 || g.Co > 65535 * 32 || g.Ci > 65535 * 64 || terms < 3e9) return 0;
-    return (size_t)KK * g.Co * g.Ci * sizeof(float);
+    if (KK == 1 || KK > 128 || g.Ci % 4 != 0 || g.Ci > 65535 * 64 || terms < 3e9) return false;
+    GxGatherArgs a;
+    dim3 grid;
+    bool more;
+    const int tile = plan(g, 0, fast, a, grid, more);
+    return copy_pays(g, a, (int)grid.z, kTiles[tile], fast);
+}
+
+// Bytes of the copy of w by taps; 0 where the layer does without in both forms.
+size_t gx_gather_workspace_bytes(const ConvGeom& g) {
+    return uses_copy(g, false) || uses_copy(g, true) ? (size_t)g.kh * g.kw * g.Co * g.Ci * sizeof(float) : 0;
 }
 
 int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const float* w, float* gx, int fast, int accumulate,
                      cudaStream_t stream, void* workspace, size_t workspace_bytes) {
     float* by_taps = nullptr;
-    const size_t need = gx_gather_workspace_bytes(g);
-    if (workspace != nullptr && need > 0 && workspace_bytes >= need && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0) {
+    if (workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && uses_copy(g, fast != 0) &&
+        workspace_bytes >= (size_t)g.kh * g.kw * g.Co * g.Ci * sizeof(float)) {
         by_taps = static_cast<float*>(workspace);
         by_taps_kernel<<<dim3((unsigned)g.Co, (unsigned)ceil_div(g.Ci, 64)), 256, (size_t)64 * g.kh * g.kw * sizeof(float), stream>>>(w, by_taps, g.Co, g.Ci, g.kh * g.kw);
         const int st = launched();
@@ -572,7 +620,8 @@ int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const
         const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gx)) & 15) == 0;
         const bool unit = g.sh == 1 && g.sw == 1;
         a.vec_io = unit && (g.H * g.W) % 4 == 0 && aligned;
-        if (by_taps != nullptr) a.w = by_taps;
+        const bool copied = by_taps != nullptr && takes_copy(kTiles[tile].rc, kTiles[tile].rp, kTiles[tile].tc / kTiles[tile].rc);
+        if (copied) a.w = by_taps;
         a.w_quads = a.KK == 1 && g.Ci % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
         a.fill_block = single_class(g) && !accumulate;
         a.fill_quads = a.fill_block && g.sh == 2 && g.sw == 2 && g.W == 2 * a.m[0].PW && g.H == 2 * a.m[0].PH && a.m[0].PW % 4 == 0 &&
@@ -580,7 +629,7 @@ int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const
         // (planes of an odd height keep an even number of values, so that every plane starts aligned)
         a.fill_pairs = a.fill_block && !a.fill_quads && g.sh == 2 && g.sw == 2 && g.W % 2 == 0 && (reinterpret_cast<uintptr_t>(gx) & 7) == 0;
         const bool quads = gx_quads(g, a, grid, first, (reinterpret_cast<uintptr_t>(gout) & 15) == 0);
-        const int mode = by_taps != nullptr ? GATHER_TAP_ROWS : quads ? GATHER_QUADS : GATHER_TAP;
+        const int mode = copied ? GATHER_TAP_ROWS : quads ? GATHER_QUADS : GATHER_TAP;
         const int rows = stage_rows(kTiles[tile], mode);
         a.CK = g.Co < rows ? g.Co : rows;      // full blocks have the cheaper staging loops, so one ragged block rather than even ones
         const size_t smem = smem_bytes(kTiles[tile], mode);

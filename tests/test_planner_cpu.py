@@ -196,3 +196,20 @@ def test_statistics_pass_has_a_row_of_blocks_per_channel():
     for co, some in ((65535, True), (65536, False)):
         assert (lib.adder_b200_forward_stat_slices(8, 4, 3, 3, co, 1, 1, 0) > 0) == some
         assert (lib.adder_b200_forward_stat_slices(8, 128, 3, 3, co, 3, 1, 1) > 0) == some
+
+
+def test_copy_by_taps_where_it_pays():
+    """The input gradient's copy of w by taps costs by the weight and saves by the term: scratch is asked for where outputs enough share
+    a weight, and where a tile that gains by it is launched (of at least 32 input channels, mostly)."""
+    lib = _lib.load()
+
+    def scratch(n, ci, h, w, co, k, s):
+        return lib.adder_b200_conv_backward_input_workspace_bytes(n, ci, h, w, co, k, k, s, s, k // 2, k // 2, 1, 1)
+
+    # few outputs a weight (the copy took 5 to 30 % more than it saved), tiles of 8 and 16 channels (7 % slower with it), small layers
+    for shape in ((2, 2048, 7, 7, 2048, 3, 1), (1, 4096, 5, 5, 4096, 3, 1), (7, 1024, 7, 7, 1024, 3, 1), (9, 72, 56, 56, 176, 3, 1),
+                  (152, 48, 59, 11, 80, 3, 1), (47, 176, 8, 8, 176, 3, 1), (256, 1024, 14, 14, 256, 1, 1)):
+        assert scratch(*shape) == 0, shape
+    for shape in ((256, 256, 14, 14, 256, 3, 1), (64, 128, 56, 56, 128, 3, 2), (64, 512, 14, 14, 512, 3, 2), (4, 1024, 14, 14, 1024, 3, 1),
+                  (16, 256, 14, 14, 256, 5, 1), (1, 512, 16, 16, 512, 7, 1)):
+        assert scratch(*shape) == 4 * shape[1] * shape[4] * shape[5] ** 2, shape
