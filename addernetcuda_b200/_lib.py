@@ -16,6 +16,7 @@ TUNING_LIB_PATH = _PKG / "libadder_b200_tuning.so"
 ADDER_OK = 0
 FLAG_FAST_CLAMP = 1
 FLAG_ACCUMULATE = 2
+FLAG_UNALIGNED = 4
 # status codes of include/adder_b200.h
 (OK, ERR_NULL_POINTER, ERR_BAD_SHAPE, ERR_UNSUPPORTED, ERR_ALIGNMENT, ERR_WORKSPACE, ERR_CUDA, ERR_INTERNAL,
  ERR_TOO_LARGE, ERR_TIMEOUT) = range(10)

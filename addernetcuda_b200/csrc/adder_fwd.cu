@@ -426,15 +426,15 @@ static double tiled_fwd_clocks(const FwdPlan& p) {
 // time lost against the better of the two is 0.23 % on average; 15 are more than 5 % slower than with this kernel (20 of 430 with a rule
 // on channels and plane before, the worst 16->40 60x60 at batch 147 404 against 323 us, 416->33 10x24 at batch 241 1190 against 825).  Where
 // batch-norm statistics are asked for, this kernel makes them in its epilogue.
-static bool fwd_uses_gather(const Geom& g, const TileHint& hint) {
+static bool fwd_uses_gather(const Geom& g, const TileHint& hint, bool w_aligned) {
     if (g.k != 3) return true;
     TileHint h = hint;
     h.variant = 0;
     if (!h.is_default()) return false;
     if (hint.variant) return hint.variant == 2;
     if (g.stride != 1) return true;
-    bool gather = true;
-    cached_plan(g, gather, [&](bool& use) {
+    struct { bool use[2]; } gather;              // by whether w is 16-byte aligned
+    cached_plan(g, gather, [&](decltype(gather)& q) {
         int rw = 8, rm = 8;
         choose_fwd_tile(g, hint, rw, rm);
         FwdPlan p;
@@ -442,21 +442,21 @@ static bool fwd_uses_gather(const Geom& g, const TileHint& hint) {
 #define ADDER_FWD_PLAN(KS_, S_, RW_, RM_) st = plan_fwd_t<KS_, S_, RW_, RM_>(g, nullptr, hint, p);
         ADDER_FWD_DISPATCH(ADDER_FWD_PLAN)
 #undef ADDER_FWD_PLAN
-        use = st != ADDER_OK || tiled_fwd_clocks(p) >= fwd_gather_clocks(conv_geom(g));
+        for (int i = 0; i < 2; ++i) q.use[i] = st != ADDER_OK || tiled_fwd_clocks(p) >= fwd_gather_clocks(conv_geom(g), i != 0);
         return ADDER_OK;
     });
-    return gather;
+    return gather.use[w_aligned];
 }
 
-int describe_fwd(const Geom& layer, const TileHint& hint, char* buf, size_t n) {
+int describe_fwd(const Geom& layer, bool aligned, const TileHint& hint, char* buf, size_t n) {
     const Geom g = flatten_pointwise(layer);
     if (hint.is_default() && pointwise_applicable(g)) {
         snprintf(buf, n, "fwd k=1 s=%d pointwise: one thread per output position, 16 output channels per CTA, threads=256 "
                  "grid=(%d,%d) status=0", g.stride, ceil_div(g.N * g.Ho * g.Wo, 256), ceil_div(g.Co, 16));
         return ADDER_OK;
     }
-    if (fwd_uses_gather(layer, hint)) {
-        const int w = describe_fwd_gather(conv_geom(layer), buf, n);
+    if (fwd_uses_gather(layer, hint, aligned)) {
+        const int w = describe_fwd_gather(conv_geom(layer), aligned, buf, n);
         if (layer.k == 1 || w < 0 || (size_t)w + 16 >= n) return ADDER_OK;      // the tiled kernel has no 1x1 form
         buf += w; n -= w;
         const int w2 = snprintf(buf, n, "; tiled form: ");
@@ -559,7 +559,7 @@ int launch_fwd(const Geom& layer, const float* x, const float* w, float* out, co
                                                                                          FastDiv(ceil_div(g.Wo, rw)), FastDiv(g.Ho));
         return launched();
     }
-    if (stats == nullptr && fwd_uses_gather(layer, hint)) return launch_fwd_gather(conv_geom(layer), x, w, out, stream, ep);
+    if (stats == nullptr && fwd_uses_gather(layer, hint, (reinterpret_cast<uintptr_t>(w) & 15) == 0)) return launch_fwd_gather(conv_geom(layer), x, w, out, stream, ep);
 #define ADDER_FWD_LAUNCH(KS_, S_, RW_, RM_) \
     return launch_fwd_t<KS_, S_, RW_, RM_>(g, x, w, out, hint, stream, stats, stat_slices, ep);
     ADDER_FWD_DISPATCH(ADDER_FWD_LAUNCH)

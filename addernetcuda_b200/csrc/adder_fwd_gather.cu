@@ -335,7 +335,8 @@ constexpr Tile kTiles[] = {
 #undef X
 };
 
-// `rows`: rows of w are whole aligned quads (takes_rows), which takes 5 % off what a tile costs that profits.
+// `rows`: the layer's weights can be staged as they lie (row_layer), which takes 5 % off what a tile costs that profits.  Without aligned
+// operands nothing is taken off: 944->144 22x22 1x1 at batch 19 then runs the other tile, 136 -> 126 us.
 int choose_tile(int P, int Co, bool rows) {
     int best = 0;
     double best_cost = 1e300;
@@ -348,12 +349,14 @@ int choose_tile(int P, int Co, bool rows) {
     return best;
 }
 
-// Layers whose weights can be staged as they lie: 3x3, and 1x1 whose pixels are the input's in order.  The plan looks at the sizes alone,
-// the launch at the alignment too.
-bool row_layer(const ConvGeom& g) {
-    const bool in_order = g.kh * g.kw == 1 && g.sh == 1 && g.sw == 1 && g.ph == 0 && g.pw == 0 && (g.Ho * g.Wo) % 4 == 0;
+// 16-byte alignment of the operands.
+struct Aligned { bool x, w; };
+
+// Layers whose weights can be staged as they lie: 3x3, and 1x1 whose pixels are the input's in order and come in quads.
+bool row_layer(const ConvGeom& g, Aligned al) {
+    const bool in_order = g.kh * g.kw == 1 && g.sh == 1 && g.sw == 1 && g.ph == 0 && g.pw == 0 && (g.Ho * g.Wo) % 4 == 0 && al.x;
     const int K = g.Ci * g.kh * g.kw;            // (a row of fewer steps is mostly padding of the stage: 4->336 16x16 at batch 11 3.0 -> 3.4 us)
-    return K % 4 == 0 && K >= 32 && (in_order || (g.kh == 3 && g.kw == 3));
+    return al.w && K % 4 == 0 && K >= 32 && (in_order || (g.kh == 3 && g.kw == 3));
 }
 
 bool thin(const Tile& t) { return t.rm <= 2 && t.rp <= 2; }
@@ -399,25 +402,26 @@ int launch_mode(int tile, const FwdGatherArgs& a, dim3 grid, size_t smem, cudaSt
 
 }  // namespace
 
-double fwd_gather_clocks(const ConvGeom& g) {
+double fwd_gather_clocks(const ConvGeom& g, bool w_aligned) {
     const int P = g.N * g.Ho * g.Wo;
-    const bool rows = row_layer(g);
+    const bool rows = row_layer(g, {true, w_aligned});
     const Tile& t = kTiles[choose_tile(P, g.Co, rows)];
     return tile_cost(t.cost, (long long)ceil_div(P, t.tp) * ceil_div(g.Co, t.tc), sm_count()) * (rows && takes_rows(t.rm, t.cg) ? 0.95 : 1.0);
 }
 
-static int fwd_mode(const ConvGeom& g, const Tile& t, bool aligned, bool w_quads) {
-    const bool rows = w_quads && takes_rows(t.rm, t.cg);
+static int fwd_mode(const ConvGeom& g, const Tile& t, Aligned al) {
+    const bool rows = row_layer(g, al) && takes_rows(t.rm, t.cg);
     if (g.kh == 3 && g.kw == 3) return rows ? GATHER_NINE_ROWS : GATHER_NINE;
     const bool in_order = g.kh * g.kw == 1 && g.sh == 1 && g.sw == 1 && g.ph == 0 && g.pw == 0;
-    if (!in_order || !aligned || (g.Ho * g.Wo) % 4 != 0) return GATHER_TAP;
+    if (!in_order || !al.x || (g.Ho * g.Wo) % 4 != 0) return GATHER_TAP;
     return rows ? GATHER_QUADS_ROWS : GATHER_QUADS;
 }
 
-int describe_fwd_gather(const ConvGeom& g, char* buf, size_t n) {
+int describe_fwd_gather(const ConvGeom& g, bool aligned, char* buf, size_t n) {
     const int P = g.N * g.Ho * g.Wo;
-    const Tile& t = kTiles[choose_tile(P, g.Co, row_layer(g))];
-    const size_t smem = smem_bytes(t, fwd_mode(g, t, true, row_layer(g)));
+    const Aligned al{aligned, aligned};
+    const Tile& t = kTiles[choose_tile(P, g.Co, row_layer(g, al))];
+    const size_t smem = smem_bytes(t, fwd_mode(g, t, al));
     return snprintf(buf, n, "fwd gather k=%dx%d RM=%d RP=%d TC=%d TP=%d threads=%d smem=%zu grid=(%d,%d) status=%d", g.kh, g.kw, t.rm,
                     t.rp, t.tc, t.tp, GATHER_THREADS, smem, ceil_div(P, t.tp), ceil_div(g.Co, t.tc), gather_status(ceil_div(g.Co, t.tc), smem));
 }
@@ -428,11 +432,12 @@ int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* 
     a.x = x; a.w = w; a.out = out; a.ep = ep;
     a.Ci = g.Ci; a.H = g.H; a.W = g.W; a.Co = g.Co; a.KK = g.kh * g.kw;
     const bool whole_quads = (g.Ho * g.Wo) % 4 == 0;
-    a.vec_w = (a.KK == 1 || (g.kh == 3 && g.kw == 3)) && (g.Ci * a.KK) % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
+    const Aligned al{(reinterpret_cast<uintptr_t>(x) & 15) == 0, (reinterpret_cast<uintptr_t>(w) & 15) == 0};
+    a.vec_w = (a.KK == 1 || (g.kh == 3 && g.kw == 3)) && (g.Ci * a.KK) % 4 == 0 && al.w;
     a.vec_store = whole_quads && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(ep.residual)) & 15) == 0;
-    const int tile = choose_tile(a.m.P, g.Co, row_layer(g));
+    const int tile = choose_tile(a.m.P, g.Co, row_layer(g, al));
     const Tile& t = kTiles[tile];
-    const int mode = fwd_mode(g, t, (reinterpret_cast<uintptr_t>(x) & 15) == 0, a.vec_w && row_layer(g));
+    const int mode = fwd_mode(g, t, al);
     const int rows = stage_rows(t, mode);
     // Windows of several taps are added up in the order (block of 16 channels, tap, channel) by every tile: the tile follows the batch,
     // and an image's result must not.  A thin tile, whose stages have 32 rows, takes two such blocks a stage.

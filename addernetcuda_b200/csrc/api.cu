@@ -346,7 +346,7 @@ int adder_b200_describe_plan(int op, int n, int ci, int h, int wd, int co, int k
     const int st = make_geom(n, ci, h, wd, co, k, stride, pad, &g);
     if (st != ADDER_OK) return st;
     buf[0] = 0;
-    if (op == 0) return describe_fwd(g, current_hint(0), buf, buf_bytes);
+    if (op == 0) return describe_fwd(g, (flags & ADDER_FLAG_UNALIGNED) == 0, current_hint(0), buf, buf_bytes);
     if (op == 1) return describe_gx(g, (flags & ADDER_FLAG_FAST_CLAMP) != 0, current_hint(1), buf, buf_bytes);
     if (op == 2) return describe_gw(g, current_hint(2), buf, buf_bytes);
     return ADDER_ERR_BAD_SHAPE;

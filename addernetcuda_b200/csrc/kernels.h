@@ -138,8 +138,8 @@ int launch_conv_gw(const ConvGeom& g, const float* gout, const float* x, const f
 // Channels x pixels tiles with a gathered operand (adder_fwd_gather.cu, adder_gx_gather.cu)
 int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* out, cudaStream_t s,
                       const Epilogue& ep = Epilogue());
-double fwd_gather_clocks(const ConvGeom& g);      // predicted time of its launch, in clocks per reduction step
-int describe_fwd_gather(const ConvGeom& g, char* buf, size_t n);
+double fwd_gather_clocks(const ConvGeom& g, bool w_aligned);      // predicted time of its launch, in clocks per reduction step
+int describe_fwd_gather(const ConvGeom& g, bool aligned, char* buf, size_t n);
 int launch_gx_gather(const ConvGeom& g, const float* gout, const float* x, const float* w, float* gx, int fast, int accumulate,
                      cudaStream_t s, void* workspace = nullptr, size_t workspace_bytes = 0);
 size_t gx_gather_workspace_bytes(const ConvGeom& g);
@@ -182,7 +182,7 @@ int gw1x1_splits(const Geom& g);
 int launch_gw1x1(const Geom& g, const float* gout, const float* x, float* part, float* gsum_part,
                  unsigned int* ticket, int splits, cudaStream_t stream);
 
-int describe_fwd(const Geom& g, const TileHint& hint, char* buf, size_t n);
+int describe_fwd(const Geom& g, bool aligned, const TileHint& hint, char* buf, size_t n);      // aligned: 16-byte alignment of x and w
 int describe_gx(const Geom& g, int fast, const TileHint& hint, char* buf, size_t n);
 int describe_gw(const Geom& g, const TileHint& hint, char* buf, size_t n);
 

@@ -54,6 +54,7 @@ enum {
 #define ADDER_FLAG_FAST_CLAMP 1  /* input gradient: saturating-add form of clamp(); differs from the
                                     exact form by about 1e-7 per term */
 #define ADDER_FLAG_ACCUMULATE 2  /* add into the output buffer(s) instead of overwriting them */
+#define ADDER_FLAG_UNALIGNED 4   /* adder_b200_describe_plan, forward: x and w are not 16-byte aligned */
 
 /* Human-readable name of a status code (static storage, never NULL). */
 ADDER_API const char* adder_b200_status_string(int status);

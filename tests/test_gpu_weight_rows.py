@@ -26,7 +26,7 @@ def _shifted(t):
 
 # one block of channels and less, ragged outputs and inputs, odd and even numbers of channel pairs, several blocks
 @pytest.mark.parametrize("shape", [(64, 64, 64, 14, 14, 3, 1, 1), (40, 36, 100, 17, 9, 3, 1, 1), (64, 128, 128, 28, 28, 3, 1, 1),
-                                   (20, 32, 64, 20, 20, 1, 1, 0), (64, 512, 128, 14, 14, 1, 1, 0), (48, 68, 60, 12, 20, 1, 1, 0)],
+                                   (73, 4, 96, 8, 12, 3, 1, 1), (20, 32, 64, 20, 20, 1, 1, 0), (64, 512, 128, 14, 14, 1, 1, 0), (48, 68, 60, 12, 20, 1, 1, 0)],
                          ids=lambda s: "n%d_c%dto%d_%dx%d_k%ds%dp%d" % s)
 def test_forward_rows(shape):
     from addernetcuda_b200 import adder_cuda as ac
