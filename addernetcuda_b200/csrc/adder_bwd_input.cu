@@ -120,7 +120,7 @@ __device__ __forceinline__ void gx_scale_weights(const GxArgs& a, float* wt, int
 
 // MB = CTAs per SM the register budget is cut for.  A layer whose output channels fit one chunk needs one
 // stage of shared memory only, and with 4-pixel segments few enough registers for three CTAs per SM: the
-// third CTA's loads and stores then run under the other two's arithmetic (16->16 32x32: 69 -> 66 us).
+// third CTA's loads and stores then run under the other two's arithmetic (16->16 32x32: 69 -> 66 us).  gx_budget has the rule.
 template <int KS, int S, int RW, int RC, bool FAST, int MB = 2>
 __global__ void __launch_bounds__(256, MB) adder_gx_kernel(const GxArgs a) {
     constexpr int KK = KS * KS;
@@ -827,6 +827,17 @@ static Geom gx_tiling_geom(const Geom& g) {
     return t;
 }
 
+// MB of a launch of adder_gx_kernel.  Saturating form: three CTAs where they fit, the layer needing one stage only.  The packed loop of the exact
+// form is the faster one with that budget (80 registers for 101) wherever several CTAs share an SM, also where two are all that
+// fits: at two of 5 or 6 warps it fell behind the scalar loop otherwise (144->48 6x12 at batch 355: scalar 283 us, packed 315, now
+// 254; 64->64 8x8 at batch 256 83, 78, 76).  Few warps are a chain of latencies, which the larger budget shortens: up to 8 an SM (64->64 8x8
+// at batch 128, 7 warps: 44.7 us with 80 registers, 43.6; 3->208 4x4 at batch 3 200, 185).
+static int gx_budget(const GxPlan& p) {
+    if (p.ks != 3 || p.s != 1 || p.rw != 4) return 2;
+    if (p.fast) return p.a.nstages == 1 && 3 * (p.smem + 1024) <= 227 * 1024 ? 3 : 2;
+    return p.gx * p.gy * (p.threads / 32) > 8LL * sm_count() ? 3 : 2;
+}
+
 template <int KS, int S, int RW, int RC, bool FAST>
 static int launch_gx_t(const Geom& real, const float* gout, const float* x, const float* w, float* gx,
                        int accumulate, const TileHint& hint, cudaStream_t stream) {
@@ -850,7 +861,7 @@ static int launch_gx_t(const Geom& real, const float* gout, const float* x, cons
         }
     }
     if constexpr (S == 1 && RW == 4 && KS == 3) {
-        if (p.a.nstages == 1 && 3 * (p.smem + 1024) <= 227 * 1024) {
+        if (gx_budget(p) == 3) {
             auto kern3 = adder_gx_kernel<KS, S, RW, RC, FAST, 3>;
             if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern3), p.smem) != ADDER_OK) return ADDER_ERR_CUDA;
             kern3<<<dim3((unsigned)p.gx, (unsigned)p.gy), p.threads, p.smem, stream>>>(p.a);
@@ -927,9 +938,9 @@ int describe_gx(const Geom& layer, int fast, const TileHint& hint, char* buf, si
     if (st == ADDER_ERR_UNSUPPORTED && !((g.k == 1 || g.k == 3) && (g.stride == 1 || g.stride == 2))) return st;
     snprintf(buf, n,
              "gx k=%d s=%d RW=%d RC=%d fast=%d segs/thread=%d CGI=%d TCI=%d TI=%d TH=%d SPRC=%d SEGS=%d CKO=%d rows=%d cols=%d pitch=%d "
-             "threads=%d smem=%zu grid=(%lld,%d) status=%d",
+             "MB=%d threads=%d smem=%zu grid=(%lld,%d) status=%d",
              p.ks, p.s, p.rw, p.rc, p.fast, p.a.nseg, p.a.CGI, p.a.TCI, p.a.TI, p.a.TH, p.a.SPRC, p.a.SEGS, p.a.CKO, p.a.pd.ROWS,
-             p.a.pd.COLS, p.a.pd.PITCH, p.threads, p.smem, p.gx, p.gy, st);
+             p.a.pd.COLS, p.a.pd.PITCH, gx_budget(p), p.threads, p.smem, p.gx, p.gy, st);
     return ADDER_OK;
 }
 

@@ -215,6 +215,16 @@ def test_copy_by_taps_where_it_pays():
         assert scratch(*shape) == 4 * shape[1] * shape[4] * shape[5] ** 2, shape
 
 
+def test_register_budget_of_the_exact_input_gradient():
+    """Tiled 3x3 stride-1 layers: the budget of three CTAs an SM where more than 8 warps share one (with that of two, two CTAs of 5 warps
+    were 11 % slower than before the packed loop), that of two below; the saturating form by what fits."""
+    for shape, exact, fast in (((355, 144, 6, 12, 48), 3, 2), ((173, 144, 12, 24, 48), 3, 2), ((256, 64, 8, 8, 64), 3, 2),
+                               ((128, 64, 8, 8, 64), 2, 2), ((3, 3, 4, 4, 208), 2, 2), ((256, 16, 32, 32, 16), 3, 3), ((1, 16, 32, 32, 16), 2, 3),
+                               ((256, 32, 14, 14, 32), 2, 2)):
+        assert _field(_launched(1, *shape, 3, 1, 1, 0), "MB") == exact, shape
+        assert _field(_launched(1, *shape, 3, 1, 1, 1), "MB") == fast, shape
+
+
 def test_forward_plan_by_alignment():
     """Tiles that profit from weights in 16-byte copies are planned as cheaper only where the operands allow those: without
     alignment the layers below ran 5 to 8 % slower on them than on the tile (the last one: kernel) that is planned otherwise."""
