@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
     constexpr int PARTS = 4, MINE = PARTS / ROWS;      // partial sums of g per pixel, and those of one thread
     static_assert(PARTS % ROWS == 0 && (PARTS > ROWS || CK == 16), "whole partial sums per thread, a stage at a time");
     constexpr int FOLD = 64 / CK;                // chunks per partial sum: 64 terms before it is folded into the total
+    constexpr bool PACKED = !FAST && RP == 8 && CG >= 8;      // exact form: differences of two pixels at a time
     constexpr int GS = CK * TP, WS = CK * WP;
     extern __shared__ __align__(16) float smem[];
     float* const Gs = smem;
@@ -205,7 +206,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
                 for (int r = 0; r < RC; ++r)
 #pragma unroll
                     for (int j = 0; j < RP; ++j) acc[r][j] = fmaf(__saturatef(fmaf(wv[r], 0.5f, xv[r][j])), gv[j], acc[r][j]);
-            } else if constexpr (RP == 8 && CG >= 8) {
+            } else if constexpr (PACKED) {
                 // both steps of a pair of pixels packed but the clamp: 2.97 lane-clocks a term with nothing around it, 3.31 with a scalar
                 // subtraction (1024->256 14x14 at batch 256: 1308 -> 1179 us)
 #pragma unroll
@@ -384,7 +385,14 @@ __global__ void __launch_bounds__(GATHER_THREADS, T::MB) adder_gx_gather_kernel(
                 const float v = acc[c][PQ * h + j];
                 if (a.accumulate) { *oc += v; continue; }
                 *oc = v;
-                if (a.fill_block)
+                // (stride 2 without loops, whose code the packed tiles' register allocation made the slower: 960->24 29x31 at batch 60
+                // 340 us scalar, 364 packed, now 302.  The other tiles have the loops: the branch cost some of them 1 to 3 %.)
+                if (PACKED && a.fill_block && a.sh == 2 && a.sw == 2) {
+                    const bool right = xi + 1 < a.W, below = yi + 1 < a.H;
+                    if (right) oc[1] = 0.f;
+                    if (below) oc[a.W] = 0.f;
+                    if (right & below) oc[a.W + 1] = 0.f;
+                } else if (a.fill_block)
                     for (int dy = 0; dy < a.sh && yi + dy < a.H; ++dy)
                         for (int dx = 0; dx < a.sw && xi + dx < a.W; ++dx)
                             if (dy | dx) oc[dy * a.W + dx] = 0.f;

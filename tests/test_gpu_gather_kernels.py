@@ -79,3 +79,25 @@ def test_gathering_kernels(case):
         size = back(g64.abs().sum(0).expand(terms, -1))
         for got in grads:
             assert ((got[i].double() - want_gx).abs() <= 4 * (co * k * k + 4) * U * size).all()
+
+
+@pytest.mark.parametrize("fast", [0, 1], ids=["exact", "saturating"])
+@pytest.mark.parametrize("hw", [(9, 11), (10, 11), (9, 12), (10, 12), (8, 16), (1, 1), (2, 1), (1, 2)], ids=lambda v: "%dx%d" % v)
+@pytest.mark.parametrize("strides", [(2, 2), (2, 3), (3, 2), (3, 3), (1, 2), (2, 1), (5, 2)], ids=lambda v: "s%dx%d" % v)
+def test_unsampled_pixels_get_zeros(strides, hw, fast):
+    """A strided 1x1 layer reads one pixel of each block: the input gradient writes a zero to every other one, whatever lay there, with
+    16-byte, 8-byte or single stores."""
+    from addernetcuda_b200 import _lib
+    (h, w), (sh, sw), n, ci, co = hw, strides, 3, 70, 66
+    gen = torch.Generator(device=DEV).manual_seed(h * w + sh)
+    x, wt = torch.randn(n, ci, h, w, device=DEV, generator=gen), torch.randn(co, ci, device=DEV, generator=gen)
+    g = torch.randn(n, co, -(-h // sh), -(-w // sw), device=DEV, generator=gen)
+    gx = torch.full_like(x, float("nan"))
+    _lib.check(_lib.load().adder_b200_conv_backward_input(g.data_ptr(), x.data_ptr(), wt.data_ptr(), gx.data_ptr(), n, ci, h, w, co, 1, 1,
+                                                          sh, sw, 0, 0, 1, 1, fast, torch.cuda.current_stream().cuda_stream), "backward_input")
+    want = torch.zeros(n, ci, h, w, device=DEV, dtype=torch.float64)
+    d = (wt.double()[None, :, :, None, None] - x.double()[:, None, :, ::sh, ::sw]).clamp(-1, 1)
+    want[:, :, ::sh, ::sw] = (d * g.double()[:, :, None]).sum(1)
+    size = torch.zeros_like(want)
+    size[:, :, ::sh, ::sw] = g.double().abs().sum(1, keepdim=True)
+    assert ((gx.double() - want).abs() <= 4 * (co + 4) * U * size).all()
