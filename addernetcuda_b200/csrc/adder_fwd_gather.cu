@@ -421,9 +421,10 @@ int describe_fwd_gather(const ConvGeom& g, bool aligned, char* buf, size_t n) {
     const int P = g.N * g.Ho * g.Wo;
     const Aligned al{aligned, aligned};
     const Tile& t = kTiles[choose_tile(P, g.Co, row_layer(g, al))];
-    const size_t smem = smem_bytes(t, fwd_mode(g, t, al));
-    return snprintf(buf, n, "fwd gather k=%dx%d RM=%d RP=%d TC=%d TP=%d threads=%d smem=%zu grid=(%d,%d) status=%d", g.kh, g.kw, t.rm,
-                    t.rp, t.tc, t.tp, GATHER_THREADS, smem, ceil_div(P, t.tp), ceil_div(g.Co, t.tc), gather_status(ceil_div(g.Co, t.tc), smem));
+    const int mode = fwd_mode(g, t, al);
+    const size_t smem = smem_bytes(t, mode);
+    return snprintf(buf, n, "fwd gather k=%dx%d RM=%d RP=%d TC=%d TP=%d staging=%s threads=%d smem=%zu grid=(%d,%d) status=%d", g.kh, g.kw, t.rm,
+                    t.rp, t.tc, t.tp, staging_name(mode), GATHER_THREADS, smem, ceil_div(P, t.tp), ceil_div(g.Co, t.tc), gather_status(ceil_div(g.Co, t.tc), smem));
 }
 
 int launch_fwd_gather(const ConvGeom& g, const float* x, const float* w, float* out, cudaStream_t stream, const Epilogue& ep) {

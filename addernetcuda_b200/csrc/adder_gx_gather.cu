@@ -539,16 +539,6 @@ static bool gx_quads(const ConvGeom& g, const GxGatherArgs& a, const dim3& grid,
            (g.Ho * g.Wo) % 4 == 0 && aligned;
 }
 
-int describe_gx_gather(const ConvGeom& g, int fast, char* buf, size_t n) {
-    GxGatherArgs a;
-    dim3 grid;
-    bool more;
-    const Tile& t = kTiles[plan(g, 0, fast != 0, a, grid, more)];
-    const size_t smem = smem_bytes(t, gx_quads(g, a, grid, 0, true) ? GATHER_QUADS : GATHER_TAP);
-    return snprintf(buf, n, "gx gather k=%dx%d fast=%d classes=%u RC=%d RP=%d TC=%d TP=%d threads=%d smem=%zu grid=(%u,%u) status=%d",
-                    g.kh, g.kw, fast, grid.z, t.rc, t.rp, t.tc, t.tp, GATHER_THREADS, smem, grid.x, grid.y, gather_status((int)grid.y, smem));
-}
-
 // w[Co][Ci][KK] -> [KK][Co][Ci]: a block has 64 input channels of one output channel, which are consecutive on both sides.
 __global__ void __launch_bounds__(256) by_taps_kernel(const float* __restrict__ w, float* __restrict__ wt, int Co, int Ci, int KK) {
     extern __shared__ float taps[];              // [64][KK]
@@ -602,6 +592,19 @@ static bool uses_copy(const ConvGeom& g, bool fast) {
     bool more;
     const int tile = plan(g, 0, fast, a, grid, more);
     return copy_pays(g, a, (int)grid.z, kTiles[tile], fast);
+}
+
+// With scratch (staging=tap_rows: the copy by taps is a launch in front).
+int describe_gx_gather(const ConvGeom& g, int fast, char* buf, size_t n) {
+    GxGatherArgs a;
+    dim3 grid;
+    bool more;
+    const Tile& t = kTiles[plan(g, 0, fast != 0, a, grid, more)];
+    const int mode = uses_copy(g, fast != 0) ? GATHER_TAP_ROWS : gx_quads(g, a, grid, 0, true) ? GATHER_QUADS : GATHER_TAP;
+    const size_t smem = smem_bytes(t, mode);
+    return snprintf(buf, n, "gx gather k=%dx%d fast=%d classes=%u RC=%d RP=%d TC=%d TP=%d staging=%s threads=%d smem=%zu grid=(%u,%u) status=%d",
+                    g.kh, g.kw, fast, grid.z, t.rc, t.rp, t.tc, t.tp, staging_name(mode), GATHER_THREADS, smem, grid.x, grid.y,
+                    gather_status((int)grid.y, smem));
 }
 
 // Bytes of the copy of w by taps; 0 where the layer does without in both forms.

@@ -22,6 +22,10 @@ namespace adder {
 constexpr int GATHER_CK = 16;
 constexpr int GATHER_THREADS = 128;
 enum GatherMode { GATHER_TAP, GATHER_QUADS, GATHER_NINE, GATHER_HALVES, GATHER_QUADS_ROWS, GATHER_NINE_ROWS, GATHER_TAP_ROWS };
+inline const char* staging_name(int mode) {
+    constexpr const char* names[] = {"tap", "quads", "nine", "halves", "quads_rows", "nine_rows", "tap_rows"};
+    return names[mode];
+}
 
 // Channels of a chunk of GATHER_NINE; thin tiles (a few outputs a thread) spend their time on the instructions around a stage
 // rather than on its terms, so their stages are twice as long.
