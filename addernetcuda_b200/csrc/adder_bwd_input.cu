@@ -17,7 +17,8 @@
 // FAST variant: clamp(d,-1,1) = 2*sat(d/2 + 1/2) - 1, so with w' = w/2 + 1/2 staged in shared
 // memory and x' = -x/2 in registers a term costs one saturating add and one fused multiply-add;
 // the correction sum(g) over the same taps is the box sum of the channel-summed g patch, which
-// the CTA accumulates on the side.  The exact variant evaluates the formula as written.
+// the CTA accumulates on the side.  The exact variant evaluates the formula as written; at stride 1 it forms the differences, and both
+// variants the sums, of two channels in one packed instruction.
 #include <type_traits>
 #include "common.cuh"
 #include "kernels.h"
@@ -35,7 +36,8 @@ __device__ __forceinline__ float gx_term(float wv, float xv) {
 // Stride-2 taps of one output channel for a thread whose pixels have row phase PH = (y+pad) mod 2 and
 // column phase PW = (x+pad) mod 2: only the taps kh = PH, PH+2, ... and kw = PW, PW+2, ... reach an
 // output pixel, so the loops are compile-time and nothing is predicated.  row0/col0 locate the tap
-// (PH, PW) in the shared-memory patch of g; later taps sit one row / one column before it.
+// (PH, PW) in the shared-memory patch of g; later taps sit one row / one column before it.  Differences and sums are scalar here in both
+// forms: the packed ones of the stride-1 loop were not tried.
 template <int KS, int RW, int RC, bool FAST, int PH, int PW>
 __device__ __forceinline__ void gx_taps_stride2(float (&acc)[RC][RW], const float (&xv)[RC][RW], const float* gch,
                                                 const float* wch, int row0, int col0, int pitch) {
@@ -274,7 +276,7 @@ __global__ void __launch_bounds__(256, MB) adder_gx_kernel(const GxArgs a) {
                                     if constexpr (FAST) {
                                         s0 = gx_term<true>(wv[cc], xv[cc][j]);
                                         s1 = gx_term<true>(wv[cc + 1], xv[cc + 1][j]);
-                                    } else {         // (one packed subtraction: 16->16 32x32 at batch 256 74.3 -> 65.2 us, 64->64 8x8 83.3 -> 78.0)
+                                    } else {         // (one packed subtraction: 16->16 32x32 at batch 256 74.3 -> 65.3 us, 64->64 8x8 83.3 -> 76.1)
                                         unpack2(add2(pack2(wv[cc], wv[cc + 1]), pack2(xv[cc][j], xv[cc + 1][j])), s0, s1);
                                         s0 = clamp_unit(s0);
                                         s1 = clamp_unit(s1);

@@ -424,7 +424,8 @@ static double tiled_fwd_clocks(const FwdPlan& p) {
 // same order, so the choice does not show in the result.  1x1 kernels and stride 2 (16->32 at batch 256: 36 against 30 us) are the
 // gathering kernel's; of the stride-1 3x3 layers each kernel takes those it is predicted to be faster on.  Over 1400 drawn ones the
 // time lost against the better of the two is 0.23 % on average; 15 are more than 5 % slower than with this kernel (20 of 430 with a rule
-// on channels and plane before, the worst 16->40 60x60 at batch 147 404 against 323 us, 416->33 10x24 at batch 241 1190 against 825).  Where
+// on channels and plane before, the worst 16->40 60x60 at batch 147 404 against 323 us, 416->33 10x24 at batch 241 1190 against 825);
+// those figures are from before the gathering kernel's tiles that take the weights as they lie (choose_tile there).  Where
 // batch-norm statistics are asked for, this kernel makes them in its epilogue.
 static bool fwd_uses_gather(const Geom& g, const TileHint& hint, bool w_aligned) {
     if (g.k != 3) return true;

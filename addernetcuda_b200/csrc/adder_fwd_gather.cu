@@ -335,8 +335,10 @@ constexpr Tile kTiles[] = {
 #undef X
 };
 
-// `rows`: the layer's weights can be staged as they lie (row_layer), which takes 5 % off what a tile costs that profits.  Without aligned
-// operands nothing is taken off: 944->144 22x22 1x1 at batch 19 then runs the other tile, 136 -> 126 us.
+// `rows`: the layer's weights can be staged as they lie (row_layer), which takes 5 % off what a tile costs that profits: 500 layers whose
+// tile, or kernel, that changes gain 3.7 %, 9 of them lose more than 5 %, 12 % at worst (taking nothing off beyond 8 CTAs an SM halves the
+// losers and a part of the gains: the same sum).  Without aligned operands nothing is taken off: 944->144 22x22 1x1 at batch 19 then runs
+// the other tile, 136 -> 126 us.
 int choose_tile(int P, int Co, bool rows) {
     int best = 0;
     double best_cost = 1e300;

@@ -10,8 +10,8 @@
 // stages pass by: in four partial sums, of rows r, r + 4, r + 8 and r + 12 of every 16, whichever threads share the pixel, so that
 // the tile - which follows the size of the batch - does not show in the result.  Exact form: min.xorsign.abs is the clamp in one instruction (magnitude min(|d|, 1), sign of d),
 // where fminf(fmaxf(d, -1), 1) takes two; differences (large tiles) and sums are packed pairs of pixels.
-// Both are bound by the register operands they read (5 a term, 2 a cycle and scheduler): 2.5 and 3.0 lane cycles a term
-// with nothing around them.  What stands around them is the staging: without it the saturating form of 256->256 14x14 at batch 256
+// With nothing around it the saturating form takes 2.5 lane cycles a term, the register operands that it reads (5 a term, 2 a cycle and
+// scheduler); the exact form, a clamp and two halves of packed instructions, is measured at 3.0.  What stands around them is the staging: without it the saturating form of 256->256 14x14 at batch 256
 // takes 2.90 lane cycles a term, with it 3.43 from w as it lies and 3.27 from a copy by taps (gx_gather_workspace_bytes).
 #include <cstdio>
 #include "common.cuh"

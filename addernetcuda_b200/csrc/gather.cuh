@@ -32,8 +32,8 @@ inline const char* staging_name(int mode) {
 __host__ __device__ constexpr int nine_channels(bool thin) { return thin ? 4 : 2; }
 
 // Rows of a stage.  1x1 layers take 32 channels at a time where four CTAs still fit an SM: half the barriers (1024->256 on 75,776
-// pixels: input gradient 1687 -> 1549 us saturating, 2013 -> 1937 exact, forward 1344 -> 1326; 3x3 layers lose 1-6 %, the weights of
-// a chunk being strided).
+// pixels: input gradient 1687 -> 1549 us saturating, 2013 -> 1937 exact, forward 1344 -> 1326).  3x3 layers
+// lost 1-6 % by it, measured with weights staged as they lie, a tap's words apart; the _ROWS modes were not measured with more rows.
 __host__ __device__ constexpr int gather_rows(int mode, int stages, int tc, int tp, int more_bytes, int ctas, bool thin = false) {
     if (mode == GATHER_NINE || mode == GATHER_NINE_ROWS) return 9 * nine_channels(thin);
     if (thin) return 2 * GATHER_CK;
